@@ -106,7 +106,7 @@ struct ssg_index {
     DevBuf st_db, st_scale, st_alpha, st_beta, st_q, st_qscale;
     // plain FP32 GEMM-form path: |x|^2 per row and its maximum, query flags of
     // the completeness check and the fallback's buffers
-    DevBuf sq_norm, sq_max, flags, qsq, fb_list, fb_q, fb_out, fb_cand, fb_qn;
+    DevBuf sq_norm, sq_max, flags, fb_list, fb_q, fb_out, fb_cand, fb_qn;
     // BF16 threshold-filter path (candidate counts beyond the on-chip heaps):
     // tiles of every smp_r-th database row, filtered lists, counts, bounds
     DevBuf tc_smp, tc_smp_norm, f_out, f_cnt, f_thr, gbound;
@@ -601,7 +601,6 @@ int run_gemm(ssg_index *idx, const float *dq, const float *dqn, int64_t m, int k
     }
     if (sq) {
         SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
-        SSG_CK(idx->qsq.ensure(size_t(chunk) * 4 + 16), "allocating query norms");
         SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
     }
     int *flags = static_cast<int *>(idx->flags.p);
@@ -642,11 +641,7 @@ int run_gemm(ssg_index *idx, const float *dq, const float *dqn, int64_t m, int k
         f.out_ids = d_ids + size_t(c0) * k;
         f.out_dists = d_dists + size_t(c0) * k;
         if (sq) {
-            float *qsq = static_cast<float *>(idx->qsq.p);
-            SSG_CK(ssg::launch_row_sq_norms(qc, mc, idx->dim, qsq, qsq + chunk, idx->stream, &idx->last_launches),
-                   "computing query norms");
             f.check = 1;
-            f.q_sq = qsq;
             f.max_x_sq = idx->max_x_sq;
             f.err_scale = 4.0f * float(idx->dim + 2) * 5.9604645e-8f;
             f.n_total = idx->n;
@@ -854,7 +849,6 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
     SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
-    SSG_CK(idx->qsq.ensure(size_t(chunk) * 4 + 16), "allocating query norms");
     const size_t tb = ssg::tc_tile_bytes(k3);
     const uint8_t *qtiles = static_cast<const uint8_t *>(idx->ps_dbq.p);
     if (!queries_are_db) {
@@ -896,7 +890,6 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     const float ulp24 = 5.9604645e-8f;
     int *flags = static_cast<int *>(idx->flags.p);
     int *flag_count = flags + m;
-    float *qsq = static_cast<float *>(idx->qsq.p);
     ScanTimer timer(idx);
     for (int64_t c0 = 0; c0 < m; c0 += chunk) {
         const int64_t mc = std::min<int64_t>(chunk, m - c0);
@@ -909,8 +902,6 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
                "launching the split tensor-core scan");
         SSG_RC(timer.end());
         const float *qc = dq + size_t(c0) * idx->dim;
-        SSG_CK(ssg::launch_row_sq_norms(qc, mc, idx->dim, qsq, qsq + chunk, idx->stream, &idx->last_launches),
-               "computing query norms");
         ssg::FinalizeArgs f{};
         SSG_RC(reduce_segments(idx, static_cast<const uint64_t *>(idx->cand.p), mc, segs, kk, &f.cand, &f.segs));
         f.kk = kk;
@@ -923,7 +914,6 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
         f.n_rows = idx->n;
         f.rerank = std::min(plan.rr, f.segs * kk);
         f.check = sq ? 1 : (idx->metric == SSG_METRIC_COSINE ? 3 : 2);
-        f.q_sq = qsq;
         f.max_x_sq = idx->max_x_sq;
         f.err_scale = sq ? 4.0f * float(idx->dim + 2) * ulp24 + 0.5f * c
                          : (f.check == 3 ? c + float(2 * idx->dim + 16) * ulp24 : c + float(idx->dim + 2) * ulp24);
@@ -1018,7 +1008,6 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
     SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
-    SSG_CK(idx->qsq.ensure(size_t(chunk) * 4 + 16), "allocating query norms");
     const size_t tb = 3 * ssg::stream_tile_bytes(idx->dim, 0);
     const uint8_t *qt = static_cast<const uint8_t *>(idx->pss_dbq.p);
     if (!queries_are_db) {
@@ -1039,7 +1028,6 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     const float ulp24 = 5.9604645e-8f;
     int *flags = static_cast<int *>(idx->flags.p);
     int *flag_count = flags + m;
-    float *qsq = static_cast<float *>(idx->qsq.p);
     ScanTimer timer(idx);
     for (int64_t c0 = 0; c0 < m; c0 += chunk) {
         const int64_t mc = std::min<int64_t>(chunk, m - c0);
@@ -1055,8 +1043,6 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
                "launching the split streaming scan");
         SSG_RC(timer.end());
         const float *qc = dq + size_t(c0) * idx->dim;
-        SSG_CK(ssg::launch_row_sq_norms(qc, mc, idx->dim, qsq, qsq + chunk, idx->stream, &idx->last_launches),
-               "computing query norms");
         ssg::FinalizeArgs f{};
         SSG_RC(reduce_segments(idx, static_cast<const uint64_t *>(idx->cand.p), mc, segs, kk, &f.cand, &f.segs));
         f.kk = kk;
@@ -1068,7 +1054,6 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
         f.out_dists = d_dists + size_t(c0) * k;
         f.n_rows = idx->n;
         f.check = sq ? 1 : (idx->metric == SSG_METRIC_COSINE ? 3 : 2);
-        f.q_sq = qsq;
         f.max_x_sq = idx->max_x_sq;
         f.err_scale = sq ? 4.0f * float(idx->dim + 2) * ulp24 + 0.5f * c
                          : (f.check == 3 ? c + float(2 * idx->dim + 16) * ulp24 : c + float(idx->dim + 2) * ulp24);
@@ -2552,7 +2537,7 @@ void ssg_destroy(ssg_index *idx) {
     for (DevBuf *b : {&idx->st_db, &idx->st_scale, &idx->st_alpha, &idx->st_beta, &idx->st_q, &idx->st_qscale,
                       &idx->red[0], &idx->red[1]})
         b->release();
-    for (DevBuf *b : {&idx->sq_norm, &idx->sq_max, &idx->flags, &idx->qsq, &idx->fb_list, &idx->fb_q, &idx->fb_out,
+    for (DevBuf *b : {&idx->sq_norm, &idx->sq_max, &idx->flags, &idx->fb_list, &idx->fb_q, &idx->fb_out,
                       &idx->fb_cand, &idx->fb_qn, &idx->tc_smp, &idx->tc_smp_norm, &idx->f_out, &idx->f_cnt,
                       &idx->f_thr, &idx->gbound, &idx->pack_q, &idx->pack_out, &idx->gm_db, &idx->gm_q,
                       &idx->ps_db, &idx->ps_dbq, &idx->ps_norm, &idx->ps_q, &idx->qbound, &idx->pss_db,

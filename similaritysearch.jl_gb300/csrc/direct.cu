@@ -192,39 +192,7 @@ cudaError_t launch_direct_f32(const ScanArgs &a, const float *db, const float *d
 #undef SSG_DIRECT_CASE
 }
 
-// ---------------------------------------------------------------------------
-// Finalize: merge per-split sorted key lists, cut to k, decode to the
-// reference's output form (1-based UInt32 ids, Float32 dists, 0 / Inf32 when
-// fewer than k exist -- src/SimilaritySearch.jl:309-313, allknn.jl:43-46).
-// ---------------------------------------------------------------------------
 namespace {
-
-__global__ void finalize_kernel(FinalizeArgs a, int P) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint64_t *s = reinterpret_cast<uint64_t *>(smem);
-    const int64_t j = blockIdx.x;
-    const int total = a.segs * a.kk;
-    const uint64_t *src = a.cand + size_t(j) * total;
-    for (int i = threadIdx.x; i < P; i += blockDim.x) s[i] = i < total ? src[i] : KEY_EMPTY;
-    if (a.segs > 1) block_bitonic_sort(s, P);
-    else __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t *oi = a.out_ids + size_t(j) * a.k_out;
-        float *od = a.out_dists + size_t(j) * a.k_out;
-        int w = 0;
-        const uint32_t self0 = uint32_t(a.self_ids ? a.self_ids[j] : j + a.self_base);
-        bool dropped = !a.exclude_self;
-        const int limit = a.k_out + (a.exclude_self ? 1 : 0);
-        for (int i = 0; i < limit && i < P && w < a.k_out; ++i) {
-            uint64_t key = s[i];
-            if (!dropped && key != KEY_EMPTY && key_id0(key) == self0) { dropped = true; continue; }
-            if (key == KEY_EMPTY) { oi[w] = 0; od[w] = INFINITY; }
-            else { oi[w] = key_id0(key) + 1; od[w] = key_dist(key); }
-            ++w;
-        }
-        for (; w < a.k_out; ++w) { oi[w] = 0; od[w] = INFINITY; }
-    }
-}
 
 // Merges groups of `group` sorted segments of kk keys into one sorted
 // segment of the group's kk smallest keys: the pass used when a query's
@@ -257,17 +225,6 @@ cudaError_t launch_merge_groups(const uint64_t *in, int64_t m, int segs, int kk,
     if (launches) *launches += 1;
     merge_groups_kernel<<<dim3(unsigned(m), unsigned(out_segs)), 256, smem, st>>>(in, segs, kk, group, out_segs, P,
                                                                                   out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_finalize(const FinalizeArgs &a, cudaStream_t st, int *launches) {
-    const int P = next_pow2(int64_t(a.segs) * a.kk);
-    size_t smem = size_t(P) * 8;
-    cudaError_t e = cudaFuncSetAttribute(finalize_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(smem));
-    if (e != cudaSuccess) return e;
-    if (launches) *launches += 1;
-    finalize_kernel<<<unsigned(a.m), 256, smem, st>>>(a, P);
     return cudaGetLastError();
 }
 

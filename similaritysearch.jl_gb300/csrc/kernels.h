@@ -65,7 +65,6 @@ struct FinalizeArgs {
     // of SqL2 / L2 (|x|^2 - 2 x.q), error err_scale (|x|max + |q|)^2; 2:
     // dot-product keys (-x.q), error err_scale |x|max |q|.
     int check = 0;
-    const float *q_sq = nullptr;   // |q|^2 per query
     float max_x_sq = 0.0f;         // max |x|^2 over the database (the metric's rows as stored)
     float err_scale = 0.0f;        // the error bound's scale (see the check's kinds above)
     int64_t n_total = 0;           // database rows

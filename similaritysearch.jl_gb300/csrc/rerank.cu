@@ -9,6 +9,9 @@
 #include "exact.cuh"
 #include "kernels.h"
 
+#include <algorithm>
+#include <climits>
+
 namespace ssg {
 
 namespace {
@@ -77,152 +80,588 @@ cudaError_t launch_rerank(int metric, const void *db, const float *db_norm, int6
 }
 
 // ---------------------------------------------------------------------------
-// Merge the per-split approximate candidates, re-rank them with the exact
-// FP32 distance and write the k best in (distance, id) order.
+// Finalize: select a query's best keys among its candidate segments, re-rank
+// them with the exact FP32 distance (RERANK) and write the k best in
+// (distance, id) order.
+//
+// What bounds it: for many queries the gather of the candidates' rows (C2:
+// 1e6 queries x 50 rows x 384 bytes = 19.2 GB); for few queries the latency
+// of one block.  So nothing here sorts the candidates: the `need` smallest of
+// a query's unique 64-bit keys are selected by bisection on the key's bits
+// (one compare and count per key and step), the rows of the selected
+// candidates stream through shared memory 32 dimensions at a time (coalesced
+// cp.async copies, three or four steps in flight), one thread then walks each
+// candidate's sequential fma chain, and the order is found by counting the
+// smaller keys.  Two shapes: a warp per query (up to 256 keys in, 64 out:
+// allknn and ordinary batches, where a block per query left most threads idle
+// at its barriers), a block per query beyond.  Against the block-wide bitonic sorts
+// with a thread per gathered row that stood here: C1's 1,000 queries x 684
+// keys 71 us (with the query norms' own launch) -> 26 us, one query of 5,472
+// keys 171 -> 21 us, 4,096 queries x 125 rows of 768 dimensions 1,229 ->
+// 391 us, C2's 1e6 queries x 50 rows of 96 10.2 -> 6.5 ms (3.0 TB/s of
+// gathered rows).
 // ---------------------------------------------------------------------------
 namespace {
 
-template <int METRIC>
-__global__ void finalize_rerank_kernel(FinalizeArgs f, const float *db, const float *db_norm, int64_t dim,
-                                       const float *q, const float *q_norm, int P1, int P2) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint64_t *s1 = reinterpret_cast<uint64_t *>(smem);
-    uint64_t *s2 = s1 + P1;
-    const int64_t j = blockIdx.x;
-    const int total = f.segs * f.kk;
-    const uint64_t *src = f.cand + size_t(j) * total;
-    for (int i = threadIdx.x; i < P1; i += blockDim.x) s1[i] = i < total ? src[i] : KEY_EMPTY;
-    if (f.segs > 1) block_bitonic_sort(s1, P1);
-    else __syncthreads();
-    const int rr = f.rerank ? f.rerank : f.kk;
-    for (int i = threadIdx.x; i < P2; i += blockDim.x) {
-        uint64_t key = KEY_EMPTY;
-        if (i < rr) {
-            const uint64_t ak = s1[i];
-            if (ak != KEY_EMPTY && int64_t(key_id0(ak)) < f.n_rows) {
-                const uint32_t id0 = key_id0(ak);
-                const float d = exact_pair<METRIC>(db, int64_t(id0), dim, q, j, db_norm, q_norm);
-                key = make_key(d, id0);
-            }
+constexpr int kDimStep = 32;               // dimensions staged per step
+constexpr int kRowStride = kDimStep + 4;   // floats: 16-byte rows, float4 reads of 8 lanes on distinct banks
+constexpr int kWarpKeys = 8;               // keys per lane in the warp shape (256 in all)
+constexpr int kWarpOut = 64;               // candidates re-ranked per query in the warp shape
+constexpr int kWarpsPerBlock = 4;
+constexpr int kWarpStages = 3;
+constexpr int kBlockThreads = 256;
+constexpr int kBlockRows = 128;            // candidates staged together in the block shape
+constexpr int kBlockStages = 4;
+
+struct RowSource {
+    const float *db, *q;  // database rows, this query's row
+    int dim;
+    bool vec;             // 16-byte copies: dim % 4 == 0 and both bases 16-byte aligned
+};
+
+// Copies dimensions [c0, c0 + kDimStep) of `rows` candidate rows (ids key_id0(sel[r]))
+// and of the query (row `rows`) into buf, `threads` threads taking part.
+__device__ __forceinline__ void stage_rows(const RowSource &s, const uint64_t *sel, int rows, int c0, float *buf,
+                                           int tid, int threads) {
+    if (s.vec) {
+        constexpr int per = kDimStep / 4;
+        for (int e = tid; e < (rows + 1) * per; e += threads) {
+            const int r = e / per, c = c0 + 4 * (e % per);
+            if (c >= s.dim) continue;
+            const float *src = (r < rows ? s.db + size_t(key_id0(sel[r])) * s.dim : s.q) + c;
+            const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(buf + r * kRowStride + (c - c0)));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
         }
-        s2[i] = key;
+    } else {
+        for (int e = tid; e < (rows + 1) * kDimStep; e += threads) {
+            const int r = e / kDimStep, c = c0 + e % kDimStep;
+            if (c >= s.dim) continue;
+            const float *src = (r < rows ? s.db + size_t(key_id0(sel[r])) * s.dim : s.q) + c;
+            const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(buf + r * kRowStride + (c - c0)));
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+        }
     }
-    block_bitonic_sort(s2, P2);
-    if (f.check && threadIdx.x == 0) {
-        // Completeness of an approximate candidate list.  An object y left
-        // out was either dropped by a full heap (or a merge of segments), so
-        // its approximate key a(y) is at least that segment's last key, or
-        // sits in a segment behind the re-ranked list: a(y) >= a_low =
-        // min(last key of every full segment, last re-ranked key).  Its exact
-        // FP32 distance D(y) >= a(y) + c - E, where c turns keys into
-        // distances and E bounds the approximation and evaluation errors:
-        //   check 1 (keys |x|^2 - 2 x.q of SqL2 / L2): c = |q|^2,
-        //           E = err_scale (R + |q|)^2, R a bound on |y| for every y
-        //           that could rank at or before the take-th candidate:
-        //           |y - q|^2 <= D_take (up to the FP32 evaluation's relative
-        //           error t^2 = (d + 2) 2^-24 of (|y| + |q|)^2) gives
-        //           |y| <= ((1 + t) |q| + sqrt(D_take)) / (1 - t), and
-        //           |y| <= sqrt(max |x|^2) always;
-        //   check 2 (keys -x.q): c = 1 for NormCosine, 0 for InnerProduct,
-        //           E = err_scale sqrt(max |x|^2) |q| + 2^-22;
-        //   check 3 (Cosine's keys -x.q / |x|): distances 1 + a / |q|, so
-        //           a_low enters as 1 + a_low / |q| and E = err_scale (the
-        //           split's c plus the FP32 dot, norms, division and
-        //           subtraction, (2 d + 16) 2^-24, all relative to 1).
-        // If a_low + c - E exceeds the exact distance of the take-th
-        // re-ranked candidate (for L2 its square, widened by 2^-20 so that
-        // sqrt rounding cannot tie), y ranks behind it: the list holds the
-        // exact top `take`.  Evaluated in double.
-        // A list shorter than rr (heaps that a shared bound kept from
-        // filling) holds every candidate no heap dropped: a_low is then the
-        // full segments' smallest last key alone.  A list that holds every
-        // row needs no check; one shorter than `take` cannot be certified.
-        const int take = f.k_out + (f.exclude_self ? 1 : 0);
-        int nv = 0;
-        while (nv < rr && s1[nv] != KEY_EMPTY) ++nv;
-        if (int64_t(nv) < f.n_total) {
-            uint64_t low = nv == rr ? s1[rr - 1] : KEY_EMPTY;
-            for (int sgi = 0; sgi < f.segs; ++sgi) {
-                const uint64_t last = src[size_t(sgi) * f.kk + f.kk - 1];
-                if (last != KEY_EMPTY && last < low) low = last;
+}
+
+// Continues the sequential chain of one staged row over `dims` dimensions:
+// squared difference or product, in index order, one fma each.  qs = 0 turns
+// the squared difference into the row's own square (the query's |q|^2).
+template <int METRIC>
+__device__ __forceinline__ float chain_step(float acc, const float *x, const float *q, int dims, float qs) {
+    auto one = [&](float a, float b) {
+        if constexpr (METRIC == SQL2 || METRIC == L2) {
+            const float m = a - b * qs;
+            acc = fmaf(m, m, acc);
+        } else {
+            acc = fmaf(a, b, acc);
+        }
+    };
+    if (dims == kDimStep) {
+#pragma unroll
+        for (int c = 0; c < kDimStep; c += 4) {
+            const float4 a = *reinterpret_cast<const float4 *>(x + c);
+            const float4 b = *reinterpret_cast<const float4 *>(q + c);
+            one(a.x, b.x); one(a.y, b.y); one(a.z, b.z); one(a.w, b.w);
+        }
+    } else {
+        for (int c = 0; c < dims; ++c) one(x[c], q[c]);
+    }
+    return acc;
+}
+
+template <int METRIC>
+__device__ __forceinline__ float chain_distance(float acc, uint32_t id0, const float *xn, float qn) {
+    if constexpr (METRIC == SQL2) return acc;
+    if constexpr (METRIC == L2) return sqrtf(acc);
+    if constexpr (METRIC == NORMCOSINE) return 1.0f - acc;
+    if constexpr (METRIC == IP) return -acc;
+    return 1.0f - acc / (xn[id0] * qn);
+}
+
+// Completeness of an approximate candidate list.  An object y left out was
+// either dropped by a full heap (or a merge of segments), so its approximate
+// key a(y) is at least that segment's last key, or sits in a segment behind
+// the re-ranked list: a(y) >= a_low = min(last key of every full segment,
+// last re-ranked key).  Its exact FP32 distance D(y) >= a(y) + c - E, where
+// c turns keys into distances and E bounds the approximation and evaluation
+// errors:
+//   check 1 (keys |x|^2 - 2 x.q of SqL2 / L2): c = |q|^2,
+//           E = err_scale (R + |q|)^2, R a bound on |y| for every y
+//           that could rank at or before the take-th candidate:
+//           |y - q|^2 <= D_take (up to the FP32 evaluation's relative
+//           error t^2 = (d + 2) 2^-24 of (|y| + |q|)^2) gives
+//           |y| <= ((1 + t) |q| + sqrt(D_take)) / (1 - t), and
+//           |y| <= sqrt(max |x|^2) always;
+//   check 2 (keys -x.q): c = 1 for NormCosine, 0 for InnerProduct,
+//           E = err_scale sqrt(max |x|^2) |q| + 2^-22;
+//   check 3 (Cosine's keys -x.q / |x|): distances 1 + a / |q|, so
+//           a_low enters as 1 + a_low / |q| and E = err_scale (the
+//           split's c plus the FP32 dot, norms, division and
+//           subtraction, (2 d + 16) 2^-24, all relative to 1).
+// If a_low + c - E exceeds the exact distance of the take-th re-ranked
+// candidate (for L2 its square, widened by 2^-20 so that sqrt rounding
+// cannot tie), y ranks behind it: the list holds the exact top `take`.
+// Evaluated in double.  A list shorter than asked for (heaps that a shared
+// bound kept from filling) holds every candidate no heap dropped: a_low is
+// then the full segments' smallest last key alone.  A list that holds every
+// row needs no check (the caller's business); one shorter than `take`
+// cannot be certified.  low: a_low's key, KEY_EMPTY if there is none.
+template <int METRIC>
+__device__ bool list_complete(const FinalizeArgs &f, int64_t dim, int nv, uint64_t low, float q_sq, float d_take) {
+    const int take = f.k_out + (f.exclude_self ? 1 : 0);
+    if (nv < take || low == KEY_EMPTY) return false;
+    const double qs = double(q_sq);
+    const double xm = sqrt(double(f.max_x_sq));
+    double dtake = double(d_take);
+    if (METRIC == L2) dtake = dtake * dtake * (1.0 + 9.5367431640625e-7);
+    double c, E;
+    if (f.check == 1) {
+        double r = xm + sqrt(qs);
+        if (dtake >= 0.0) {
+            const double t = sqrt(double(dim + 2) * 5.9604644775390625e-8);
+            r = fmin(xm, ((1.0 + t) * sqrt(qs) + sqrt(dtake)) / (1.0 - t)) + sqrt(qs);
+        }
+        c = qs;
+        E = double(f.err_scale) * r * r;
+    } else if (f.check == 3) {
+        c = 1.0;
+        E = double(f.err_scale);
+    } else {
+        c = METRIC == NORMCOSINE ? 1.0 : 0.0;
+        E = double(f.err_scale) * xm * sqrt(qs) + 2.384185791015625e-7;
+    }
+    const double a_low = f.check == 3 ? double(key_dist(low)) / sqrt(qs) : double(key_dist(low));
+    return a_low + c - E > dtake;
+}
+
+// Writes the result row from the sorted keys: the object itself left out when
+// exclude_self finds it among the first k_out + 1, 0 / +Inf past the end.
+// `at` is the calling thread's number of `threads`; self_pos (a place in
+// sorted, or a large number) comes from the caller.
+__device__ __forceinline__ void write_row(const FinalizeArgs &f, int64_t j, const uint64_t *sorted, int nv,
+                                          int self_pos, int at, int threads) {
+    uint32_t *oi = f.out_ids + size_t(j) * f.k_out;
+    float *od = f.out_dists + size_t(j) * f.k_out;
+    for (int w = at; w < f.k_out; w += threads) {
+        const int i = w + (self_pos <= w ? 1 : 0);
+        const uint64_t key = i < nv ? sorted[i] : KEY_EMPTY;
+        oi[w] = key == KEY_EMPTY ? 0u : key_id0(key) + 1;
+        od[w] = key == KEY_EMPTY ? INFINITY : key_dist(key);
+    }
+}
+
+__device__ __forceinline__ uint32_t self_id(const FinalizeArgs &f, int64_t j) {
+    return uint32_t(f.self_ids ? f.self_ids[j] : j + f.self_base);
+}
+
+__device__ __forceinline__ uint64_t warp_min64(uint64_t v) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t w = __shfl_xor_sync(0xffffffffu, v, o);
+        if (w < v) v = w;
+    }
+    return v;
+}
+__device__ __forceinline__ uint64_t warp_max64(uint64_t v) {
+    for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t w = __shfl_xor_sync(0xffffffffu, v, o);
+        if (w > v) v = w;
+    }
+    return v;
+}
+
+// A warp per query: its segs * kk <= 32 * kWarpKeys keys in registers.
+template <int METRIC, bool RERANK>
+__global__ void __launch_bounds__(32 * kWarpsPerBlock)
+finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *__restrict__ db_norm, int64_t dim,
+                     const float *__restrict__ q, const float *__restrict__ q_norm, int need, int vec) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint64_t s_sel[kWarpsPerBlock][kWarpOut];
+    __shared__ uint64_t s_key[kWarpsPerBlock][kWarpOut];
+    // the certificates of the block's queries, evaluated side by side: one
+    // lane alone would hold the FP64 pipe for as long as eight
+    __shared__ uint64_t s_low[kWarpsPerBlock];
+    __shared__ float s_qsq[kWarpsPerBlock], s_take[kWarpsPerBlock];
+    __shared__ int s_nv[kWarpsPerBlock];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int64_t j = int64_t(blockIdx.x) * kWarpsPerBlock + warp;
+    const bool live = j < f.m;
+    uint64_t *sel = s_sel[warp], *out = s_key[warp];
+    if (live) {
+        const int total = f.segs * f.kk;
+        const uint64_t *src = f.cand + size_t(j) * total;
+        uint64_t key[kWarpKeys];
+        int cnt = 0;
+#pragma unroll
+        for (int i = 0; i < kWarpKeys; ++i) {
+            const int at = i * 32 + lane;
+            key[i] = at < total ? src[at] : KEY_EMPTY;
+            if (RERANK && int64_t(key_id0(key[i])) >= f.n_rows) key[i] = KEY_EMPTY;
+            cnt += key[i] != KEY_EMPTY;
+        }
+        const int nvt = __reduce_add_sync(0xffffffffu, cnt);
+        uint64_t low = KEY_EMPTY;
+        if (RERANK && f.check) {
+            for (int s = lane; s < f.segs; s += 32) low = min(low, src[size_t(s) * f.kk + f.kk - 1]);
+            low = warp_min64(low);
+        }
+        const int nv = min(need, nvt);
+        // below: every selected key is smaller; found bit by bit from the top
+        uint64_t below = KEY_EMPTY;
+        if (nvt > need) {
+            uint64_t mx = 0, mn = KEY_EMPTY;
+#pragma unroll
+            for (int i = 0; i < kWarpKeys; ++i) {
+                mn = min(mn, key[i]);
+                if (key[i] != KEY_EMPTY) mx = max(mx, key[i]);
             }
-            bool certified = nv >= take && low != KEY_EMPTY;
-            const double qs = double(f.q_sq[j]);
-            const double xm = sqrt(double(f.max_x_sq));
-            double c, E;
-            if (f.check == 1) {
-                const double r = xm + sqrt(qs);
-                c = qs;
-                E = double(f.err_scale) * r * r;
-            } else if (f.check == 3) {
-                c = 1.0;
-                E = double(f.err_scale);
-            } else {
-                c = METRIC == NORMCOSINE ? 1.0 : 0.0;
-                E = double(f.err_scale) * xm * sqrt(qs) + 2.384185791015625e-7;
+            mn = warp_min64(mn);
+            mx = warp_max64(mx);
+            const int top = 63 - __clzll(mn ^ mx);
+            uint64_t p = top >= 63 ? 0ull : (mn >> (top + 1)) << (top + 1);
+            bool done = false;
+            for (int b = top; b >= 0; --b) {
+                const uint64_t t = p | (1ull << b);
+                int c = 0;
+#pragma unroll
+                for (int i = 0; i < kWarpKeys; ++i) c += key[i] < t;
+                c = __reduce_add_sync(0xffffffffu, c);
+                if (c == need) { below = t; done = true; break; }
+                if (c < need) p = t;
             }
-            double dtake = certified ? double(key_dist(s2[take - 1])) : 0.0;
-            if (METRIC == L2) dtake = dtake * dtake * (1.0 + 9.5367431640625e-7);
-            if (f.check == 1 && dtake >= 0.0) {
-                const double t = sqrt(double(dim + 2) * 5.9604644775390625e-8);
-                const double r = fmin(xm, ((1.0 + t) * sqrt(qs) + sqrt(dtake)) / (1.0 - t)) + sqrt(qs);
-                E = double(f.err_scale) * r * r;
+            if (!done) below = p + 1;
+        }
+        int base = 0;
+#pragma unroll
+        for (int i = 0; i < kWarpKeys; ++i) {
+            const bool take = key[i] < below;
+            const uint32_t vote = __ballot_sync(0xffffffffu, take);
+            const int at = base + __popc(vote & ((1u << lane) - 1u));
+            if (take && at < need) sel[at] = key[i];
+            base += __popc(vote);
+        }
+        __syncwarp();
+        uint64_t k0 = KEY_EMPTY, k1 = KEY_EMPTY;  // this lane's candidates lane, lane + 32
+        if (lane < nv) k0 = sel[lane];
+        if (lane + 32 < nv) k1 = sel[lane + 32];
+        if constexpr (RERANK) {
+            if (f.check && nv == need) {
+                uint64_t last = lane < nv ? k0 : 0;
+                if (lane + 32 < nv) last = max(last, k1);
+                low = min(low, warp_max64(last));
             }
-            const double a_low = f.check == 3 ? double(key_dist(low)) / sqrt(qs) : double(key_dist(low));
-            const double lower = certified ? a_low + c - E : 0.0;
-            if (!certified || !(lower > dtake)) {
-                f.flags[j] = 1;
+            // the query's row is staged behind the candidates; the lane of
+            // that row sums |q|^2 for the certificate
+            const int rows_s = need + 1;
+            float *ring = reinterpret_cast<float *>(smem) + size_t(warp) * kWarpStages * rows_s * kRowStride;
+            const RowSource rs{db, q + size_t(j) * dim, int(dim), vec != 0};
+            const int steps = (int(dim) + kDimStep - 1) / kDimStep;
+            float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
+            const float s0 = lane == nv ? 0.0f : 1.0f, s1 = lane + 32 == nv ? 0.0f : 1.0f;
+#pragma unroll
+            for (int p = 0; p < kWarpStages - 1; ++p) {
+                if (p < steps) stage_rows(rs, sel, nv, p * kDimStep, ring + size_t(p) * rows_s * kRowStride, lane, 32);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            for (int c = 0; c < steps; ++c) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kWarpStages - 2) : "memory");
+                __syncwarp();
+                const int nx = c + kWarpStages - 1;
+                if (nx < steps)
+                    stage_rows(rs, sel, nv, nx * kDimStep, ring + size_t(nx % kWarpStages) * rows_s * kRowStride, lane,
+                               32);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                const float *buf = ring + size_t(c % kWarpStages) * rows_s * kRowStride;
+                const float *qr = buf + nv * kRowStride;
+                const int dims = min(kDimStep, int(dim) - c * kDimStep);
+                if (lane <= nv) a0 = chain_step<METRIC>(a0, buf + lane * kRowStride, qr, dims, s0);
+                if (lane + 32 <= nv) a1 = chain_step<METRIC>(a1, buf + (lane + 32) * kRowStride, qr, dims, s1);
+                if (nv == 64 && lane == 0) a2 = chain_step<METRIC>(a2, qr, qr, dims, 0.0f);
+            }
+            const float qn = METRIC == COSINE ? q_norm[j] : 0.0f;
+            if (k0 != KEY_EMPTY) k0 = make_key(chain_distance<METRIC>(a0, key_id0(k0), db_norm, qn), key_id0(k0));
+            if (k1 != KEY_EMPTY) k1 = make_key(chain_distance<METRIC>(a1, key_id0(k1), db_norm, qn), key_id0(k1));
+            if (lane == nv) s_qsq[warp] = a0;
+            if (lane + 32 == nv) s_qsq[warp] = a1;
+            if (nv == 64 && lane == 0) s_qsq[warp] = a2;
+            __syncwarp();
+            sel[lane] = k0;
+            if (lane + 32 < kWarpOut) sel[lane + 32] = k1;
+            __syncwarp();
+        }
+        // place by counting the smaller keys (ids make them unique)
+        int r0 = 0, r1 = 0;
+        for (int i = 0; i < nv; ++i) {
+            const uint64_t v = sel[i];
+            r0 += v < k0;
+            r1 += v < k1;
+        }
+        __syncwarp();
+        if (lane < nv) out[r0] = k0;
+        if (lane + 32 < nv) out[r1] = k1;
+        __syncwarp();
+        int self_pos = INT_MAX;
+        if (f.exclude_self) {
+            const uint32_t id = self_id(f, j);
+            const int limit = min(nv, f.k_out + 1);
+            for (int i = lane; i < limit; i += 32)
+                if (key_id0(out[i]) == id) self_pos = i;
+            self_pos = __reduce_min_sync(0xffffffffu, self_pos);
+        }
+        write_row(f, j, out, nv, self_pos, lane, 32);
+        if (RERANK && f.check && lane == 0) {
+            const int take = f.k_out + (f.exclude_self ? 1 : 0);
+            s_low[warp] = low;
+            s_nv[warp] = nv;
+            s_take[warp] = nv >= take ? key_dist(out[take - 1]) : 0.0f;
+        }
+    }
+    if constexpr (RERANK) {
+        if (!f.check) return;
+        __syncthreads();
+        const int64_t jq = int64_t(blockIdx.x) * kWarpsPerBlock + threadIdx.x;
+        if (threadIdx.x < kWarpsPerBlock && jq < f.m) {
+            const int nv = s_nv[threadIdx.x];
+            if (int64_t(nv) < f.n_total &&
+                !list_complete<METRIC>(f, dim, nv, s_low[threadIdx.x], s_qsq[threadIdx.x], s_take[threadIdx.x])) {
+                f.flags[jq] = 1;
                 atomicAdd(f.flag_count, 1);
             }
         }
     }
-    if (threadIdx.x == 0) {
-        uint32_t *oi = f.out_ids + size_t(j) * f.k_out;
-        float *od = f.out_dists + size_t(j) * f.k_out;
-        int w = 0;
-        const uint32_t self0 = uint32_t(f.self_ids ? f.self_ids[j] : j + f.self_base);
-        bool dropped = !f.exclude_self;
-        const int limit = f.k_out + (f.exclude_self ? 1 : 0);
-        for (int i = 0; i < limit && i < P2 && w < f.k_out; ++i) {
-            const uint64_t key = s2[i];
-            if (!dropped && key != KEY_EMPTY && key_id0(key) == self0) { dropped = true; continue; }
-            if (key == KEY_EMPTY) { oi[w] = 0; od[w] = INFINITY; }
-            else { oi[w] = key_id0(key) + 1; od[w] = key_dist(key); }
-            ++w;
-        }
-        for (; w < f.k_out; ++w) { oi[w] = 0; od[w] = INFINITY; }
+}
+
+// A block per query.  cap: room for keys in shared memory (every key of the
+// query); sel_cap: room for the selected ones (0: they take the keys' place,
+// when nothing is left out).
+template <int METRIC, bool RERANK>
+__global__ void __launch_bounds__(kBlockThreads)
+finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float *__restrict__ db_norm, int64_t dim,
+                      const float *__restrict__ q, const float *__restrict__ q_norm, int need, int cap, int sel_cap,
+                      int vec) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint64_t *keys = reinterpret_cast<uint64_t *>(smem);
+    uint64_t *sel = sel_cap ? keys + cap : keys;
+    uint64_t *out = sel_cap ? sel + sel_cap : keys + cap;  // as long as sel
+    float *ring = reinterpret_cast<float *>(out + (sel_cap ? sel_cap : cap));
+    __shared__ int s_cnt[3], s_n, s_self;
+    __shared__ unsigned long long s_min, s_max, s_low, s_last;
+    __shared__ float s_qsq;
+    const int tid = threadIdx.x, lane = tid % 32;
+    const int64_t j = blockIdx.x;
+    const int total = f.segs * f.kk;
+    const uint64_t *src = f.cand + size_t(j) * total;
+    if (tid == 0) {
+        s_n = 0;
+        s_cnt[0] = s_cnt[1] = s_cnt[2] = 0;
+        s_min = s_low = KEY_EMPTY;
+        s_max = s_last = 0;
+        s_self = INT_MAX;
     }
+    __syncthreads();
+    // the query's keys, empty slots left out
+    uint64_t mn = KEY_EMPTY, mx = 0;
+    for (int i0 = 0; i0 < total; i0 += kBlockThreads) {
+        const int i = i0 + tid;
+        uint64_t key = i < total ? src[i] : KEY_EMPTY;
+        if (RERANK && int64_t(key_id0(key)) >= f.n_rows) key = KEY_EMPTY;
+        const bool have = key != KEY_EMPTY;
+        const uint32_t vote = __ballot_sync(0xffffffffu, have);
+        int base = 0;
+        if (lane == 0 && vote) base = atomicAdd(&s_n, __popc(vote));
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (have) {
+            keys[base + __popc(vote & ((1u << lane) - 1u))] = key;
+            mn = min(mn, key);
+            mx = max(mx, key);
+        }
+    }
+    mn = warp_min64(mn);
+    mx = warp_max64(mx);
+    uint64_t low = KEY_EMPTY;
+    if (RERANK && f.check) {
+        for (int s = tid; s < f.segs; s += kBlockThreads) low = min(low, src[size_t(s) * f.kk + f.kk - 1]);
+        low = warp_min64(low);
+    }
+    if (lane == 0) {
+        atomicMin(&s_min, mn);
+        atomicMax(&s_max, mx);
+        if (RERANK && f.check) atomicMin(&s_low, low);
+    }
+    __syncthreads();
+    const int nvt = s_n;
+    const int nv = min(need, nvt);
+    if (nvt > need) {
+        const uint64_t lo = s_min, hi = s_max;
+        const int top = 63 - __clzll(lo ^ hi);
+        uint64_t p = top >= 63 ? 0ull : (lo >> (top + 1)) << (top + 1), below = KEY_EMPTY;
+        bool done = false;
+        int it = 0;
+        for (int b = top; b >= 0; --b, ++it) {
+            const uint64_t t = p | (1ull << b);
+            int c = 0;
+            for (int i = tid; i < nvt; i += kBlockThreads) c += keys[i] < t;
+            c = __reduce_add_sync(0xffffffffu, c);
+            int *slot = &s_cnt[it % 3];
+            if (lane == 0 && c) atomicAdd(slot, c);
+            __syncthreads();
+            c = *slot;
+            if (tid == 0) s_cnt[(it + 2) % 3] = 0;  // read by all before the last barrier, written after the next
+            if (c == need) { below = t; done = true; break; }
+            if (c < need) p = t;
+        }
+        if (!done) below = p + 1;
+        __syncthreads();
+        if (tid == 0) s_n = 0;
+        __syncthreads();
+        for (int i0 = 0; i0 < nvt; i0 += kBlockThreads) {
+            const int i = i0 + tid;
+            const uint64_t key = i < nvt ? keys[i] : KEY_EMPTY;
+            const bool take = key < below;
+            const uint32_t vote = __ballot_sync(0xffffffffu, take);
+            int base = 0;
+            if (lane == 0 && vote) base = atomicAdd(&s_n, __popc(vote));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            const int at = base + __popc(vote & ((1u << lane) - 1u));
+            if (take && at < need) sel[at] = key;
+        }
+        __syncthreads();
+    } else if (sel != keys) {
+        for (int i = tid; i < nv; i += kBlockThreads) sel[i] = keys[i];
+        __syncthreads();
+    }
+    if constexpr (RERANK) {
+        if (f.check && nv == need) {
+            uint64_t last = 0;
+            for (int i = tid; i < nv; i += kBlockThreads) last = max(last, sel[i]);
+            last = warp_max64(last);
+            if (lane == 0) atomicMax(&s_last, last);
+            __syncthreads();
+            if (tid == 0 && s_last < s_low) s_low = s_last;
+        }
+        const RowSource rs{db, q + size_t(j) * dim, int(dim), vec != 0};
+        const int steps = (int(dim) + kDimStep - 1) / kDimStep;
+        const float qn = METRIC == COSINE ? q_norm[j] : 0.0f;
+        const int rows_s = min(need, kBlockRows) + 1;
+        for (int r0 = 0; r0 < nv || r0 == 0; r0 += kBlockRows) {
+            const int rows = min(kBlockRows, nv - r0);
+            float acc = 0.0f;
+            const float qs = tid == rows ? 0.0f : 1.0f;
+#pragma unroll
+            for (int p = 0; p < kBlockStages - 1; ++p) {
+                if (p < steps)
+                    stage_rows(rs, sel + r0, rows, p * kDimStep, ring + size_t(p) * rows_s * kRowStride, tid,
+                               kBlockThreads);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+            for (int c = 0; c < steps; ++c) {
+                asm volatile("cp.async.wait_group %0;" ::"n"(kBlockStages - 2) : "memory");
+                __syncthreads();
+                const int nx = c + kBlockStages - 1;
+                if (nx < steps)
+                    stage_rows(rs, sel + r0, rows, nx * kDimStep,
+                               ring + size_t(nx % kBlockStages) * rows_s * kRowStride, tid, kBlockThreads);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                const float *buf = ring + size_t(c % kBlockStages) * rows_s * kRowStride;
+                if (tid <= rows)
+                    acc = chain_step<METRIC>(acc, buf + tid * kRowStride, buf + rows * kRowStride,
+                                             min(kDimStep, int(dim) - c * kDimStep), qs);
+            }
+            if (tid < rows) {
+                const uint32_t id0 = key_id0(sel[r0 + tid]);
+                out[r0 + tid] = make_key(chain_distance<METRIC>(acc, id0, db_norm, qn), id0);
+            }
+            if (r0 == 0 && tid == rows) s_qsq = acc;  // the query's row: |q|^2
+            __syncthreads();  // the ring is refilled
+        }
+        uint64_t *t = sel;
+        sel = out;
+        out = t;
+    }
+    // place by counting the smaller keys; long lists by a bitonic sort
+    if (nv <= 512) {
+        for (int i = tid; i < nv; i += kBlockThreads) {
+            const uint64_t v = sel[i];
+            int r = 0;
+            for (int k = 0; k < nv; ++k) r += sel[k] < v;
+            out[r] = v;
+        }
+        __syncthreads();
+    } else {
+        int P = 1024;
+        while (P < nv) P <<= 1;
+        for (int i = tid; i < P; i += kBlockThreads) out[i] = i < nv ? sel[i] : KEY_EMPTY;
+        block_bitonic_sort(out, P);
+    }
+    if (f.exclude_self) {
+        const uint32_t id = self_id(f, j);
+        const int limit = min(nv, f.k_out + 1);
+        for (int i = tid; i < limit; i += kBlockThreads)
+            if (key_id0(out[i]) == id) atomicMin(&s_self, i);
+        __syncthreads();
+    }
+    write_row(f, j, out, nv, s_self, tid, kBlockThreads);
+    if (RERANK && f.check && tid == 0 && int64_t(nv) < f.n_total) {
+        const int take = f.k_out + (f.exclude_self ? 1 : 0);
+        if (!list_complete<METRIC>(f, dim, nv, s_low, s_qsq, nv >= take ? key_dist(out[take - 1]) : 0.0f)) {
+            f.flags[j] = 1;
+            atomicAdd(f.flag_count, 1);
+        }
+    }
+}
+
+template <int METRIC, bool RERANK>
+cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const float *db_norm, int64_t dim,
+                              const float *q, const float *q_norm, int need, cudaStream_t st) {
+    const int total = f.segs * f.kk;
+    const bool vec = RERANK && dim % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(db) | reinterpret_cast<uintptr_t>(q)) & 15) == 0;
+    if (total <= 32 * kWarpKeys && need <= kWarpOut) {
+        const size_t smem = RERANK ? size_t(kWarpsPerBlock) * kWarpStages * (need + 1) * kRowStride * 4 : 0;
+        auto kern = finalize_warp_kernel<METRIC, RERANK>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+        if (e != cudaSuccess) return e;
+        const unsigned blocks = unsigned((f.m + kWarpsPerBlock - 1) / kWarpsPerBlock);
+        kern<<<blocks, 32 * kWarpsPerBlock, smem, st>>>(f, db, db_norm, dim, q, q_norm, need, vec ? 1 : 0);
+        return cudaGetLastError();
+    }
+    // the sorted order of more than 512 selected keys takes a power of two
+    const int out_cap = need <= 512 ? (need + 1) / 2 * 2 : next_pow2(need);  // even: the ring behind is 16-byte aligned
+    const bool in_place = total <= need;
+    const int cap = in_place ? std::max((total + 1) / 2 * 2, out_cap) : (total + 1) / 2 * 2;
+    const size_t keys = in_place ? 2 * size_t(cap) : size_t(cap) + 2 * size_t(out_cap);
+    const size_t ring = RERANK ? size_t(kBlockStages) * (std::min(need, kBlockRows) + 1) * kRowStride * 4 : 0;
+    const size_t smem = keys * 8 + ring;
+    if (smem > 226 * 1024) return cudaErrorInvalidValue;
+    auto kern = finalize_block_kernel<METRIC, RERANK>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    kern<<<unsigned(f.m), kBlockThreads, smem, st>>>(f, db, db_norm, dim, q, q_norm, need, cap,
+                                                     in_place ? 0 : out_cap, vec ? 1 : 0);
+    return cudaGetLastError();
 }
 
 }  // namespace
 
+cudaError_t launch_finalize(const FinalizeArgs &f, cudaStream_t st, int *launches) {
+    const int need = std::min(f.segs * f.kk, f.k_out + (f.exclude_self ? 1 : 0));
+    if (launches) *launches += 1;
+    return launch_finalize_t<SQL2, false>(f, nullptr, nullptr, 0, nullptr, nullptr, need, st);
+}
+
 cudaError_t launch_finalize_rerank(int metric, const FinalizeArgs &f, const float *db, const float *db_norm,
                                    int64_t dim, const float *q, const float *q_norm, cudaStream_t st,
                                    int *launches) {
-    const int P1 = next_pow2(int64_t(f.segs) * f.kk);
     const int rr = f.rerank ? f.rerank : f.kk;
     if (rr > f.segs * f.kk) return cudaErrorInvalidValue;
-    const int P2 = next_pow2(rr);
-    const size_t smem = size_t(P1 + P2) * 8;
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
     if (launches) *launches += 1;
-#define SSG_FR(MET)                                                                                      \
-    case MET: {                                                                                          \
-        cudaError_t e = cudaFuncSetAttribute(finalize_rerank_kernel<MET>,                                \
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));   \
-        if (e != cudaSuccess) return e;                                                                  \
-        finalize_rerank_kernel<MET><<<unsigned(f.m), 128, smem, st>>>(f, db, db_norm, dim, q, q_norm, P1, P2); \
-        return cudaGetLastError();                                                                       \
-    }
     switch (metric) {
-        SSG_FR(SQL2)
-        SSG_FR(L2)
-        SSG_FR(NORMCOSINE)
-        SSG_FR(COSINE)
-        SSG_FR(IP)
+        case SQL2: return launch_finalize_t<SQL2, true>(f, db, db_norm, dim, q, q_norm, rr, st);
+        case L2: return launch_finalize_t<L2, true>(f, db, db_norm, dim, q, q_norm, rr, st);
+        case NORMCOSINE: return launch_finalize_t<NORMCOSINE, true>(f, db, db_norm, dim, q, q_norm, rr, st);
+        case COSINE: return launch_finalize_t<COSINE, true>(f, db, db_norm, dim, q, q_norm, rr, st);
+        case IP: return launch_finalize_t<IP, true>(f, db, db_norm, dim, q, q_norm, rr, st);
         default: return cudaErrorInvalidValue;
     }
-#undef SSG_FR
 }
 
 }  // namespace ssg
