@@ -126,6 +126,11 @@ struct ssg_index {
     // database (both roles), its epilogue coefficients, the queries' tiles
     DevBuf pss_db, pss_dbq, pss_alpha, pss_beta, pss_q;
     int64_t pss_rows = -1, pss_qrows = -1;
+    // list scan (tc_list.cu): candidate lists, their counts, the seed's group
+    // minima; +-1 FP8 tiles of the sketches (built for sk_rows rows) and of
+    // the current queries
+    DevBuf l_lists, l_counts, l_minima, sk_db, sk_q;
+    int64_t sk_rows = -1;
     int plain_tc_param = 1;
     int last_plain_tc = 0;  // 1: the last plain-method search ran on the tensor cores
     int64_t smp_r = 0, smp_n = -1, smp_rows = 0;
@@ -417,6 +422,46 @@ int64_t wave_splits(int64_t qctas, int64_t cap, int64_t max_s) {
     return best;
 }
 
+// How a list scan (tc_list.cu) of kk candidates for m queries runs.
+struct ListPlan {
+    int splits = 0, cap = 0, groups = 0, fine = 0, keys = 0;
+    int64_t samples = 0, stride = 0;
+    int64_t chunk = 0;  // queries per pass: the lists stay within 1 GiB
+};
+
+// False when the scan does not apply: too few whole wide tiles for a bound
+// (four groups of columns per candidate from at most a quarter of the
+// database), or lists longer than a list's room.
+bool list_plan(const ssg_index *idx, int64_t m, int kk, ListPlan *p) {
+    const int64_t n_full = idx->n / 256, n_wide = (idx->n + 255) / 256;
+    if (kk > (ssg::kListMaxCap - 64) / 2 || n_full < 8) return false;
+    // The sample costs its share of a scan, and a bound from one row in f
+    // lets about 1.2 kk f candidates per query through.  With few queries the
+    // scan reads memory and hardly appends: a smaller sample.
+    const int64_t f = m > 256 ? 8 : 16;
+    const int64_t least = (int64_t(4) * kk + 7) / 8;  // wide tiles for 4 kk groups of 32 columns
+    if (least > n_full / 4) return false;
+    p->samples = std::max<int64_t>(least, n_full / f);
+    p->stride = n_full / p->samples;
+    p->fine = 2 * p->samples < 4 * kk;
+    p->groups = int(p->samples * (p->fine ? 8 : 2));
+    const int64_t qtiles = (m + 127) / 128;
+    const int64_t pairs = (qtiles + 1) / 2;
+    int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(pairs, ssg::device_sm_count() / 2, n_wide);
+    splits = std::max<int64_t>(1, std::min<int64_t>(splits, n_wide));
+    p->splits = int(splits);
+    const int64_t expect = int64_t(1.25 * kk * double(n_wide) / double(p->samples)) + kk;
+    const int64_t cap = std::max<int64_t>(2 * kk + 64, 4 * expect / (2 * splits) + 64);
+    p->cap = int(std::min<int64_t>(ssg::kListMaxCap, std::max<int64_t>(128, (cap + 31) / 32 * 32)));
+    int64_t keys = 1024;
+    while (keys < 2 * expect && keys < 8192) keys *= 2;
+    p->keys = int(keys);
+    const size_t per_query = size_t(2 * splits) * p->cap * 8;
+    p->chunk = std::max<int64_t>(256, int64_t((size_t(1) << 30) / per_query) / 256 * 256);
+    p->chunk = std::min<int64_t>(p->chunk, (m + 255) / 256 * 256);
+    return true;
+}
+
 int choose_splits(ssg_index *idx, int64_t m, int kk, int qpb) {
     if (idx->splits_param > 0) return idx->splits_param;
     const int64_t qtiles = (m + qpb - 1) / qpb;
@@ -480,6 +525,126 @@ int reduce_segments(ssg_index *idx, const uint64_t *cand, int64_t m, int segs, i
     *out = cur;
     *out_segs = cs;
     return SSG_OK;
+}
+
+// Sizes the list scan's buffers for one chunk and points the scan at them.
+int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
+    const size_t segs = size_t(p.splits) * 2;
+    SSG_CK(idx->l_lists.ensure(size_t(p.chunk) * segs * p.cap * 8), "allocating candidate lists");
+    SSG_CK(idx->l_counts.ensure(size_t(p.chunk) * segs * 4), "allocating list counts");
+    SSG_CK(idx->l_minima.ensure(size_t(p.chunk) * p.groups * 4), "allocating the seed's minima");
+    SSG_CK(idx->qbound.ensure(size_t(p.chunk) * 4), "allocating query bounds");
+    SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
+    s->cap = p.cap;
+    s->splits = p.splits;
+    s->samples = p.samples;
+    s->sample_stride = p.stride;
+    s->groups = p.groups;
+    s->fine_groups = p.fine;
+    s->bound = static_cast<uint32_t *>(idx->qbound.p);
+    s->lists = static_cast<uint64_t *>(idx->l_lists.p);
+    s->counts = static_cast<int *>(idx->l_counts.p);
+    s->minima = static_cast<float *>(idx->l_minima.p);
+    s->err = static_cast<int *>(idx->status.p);
+    return SSG_OK;
+}
+
+// The finalize side of a chunk's lists.
+void list_finalize(const ListPlan &p, const ssg::ListScan &s, ssg::FinalizeArgs *f) {
+    f->cand = s.lists;
+    f->counts = s.counts;
+    f->segs = p.splits * 2;
+    f->list_cap = p.cap;
+    f->list_keys = p.keys;
+    f->kk = s.kk;
+}
+
+// Seed, scan and finalize, chunk by chunk of the queries.  s holds the
+// operands (dt, row form, epilogue, n, kk; gamma of the first query), qtiles
+// the query tiles of tb bytes each; finish(c0, f) launches the chunk's
+// finalize kernel.
+template <typename F>
+int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, const uint8_t *qtiles, size_t tb, int64_t m,
+                int k, int exclude_self, uint32_t *d_ids, float *d_dists, F &&finish) {
+    SSG_RC(list_buffers(idx, plan, &s));
+    SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
+    const float *gamma = s.gamma;
+    ScanTimer timer(idx);
+    for (int64_t c0 = 0; c0 < m; c0 += plan.chunk) {
+        const int64_t mc = std::min<int64_t>(plan.chunk, m - c0);
+        s.qt = qtiles + size_t(c0 / 128) * tb;
+        s.m = mc;
+        s.gamma = gamma ? gamma + c0 : nullptr;
+        SSG_RC(timer.begin());
+        SSG_CK(ssg::launch_list_seed(s, idx->stream, &idx->last_launches), "launching the scan's seed");
+        SSG_CK(ssg::launch_list_scan(s, idx->stream, &idx->last_launches), "launching the list scan");
+        SSG_RC(timer.end());
+        ssg::FinalizeArgs f{};
+        list_finalize(plan, s, &f);
+        f.m = mc;
+        f.k_out = k;
+        f.exclude_self = exclude_self;
+        f.self_base = c0;
+        f.out_ids = d_ids + size_t(c0) * k;
+        f.out_dists = d_dists + size_t(c0) * k;
+        f.n_rows = idx->n;
+        f.n_total = idx->n;
+        SSG_CK(finish(c0, f), "launching the merge kernel");
+        SSG_RC(timer.collect());
+    }
+    return SSG_OK;
+}
+
+// Waits for the scan and turns its status word into an error (under capture
+// it is read after the graph launch).
+int scan_status(ssg_index *idx, const char *what) {
+    if (idx->capturing) return SSG_OK;
+    int status = 0;
+    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
+           "reading the status word");
+    SSG_CK(cudaStreamSynchronize(idx->stream), "running the scan");
+    if (status != 0) return fail(idx, SSG_ETIMEOUT, "a bounded wait in the %s scan gave up (code %d)", what, status);
+    return SSG_OK;
+}
+
+// Hamming on the tensor cores: sketches as +-1 FP8 rows, products exact in
+// FP32 (at most 2,048 terms of +-1), distance = (bits - product) / 2, so the
+// keys are the ones hamming_kernel makes.
+int run_hamming_tc(ssg_index *idx, const void *dq, int64_t m, int k, int exclude_self, uint32_t *d_ids,
+                   float *d_dists, bool queries_are_db, int kk, const ListPlan &plan) {
+    const int row_bytes = ssg::sketch_row_bytes(idx->dim);
+    const size_t tb = size_t(128) * row_bytes;
+    const int64_t tiles = (ssg::tc_tiles(idx->n) + 1) / 2 * 2;
+    if (idx->sk_rows != idx->n) {
+        SSG_CK(idx->sk_db.ensure(size_t(tiles) * tb), "allocating sketch tiles");
+        SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(idx->db.p), idx->n, idx->dim, tiles,
+                                        static_cast<uint8_t *>(idx->sk_db.p), idx->stream, &idx->last_launches),
+               "building sketch tiles");
+        idx->sk_rows = idx->n;
+    }
+    const uint8_t *qtiles = static_cast<const uint8_t *>(idx->sk_db.p);
+    if (!queries_are_db) {
+        const int64_t qt = (ssg::tc_tiles(m) + 1) / 2 * 2;
+        SSG_CK(idx->sk_q.ensure(size_t(qt) * tb), "allocating query sketch tiles");
+        SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(dq), m, idx->dim, qt,
+                                        static_cast<uint8_t *>(idx->sk_q.p), idx->stream, &idx->last_launches),
+               "building query sketch tiles");
+        qtiles = static_cast<const uint8_t *>(idx->sk_q.p);
+    }
+    ssg::ListScan s{};
+    s.dt = static_cast<const uint8_t *>(idx->sk_db.p);
+    s.row_bytes = row_bytes;
+    s.swb = 128;
+    s.fp8 = 1;
+    s.epi = ssg::LIST_HAMMING;
+    s.bits = float(64 * idx->dim);
+    s.n = idx->n;
+    s.kk = kk;
+    SSG_RC(list_search(idx, s, plan, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+                       [&](int64_t, ssg::FinalizeArgs &f) {
+                           return ssg::launch_finalize(f, idx->stream, &idx->last_launches);
+                       }));
+    return scan_status(idx, "sketch");
 }
 
 // The exact scan (direct FP32 or Hamming) then merge and decode.  dq are
@@ -1135,6 +1300,24 @@ int run_knn(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, 
         kk = std::min<int64_t>(kk, std::max<int64_t>(1, idx->n));
         if (ssg::gemm_fits(int(kk)))
             return run_gemm(idx, static_cast<const float *>(dq), dqn, m, k, exclude_self, d_ids, d_dists, int(kk));
+    }
+    if (idx->metric == SSG_METRIC_HAMMING && !idx->exact_scan_param) {
+        // On the tensor cores wherever the seed has its groups: measured
+        // against the POPC scan for 1 to 1,024 queries x 1 to 16 words x
+        // 8,192 to 2e6 sketches it is the faster one throughout (8,192
+        // sketches of 64 bits, one query: 85 against 95 us; 2e6 of 1,024
+        // bits: one query 409 against 1,631 us, 1,024 queries 1.45 against
+        // 18.8 ms).
+        const int kk = int(std::min<int64_t>(int64_t(k) + (exclude_self ? 1 : 0), idx->n));
+        ListPlan plan;
+        if (ssg::list_fits(ssg::sketch_row_bytes(idx->dim), 128, idx->n) && list_plan(idx, m, kk, &plan)) {
+            // the tiles take 8 times the sketches: without the memory the
+            // sketches are scanned as they are
+            const int rc = run_hamming_tc(idx, dq, m, k, exclude_self, d_ids, d_dists, queries_are_db, kk, plan);
+            if (rc != SSG_ENOMEM) return rc;
+            for (DevBuf *b : {&idx->sk_db, &idx->sk_q, &idx->l_lists, &idx->l_minima}) b->release();
+            idx->sk_rows = -1;
+        }
     }
     return run_exact_scan(idx, dq, dqn, m, k, exclude_self, nullptr, d_ids, d_dists, idx->cand);
 }
@@ -1836,7 +2019,7 @@ std::vector<uint64_t> graph_key(const ssg_index *idx, int64_t m, int k) {
     for (const DevBuf *b : {&idx->db, &idx->db_norm, &idx->tc_db, &idx->tc_norm, &idx->tc_q, &idx->st_db,
                             &idx->st_scale, &idx->st_alpha, &idx->st_beta, &idx->st_q, &idx->st_qscale, &idx->cand,
                             &idx->red[0], &idx->red[1], &idx->status, &idx->gbound, &idx->qnorm, &idx->pack_q,
-                            &idx->pack_out, &idx->qbound})
+                            &idx->pack_out, &idx->qbound, &idx->l_lists, &idx->l_counts, &idx->l_minima})
         key.push_back(uint64_t(reinterpret_cast<uintptr_t>(b->p)));
     return key;
 }
@@ -2541,7 +2724,8 @@ void ssg_destroy(ssg_index *idx) {
                       &idx->fb_cand, &idx->fb_qn, &idx->tc_smp, &idx->tc_smp_norm, &idx->f_out, &idx->f_cnt,
                       &idx->f_thr, &idx->gbound, &idx->pack_q, &idx->pack_out, &idx->gm_db, &idx->gm_q,
                       &idx->ps_db, &idx->ps_dbq, &idx->ps_norm, &idx->ps_q, &idx->qbound, &idx->pss_db,
-                      &idx->pss_dbq, &idx->pss_alpha, &idx->pss_beta, &idx->pss_q})
+                      &idx->pss_dbq, &idx->pss_alpha, &idx->pss_beta, &idx->pss_q, &idx->l_lists, &idx->l_counts,
+                      &idx->l_minima, &idx->sk_db, &idx->sk_q})
         b->release();
     if (idx->ev0) cudaEventDestroy(idx->ev0);
     if (idx->ev1) cudaEventDestroy(idx->ev1);

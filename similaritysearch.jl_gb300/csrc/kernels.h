@@ -77,6 +77,12 @@ struct FinalizeArgs {
     // segment length).  More than kk when each heap kept only part of the
     // list (the plain method's half heaps on the tensor cores).
     int rerank = 0;
+    // candidate lists instead of segments (tc_list.cu): counts[j * segs + s]
+    // unsorted keys at cand[(j * segs + s) * list_cap]; kk of them are wanted
+    // and together the lists hold the query's kk smallest keys
+    const int *counts = nullptr;
+    int list_cap = 0;
+    int list_keys = 0;  // keys per query kept on chip while selecting (more take extra passes)
 };
 cudaError_t launch_finalize(const FinalizeArgs &a, cudaStream_t st, int *launches);
 
@@ -196,6 +202,40 @@ cudaError_t launch_stream_scan(const uint8_t *q_tiles, const uint8_t *d_tiles, c
                                const float *qgamma, int64_t n, int64_t m, int64_t dim, int fp8, int kk, int splits,
                                int heap_rows, uint32_t *gbound, uint64_t *cand, int *err, cudaStream_t st,
                                int *launches, int *segs_per_split);
+
+// ---- resident-query scan with candidate lists (tc_list.cu) ----
+enum { LIST_DOT = 0, LIST_SQ = 1, LIST_COS = 2, LIST_AFFINE = 3, LIST_HAMMING = 4 };
+constexpr int kListMaxCap = 1024;  // entries of one list at most
+// One scan of n database rows for m queries: query (q, seg) of 2 * splits
+// segments leaves counts[q * segs + seg] unsorted keys at
+// lists[(q * segs + seg) * cap]; together they hold the query's kk smallest.
+struct ListScan {
+    const uint8_t *qt, *dt;   // operand tiles (an even number of each)
+    int row_bytes, swb, fp8;  // bytes per padded row, per K-block row (64 / 128), FP8 or BF16
+    int epi;                  // LIST_*
+    const float *alpha;       // per padded row: |x|^2 (SQ), 1 / |x| (COS), alpha (AFFINE)
+    const float *beta;        // AFFINE
+    const float *gamma;       // AFFINE: per query, null: 1
+    float bits;               // HAMMING: bits per sketch
+    int64_t n, m;
+    int kk, cap, splits;
+    uint32_t *bound;          // per query (ordered distance; all ones: none), written by the seed
+    uint64_t *lists;
+    int *counts;
+    // the seed: `samples` wide tiles (256 rows), every sample_stride-th of the
+    // database, all of whole rows; groups = 2 (or 8, fine_groups) minima each
+    int64_t samples, sample_stride;
+    int groups, fine_groups;
+    float *minima;            // m * groups
+    int *err;
+};
+bool list_fits(int row_bytes, int swb, int64_t n);
+cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches);
+cudaError_t launch_list_scan(const ListScan &s, cudaStream_t st, int *launches);
+// Sketches as +-1 FP8 rows (128-byte K-blocks).
+int sketch_row_bytes(int64_t words);
+cudaError_t launch_sketch_tiles(const uint64_t *x, int64_t rows, int64_t words, int64_t tiles, uint8_t *out,
+                                cudaStream_t st, int *launches);
 
 // ---- plain FP32 GEMM-form scan (gemm_f32.cu) ----
 // Writes `splits` sorted segments of kk keys per query.

@@ -431,7 +431,8 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
 }
 
 // A block per query.  cap: room for keys in shared memory (every key of the
-// query); sel_cap: room for the selected ones (0: they take the keys' place,
+// query's segments; of lists with more than that, only keys below a limit
+// found by counting are taken); sel_cap: room for the selected ones (0: they take the keys' place,
 // when nothing is left out).
 template <int METRIC, bool RERANK>
 __global__ void __launch_bounds__(kBlockThreads)
@@ -460,25 +461,76 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
     __syncthreads();
     // the query's keys, empty slots left out
     uint64_t mn = KEY_EMPTY, mx = 0;
-    for (int i0 = 0; i0 < total; i0 += kBlockThreads) {
-        const int i = i0 + tid;
-        uint64_t key = i < total ? src[i] : KEY_EMPTY;
+    auto push = [&](uint64_t key) {  // by whole warps
         if (RERANK && int64_t(key_id0(key)) >= f.n_rows) key = KEY_EMPTY;
         const bool have = key != KEY_EMPTY;
         const uint32_t vote = __ballot_sync(0xffffffffu, have);
         int base = 0;
         if (lane == 0 && vote) base = atomicAdd(&s_n, __popc(vote));
         base = __shfl_sync(0xffffffffu, base, 0);
-        if (have) {
-            keys[base + __popc(vote & ((1u << lane) - 1u))] = key;
+        const int at = base + __popc(vote & ((1u << lane) - 1u));
+        if (have && at < cap) {
+            keys[at] = key;
             mn = min(mn, key);
             mx = max(mx, key);
         }
+    };
+    if (f.counts) {
+        // eight lanes per list
+        const int *cn = f.counts + size_t(j) * f.segs;
+        const uint64_t *lists = f.cand + size_t(j) * f.segs * f.list_cap;
+        const int sub = lane % 8;
+        auto each_key = [&](auto &&body) {
+            for (int s0 = (tid / 32) * 4; s0 < f.segs; s0 += kBlockThreads / 8) {
+                const int sg = s0 + lane / 8;
+                const int c = sg < f.segs ? cn[sg] : 0;
+                const uint64_t *l = lists + size_t(sg) * f.list_cap;
+                const int most = __reduce_max_sync(0xffffffffu, c);
+                for (int i = sub; i < most + sub; i += 8) body(i < c ? l[i] : KEY_EMPTY);
+            }
+        };
+        int sum = 0;
+        for (int s = tid; s < f.segs; s += kBlockThreads) sum += cn[s];
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0 && sum) atomicAdd(&s_cnt[0], sum);
+        __syncthreads();
+        const int all = s_cnt[0];
+        uint64_t lim = KEY_EMPTY;
+        if (all > cap) {
+            // more keys than fit: a limit with at least `need` and at most
+            // cap keys below it (keys are unique, so one exists)
+            __syncthreads();
+            if (tid == 0) s_cnt[0] = 0;
+            __syncthreads();
+            uint64_t p = 0;
+            int it = 0;
+            for (int b = 63; b >= 0; --b, ++it) {
+                const uint64_t t = p | (1ull << b);
+                int c = 0;
+                each_key([&](uint64_t key) { c += key < t; });
+                c = __reduce_add_sync(0xffffffffu, c);
+                if (lane == 0 && c) atomicAdd(&s_cnt[it % 3], c);
+                __syncthreads();
+                c = s_cnt[it % 3];
+                if (tid == 0) s_cnt[(it + 2) % 3] = 0;
+                if (c >= need && c <= cap) { lim = t; break; }
+                if (c < need) p = t;
+            }
+            __syncthreads();
+            if (tid < 3) s_cnt[tid] = 0;
+            __syncthreads();
+        } else {
+            __syncthreads();
+            if (tid == 0) s_cnt[0] = 0;
+        }
+        each_key([&](uint64_t key) { push(key < lim ? key : KEY_EMPTY); });
+    } else {
+        for (int i0 = 0; i0 < total; i0 += kBlockThreads) push(i0 + tid < total ? src[i0 + tid] : KEY_EMPTY);
     }
     mn = warp_min64(mn);
     mx = warp_max64(mx);
     uint64_t low = KEY_EMPTY;
-    if (RERANK && f.check) {
+    if (RERANK && f.check && !f.counts) {
         for (int s = tid; s < f.segs; s += kBlockThreads) low = min(low, src[size_t(s) * f.kk + f.kk - 1]);
         low = warp_min64(low);
     }
@@ -488,7 +540,7 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
         if (RERANK && f.check) atomicMin(&s_low, low);
     }
     __syncthreads();
-    const int nvt = s_n;
+    const int nvt = min(s_n, cap);
     const int nv = min(need, nvt);
     if (nvt > need) {
         const uint64_t lo = s_min, hi = s_max;
@@ -612,10 +664,11 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
 template <int METRIC, bool RERANK>
 cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const float *db_norm, int64_t dim,
                               const float *q, const float *q_norm, int need, cudaStream_t st) {
-    const int total = f.segs * f.kk;
+    // lists: room for twice the keys a seeded bound leaves on average
+    const int total = f.counts ? std::max(f.list_keys, 2 * need) : f.segs * f.kk;
     const bool vec = RERANK && dim % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(db) | reinterpret_cast<uintptr_t>(q)) & 15) == 0;
-    if (total <= 32 * kWarpKeys && need <= kWarpOut) {
+    if (!f.counts && total <= 32 * kWarpKeys && need <= kWarpOut) {
         const size_t smem = RERANK ? size_t(kWarpsPerBlock) * kWarpStages * (need + 1) * kRowStride * 4 : 0;
         auto kern = finalize_warp_kernel<METRIC, RERANK>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
@@ -643,7 +696,7 @@ cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const floa
 }  // namespace
 
 cudaError_t launch_finalize(const FinalizeArgs &f, cudaStream_t st, int *launches) {
-    const int need = std::min(f.segs * f.kk, f.k_out + (f.exclude_self ? 1 : 0));
+    const int need = std::min(f.counts ? f.kk : f.segs * f.kk, f.k_out + (f.exclude_self ? 1 : 0));
     if (launches) *launches += 1;
     return launch_finalize_t<SQL2, false>(f, nullptr, nullptr, 0, nullptr, nullptr, need, st);
 }
@@ -652,7 +705,7 @@ cudaError_t launch_finalize_rerank(int metric, const FinalizeArgs &f, const floa
                                    int64_t dim, const float *q, const float *q_norm, cudaStream_t st,
                                    int *launches) {
     const int rr = f.rerank ? f.rerank : f.kk;
-    if (rr > f.segs * f.kk) return cudaErrorInvalidValue;
+    if (rr > (f.counts ? f.kk : f.segs * f.kk)) return cudaErrorInvalidValue;
     if (launches) *launches += 1;
     switch (metric) {
         case SQL2: return launch_finalize_t<SQL2, true>(f, db, db_norm, dim, q, q_norm, rr, st);

@@ -1,0 +1,658 @@
+// tc_list.cu -- tensor-core scan on CTA pairs with the query tile resident and
+// append-only candidate lists (tcgen05, cta_group::2).
+//
+// One scan for every operand form whose 128-query tile fits on chip beside a
+// ring of database K-blocks: BF16 and two-piece BF16 rows (64-byte K-blocks,
+// tc_bf16.cu), FP8 and wide BF16 rows (128-byte K-blocks, tc_stream.cu), and
+// bit sketches as +-1 FP8 rows (Hamming distance = (bits - dot) / 2, exact).
+//
+// Why lists and a seeded bound.  A search over S splits fills 2 S heaps per
+// query, each from scratch: kk (1 + ln(rows / kk)) insertions per heap, and
+// while they fill, the slowest of the warps holds its accumulator and with it
+// the MMAs (2,048 queries x 1e6 rows x 96 dimensions: 6,400 cycles per
+// 128 x 256 tile against 1,940 in allknn, whose order fills the heaps in the
+// first tiles).  Long heaps also take the shared memory that the resident
+// query tile needs.  Here a first pass over an evenly spaced sample of the
+// database (SEED) keeps only the smallest distance of each group of columns;
+// the kk-th smallest of a query's group minima is a bound with at least kk
+// rows at or below it.  The scan then appends what lies at or below that
+// bound (about 1.2 kk rows / sample rows per query) to a list in global
+// memory: no heap, no sort, no shared memory, and the same kk best keys.
+//
+// Why pairs.  Each CTA holds its own query tile and half of every database
+// K-block; one 256 x 256 MMA reads both.  A K-block byte so feeds 256 query
+// rows per SM load: 32 bytes per clock and SM at the full MMA rate instead of
+// 64 with one CTA (L2 gives about 35) and 128 for 128 x 128 tiles with both
+// operands streamed.
+//
+// Roles (320 threads per CTA, as in tc_pair_kernel): warp 0 producer, warp 1
+// TMEM owner and, in the even CTA, MMA issuer, warps 2..9 epilogue (two per
+// TMEM lane quarter, alternate 32-column chunks, a list each).  Every
+// mbarrier wait is bounded (tc_ptx.cuh); both CTAs meet at a cluster barrier
+// before TMEM is freed.
+#include "common.cuh"
+#include "kernels.h"
+#include "tc_ptx.cuh"
+
+#include <cuda.h>
+
+#include <algorithm>
+
+namespace ssg {
+
+namespace {
+
+constexpr int TILE = 128;
+constexpr int WIDE = 2 * TILE;
+constexpr int NACC = 2;
+constexpr int kThreads = 64 + 2 * TILE;
+constexpr int kMaxStages = 16;
+constexpr size_t kMaxSmem = 227 * 1024;
+constexpr size_t kAloneSmem = 120 * 1024;  // all 512 TMEM columns: alone on the SM
+constexpr int kSlack = 8;                  // appends between two checks of a list's room
+
+enum { EPI_DOT = LIST_DOT, EPI_SQ = LIST_SQ, EPI_COS = LIST_COS, EPI_AFF = LIST_AFFINE, EPI_HAM = LIST_HAMMING };
+
+// EPI_DOT and EPI_HAM rank by the raw product, largest first; the distance is
+// made from it only for a candidate.
+__host__ __device__ constexpr bool raw_rank(int epi) { return epi == EPI_DOT || epi == EPI_HAM; }
+
+struct KernelArgs {
+    ListScan s;
+    int kblocks;        // K-blocks per row
+    int stages;         // ring depth
+    int64_t n_wide;     // wide tiles of this pass (the sample's in SEED)
+};
+
+// Keeps the kk smallest of each full list (more than `room` entries): the
+// warp takes its lanes' full lists in turn, holds one in registers, finds the
+// kk-th key bit by bit and writes the kept keys back.  Returns the calling
+// lane's new count and sets *top to its largest kept key.  Rare: a bound
+// seeded from the sample leaves the lists far from full unless most of a
+// query's neighbours lie in one split.
+__device__ __noinline__ int compact_lists(uint64_t *list, int nb, int room, int kk, uint64_t *top) {
+    constexpr int PER = kListMaxCap / 32;
+    const int lane = threadIdx.x % 32;
+    uint32_t todo = __ballot_sync(0xffffffffu, nb > room);
+    while (todo) {
+        const int who = __ffs(todo) - 1;
+        todo &= todo - 1;
+        uint64_t *l = reinterpret_cast<uint64_t *>(
+            __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(list), who));
+        const int cnt = __shfl_sync(0xffffffffu, nb, who);
+        __syncwarp();
+        uint64_t key[PER];
+        uint64_t all = ~0ull, any = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const int at = i * 32 + lane;
+            key[i] = at < cnt ? l[at] : KEY_EMPTY;
+            if (at < cnt) { all &= key[i]; any |= key[i]; }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            all &= __shfl_xor_sync(0xffffffffu, all, o);
+            any |= __shfl_xor_sync(0xffffffffu, any, o);
+        }
+        // bits above the highest one in which two keys differ are common
+        const int hi = 63 - __clzll((all ^ any) | 1ull);
+        uint64_t p = hi >= 63 ? 0ull : (all >> (hi + 1)) << (hi + 1), below = KEY_EMPTY;
+        bool done = false;
+        for (int b = hi; b >= 0; --b) {
+            const uint64_t t = p | (1ull << b);
+            int c = 0;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) c += key[i] < t;
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (c == kk) { below = t; done = true; break; }
+            if (c < kk) p = t;
+        }
+        if (!done) below = p + 1;
+        int base = 0;
+        uint64_t mx = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            const bool take = key[i] < below;
+            const uint32_t vote = __ballot_sync(0xffffffffu, take);
+            const int at = base + __popc(vote & ((1u << lane) - 1u));
+            if (take && at < kk) {
+                l[at] = key[i];
+                mx = key[i] > mx ? key[i] : mx;
+            }
+            base += __popc(vote);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const uint64_t w = __shfl_xor_sync(0xffffffffu, mx, o);
+            mx = w > mx ? w : mx;
+        }
+        __syncwarp();
+        if (lane == who) {
+            nb = kk;
+            *top = mx;
+        }
+    }
+    return nb;
+}
+
+// The distance of a ranking value.
+template <int EPI>
+__device__ __forceinline__ float rank_distance(float x, float bits) {
+    return EPI == EPI_DOT ? -x : EPI == EPI_HAM ? (bits - x) * 0.5f : x;
+}
+
+// Appends those of eight columns' values v (columns id0.. of which lim are
+// rows) that pass the limit t (products >= t, distances <= t) to the lane's
+// list; full lists of the warp are compacted.  All 32 lanes call it.  Returns
+// the count (low word) and the limit, tightened by a compaction (high word).
+// One copy of this code for every call site: unrolled at the sites, the
+// kernel overflowed the instruction cache and an append took ~2,400 cycles
+// (10,000 queries x 2e6 sketches: 27.9 ms; with this function 12.2).
+template <int EPI>
+__device__ __noinline__ uint64_t append_group(uint64_t *list, int nb, int cap, int kk, float t, float bits,
+                                              uint32_t id0, int lim, float v0, float v1, float v2, float v3, float v4,
+                                              float v5, float v6, float v7) {
+    const float v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        if ((raw_rank(EPI) ? v[j] >= t : v[j] <= t) && j < lim) {
+            list[nb] = make_key(rank_distance<EPI>(v[j], bits), id0 + uint32_t(j));
+            ++nb;
+        }
+    }
+    if (__any_sync(0xffffffffu, nb > cap - kSlack)) {
+        uint64_t top = 0;
+        const bool full = nb > cap - kSlack;
+        nb = compact_lists(list, nb, cap - kSlack, kk, &top);
+        if (full) {
+            // kk keys up to `top` are kept and ids only grow from here: an
+            // equal distance no longer counts
+            const float d = key_dist(top);
+            if (EPI == EPI_HAM) t = fmaxf(t, bits - 2.0f * d + 1.0f);
+            else {
+                const float below = ordered_to_float(float_to_ordered(d) - 1u);
+                t = EPI == EPI_DOT ? fmaxf(t, -below) : fminf(t, below);
+            }
+        }
+    }
+    return (uint64_t(__float_as_uint(t)) << 32) | uint32_t(nb);
+}
+
+// One query row's candidates (one lane).
+template <int EPI>
+struct RowList {
+    uint64_t *list;
+    int nb, cap, kk;
+    int64_t n;
+    bool valid;
+    float lim_v;       // a candidate's ranking value: product >= lim_v (raw_rank) or distance <= lim_v
+    float bits;        // EPI_HAM: bits per sketch
+    float gamma;       // EPI_AFF: the query's scale
+
+    // the limit for a bound t on the distance; a row that is no query's lets nothing through
+    __device__ __forceinline__ void set(float t) {
+        if (!valid) t = -INFINITY;
+        lim_v = EPI == EPI_HAM ? bits - 2.0f * t : EPI == EPI_DOT ? -t : t;
+    }
+    // ranking values of a chunk's 32 columns: products (raw_rank) or distances
+    __device__ __forceinline__ void values(const uint32_t (&r)[32], int64_t id0, const ListScan &s,
+                                           float (&dv)[32]) const {
+        if constexpr (raw_rank(EPI)) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) dv[j] = __uint_as_float(r[j]);
+        } else {
+            const float4 *al = reinterpret_cast<const float4 *>(s.alpha + id0);
+            const float4 *be = EPI == EPI_AFF ? reinterpret_cast<const float4 *>(s.beta + id0) : nullptr;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 a = __ldg(al + j);
+                const float v0 = __uint_as_float(r[4 * j]), v1 = __uint_as_float(r[4 * j + 1]);
+                const float v2 = __uint_as_float(r[4 * j + 2]), v3 = __uint_as_float(r[4 * j + 3]);
+                if constexpr (EPI == EPI_SQ) {
+                    dv[4 * j] = fmaf(-2.0f, v0, a.x);
+                    dv[4 * j + 1] = fmaf(-2.0f, v1, a.y);
+                    dv[4 * j + 2] = fmaf(-2.0f, v2, a.z);
+                    dv[4 * j + 3] = fmaf(-2.0f, v3, a.w);
+                } else if constexpr (EPI == EPI_COS) {
+                    dv[4 * j] = -v0 * a.x;
+                    dv[4 * j + 1] = -v1 * a.y;
+                    dv[4 * j + 2] = -v2 * a.z;
+                    dv[4 * j + 3] = -v3 * a.w;
+                } else {
+                    const float4 b = __ldg(be + j);
+                    dv[4 * j] = fmaf(v0 * gamma, a.x, b.x);
+                    dv[4 * j + 1] = fmaf(v1 * gamma, a.y, b.y);
+                    dv[4 * j + 2] = fmaf(v2 * gamma, a.z, b.z);
+                    dv[4 * j + 3] = fmaf(v3 * gamma, a.w, b.w);
+                }
+            }
+        }
+    }
+    __device__ __forceinline__ static float best8(const float *v) { return raw_rank(EPI) ? fmax8(v) : fmin8(v); }
+    __device__ __forceinline__ static float best(float a, float b) { return raw_rank(EPI) ? fmaxf(a, b) : fminf(a, b); }
+    __device__ __forceinline__ bool passes(float x) const { return raw_rank(EPI) ? x >= lim_v : x <= lim_v; }
+
+    // the smallest distance among the chunk's columns (all of them rows)
+    __device__ __forceinline__ float chunk_min(const uint32_t (&r)[32], int64_t id0, const ListScan &s) const {
+        float dv[32];
+        values(r, id0, s, dv);
+        const float b = best(best(best8(dv), best8(dv + 8)), best(best8(dv + 16), best8(dv + 24)));
+        return fminf(rank_distance<EPI>(b, bits), INFINITY);  // NaN products: +inf
+    }
+    __device__ __forceinline__ void chunk(const uint32_t (&r)[32], int64_t id0, const ListScan &s) {
+        float dv[32], g[4];
+        values(r, id0, s, dv);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) g[i] = best8(dv + 8 * i);
+        if (!__any_sync(0xffffffffu, passes(best(best(g[0], g[1]), best(g[2], g[3]))))) return;
+        const int lim = int(id0 + 32 <= n ? 32 : n - id0);  // columns that are rows
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (!__any_sync(0xffffffffu, passes(g[i]))) continue;
+            const float *v = dv + 8 * i;
+            const uint64_t r2 = append_group<EPI>(list, nb, cap, kk, lim_v, bits, uint32_t(id0) + 8u * i,
+                                                  valid ? lim - 8 * i : 0, v[0], v[1], v[2], v[3], v[4], v[5], v[6],
+                                                  v[7]);
+            nb = int(uint32_t(r2));
+            lim_v = __uint_as_float(uint32_t(r2 >> 32));
+        }
+    }
+};
+
+template <int SWB, bool F8, int EPI, bool SEED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+    tc_list_kernel(KernelArgs ka, const __grid_constant__ CUtensorMap dmap) {
+    constexpr int KBLK = TILE * SWB;   // bytes of a K-block of one 128-row tile
+    constexpr int KSTEPS = SWB / 32;   // MMAs per K-block (32 bytes of K each)
+    const ListScan &a = ka.s;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int kblocks = ka.kblocks, stages = ka.stages;
+    const size_t tile_bytes = size_t(kblocks) * KBLK;
+    uint8_t *sA = smem;
+    uint8_t *sB = sA + tile_bytes;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sB + size_t(stages) * KBLK);
+    uint64_t *a_full = bars;                  // this CTA's query tile landed
+    uint64_t *pa_full = a_full + 1;           // (even CTA) the odd CTA's query tile landed
+    uint64_t *full = pa_full + 1;             // (even CTA) both halves of stage s landed
+    uint64_t *empty = full + kMaxStages;      // the MMAs of stage s are done
+    uint64_t *acc_full = empty + kMaxStages;  // accumulator b holds a finished wide tile
+    uint64_t *acc_empty = acc_full + NACC;    // (even CTA) its epilogue warps released b
+    uint64_t *pacc_empty = acc_empty + NACC;  // (even CTA) the odd CTA's epilogue warps released b
+    uint64_t *mma_done = pacc_empty + NACC;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
+    const int warp = threadIdx.x / 32;
+    const int lane = threadIdx.x % 32;
+    const uint32_t rank = tc::cluster_ctarank();  // 0: the even CTA (issues the MMAs)
+    const uint32_t peer = rank ^ 1u;
+    const int64_t qx = blockIdx.x;                // this CTA's query tile
+    const int64_t qpair = qx - int64_t(rank);
+    // epilogue warps of a query tile whose lane quarter holds a query
+    auto live_warps = [&](int64_t tile) {
+        int live = 0;
+        for (int w = 0; w < 4; ++w)
+            if (tile * TILE + w * 32 < a.m) live += 2;
+        return live;
+    };
+    const int live_self = live_warps(qx), live_peer = live_warps(qpair + int64_t(peer));
+
+    if (threadIdx.x == 0) {
+        tc::mbar_init(a_full, 1);
+        tc::mbar_init(pa_full, 1);
+        for (int s = 0; s < stages; ++s) {
+            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < NACC; ++b) {
+            tc::mbar_init(&acc_full[b], 1);
+            tc::mbar_init(&acc_empty[b], live_self > 0 ? live_self : 1);
+            tc::mbar_init(&pacc_empty[b], live_peer > 0 ? live_peer : 1);
+        }
+        tc::mbar_init(mma_done, 1);
+        tc::fence_mbarrier_init();
+    }
+    if (warp == 1) tc::tmem_alloc_pair<512>(tmem_slot);
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::cluster_sync();  // both CTAs' barriers exist before any cross-CTA arrive
+    tc::tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    // this split's wide tiles (places in the sample when SEED)
+    const int64_t split_w = (ka.n_wide + a.splits - 1) / a.splits;
+    const int64_t w_lo = int64_t(blockIdx.y) * split_w;
+    const int64_t w_hi = w_lo + split_w < ka.n_wide ? w_lo + split_w : ka.n_wide;
+    const int W = w_hi > w_lo ? int(w_hi - w_lo) : 0;
+    auto wide_tile = [&](int u) { return SEED ? (w_lo + u) * a.sample_stride : w_lo + u; };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // producer: this CTA's query tile, then its half of every K-block;
+            // both halves of a stage complete on the even CTA's full[s]
+            tc::mbar_arrive_expect_tx(a_full, uint32_t(tile_bytes));
+            for (int kb = 0; kb < kblocks; ++kb)
+                tc::bulk_g2s(sA + size_t(kb) * KBLK, a.qt + size_t(qx) * tile_bytes + size_t(kb) * KBLK, KBLK, a_full);
+            const uint32_t full0 = tc::mapa_shared(tc::smem_u32(full), 0);
+            int s = 0, issued = 0;
+            uint32_t ph = 1;
+            bool ok = true;
+            for (int u = 0; ok && u < W; ++u) {
+                const int64_t tile = 2 * wide_tile(u) + rank;
+                const uint8_t *src = a.dt + size_t(tile) * tile_bytes;
+                int line = int(tile * kblocks * TILE);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!tc::mbar_wait(&empty[s], ph, a.err, 21)) { ok = false; break; }
+                    uint8_t *dst = sB + size_t(s) * KBLK;
+                    if (rank == 0) {
+                        tc::mbar_arrive_expect_tx(&full[s], uint32_t(2 * KBLK));
+                        tc::bulk_g2s(dst, src, uint32_t(KBLK), &full[s]);
+                    } else {
+                        tc::tma_load_2d_pair(dst, &dmap, 0, line, full0 + uint32_t(s * 8));
+                    }
+                    src += KBLK;
+                    line += TILE;
+                    issued = issued < stages ? issued + 1 : stages;
+                    if (++s == stages) { s = 0; ph ^= 1; }
+                }
+            }
+            // wait (bounded) until every copy of this pair has landed (the
+            // even CTA's barriers count both halves; the final cluster
+            // barrier keeps the odd CTA alive until then)
+            tc::mbar_wait(a_full, 0, a.err, 22);
+            if (rank == 0) {
+                // the last `issued` stages, newest first: a stage's landing
+                // phase is the opposite of the one its emptiness was waited for
+                for (int i = 0; i < issued; ++i) {
+                    if (--s < 0) { s = stages - 1; ph ^= 1; }
+                    tc::mbar_wait(&full[s], ph ^ 1, a.err, 22);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 1) {
+            // the odd CTA tells the even CTA that its query tile landed
+            if (tc::mbar_wait(a_full, 0, a.err, 28)) tc::mbar_arrive_cluster(tc::mapa_shared(tc::smem_u32(pa_full), peer));
+        } else if (lane == 0) {
+            // the even CTA issues the pair's MMAs
+            constexpr uint32_t idesc = F8 ? tc::idesc_e4m3_f32(2 * TILE, WIDE) : tc::idesc_bf16_f32(2 * TILE, WIDE);
+            bool ok = tc::mbar_wait(a_full, 0, a.err, 23) && tc::mbar_wait(pa_full, 0, a.err, 23);
+            const uint64_t a_desc = tc::smem_desc(tc::smem_u32(sA), SWB);
+            const uint64_t b_desc = tc::smem_desc(tc::smem_u32(sB), SWB);
+            int s = 0;
+            uint32_t ph = 0;
+            for (int u = 0; ok && u < W; ++u) {
+                const int b = u & 1;
+                const uint32_t aph = ((u >> 1) & 1) ^ 1;
+                if (live_self > 0 && !tc::mbar_wait(&acc_empty[b], aph, a.err, 25)) break;
+                if (live_peer > 0 && !tc::mbar_wait(&pacc_empty[b], aph, a.err, 25)) break;
+                const uint32_t d_tmem = tmem_base + uint32_t(b * WIDE);
+                for (int kb = 0; kb < kblocks; ++kb) {
+                    if (!tc::mbar_wait(&full[s], ph, a.err, 24)) { ok = false; break; }
+                    tc::tc_fence_after();
+#pragma unroll
+                    for (int k = 0; k < KSTEPS; ++k) {
+                        // descriptors address 16-byte units
+                        const uint64_t ad = a_desc + uint64_t((kb * KBLK + k * 32) >> 4);
+                        const uint64_t bd = b_desc + uint64_t((s * KBLK + k * 32) >> 4);
+                        if (F8) tc::mma_f8_pair(d_tmem, ad, bd, idesc, (kb | k) ? 1u : 0u);
+                        else tc::mma_f16_pair(d_tmem, ad, bd, idesc, (kb | k) ? 1u : 0u);
+                    }
+                    tc::mma_commit_both(&empty[s]);
+                    if (++s == stages) { s = 0; ph ^= 1; }
+                }
+                if (!ok) break;
+                tc::mma_commit_both(&acc_full[b]);
+            }
+            tc::mma_commit_pair(tc::smem_u32(mma_done));
+            tc::mbar_wait(mma_done, 0, a.err, 26);
+        }
+        __syncwarp();
+    } else {
+        const int cs = (warp - 2) / 4;
+        const int quarter = warp % 4;
+        const int64_t query = qx * TILE + quarter * 32 + lane;
+        const uint32_t r_pacc0 = tc::mapa_shared(tc::smem_u32(pacc_empty), peer);
+        const int seg = int(blockIdx.y) * 2 + cs, segs = a.splits * 2;
+        RowList<EPI> T;
+        T.valid = query < a.m;
+        T.list = SEED ? nullptr : a.lists + (size_t(T.valid ? query : 0) * segs + seg) * a.cap;
+        T.nb = 0;
+        T.cap = a.cap;
+        T.kk = a.kk;
+        T.n = a.n;
+        T.bits = a.bits;
+        T.gamma = (EPI == EPI_AFF && a.gamma && T.valid) ? a.gamma[query] : 1.0f;
+        T.set((!SEED && T.valid) ? bound_read(a.bound + query) : INFINITY);
+        const bool warp_live = qx * TILE + quarter * 32 < a.m;
+        for (int u = 0; warp_live && u < W; ++u) {
+            const int b = u & 1;
+            int ok = 1;
+            if (lane == 0) ok = tc::mbar_wait(&acc_full[b], (u >> 1) & 1, a.err, 27) ? 1 : 0;
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            if (!ok) break;
+            tc::tc_fence_after();
+            // this warp's chunks cs, cs + 2, ... of the wide tile, two in
+            // flight per round (four spill beside the list's state: 13.5 ms
+            // against 12.2 for 10,000 queries x 2e6 sketches); the
+            // accumulator goes back after the last load
+            constexpr int LDC = 2;
+            const int64_t row0 = wide_tile(u) * WIDE + cs * 32;
+            const uint32_t tbase = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(b * WIDE + cs * 32);
+            uint32_t r[LDC][32];
+            float gmin[4];
+#pragma unroll
+            for (int round = 0; round < 4 / LDC; ++round) {
+                __syncwarp();
+#pragma unroll
+                for (int c = 0; c < LDC; ++c)
+                    tc::tmem_ld_32x32b_x32_async(tbase + uint32_t((round * LDC + c) * 64), r[c]);
+                tc::tmem_wait_ld();
+                if (round == 4 / LDC - 1) {
+                    tc::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (rank == 0) tc::mbar_arrive(&acc_empty[b]);
+                        else tc::mbar_arrive_cluster(r_pacc0 + uint32_t(b * 8));
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < LDC; ++c) {
+                    const int64_t id0 = row0 + (round * LDC + c) * 64;
+                    if constexpr (SEED) gmin[round * LDC + c] = T.chunk_min(r[c], id0, a);
+                    else T.chunk(r[c], id0, a);
+                }
+            }
+            if constexpr (SEED) {
+                if (T.valid) {
+                    float *g = a.minima + size_t(query) * a.groups;
+                    const int64_t at = w_lo + u;
+                    if (a.fine_groups) {
+                        *reinterpret_cast<float4 *>(g + at * 8 + cs * 4) = make_float4(gmin[0], gmin[1], gmin[2], gmin[3]);
+                    } else {
+                        g[at * 2 + cs] = fminf(fminf(gmin[0], gmin[1]), fminf(gmin[2], gmin[3]));
+                    }
+                }
+            }
+        }
+        if (!SEED && T.valid) a.counts[size_t(query) * segs + seg] = T.nb;
+    }
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::cluster_sync();  // the even CTA's MMAs are done with both CTAs' shared memory
+    if (warp == 1) {
+        tc::tc_fence_after();
+        tc::tmem_dealloc_pair<512>(tmem_base);
+    }
+}
+
+// bound[q] = the kk-th smallest of the query's group minima (all ones, no
+// bound, when they are not that many): each is the distance of another row.
+// A warp per query; groups beyond 32 * NV are joined (their minimum is still
+// a row's distance), the kk-th value is found bit by bit from registers.
+template <int NV>
+__global__ void __launch_bounds__(128) seed_bound_kernel(const float *__restrict__ minima, int64_t m, int groups, int kk,
+                                                         uint32_t *__restrict__ bound) {
+    const int64_t q = int64_t(blockIdx.x) * 4 + threadIdx.x / 32;
+    const int lane = threadIdx.x % 32;
+    if (q >= m) return;
+    const float *g = minima + size_t(q) * groups;
+    float f[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) f[i] = i * 32 + lane < groups ? g[i * 32 + lane] : INFINITY;
+    for (int at = NV * 32 + lane; at < groups; at += NV * 32) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+            if (at + i * 32 < groups) f[i] = fminf(f[i], g[at + i * 32]);
+    }
+    uint32_t v[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] = float_to_ordered(f[i]);
+    uint32_t p = 0;
+    for (int b = 31; b >= 0; --b) {
+        const uint32_t t = p | (1u << b);
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) c += v[i] < t;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c < kk) p = t;
+    }
+    if (lane == 0) bound[q] = kk <= groups ? p : 0xffffffffu;
+}
+
+// Sketches -> +-1 FP8 (e4m3) tiles in the 128-byte K-block layout: bit 0 is
+// +1, bit 1 is -1, words past the sketch and rows past the end are zeros.
+// Thread = 16 bits = one 16-byte chunk.
+__global__ void sketch_tile_kernel(const uint64_t *__restrict__ x, int64_t rows, int words, int kblocks, int64_t tiles,
+                                   uint8_t *__restrict__ out) {
+    const int chunks = kblocks * 8;  // 16-bit chunks per padded row
+    const int64_t total = tiles * TILE * chunks;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
+        const int ch = int(i % chunks);
+        const int64_t row = i / chunks;
+        uint32_t w[4] = {0, 0, 0, 0};
+        if (row < rows && ch < words * 4) {
+            const uint32_t bits = uint32_t(x[row * words + ch / 4] >> ((ch % 4) * 16)) & 0xffffu;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                // four bits spread to the bytes' sign bits
+                const uint32_t nib = (bits >> (4 * k)) & 0xfu;
+                w[k] = (((nib * 0x00204081u) & 0x01010101u) << 7) | 0x38383838u;
+            }
+        }
+        const int64_t tile = row / TILE;
+        const uint32_t off = tc::swizzled_offset(uint32_t(row % TILE), uint32_t((ch % 8) * 16), 128);
+        uint8_t *dst = out + (size_t(tile) * kblocks + ch / 8) * (TILE * 128) + off;
+        *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// The database tiles as a 2D array of K-block lines (swb bytes each, already
+// swizzled); a box of 128 lines is one tile's K-block, copied verbatim.
+cudaError_t line_map(const ListScan &s, int kblocks, CUtensorMap *map) {
+    using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static EncodeFn encode = nullptr;
+    if (!encode) {
+        void *fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q);
+        if (e != cudaSuccess) return e;
+        if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
+        encode = reinterpret_cast<EncodeFn>(fn);
+    }
+    if (reinterpret_cast<uintptr_t>(s.dt) % 16 != 0) return cudaErrorInvalidValue;
+    const int64_t tiles = ((s.n + TILE - 1) / TILE + 1) / 2 * 2;
+    const cuuint64_t dims[2] = {cuuint64_t(s.swb), cuuint64_t(tiles) * kblocks * TILE};
+    const cuuint64_t strides[1] = {cuuint64_t(s.swb)};
+    const cuuint32_t box[2] = {cuuint32_t(s.swb), cuuint32_t(TILE)};
+    const cuuint32_t estr[2] = {1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(s.dt), dims, strides, box,
+                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+size_t list_smem(int tile_bytes, int kblk, int stages) {
+    return 1024 + size_t(tile_bytes) + size_t(stages) * kblk + (2 + 2 * kMaxStages + 3 * NACC + 1) * 8 + 16;
+}
+
+int list_stages(int row_bytes, int swb) {
+    int st = kMaxStages;
+    while (st > 0 && list_smem(TILE * row_bytes, TILE * swb, st) > kMaxSmem) --st;
+    return st;
+}
+
+template <int SWB, bool F8, int EPI, bool SEED>
+cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
+    KernelArgs ka;
+    ka.s = s;
+    ka.kblocks = s.row_bytes / SWB;
+    ka.stages = list_stages(s.row_bytes, SWB);
+    ka.n_wide = SEED ? s.samples : (s.n + WIDE - 1) / WIDE;
+    size_t smem = list_smem(TILE * s.row_bytes, TILE * SWB, ka.stages);
+    if (smem < kAloneSmem) smem = kAloneSmem;
+    auto kern = tc_list_kernel<SWB, F8, EPI, SEED>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    CUtensorMap map;
+    e = line_map(s, ka.kblocks, &map);
+    if (e != cudaSuccess) return e;
+    const int64_t qtiles = ((s.m + TILE - 1) / TILE + 1) / 2 * 2;
+    kern<<<dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st>>>(ka, map);
+    return cudaGetLastError();
+}
+
+template <bool SEED>
+cudaError_t launch_list_any(const ListScan &s, cudaStream_t st) {
+    if (s.swb == 128 && s.fp8) {
+        if (s.epi == LIST_HAMMING) return launch_list_t<128, true, EPI_HAM, SEED>(s, st);
+        if (s.epi == LIST_AFFINE) return launch_list_t<128, true, EPI_AFF, SEED>(s, st);
+        return cudaErrorInvalidValue;
+    }
+    if (s.swb == 128) return s.epi == LIST_AFFINE ? launch_list_t<128, false, EPI_AFF, SEED>(s, st) : cudaErrorInvalidValue;
+    switch (s.epi) {
+        case LIST_DOT: return launch_list_t<64, false, EPI_DOT, SEED>(s, st);
+        case LIST_SQ: return launch_list_t<64, false, EPI_SQ, SEED>(s, st);
+        case LIST_COS: return launch_list_t<64, false, EPI_COS, SEED>(s, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+}  // namespace
+
+// At least four ring stages beside the query tile, and the database's K-block
+// lines within the tensor map's 32-bit coordinates.
+bool list_fits(int row_bytes, int swb, int64_t n) {
+    return list_stages(row_bytes, swb) >= 4 && (n + 2 * WIDE) * (row_bytes / swb) < (int64_t(1) << 31);
+}
+
+cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches) {
+    cudaError_t e = launch_list_any<true>(s, st);
+    if (e != cudaSuccess) return e;
+    // about four groups per candidate keep the bound within a fifth of the
+    // sample's own kk-th distance in rank
+    const unsigned blocks = unsigned((s.m + 3) / 4);
+    if (s.kk <= 64) seed_bound_kernel<8><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
+    else if (s.kk <= 160) seed_bound_kernel<20><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
+    else seed_bound_kernel<60><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
+    if (launches) *launches += 2;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_list_scan(const ListScan &s, cudaStream_t st, int *launches) {
+    if (launches) *launches += 1;
+    return launch_list_any<false>(s, st);
+}
+
+int sketch_row_bytes(int64_t words) { return int((words + 1) / 2 * 128); }
+
+cudaError_t launch_sketch_tiles(const uint64_t *x, int64_t rows, int64_t words, int64_t tiles, uint8_t *out,
+                                cudaStream_t st, int *launches) {
+    const int kblocks = sketch_row_bytes(words) / 128;
+    const int64_t total = tiles * TILE * kblocks * 8;
+    const int64_t blocks = std::min<int64_t>((total + 255) / 256, 152 * 64);
+    if (launches) *launches += 1;
+    sketch_tile_kernel<<<unsigned(std::max<int64_t>(1, blocks)), 256, 0, st>>>(x, rows, int(words), kblocks, tiles, out);
+    return cudaGetLastError();
+}
+
+}  // namespace ssg

@@ -290,5 +290,26 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t cluster_addr) {
                  : "memory");
 }
 
+// The same for kind::f8f6f4 (FP8 in, FP32 accumulator).
+__device__ __forceinline__ void mma_f8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// Arrives once on the mbarrier at this offset in both CTAs of the pair when
+// the pair MMAs this thread issued so far have completed.
+__device__ __forceinline__ void mma_commit_both(uint64_t *bar) {
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            smem_u32(bar)),
+        "h"(uint16_t(3))
+        : "memory");
+}
+
 }  // namespace tc
 }  // namespace ssg
