@@ -293,7 +293,7 @@ bool uses_stream(const ssg_index *idx) {
 // (Re)builds the K-block operand tiles, FP8 scales and epilogue coefficients.
 int build_stream_tiles(ssg_index *idx) {
     const int fp8 = idx->prec == SSG_PREC_FP8;
-    const int64_t tiles = ssg::tc_tiles(idx->n);
+    const int64_t tiles = (ssg::tc_tiles(idx->n) + 1) / 2 * 2;  // the list scan reads pairs of tiles
     SSG_CK(idx->st_db.ensure(size_t(tiles) * ssg::stream_tile_bytes(idx->dim, fp8)), "allocating operand tiles");
     float *scale = nullptr;
     if (fp8) {
@@ -605,6 +605,11 @@ int scan_status(ssg_index *idx, const char *what) {
     SSG_CK(cudaStreamSynchronize(idx->stream), "running the scan");
     if (status != 0) return fail(idx, SSG_ETIMEOUT, "a bounded wait in the %s scan gave up (code %d)", what, status);
     return SSG_OK;
+}
+
+// The BF16 tiles' epilogue of a metric.
+int list_epilogue(int metric) {
+    return is_sq_metric(metric) ? ssg::LIST_SQ : metric == SSG_METRIC_COSINE ? ssg::LIST_COS : ssg::LIST_DOT;
 }
 
 // Hamming on the tensor cores: sketches as +-1 FP8 rows, products exact in
@@ -995,12 +1000,80 @@ constexpr int64_t kLocalityMinRows = 32768;
 
 int ensure_plain_locality(ssg_index *idx);
 
+// The certificate's fields of the plain method's finalize: kp elements per
+// piece, flags of the chunk's queries.  |a - a_exact| <= c |x| |q| (see above)
+// plus the exact evaluation's own error: (d + 2) 2^-24 |x| |q| for a dot
+// product; the squared-distance metrics add c |x| |q| <= c/2 (|x| + |q|)^2 to
+// the GEMM-form allowance 4 (d + 2) 2^-24 (|x| + |q|)^2.
+void plain_certificate(const ssg_index *idx, int kp, int *flags, int *flag_count, ssg::FinalizeArgs *f) {
+    const bool sq = is_sq_metric(idx->metric);
+    const float c = 3.05f * 1.52587890625e-5f + 2.2f * float(kp) * 1.1920929e-7f;
+    const float ulp24 = 5.9604645e-8f;
+    f->n_rows = idx->n;
+    f->check = sq ? 1 : (idx->metric == SSG_METRIC_COSINE ? 3 : 2);
+    f->max_x_sq = idx->max_x_sq;
+    f->err_scale = sq ? 4.0f * float(idx->dim + 2) * ulp24 + 0.5f * c
+                      : (f->check == 3 ? c + float(2 * idx->dim + 16) * ulp24 : c + float(idx->dim + 2) * ulp24);
+    f->n_total = idx->n;
+    f->flags = flags;
+    f->flag_count = flag_count;
+}
+
+// Waits for the plain method's scan, then recomputes the queries that were
+// not certified.
+int plain_finish(ssg_index *idx, const char *what, const float *dq, int64_t m, int k, int exclude_self, int *flags,
+                 uint32_t *d_ids, float *d_dists) {
+    int status = 0, nflag = 0;
+    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
+           "reading the status word");
+    SSG_CK(cudaMemcpyAsync(&nflag, flags + m, sizeof(int), cudaMemcpyDeviceToHost, idx->stream), "reading flags");
+    SSG_CK(cudaStreamSynchronize(idx->stream), "running the plain method's scan");
+    if (status != 0) return fail(idx, SSG_ETIMEOUT, "a bounded wait in the split %s scan gave up (code %d)", what, status);
+    idx->last_fallbacks = nflag;
+    return run_fallback(idx, dq, m, k, exclude_self, flags, nflag, d_ids, d_dists);
+}
+
 int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, int k, int exclude_self,
                  uint32_t *d_ids, float *d_dists, bool queries_are_db, const PlainTcPlan &plan) {
     const int kk = plan.h, k3 = plan.k3;
-    const bool sq = is_sq_metric(idx->metric);
     const int kp = ssg::tc_padded_k(idx->dim);
     SSG_RC(ensure_plain_tiles(idx, queries_are_db));
+    SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
+    SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
+    const size_t tb = ssg::tc_tile_bytes(k3);
+    const uint8_t *qtiles = static_cast<const uint8_t *>(idx->ps_dbq.p);
+    if (!queries_are_db) {
+        const int64_t qt_alloc = ((m + 127) / 128 + 1) / 2 * 2;  // even: the pair scans read query tiles in pairs
+        SSG_CK(idx->ps_q.ensure(size_t(qt_alloc) * tb), "allocating split query tiles");
+        SSG_CK(ssg::launch_bf16_tiles(dq, m, idx->dim, qt_alloc, static_cast<uint8_t *>(idx->ps_q.p), idx->stream,
+                                      &idx->last_launches, nullptr, 2),
+               "building split query tiles");
+        qtiles = static_cast<const uint8_t *>(idx->ps_q.p);
+    }
+    int *flags = static_cast<int *>(idx->flags.p);
+    int *flag_count = flags + m;
+    // a batch of queries (allknn scans its locality order, below): the list scan
+    ListPlan lp;
+    const bool locality = queries_are_db && idx->locality_param && m == idx->n && idx->n >= kLocalityMinRows;
+    if (!locality && !idx->pair_param && ssg::list_fits(2 * k3, 64, idx->n) && list_plan(idx, m, plan.rr, &lp)) {
+        ssg::ListScan s{};
+        s.dt = static_cast<const uint8_t *>(idx->ps_db.p);
+        s.row_bytes = 2 * k3;
+        s.swb = 64;
+        s.epi = list_epilogue(idx->metric);
+        s.alpha = static_cast<const float *>(idx->ps_norm.p);
+        s.n = idx->n;
+        s.kk = plan.rr;
+        SSG_RC(list_search(idx, s, lp, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+                           [&](int64_t c0, ssg::FinalizeArgs &f) {
+                               plain_certificate(idx, kp, flags + c0, flag_count, &f);
+                               return ssg::launch_finalize_rerank(
+                                   idx->metric, f, static_cast<const float *>(idx->db.p),
+                                   static_cast<const float *>(idx->db_norm.p), idx->dim, dq + size_t(c0) * idx->dim,
+                                   dqn ? dqn + c0 : nullptr, idx->stream, &idx->last_launches);
+                           }));
+        return plain_finish(idx, "list", dq, m, k, exclude_self, flags, d_ids, d_dists);
+    }
     const int64_t qctas = (m + 127) / 128;
     const int64_t n_tiles = ssg::tc_tiles(idx->n);
     int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(qctas, ssg::device_sm_count(), n_tiles);
@@ -1012,18 +1085,6 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     SSG_CK(idx->cand.ensure(per_query * size_t(chunk)), "allocating candidate scratch");
     SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
-    SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
-    SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
-    const size_t tb = ssg::tc_tile_bytes(k3);
-    const uint8_t *qtiles = static_cast<const uint8_t *>(idx->ps_dbq.p);
-    if (!queries_are_db) {
-        const int64_t qt_alloc = (qctas + 1) / 2 * 2;  // even: the pair scan reads query tiles in pairs
-        SSG_CK(idx->ps_q.ensure(size_t(qt_alloc) * tb), "allocating split query tiles");
-        SSG_CK(ssg::launch_bf16_tiles(dq, m, idx->dim, qt_alloc, static_cast<uint8_t *>(idx->ps_q.p), idx->stream,
-                                      &idx->last_launches, nullptr, 2),
-               "building split query tiles");
-        qtiles = static_cast<const uint8_t *>(idx->ps_q.p);
-    }
     // allknn in one launch: the database in its locality order (rows grouped
     // by nearest pivot, each query tile starting at its own group), so the
     // heaps hold near neighbours from the first tiles on and few later
@@ -1032,7 +1093,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     const float *dnorm = static_cast<const float *>(idx->ps_norm.p);
     const uint32_t *perm = nullptr;
     const int *rot = nullptr;
-    if (queries_are_db && idx->locality_param && m == idx->n && idx->n >= kLocalityMinRows && chunk >= m) {
+    if (locality && chunk >= m) {
         SSG_RC(ensure_plain_locality(idx));
         qtiles = static_cast<const uint8_t *>(idx->loc_ps_dbq.p);
         dtiles = static_cast<const uint8_t *>(idx->loc_ps_db.p);
@@ -1047,14 +1108,6 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
         SSG_CK(idx->qbound.ensure(size_t(chunk) * 4), "allocating query bounds");
         qbound = static_cast<uint32_t *>(idx->qbound.p);
     }
-    // |a - a_exact| <= c |x| |q| (see above) plus the exact evaluation's own
-    // error: (d + 2) 2^-24 |x| |q| for a dot product; the squared-distance
-    // metrics add c |x| |q| <= c/2 (|x| + |q|)^2 to the GEMM-form allowance
-    // 4 (d + 2) 2^-24 (|x| + |q|)^2
-    const float c = 3.05f * 1.52587890625e-5f + 2.2f * float(kp) * 1.1920929e-7f;
-    const float ulp24 = 5.9604645e-8f;
-    int *flags = static_cast<int *>(idx->flags.p);
-    int *flag_count = flags + m;
     ScanTimer timer(idx);
     for (int64_t c0 = 0; c0 < m; c0 += chunk) {
         const int64_t mc = std::min<int64_t>(chunk, m - c0);
@@ -1076,15 +1129,8 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
         f.self_base = c0;
         f.out_ids = d_ids + size_t(c0) * k;
         f.out_dists = d_dists + size_t(c0) * k;
-        f.n_rows = idx->n;
         f.rerank = std::min(plan.rr, f.segs * kk);
-        f.check = sq ? 1 : (idx->metric == SSG_METRIC_COSINE ? 3 : 2);
-        f.max_x_sq = idx->max_x_sq;
-        f.err_scale = sq ? 4.0f * float(idx->dim + 2) * ulp24 + 0.5f * c
-                         : (f.check == 3 ? c + float(2 * idx->dim + 16) * ulp24 : c + float(idx->dim + 2) * ulp24);
-        f.n_total = idx->n;
-        f.flags = flags + c0;
-        f.flag_count = flag_count;
+        plain_certificate(idx, kp, flags + c0, flag_count, &f);
         SSG_CK(ssg::launch_finalize_rerank(idx->metric, f, static_cast<const float *>(idx->db.p),
                                            static_cast<const float *>(idx->db_norm.p), idx->dim, qc,
                                            dqn ? dqn + c0 : nullptr,
@@ -1092,15 +1138,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
                "launching the rerank kernel");
         SSG_RC(timer.collect());
     }
-    int status = 0, nflag = 0;
-    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
-           "reading the status word");
-    SSG_CK(cudaMemcpyAsync(&nflag, flag_count, sizeof(int), cudaMemcpyDeviceToHost, idx->stream), "reading flags");
-    SSG_CK(cudaStreamSynchronize(idx->stream), "running the split tensor-core scan");
-    if (status != 0)
-        return fail(idx, SSG_ETIMEOUT, "a bounded wait in the split tensor-core scan gave up (code %d)", status);
-    idx->last_fallbacks = nflag;
-    return run_fallback(idx, dq, m, k, exclude_self, flags, nflag, d_ids, d_dists);
+    return plain_finish(idx, "tensor-core", dq, m, k, exclude_self, flags, d_ids, d_dists);
 }
 
 // The plain method on the tensor cores for wide vectors (dim > 128, where a
@@ -1111,7 +1149,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
 constexpr int kPlainNotApplicable = 1;
 
 int ensure_plain_stream_tiles(ssg_index *idx, bool query_role) {
-    const int64_t tiles = ssg::tc_tiles(idx->n);
+    const int64_t tiles = (ssg::tc_tiles(idx->n) + 1) / 2 * 2;  // the list scan reads pairs of tiles
     const float *x = static_cast<const float *>(idx->db.p);
     const size_t tb = 3 * ssg::stream_tile_bytes(idx->dim, 0);
     if (idx->pss_rows != idx->n) {
@@ -1146,7 +1184,6 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     if (metric != SSG_METRIC_SQL2 && metric != SSG_METRIC_L2 && metric != SSG_METRIC_NORMCOSINE &&
         metric != SSG_METRIC_IP && metric != SSG_METRIC_COSINE)
         return kPlainNotApplicable;
-    const bool sq = is_sq_metric(metric);
     const int take = k + (exclude_self ? 1 : 0);
     // the margin shrinks (down to the list's basic 0.45 k) until the scan's heaps hold it
     const int margin = plain_margin(idx, take);
@@ -1160,6 +1197,43 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     const int kp = ssg::stream_kbytes(idx->dim, 0) / 2;  // elements per piece
     const int64_t k3 = 3 * int64_t(kp);
     SSG_RC(ensure_plain_stream_tiles(idx, queries_are_db));
+    SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
+    SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
+    const int64_t qt_alloc = ((m + 127) / 128 + 1) / 2 * 2;  // even: the list scan reads query tiles in pairs
+    const size_t tb = 3 * ssg::stream_tile_bytes(idx->dim, 0);
+    const uint8_t *qt = static_cast<const uint8_t *>(idx->pss_dbq.p);
+    if (!queries_are_db) {
+        SSG_CK(idx->pss_q.ensure(size_t(qt_alloc) * tb), "allocating split query tiles");
+        SSG_CK(ssg::launch_stream_tiles(dq, m, idx->dim, 0, qt_alloc, static_cast<uint8_t *>(idx->pss_q.p), nullptr,
+                                        idx->stream, &idx->last_launches, 2),
+               "building split query tiles");
+        qt = static_cast<const uint8_t *>(idx->pss_q.p);
+    }
+    int *flags = static_cast<int *>(idx->flags.p);
+    int *flag_count = flags + m;
+    // the list scan where a split query tile still fits on chip (to 192 dimensions)
+    ListPlan lp;
+    const int row_bytes = 3 * ssg::stream_kbytes(idx->dim, 0);
+    if (ssg::list_fits(row_bytes, 128, idx->n) && list_plan(idx, m, kk, &lp)) {
+        ssg::ListScan s{};
+        s.dt = static_cast<const uint8_t *>(idx->pss_db.p);
+        s.row_bytes = row_bytes;
+        s.swb = 128;
+        s.epi = ssg::LIST_AFFINE;
+        s.alpha = static_cast<const float *>(idx->pss_alpha.p);
+        s.beta = static_cast<const float *>(idx->pss_beta.p);
+        s.n = idx->n;
+        s.kk = kk;
+        SSG_RC(list_search(idx, s, lp, qt, tb, m, k, exclude_self, d_ids, d_dists,
+                           [&](int64_t c0, ssg::FinalizeArgs &f) {
+                               plain_certificate(idx, kp, flags + c0, flag_count, &f);
+                               return ssg::launch_finalize_rerank(
+                                   idx->metric, f, static_cast<const float *>(idx->db.p),
+                                   static_cast<const float *>(idx->db_norm.p), idx->dim, dq + size_t(c0) * idx->dim,
+                                   dqn ? dqn + c0 : nullptr, idx->stream, &idx->last_launches);
+                           }));
+        return plain_finish(idx, "list", dq, m, k, exclude_self, flags, d_ids, d_dists);
+    }
     const int64_t qtiles = (m + 127) / 128;
     const int64_t n_tiles = ssg::tc_tiles(idx->n);
     int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(qtiles, ssg::device_sm_count(), n_tiles);
@@ -1171,28 +1245,12 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     SSG_CK(idx->cand.ensure(per_query * size_t(chunk)), "allocating candidate scratch");
     SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
-    SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
-    SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
-    const size_t tb = 3 * ssg::stream_tile_bytes(idx->dim, 0);
-    const uint8_t *qt = static_cast<const uint8_t *>(idx->pss_dbq.p);
-    if (!queries_are_db) {
-        SSG_CK(idx->pss_q.ensure(size_t(qtiles) * tb), "allocating split query tiles");
-        SSG_CK(ssg::launch_stream_tiles(dq, m, idx->dim, 0, qtiles, static_cast<uint8_t *>(idx->pss_q.p), nullptr,
-                                        idx->stream, &idx->last_launches, 2),
-               "building split query tiles");
-        qt = static_cast<const uint8_t *>(idx->pss_q.p);
-    }
     // the K-streaming scan's shared pruning bounds, as for its reduced-precision use
     uint32_t *gbound = nullptr;
     if (kk >= 32 && 2 * splits * cs >= kk) {
         SSG_CK(idx->gbound.ensure(size_t(chunk) * ssg::kBoundWords * 4), "allocating query bounds");
         gbound = static_cast<uint32_t *>(idx->gbound.p);
     }
-    // the error bound of the split (run_plain_tc) with this kp
-    const float c = 3.05f * 1.52587890625e-5f + 2.2f * float(kp) * 1.1920929e-7f;
-    const float ulp24 = 5.9604645e-8f;
-    int *flags = static_cast<int *>(idx->flags.p);
-    int *flag_count = flags + m;
     ScanTimer timer(idx);
     for (int64_t c0 = 0; c0 < m; c0 += chunk) {
         const int64_t mc = std::min<int64_t>(chunk, m - c0);
@@ -1217,14 +1275,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
         f.self_base = c0;
         f.out_ids = d_ids + size_t(c0) * k;
         f.out_dists = d_dists + size_t(c0) * k;
-        f.n_rows = idx->n;
-        f.check = sq ? 1 : (idx->metric == SSG_METRIC_COSINE ? 3 : 2);
-        f.max_x_sq = idx->max_x_sq;
-        f.err_scale = sq ? 4.0f * float(idx->dim + 2) * ulp24 + 0.5f * c
-                         : (f.check == 3 ? c + float(2 * idx->dim + 16) * ulp24 : c + float(idx->dim + 2) * ulp24);
-        f.n_total = idx->n;
-        f.flags = flags + c0;
-        f.flag_count = flag_count;
+        plain_certificate(idx, kp, flags + c0, flag_count, &f);
         SSG_CK(ssg::launch_finalize_rerank(idx->metric, f, static_cast<const float *>(idx->db.p),
                                            static_cast<const float *>(idx->db_norm.p), idx->dim, qc,
                                            dqn ? dqn + c0 : nullptr,
@@ -1232,15 +1283,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
                "launching the rerank kernel");
         SSG_RC(timer.collect());
     }
-    int status = 0, nflag = 0;
-    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
-           "reading the status word");
-    SSG_CK(cudaMemcpyAsync(&nflag, flag_count, sizeof(int), cudaMemcpyDeviceToHost, idx->stream), "reading flags");
-    SSG_CK(cudaStreamSynchronize(idx->stream), "running the split streaming scan");
-    if (status != 0)
-        return fail(idx, SSG_ETIMEOUT, "a bounded wait in the split streaming scan gave up (code %d)", status);
-    idx->last_fallbacks = nflag;
-    return run_fallback(idx, dq, m, k, exclude_self, flags, nflag, d_ids, d_dists);
+    return plain_finish(idx, "streaming", dq, m, k, exclude_self, flags, d_ids, d_dists);
 }
 
 int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, int exclude_self,
@@ -1530,6 +1573,40 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
     int qt = 0, stages = 0;
     bool long_lists = false;
     idx->last_fallbacks = 0;
+    // a batch of queries (allknn scans its locality order, below) takes the
+    // list scan: the same kk candidates without heaps to fill in every split
+    ListPlan plan;
+    if (!(queries_are_db && idx->locality_param && !idx->capturing && idx->n >= kLocalityMinRows) &&
+        idx->wide_param && !idx->pair_param && idx->long_param && ssg::list_fits(2 * kp, 64, idx->n) &&
+        list_plan(idx, m, kk, &plan)) {
+        const size_t tb = ssg::tc_tile_bytes(idx->dim);
+        const uint8_t *qtiles = static_cast<const uint8_t *>(idx->tc_db.p);
+        if (!queries_are_db) {
+            const int64_t qt_alloc = ((m + 127) / 128 + 1) / 2 * 2;
+            SSG_CK(idx->tc_q.ensure(size_t(qt_alloc) * tb), "allocating BF16 query tiles");
+            SSG_CK(ssg::launch_bf16_tiles(static_cast<const float *>(dq), m, idx->dim, qt_alloc,
+                                          static_cast<uint8_t *>(idx->tc_q.p), idx->stream, &idx->last_launches),
+                   "building BF16 query tiles");
+            qtiles = static_cast<const uint8_t *>(idx->tc_q.p);
+        }
+        ssg::ListScan s{};
+        s.dt = static_cast<const uint8_t *>(idx->tc_db.p);
+        s.row_bytes = 2 * kp;
+        s.swb = 64;
+        s.epi = list_epilogue(idx->metric);
+        s.alpha = static_cast<const float *>(idx->tc_norm.p);
+        s.n = idx->n;
+        s.kk = kk;
+        SSG_RC(list_search(idx, s, plan, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+                           [&](int64_t c0, ssg::FinalizeArgs &f) {
+                               return ssg::launch_finalize_rerank(
+                                   idx->metric, f, static_cast<const float *>(idx->db.p),
+                                   static_cast<const float *>(idx->db_norm.p), idx->dim,
+                                   static_cast<const float *>(dq) + size_t(c0) * idx->dim, dqn ? dqn + c0 : nullptr,
+                                   idx->stream, &idx->last_launches);
+                           }));
+        return scan_status(idx, "list");
+    }
     // the wide scan (one query tile per CTA, two heaps per query) first when
     // it fits; longer lists on CTA pairs with one heap per query (8 KB ring
     // stages and one heap leave the list twice the room); beyond that the
@@ -1795,6 +1872,50 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     while (kk > take && !ssg::stream_choose(kk, heap_rows, &cs, &stages)) --kk;
     if (!ssg::stream_choose(kk, heap_rows, &cs, &stages))
         return fail(idx, SSG_EUNSUPPORTED, "k = %d does not fit the tensor-core kernel's on-chip top-k", take);
+    const int64_t qt_alloc = ((m + 127) / 128 + 1) / 2 * 2;  // even: the list scan reads query tiles in pairs
+    const size_t tb = ssg::stream_tile_bytes(idx->dim, fp8);
+    const uint8_t *qt = static_cast<const uint8_t *>(idx->st_db.p);
+    const float *qgamma = fp8 ? static_cast<const float *>(idx->st_scale.p) : nullptr;
+    if (!queries_are_db) {
+        SSG_CK(idx->st_q.ensure(size_t(qt_alloc) * tb), "allocating query tiles");
+        float *qs = nullptr;
+        if (fp8) {
+            SSG_CK(idx->st_qscale.ensure(size_t(qt_alloc) * 128 * 4), "allocating query scales");
+            qs = static_cast<float *>(idx->st_qscale.p);
+        }
+        SSG_CK(ssg::launch_stream_tiles(static_cast<const float *>(dq), m, idx->dim, fp8, qt_alloc,
+                                        static_cast<uint8_t *>(idx->st_q.p), qs, idx->stream, &idx->last_launches),
+               "building query tiles");
+        qt = static_cast<const uint8_t *>(idx->st_q.p);
+        qgamma = qs;
+    }
+    // the list scan where a query tile fits on chip (FP8 to 1,280 dimensions,
+    // BF16 to 640) and the database is large enough for its seed; the same kk
+    // candidates
+    ListPlan plan;
+    const int row_bytes = ssg::stream_kbytes(idx->dim, fp8);
+    if (ssg::list_fits(row_bytes, 128, idx->n) && list_plan(idx, m, kk, &plan)) {
+        ssg::ListScan s{};
+        s.dt = static_cast<const uint8_t *>(idx->st_db.p);
+        s.row_bytes = row_bytes;
+        s.swb = 128;
+        s.fp8 = fp8;
+        s.epi = ssg::LIST_AFFINE;
+        s.alpha = static_cast<const float *>(idx->st_alpha.p);
+        s.beta = static_cast<const float *>(idx->st_beta.p);
+        s.gamma = qgamma;
+        s.n = idx->n;
+        s.kk = kk;
+        SSG_RC(list_search(idx, s, plan, qt, tb, m, k, exclude_self, d_ids, d_dists,
+                           [&](int64_t c0, ssg::FinalizeArgs &f) {
+                               return ssg::launch_finalize_rerank(
+                                   idx->metric, f, static_cast<const float *>(idx->db.p),
+                                   static_cast<const float *>(idx->db_norm.p), idx->dim,
+                                   static_cast<const float *>(dq) + size_t(c0) * idx->dim, dqn ? dqn + c0 : nullptr,
+                                   idx->stream, &idx->last_launches);
+                           }));
+        return scan_status(idx, "list");
+    }
     const int64_t qtiles = (m + 127) / 128;
     const int64_t n_tiles = ssg::tc_tiles(idx->n);
     int64_t splits = idx->splits_param > 0 ? idx->splits_param
@@ -1808,22 +1929,6 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     SSG_CK(idx->cand.ensure(per_query * size_t(chunk)), "allocating candidate scratch");
     SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
-    const size_t tb = ssg::stream_tile_bytes(idx->dim, fp8);
-    const uint8_t *qt = static_cast<const uint8_t *>(idx->st_db.p);
-    const float *qgamma = fp8 ? static_cast<const float *>(idx->st_scale.p) : nullptr;
-    if (!queries_are_db) {
-        SSG_CK(idx->st_q.ensure(size_t(qtiles) * tb), "allocating query tiles");
-        float *qs = nullptr;
-        if (fp8) {
-            SSG_CK(idx->st_qscale.ensure(size_t(qtiles) * 128 * 4), "allocating query scales");
-            qs = static_cast<float *>(idx->st_qscale.p);
-        }
-        SSG_CK(ssg::launch_stream_tiles(static_cast<const float *>(dq), m, idx->dim, fp8, qtiles,
-                                        static_cast<uint8_t *>(idx->st_q.p), qs, idx->stream, &idx->last_launches),
-               "building query tiles");
-        qt = static_cast<const uint8_t *>(idx->st_q.p);
-        qgamma = qs;
-    }
     // shared per-query bounds pay when many splits fill long heaps of the
     // same queries (small batches, long candidate lists): with at least kk / 2
     // heaps per query the checkpoint bounds apply (two best values per heap)

@@ -45,3 +45,49 @@ def test_hamming_full_lists(ss, kind, splits):
     Q = np.zeros((40, words), dtype=np.uint64)
     Q[:, 0] = np.arange(40, dtype=np.uint64)
     hamming(ss, X, Q, k, splits)
+
+
+def clustered(n, dim, rng):
+    """Rows sorted towards the query, then a tight block between two sampled tiles."""
+    q = rng.standard_normal(dim).astype(np.float32)
+    X = rng.standard_normal((n, dim), dtype=np.float32)
+    t = np.linspace(0.0, 0.9, n, dtype=np.float32)[:, None]
+    X = (1 - t) * X + t * q
+    X[9 * 256:9 * 256 + 1700] = q + 0.3 * rng.standard_normal((1700, dim), dtype=np.float32)
+    return X, q
+
+
+@pytest.mark.parametrize("metric,dim", [("sql2", 24), ("cosine", 100), ("normcosine", 64), ("l2", 128), ("ip", 160),
+                                        ("cosine", 192)])
+@pytest.mark.parametrize("m,k,splits", [(3, 10, 0), (129, 30, 1)])
+def test_plain_full_lists(ss, metric, dim, m, k, splits):
+    rng = np.random.default_rng(dim + m)
+    X, q = clustered(24_600, dim, rng)
+    Q = (q + 0.2 * rng.standard_normal((m, dim))).astype(np.float32)
+    if metric == "normcosine":
+        X /= np.linalg.norm(X, axis=1, keepdims=True)
+        Q /= np.linalg.norm(Q, axis=1, keepdims=True)
+    dist = {"sql2": ss.Dist.SqL2, "cosine": ss.Dist.Cosine, "normcosine": ss.Dist.NormCosine, "l2": ss.Dist.L2,
+            "ip": ss.Dist.InnerProduct}[metric]()
+    idx = ss.GPUExhaustiveSearch(dist, ss.MatrixDatabase.from_rows(X), splits=splits)
+    ids, dists = ss.searchbatch(idx, ss.GenericContext(), ss.MatrixDatabase.from_rows(Q), k)
+    assert idx.get_param("last_plain_tc") == 1.0
+    ri, rd = O.searchbatch(metric, X, Q, k)
+    assert np.array_equal(ids.T, ri)
+    assert np.array_equal(dists.T, rd)
+
+
+@pytest.mark.parametrize("prec,dim", [("bf16", 96), ("bf16", 300), ("fp8", 130), ("fp8", 768)])
+@pytest.mark.parametrize("m,splits", [(1, 0), (200, 1)])
+def test_reduced_keys_do_not_depend_on_splits(ss, prec, dim, m, splits):
+    """The candidates are the kk smallest approximate keys whatever the splits,
+    the sample and the lists' compactions: one split against many."""
+    rng = np.random.default_rng(dim)
+    X, q = clustered(24_600, dim, rng)
+    Q = (q + 0.2 * rng.standard_normal((m, dim))).astype(np.float32)
+    got = []
+    for s in (splits, 17):
+        idx = ss.GPUExhaustiveSearch(ss.Dist.SqL2(), ss.MatrixDatabase.from_rows(X), precision=prec, overfetch=2.0,
+                                     splits=s)
+        got.append(ss.searchbatch(idx, ss.GenericContext(), ss.MatrixDatabase.from_rows(Q), 20))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
