@@ -439,24 +439,24 @@ bool list_plan(const ssg_index *idx, int64_t m, int kk, ListPlan *p) {
     // lets about 1.2 kk f candidates per query through.  With few queries the
     // scan reads memory and hardly appends: a smaller sample.
     const int64_t f = m > 256 ? 8 : 16;
-    const int64_t least = (int64_t(4) * kk + 7) / 8;  // wide tiles for 4 kk groups of 32 columns
+    const int64_t least = (kk + 1) / 2;  // wide tiles for 4 kk groups of 32 columns
     if (least > n_full / 4) return false;
     p->samples = std::max<int64_t>(least, n_full / f);
     p->stride = n_full / p->samples;
-    p->fine = 2 * p->samples < 4 * kk;
-    p->groups = int(p->samples * (p->fine ? 8 : 2));
+    p->fine = ssg::kListSegs * p->samples < 4 * kk;
+    p->groups = int(p->samples * (p->fine ? 8 : ssg::kListSegs));
     const int64_t qtiles = (m + 127) / 128;
     const int64_t pairs = (qtiles + 1) / 2;
     int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(pairs, ssg::device_sm_count() / 2, n_wide);
     splits = std::max<int64_t>(1, std::min<int64_t>(splits, n_wide));
     p->splits = int(splits);
     const int64_t expect = int64_t(1.25 * kk * double(n_wide) / double(p->samples)) + kk;
-    const int64_t cap = std::max<int64_t>(2 * kk + 64, 4 * expect / (2 * splits) + 64);
-    p->cap = int(std::min<int64_t>(ssg::kListMaxCap, std::max<int64_t>(128, (cap + 31) / 32 * 32)));
+    const int64_t cap = std::max<int64_t>(std::max(2 * kk, kk + 192) + ssg::kListSlack, 4 * expect / (ssg::kListSegs * splits) + 64);
+    p->cap = int(std::min<int64_t>(ssg::kListMaxCap, (cap + 31) / 32 * 32));
     int64_t keys = 1024;
     while (keys < 2 * expect && keys < 8192) keys *= 2;
     p->keys = int(keys);
-    const size_t per_query = size_t(2 * splits) * p->cap * 8;
+    const size_t per_query = size_t(ssg::kListSegs * splits) * p->cap * 8;
     p->chunk = std::max<int64_t>(256, int64_t((size_t(1) << 30) / per_query) / 256 * 256);
     p->chunk = std::min<int64_t>(p->chunk, (m + 255) / 256 * 256);
     return true;
@@ -529,7 +529,7 @@ int reduce_segments(ssg_index *idx, const uint64_t *cand, int64_t m, int segs, i
 
 // Sizes the list scan's buffers for one chunk and points the scan at them.
 int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
-    const size_t segs = size_t(p.splits) * 2;
+    const size_t segs = size_t(p.splits) * ssg::kListSegs;
     SSG_CK(idx->l_lists.ensure(size_t(p.chunk) * segs * p.cap * 8), "allocating candidate lists");
     SSG_CK(idx->l_counts.ensure(size_t(p.chunk) * segs * 4), "allocating list counts");
     SSG_CK(idx->l_minima.ensure(size_t(p.chunk) * p.groups * 4), "allocating the seed's minima");
@@ -553,7 +553,7 @@ int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
 void list_finalize(const ListPlan &p, const ssg::ListScan &s, ssg::FinalizeArgs *f) {
     f->cand = s.lists;
     f->counts = s.counts;
-    f->segs = p.splits * 2;
+    f->segs = p.splits * ssg::kListSegs;
     f->list_cap = p.cap;
     f->list_keys = p.keys;
     f->kk = s.kk;
@@ -1055,7 +1055,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     // a batch of queries (allknn scans its locality order, below): the list scan
     ListPlan lp;
     const bool locality = queries_are_db && idx->locality_param && m == idx->n && idx->n >= kLocalityMinRows;
-    if (!locality && !idx->pair_param && ssg::list_fits(2 * k3, 64, idx->n) && list_plan(idx, m, plan.rr, &lp)) {
+    if (!locality && !idx->pair_param && ssg::list_fits(2 * k3, 64, list_epilogue(idx->metric), idx->n) && list_plan(idx, m, plan.rr, &lp)) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->ps_db.p);
         s.row_bytes = 2 * k3;
@@ -1214,7 +1214,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     // the list scan where a split query tile still fits on chip (to 192 dimensions)
     ListPlan lp;
     const int row_bytes = 3 * ssg::stream_kbytes(idx->dim, 0);
-    if (ssg::list_fits(row_bytes, 128, idx->n) && list_plan(idx, m, kk, &lp)) {
+    if (ssg::list_fits(row_bytes, 128, ssg::LIST_AFFINE, idx->n) && list_plan(idx, m, kk, &lp)) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->pss_db.p);
         s.row_bytes = row_bytes;
@@ -1353,7 +1353,7 @@ int run_knn(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, 
         // 18.8 ms).
         const int kk = int(std::min<int64_t>(int64_t(k) + (exclude_self ? 1 : 0), idx->n));
         ListPlan plan;
-        if (ssg::list_fits(ssg::sketch_row_bytes(idx->dim), 128, idx->n) && list_plan(idx, m, kk, &plan)) {
+        if (ssg::list_fits(ssg::sketch_row_bytes(idx->dim), 128, ssg::LIST_HAMMING, idx->n) && list_plan(idx, m, kk, &plan)) {
             // the tiles take 8 times the sketches: without the memory the
             // sketches are scanned as they are
             const int rc = run_hamming_tc(idx, dq, m, k, exclude_self, d_ids, d_dists, queries_are_db, kk, plan);
@@ -1577,7 +1577,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
     // list scan: the same kk candidates without heaps to fill in every split
     ListPlan plan;
     if (!(queries_are_db && idx->locality_param && !idx->capturing && idx->n >= kLocalityMinRows) &&
-        idx->wide_param && !idx->pair_param && idx->long_param && ssg::list_fits(2 * kp, 64, idx->n) &&
+        idx->wide_param && !idx->pair_param && idx->long_param && ssg::list_fits(2 * kp, 64, list_epilogue(idx->metric), idx->n) &&
         list_plan(idx, m, kk, &plan)) {
         const size_t tb = ssg::tc_tile_bytes(idx->dim);
         const uint8_t *qtiles = static_cast<const uint8_t *>(idx->tc_db.p);
@@ -1894,7 +1894,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     // candidates
     ListPlan plan;
     const int row_bytes = ssg::stream_kbytes(idx->dim, fp8);
-    if (ssg::list_fits(row_bytes, 128, idx->n) && list_plan(idx, m, kk, &plan)) {
+    if (ssg::list_fits(row_bytes, 128, ssg::LIST_AFFINE, idx->n) && list_plan(idx, m, kk, &plan)) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->st_db.p);
         s.row_bytes = row_bytes;

@@ -206,7 +206,9 @@ cudaError_t launch_stream_scan(const uint8_t *q_tiles, const uint8_t *d_tiles, c
 // ---- resident-query scan with candidate lists (tc_list.cu) ----
 enum { LIST_DOT = 0, LIST_SQ = 1, LIST_COS = 2, LIST_AFFINE = 3, LIST_HAMMING = 4 };
 constexpr int kListMaxCap = 1024;  // entries of one list at most
-// One scan of n database rows for m queries: query (q, seg) of 2 * splits
+constexpr int kListSlack = 160;    // entries beyond kk that every list has room for at least
+constexpr int kListSegs = 2;       // lists of a query per split
+// One scan of n database rows for m queries: (q, seg) of kListSegs * splits
 // segments leaves counts[q * segs + seg] unsorted keys at
 // lists[(q * segs + seg) * cap]; together they hold the query's kk smallest.
 struct ListScan {
@@ -229,7 +231,7 @@ struct ListScan {
     float *minima;            // m * groups
     int *err;
 };
-bool list_fits(int row_bytes, int swb, int64_t n);
+bool list_fits(int row_bytes, int swb, int epi, int64_t n);
 cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches);
 cudaError_t launch_list_scan(const ListScan &s, cudaStream_t st, int *launches);
 // Sketches as +-1 FP8 rows (128-byte K-blocks).

@@ -25,9 +25,9 @@
 // 64 with one CTA (L2 gives about 35) and 128 for 128 x 128 tiles with both
 // operands streamed.
 //
-// Roles (320 threads per CTA, as in tc_pair_kernel): warp 0 producer, warp 1
-// TMEM owner and, in the even CTA, MMA issuer, warps 2..9 epilogue (two per
-// TMEM lane quarter, alternate 32-column chunks, a list each).  Every
+// Roles (320 threads per CTA): warp 0 producer, warp 1 TMEM owner and, in the
+// even CTA, MMA issuer, warps 2..9 epilogue (two per TMEM lane quarter,
+// alternate 32-column chunks of every wide tile, a list each).  Every
 // mbarrier wait is bounded (tc_ptx.cuh); both CTAs meet at a cluster barrier
 // before TMEM is freed.
 #include "common.cuh"
@@ -42,14 +42,21 @@ namespace ssg {
 
 namespace {
 
-constexpr int TILE = 128;
-constexpr int WIDE = 2 * TILE;
-constexpr int NACC = 2;
-constexpr int kThreads = 64 + 2 * TILE;
+constexpr int TILE = 128;      // query rows per CTA, database rows per tile
+constexpr int WIDE = 2 * TILE;  // database rows per MMA: a tile of each CTA
+constexpr int NACC = 2;         // accumulators of 256 columns: all 512 TMEM columns
+constexpr int CS = kListSegs;   // epilogue warps per TMEM lane quarter, a list each
+constexpr int kThreads = 64 + CS * TILE;
+constexpr int kStageBytes = 32 * 1024;  // most of a ring stage
+constexpr int kLine = 2048;             // bytes of a tensor-map line
 constexpr int kMaxStages = 16;
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kAloneSmem = 120 * 1024;  // all 512 TMEM columns: alone on the SM
-constexpr int kSlack = 8;                  // appends between two checks of a list's room
+constexpr int kCoefBytes = 4 * CS * 2 * (8 / CS) * 256;  // per warp two buffers of its columns' coefficients
+constexpr int kTileColumns = WIDE / CS;    // columns of a tile that one list can take
+constexpr int kBufCap = 12;                // raw candidates buffered per lane
+constexpr int kBufStride = CS * TILE * 8;  // bytes between a lane's buffer slots
+constexpr int kBufBytes = kBufCap * kBufStride;
 
 enum { EPI_DOT = LIST_DOT, EPI_SQ = LIST_SQ, EPI_COS = LIST_COS, EPI_AFF = LIST_AFFINE, EPI_HAM = LIST_HAMMING };
 
@@ -60,6 +67,7 @@ __host__ __device__ constexpr bool raw_rank(int epi) { return epi == EPI_DOT || 
 struct KernelArgs {
     ListScan s;
     int kblocks;        // K-blocks per row
+    int group;          // K-blocks per ring stage (a divisor of kblocks)
     int stages;         // ring depth
     int64_t n_wide;     // wide tiles of this pass (the sample's in SEED)
 };
@@ -139,48 +147,30 @@ __device__ __forceinline__ float rank_distance(float x, float bits) {
     return EPI == EPI_DOT ? -x : EPI == EPI_HAM ? (bits - x) * 0.5f : x;
 }
 
-// Appends those of eight columns' values v (columns id0.. of which lim are
-// rows) that pass the limit t (products >= t, distances <= t) to the lane's
-// list; full lists of the warp are compacted.  All 32 lanes call it.  Returns
-// the count (low word) and the limit, tightened by a compaction (high word).
-// One copy of this code for every call site: unrolled at the sites, the
-// kernel overflowed the instruction cache and an append took ~2,400 cycles
-// (10,000 queries x 2e6 sketches: 27.9 ms; with this function 12.2).
+// Moves the c raw candidates buffered at shared address buf (slots kBufStride
+// apart: ranking value, id) to the lane's list, as keys.  All 32 lanes call it,
+// with scalars alone and few registers of its own, so the call saves nothing.
 template <int EPI>
-__device__ __noinline__ uint64_t append_group(uint64_t *list, int nb, int cap, int kk, float t, float bits,
-                                              uint32_t id0, int lim, float v0, float v1, float v2, float v3, float v4,
-                                              float v5, float v6, float v7) {
-    const float v[8] = {v0, v1, v2, v3, v4, v5, v6, v7};
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        if ((raw_rank(EPI) ? v[j] >= t : v[j] <= t) && j < lim) {
-            list[nb] = make_key(rank_distance<EPI>(v[j], bits), id0 + uint32_t(j));
+__device__ __noinline__ int drain_raw(uint64_t *list, uint32_t buf, int c, int nb, float bits) {
+    const int cmax = __reduce_max_sync(0xffffffffu, c);
+    for (int i = 0; i < cmax; ++i) {
+        if (i < c) {
+            float v;
+            uint32_t id;
+            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=f"(v), "=r"(id) : "r"(buf + i * kBufStride) : "memory");
+            list[nb] = make_key(rank_distance<EPI>(v, bits), id);
             ++nb;
         }
     }
-    if (__any_sync(0xffffffffu, nb > cap - kSlack)) {
-        uint64_t top = 0;
-        const bool full = nb > cap - kSlack;
-        nb = compact_lists(list, nb, cap - kSlack, kk, &top);
-        if (full) {
-            // kk keys up to `top` are kept and ids only grow from here: an
-            // equal distance no longer counts
-            const float d = key_dist(top);
-            if (EPI == EPI_HAM) t = fmaxf(t, bits - 2.0f * d + 1.0f);
-            else {
-                const float below = ordered_to_float(float_to_ordered(d) - 1u);
-                t = EPI == EPI_DOT ? fmaxf(t, -below) : fminf(t, below);
-            }
-        }
-    }
-    return (uint64_t(__float_as_uint(t)) << 32) | uint32_t(nb);
+    return nb;
 }
 
 // One query row's candidates (one lane).
 template <int EPI>
 struct RowList {
     uint64_t *list;
-    int nb, cap, kk;
+    uint32_t buf;      // shared address of this lane's raw buffer
+    int nb, nbuf, cap, kk;
     int64_t n;
     bool valid;
     float lim_v;       // a candidate's ranking value: product >= lim_v (raw_rank) or distance <= lim_v
@@ -193,17 +183,16 @@ struct RowList {
         lim_v = EPI == EPI_HAM ? bits - 2.0f * t : EPI == EPI_DOT ? -t : t;
     }
     // ranking values of a chunk's 32 columns: products (raw_rank) or distances
-    __device__ __forceinline__ void values(const uint32_t (&r)[32], int64_t id0, const ListScan &s,
+    // (al, be: the columns' coefficients in shared memory)
+    __device__ __forceinline__ void values(const uint32_t (&r)[32], const float4 *al, const float4 *be,
                                            float (&dv)[32]) const {
         if constexpr (raw_rank(EPI)) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) dv[j] = __uint_as_float(r[j]);
         } else {
-            const float4 *al = reinterpret_cast<const float4 *>(s.alpha + id0);
-            const float4 *be = EPI == EPI_AFF ? reinterpret_cast<const float4 *>(s.beta + id0) : nullptr;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const float4 a = __ldg(al + j);
+                const float4 a = al[j];
                 const float v0 = __uint_as_float(r[4 * j]), v1 = __uint_as_float(r[4 * j + 1]);
                 const float v2 = __uint_as_float(r[4 * j + 2]), v3 = __uint_as_float(r[4 * j + 3]);
                 if constexpr (EPI == EPI_SQ) {
@@ -217,7 +206,7 @@ struct RowList {
                     dv[4 * j + 2] = -v2 * a.z;
                     dv[4 * j + 3] = -v3 * a.w;
                 } else {
-                    const float4 b = __ldg(be + j);
+                    const float4 b = be[j];
                     dv[4 * j] = fmaf(v0 * gamma, a.x, b.x);
                     dv[4 * j + 1] = fmaf(v1 * gamma, a.y, b.y);
                     dv[4 * j + 2] = fmaf(v2 * gamma, a.z, b.z);
@@ -231,28 +220,61 @@ struct RowList {
     __device__ __forceinline__ bool passes(float x) const { return raw_rank(EPI) ? x >= lim_v : x <= lim_v; }
 
     // the smallest distance among the chunk's columns (all of them rows)
-    __device__ __forceinline__ float chunk_min(const uint32_t (&r)[32], int64_t id0, const ListScan &s) const {
+    __device__ __forceinline__ float chunk_min(const uint32_t (&r)[32], const float4 *al, const float4 *be) const {
         float dv[32];
-        values(r, id0, s, dv);
+        values(r, al, be, dv);
         const float b = best(best(best8(dv), best8(dv + 8)), best(best8(dv + 16), best8(dv + 24)));
         return fminf(rank_distance<EPI>(b, bits), INFINITY);  // NaN products: +inf
     }
-    __device__ __forceinline__ void chunk(const uint32_t (&r)[32], int64_t id0, const ListScan &s) {
+    __device__ __forceinline__ void drain() {
+        nb = drain_raw<EPI>(list, buf, nbuf, nb, bits);
+        nbuf = 0;
+    }
+    // Between tiles (nothing of an accumulator in registers): makes room for
+    // another tile's columns in every list of the warp.
+    __device__ __forceinline__ void make_room() {
+        const int room = cap - kTileColumns - kBufCap;
+        if (!__any_sync(0xffffffffu, nb > room)) return;
+        drain();
+        uint64_t top = 0;
+        const bool full = nb > room;
+        nb = compact_lists(list, nb, room, kk, &top);
+        if (full) {
+            // kk keys up to `top` are kept and ids only grow from here: an
+            // equal distance no longer counts
+            const float d = key_dist(top);
+            if (EPI == EPI_HAM) lim_v = fmaxf(lim_v, bits - 2.0f * d + 1.0f);
+            else {
+                const float below = ordered_to_float(float_to_ordered(d) - 1u);
+                lim_v = EPI == EPI_DOT ? fmaxf(lim_v, -below) : fminf(lim_v, below);
+            }
+        }
+    }
+    // Candidates of a chunk: a vote on the chunk and on each group of 8
+    // columns, then branch-free raw appends (the slot is always written, the
+    // count only advances for a candidate) to a buffer that is drained when a
+    // lane has more than kBufCap - 8.  Anything dearer per group held up the
+    // MMAs: 2,048 queries x 1e6 rows x 96 dimensions took 691 us with the
+    // keys appended at the sites, 497 through a function (its calls spilled
+    // the accumulator's registers), 356 so.
+    __device__ __forceinline__ void chunk(const uint32_t (&r)[32], int64_t id0, const float4 *al, const float4 *be) {
         float dv[32], g[4];
-        values(r, id0, s, dv);
+        values(r, al, be, dv);
 #pragma unroll
         for (int i = 0; i < 4; ++i) g[i] = best8(dv + 8 * i);
         if (!__any_sync(0xffffffffu, passes(best(best(g[0], g[1]), best(g[2], g[3]))))) return;
-        const int lim = int(id0 + 32 <= n ? 32 : n - id0);  // columns that are rows
+        const int lim = !valid ? 0 : id0 + 32 <= n ? 32 : int(n - id0);  // columns that are rows
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (!__any_sync(0xffffffffu, passes(g[i]))) continue;
-            const float *v = dv + 8 * i;
-            const uint64_t r2 = append_group<EPI>(list, nb, cap, kk, lim_v, bits, uint32_t(id0) + 8u * i,
-                                                  valid ? lim - 8 * i : 0, v[0], v[1], v[2], v[3], v[4], v[5], v[6],
-                                                  v[7]);
-            nb = int(uint32_t(r2));
-            lim_v = __uint_as_float(uint32_t(r2 >> 32));
+#pragma unroll
+            for (int j = 8 * i; j < 8 * i + 8; ++j) {
+                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(buf + nbuf * kBufStride), "f"(dv[j]),
+                             "r"(uint32_t(id0) + uint32_t(j))
+                             : "memory");
+                nbuf += (passes(dv[j]) && j < lim) ? 1 : 0;
+            }
+            if (__any_sync(0xffffffffu, nbuf > kBufCap - 8)) drain();
         }
     }
 };
@@ -260,24 +282,28 @@ struct RowList {
 template <int SWB, bool F8, int EPI, bool SEED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     tc_list_kernel(KernelArgs ka, const __grid_constant__ CUtensorMap dmap) {
-    constexpr int KBLK = TILE * SWB;   // bytes of a K-block of one 128-row tile
+    constexpr int KBLK = TILE * SWB;   // bytes of a K-block of a tile
     constexpr int KSTEPS = SWB / 32;   // MMAs per K-block (32 bytes of K each)
     const ListScan &a = ka.s;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int kblocks = ka.kblocks, stages = ka.stages;
+    const int kblocks = ka.kblocks, stages = ka.stages, group = ka.group;
+    const int groups_per_tile = kblocks / group;
     const size_t tile_bytes = size_t(kblocks) * KBLK;
+    const uint32_t stage_bytes = uint32_t(group) * KBLK;
     uint8_t *sA = smem;
     uint8_t *sB = sA + tile_bytes;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sB + size_t(stages) * KBLK);
+    // per epilogue warp, two buffers of its 64 columns' coefficients
+    float4 *coef = reinterpret_cast<float4 *>(sB + size_t(stages) * stage_bytes);
+    uint64_t *bufs = reinterpret_cast<uint64_t *>(coef + (raw_rank(EPI) ? 0 : kCoefBytes / 16));  // raw candidates
+    uint64_t *bars = bufs + (SEED ? 0 : kBufBytes / 8);
     uint64_t *a_full = bars;                  // this CTA's query tile landed
     uint64_t *pa_full = a_full + 1;           // (even CTA) the odd CTA's query tile landed
     uint64_t *full = pa_full + 1;             // (even CTA) both halves of stage s landed
     uint64_t *empty = full + kMaxStages;      // the MMAs of stage s are done
-    uint64_t *acc_full = empty + kMaxStages;  // accumulator b holds a finished wide tile
-    uint64_t *acc_empty = acc_full + NACC;    // (even CTA) its epilogue warps released b
-    uint64_t *pacc_empty = acc_empty + NACC;  // (even CTA) the odd CTA's epilogue warps released b
-    uint64_t *mma_done = pacc_empty + NACC;
+    uint64_t *acc_full = empty + kMaxStages;  // accumulator b holds a finished tile
+    uint64_t *acc_empty = acc_full + NACC;    // (even CTA) the epilogue warps of both CTAs released b
+    uint64_t *mma_done = acc_empty + NACC;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mma_done + 1);
     const int warp = threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
@@ -285,14 +311,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const uint32_t peer = rank ^ 1u;
     const int64_t qx = blockIdx.x;                // this CTA's query tile
     const int64_t qpair = qx - int64_t(rank);
-    // epilogue warps of a query tile whose lane quarter holds a query
-    auto live_warps = [&](int64_t tile) {
-        int live = 0;
-        for (int w = 0; w < 4; ++w)
-            if (tile * TILE + w * 32 < a.m) live += 2;
-        return live;
-    };
-    const int live_self = live_warps(qx), live_peer = live_warps(qpair + int64_t(peer));
+    // epilogue warps of the pair whose lane quarter holds a query
+    int live = 0;
+    for (int w = 0; w < 8; ++w)
+        if (qpair * TILE + w * 32 < a.m) live += CS;
 
     if (threadIdx.x == 0) {
         tc::mbar_init(a_full, 1);
@@ -303,8 +325,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         }
         for (int b = 0; b < NACC; ++b) {
             tc::mbar_init(&acc_full[b], 1);
-            tc::mbar_init(&acc_empty[b], live_self > 0 ? live_self : 1);
-            tc::mbar_init(&pacc_empty[b], live_peer > 0 ? live_peer : 1);
+            tc::mbar_init(&acc_empty[b], live);
         }
         tc::mbar_init(mma_done, 1);
         tc::fence_mbarrier_init();
@@ -325,8 +346,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 
     if (warp == 0) {
         if (lane == 0) {
-            // producer: this CTA's query tile, then its half of every K-block;
-            // both halves of a stage complete on the even CTA's full[s]
+            // producer: this CTA's query tile, then its tile's part of
+            // every K-block group; both halves of a stage complete on the
+            // even CTA's full[s]
             tc::mbar_arrive_expect_tx(a_full, uint32_t(tile_bytes));
             for (int kb = 0; kb < kblocks; ++kb)
                 tc::bulk_g2s(sA + size_t(kb) * KBLK, a.qt + size_t(qx) * tile_bytes + size_t(kb) * KBLK, KBLK, a_full);
@@ -335,20 +357,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             uint32_t ph = 1;
             bool ok = true;
             for (int u = 0; ok && u < W; ++u) {
-                const int64_t tile = 2 * wide_tile(u) + rank;
-                const uint8_t *src = a.dt + size_t(tile) * tile_bytes;
-                int line = int(tile * kblocks * TILE);
-                for (int kb = 0; kb < kblocks; ++kb) {
+                int line = (int(wide_tile(u)) * 2 + int(rank)) * kblocks * (KBLK / kLine);
+                for (int g = 0; g < groups_per_tile; ++g, line += group * (KBLK / kLine)) {
                     if (!tc::mbar_wait(&empty[s], ph, a.err, 21)) { ok = false; break; }
-                    uint8_t *dst = sB + size_t(s) * KBLK;
-                    if (rank == 0) {
-                        tc::mbar_arrive_expect_tx(&full[s], uint32_t(2 * KBLK));
-                        tc::bulk_g2s(dst, src, uint32_t(KBLK), &full[s]);
-                    } else {
-                        tc::tma_load_2d_pair(dst, &dmap, 0, line, full0 + uint32_t(s * 8));
-                    }
-                    src += KBLK;
-                    line += TILE;
+                    if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
+                    tc::tma_load_2d_pair(sB + size_t(s) * stage_bytes, &dmap, 0, line, full0 + uint32_t(s * 8));
                     issued = issued < stages ? issued + 1 : stages;
                     if (++s == stages) { s = 0; ph ^= 1; }
                 }
@@ -374,32 +387,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             // the even CTA issues the pair's MMAs
             constexpr uint32_t idesc = F8 ? tc::idesc_e4m3_f32(2 * TILE, WIDE) : tc::idesc_bf16_f32(2 * TILE, WIDE);
             bool ok = tc::mbar_wait(a_full, 0, a.err, 23) && tc::mbar_wait(pa_full, 0, a.err, 23);
+            // descriptors address 16-byte units
             const uint64_t a_desc = tc::smem_desc(tc::smem_u32(sA), SWB);
             const uint64_t b_desc = tc::smem_desc(tc::smem_u32(sB), SWB);
-            int s = 0;
-            uint32_t ph = 0;
+            int s = 0, b = 0;
+            uint32_t ph = 0, aph = 1;
             for (int u = 0; ok && u < W; ++u) {
-                const int b = u & 1;
-                const uint32_t aph = ((u >> 1) & 1) ^ 1;
-                if (live_self > 0 && !tc::mbar_wait(&acc_empty[b], aph, a.err, 25)) break;
-                if (live_peer > 0 && !tc::mbar_wait(&pacc_empty[b], aph, a.err, 25)) break;
+                if (!tc::mbar_wait(&acc_empty[b], aph, a.err, 25)) break;
                 const uint32_t d_tmem = tmem_base + uint32_t(b * WIDE);
-                for (int kb = 0; kb < kblocks; ++kb) {
+                uint64_t ad = a_desc;
+                uint32_t acc = 0;
+                for (int g = 0; g < groups_per_tile; ++g) {
                     if (!tc::mbar_wait(&full[s], ph, a.err, 24)) { ok = false; break; }
                     tc::tc_fence_after();
+                    uint64_t bd = b_desc + uint64_t((uint32_t(s) * stage_bytes) >> 4);
+                    for (int kb = 0; kb < group; ++kb) {
 #pragma unroll
-                    for (int k = 0; k < KSTEPS; ++k) {
-                        // descriptors address 16-byte units
-                        const uint64_t ad = a_desc + uint64_t((kb * KBLK + k * 32) >> 4);
-                        const uint64_t bd = b_desc + uint64_t((s * KBLK + k * 32) >> 4);
-                        if (F8) tc::mma_f8_pair(d_tmem, ad, bd, idesc, (kb | k) ? 1u : 0u);
-                        else tc::mma_f16_pair(d_tmem, ad, bd, idesc, (kb | k) ? 1u : 0u);
+                        for (int k = 0; k < KSTEPS; ++k) {
+                            if (F8) tc::mma_f8_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, k ? 1u : acc);
+                            else tc::mma_f16_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, k ? 1u : acc);
+                        }
+                        acc = 1;
+                        ad += KBLK >> 4;
+                        bd += KBLK >> 4;
                     }
                     tc::mma_commit_both(&empty[s]);
                     if (++s == stages) { s = 0; ph ^= 1; }
                 }
                 if (!ok) break;
                 tc::mma_commit_both(&acc_full[b]);
+                if (++b == NACC) { b = 0; aph ^= 1; }
             }
             tc::mma_commit_pair(tc::smem_u32(mma_done));
             tc::mbar_wait(mma_done, 0, a.err, 26);
@@ -409,12 +426,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         const int cs = (warp - 2) / 4;
         const int quarter = warp % 4;
         const int64_t query = qx * TILE + quarter * 32 + lane;
-        const uint32_t r_pacc0 = tc::mapa_shared(tc::smem_u32(pacc_empty), peer);
-        const int seg = int(blockIdx.y) * 2 + cs, segs = a.splits * 2;
+        const uint32_t release0 = tc::mapa_shared(tc::smem_u32(acc_empty), 0);
+        const int seg = int(blockIdx.y) * CS + cs, segs = a.splits * CS;
         RowList<EPI> T;
         T.valid = query < a.m;
         T.list = SEED ? nullptr : a.lists + (size_t(T.valid ? query : 0) * segs + seg) * a.cap;
         T.nb = 0;
+        T.nbuf = 0;
+        T.buf = tc::smem_u32(bufs) + uint32_t((warp - 2) * 32 + lane) * 8;
         T.cap = a.cap;
         T.kk = a.kk;
         T.n = a.n;
@@ -422,56 +441,92 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         T.gamma = (EPI == EPI_AFF && a.gamma && T.valid) ? a.gamma[query] : 1.0f;
         T.set((!SEED && T.valid) ? bound_read(a.bound + query) : INFINITY);
         const bool warp_live = qx * TILE + quarter * 32 < a.m;
+        // this warp's columns of a wide tile: the 32-column chunks cs, cs + CS, ...;
+        // their coefficients are copied a tile ahead
+        constexpr int CH = 8 / CS;
+        float4 *mine = coef + (warp - 2) * CH * 32;
+        auto fetch = [&](int u, int buf) {
+            if constexpr (!raw_rank(EPI)) {
+                constexpr int PER = CH * 8;  // 16-byte pieces of alpha, and of beta
+                for (int p = lane; p < (EPI == EPI_AFF ? 2 : 1) * PER; p += 32) {
+                    const float *src = (p < PER ? a.alpha : a.beta) + wide_tile(u) * WIDE +
+                                       (cs + CS * (p % PER / 8)) * 32 + (p % 8) * 4;
+                    const uint32_t d = tc::smem_u32(mine + buf * 2 * PER + p);
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+            }
+        };
+        if (warp_live && W > 0) fetch(0, 0);
+        int b = 0;
+        uint32_t ph = 0;
         for (int u = 0; warp_live && u < W; ++u) {
-            const int b = u & 1;
             int ok = 1;
-            if (lane == 0) ok = tc::mbar_wait(&acc_full[b], (u >> 1) & 1, a.err, 27) ? 1 : 0;
+            if (lane == 0) ok = tc::mbar_wait(&acc_full[b], ph, a.err, 27) ? 1 : 0;
             ok = __shfl_sync(0xffffffffu, ok, 0);
             if (!ok) break;
             tc::tc_fence_after();
-            // this warp's chunks cs, cs + 2, ... of the wide tile, two in
-            // flight per round (four spill beside the list's state: 13.5 ms
-            // against 12.2 for 10,000 queries x 2e6 sketches); the
-            // accumulator goes back after the last load
-            constexpr int LDC = 2;
-            const int64_t row0 = wide_tile(u) * WIDE + cs * 32;
+            // all four chunks in flight together where their products are
+            // the ranking values, and the accumulator back before any is
+            // looked at; two rounds of two where the distances take registers
+            // too.  (Sixteen warps with two chunks each release as early but
+            // crowd the MMA thread: 10,000 queries x 2e6 sketches 11.8 ms
+            // against 10.4.)
+            constexpr int LDC = raw_rank(EPI) ? 4 : 2;
             const uint32_t tbase = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(b * WIDE + cs * 32);
+            const int64_t row0 = wide_tile(u) * WIDE + cs * 32;
+            const float4 *al = mine + (u & 1) * (CH * 16);  // alpha, then beta
             uint32_t r[LDC][32];
-            float gmin[4];
+            float gm[CH];
 #pragma unroll
-            for (int round = 0; round < 4 / LDC; ++round) {
+            for (int round = 0; round < CH / LDC; ++round) {
                 __syncwarp();
 #pragma unroll
                 for (int c = 0; c < LDC; ++c)
-                    tc::tmem_ld_32x32b_x32_async(tbase + uint32_t((round * LDC + c) * 64), r[c]);
-                tc::tmem_wait_ld();
-                if (round == 4 / LDC - 1) {
-                    tc::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (rank == 0) tc::mbar_arrive(&acc_empty[b]);
-                        else tc::mbar_arrive_cluster(r_pacc0 + uint32_t(b * 8));
+                    tc::tmem_ld_32x32b_x32_async(tbase + uint32_t((round * LDC + c) * CS * 32), r[c]);
+                if constexpr (!raw_rank(EPI)) {
+                    if (round == 0) {
+                        if (u + 1 < W) fetch(u + 1, (u + 1) & 1);
+                        else asm volatile("cp.async.commit_group;" ::: "memory");
+                        asm volatile("cp.async.wait_group 1;" ::: "memory");
                     }
+                }
+                tc::tmem_wait_ld();
+                if (round == CH / LDC - 1) tc::tc_fence_before();
+                __syncwarp();
+                if (round == CH / LDC - 1 && lane == 0) {
+                    if (rank == 0) tc::mbar_arrive(&acc_empty[b]);
+                    else tc::mbar_arrive_cluster_relaxed(release0 + uint32_t(b * 8));
                 }
 #pragma unroll
                 for (int c = 0; c < LDC; ++c) {
-                    const int64_t id0 = row0 + (round * LDC + c) * 64;
-                    if constexpr (SEED) gmin[round * LDC + c] = T.chunk_min(r[c], id0, a);
-                    else T.chunk(r[c], id0, a);
+                    const int ch = round * LDC + c;
+                    if constexpr (SEED) gm[ch] = T.chunk_min(r[c], al + ch * 8, al + CH * 8 + ch * 8);
+                    else T.chunk(r[c], row0 + ch * CS * 32, al + ch * 8, al + CH * 8 + ch * 8);
                 }
             }
+            if (++b == NACC) { b = 0; ph ^= 1; }
             if constexpr (SEED) {
                 if (T.valid) {
                     float *g = a.minima + size_t(query) * a.groups;
                     const int64_t at = w_lo + u;
                     if (a.fine_groups) {
-                        *reinterpret_cast<float4 *>(g + at * 8 + cs * 4) = make_float4(gmin[0], gmin[1], gmin[2], gmin[3]);
+                        // (groups of a wide tile: 8, or one per epilogue warp of a quarter)
+#pragma unroll
+                        for (int ch = 0; ch < CH; ++ch) g[at * 8 + cs * CH + ch] = gm[ch];
                     } else {
-                        g[at * 2 + cs] = fminf(fminf(gmin[0], gmin[1]), fminf(gmin[2], gmin[3]));
+                        float v = gm[0];
+#pragma unroll
+                        for (int ch = 1; ch < CH; ++ch) v = fminf(v, gm[ch]);
+                        g[at * CS + cs] = v;
                     }
                 }
             }
+            if constexpr (!SEED) T.make_room();
+            if constexpr (!raw_rank(EPI)) __syncwarp();  // the buffer is refilled a tile later
         }
+        if (!raw_rank(EPI)) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (!SEED && warp_live) T.drain();
         if (!SEED && T.valid) a.counts[size_t(query) * segs + seg] = T.nb;
     }
     tc::tc_fence_before();
@@ -544,9 +599,10 @@ __global__ void sketch_tile_kernel(const uint64_t *__restrict__ x, int64_t rows,
     }
 }
 
-// The database tiles as a 2D array of K-block lines (swb bytes each, already
-// swizzled); a box of 128 lines is one tile's K-block, copied verbatim.
-cudaError_t line_map(const ListScan &s, int kblocks, CUtensorMap *map) {
+// The database tiles as lines of 2 KB (256 eight-byte elements; the bytes are
+// already swizzled, so a box is copied verbatim): a box is one tile's part of
+// a ring stage, a whole row's K-blocks where they fit.
+cudaError_t line_map(const ListScan &s, int kblocks, int group, CUtensorMap *map) {
     using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -560,25 +616,39 @@ cudaError_t line_map(const ListScan &s, int kblocks, CUtensorMap *map) {
         encode = reinterpret_cast<EncodeFn>(fn);
     }
     if (reinterpret_cast<uintptr_t>(s.dt) % 16 != 0) return cudaErrorInvalidValue;
-    const int64_t tiles = ((s.n + TILE - 1) / TILE + 1) / 2 * 2;
-    const cuuint64_t dims[2] = {cuuint64_t(s.swb), cuuint64_t(tiles) * kblocks * TILE};
-    const cuuint64_t strides[1] = {cuuint64_t(s.swb)};
-    const cuuint32_t box[2] = {cuuint32_t(s.swb), cuuint32_t(TILE)};
+    const int64_t tiles = (s.n + WIDE - 1) / WIDE * 2;
+    const cuuint64_t dims[2] = {cuuint64_t(kLine / 8), cuuint64_t(tiles) * kblocks * (TILE * s.swb / kLine)};
+    const cuuint64_t strides[1] = {cuuint64_t(kLine)};
+    const cuuint32_t box[2] = {cuuint32_t(kLine / 8), cuuint32_t(group * (TILE * s.swb / kLine))};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<uint8_t *>(s.dt), dims, strides, box,
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<uint8_t *>(s.dt), dims, strides, box,
                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-size_t list_smem(int tile_bytes, int kblk, int stages) {
-    return 1024 + size_t(tile_bytes) + size_t(stages) * kblk + (2 + 2 * kMaxStages + 3 * NACC + 1) * 8 + 16;
+size_t list_smem(int row_bytes, int stage_bytes, int stages, int epi) {
+    return 1024 + size_t(TILE) * row_bytes + size_t(stages) * stage_bytes + (raw_rank(epi) ? 0 : kCoefBytes) + kBufBytes +
+           (2 + 2 * kMaxStages + 2 * NACC + 1) * 8 + 16;
 }
 
-int list_stages(int row_bytes, int swb) {
-    int st = kMaxStages;
-    while (st > 0 && list_smem(TILE * row_bytes, TILE * swb, st) > kMaxSmem) --st;
-    return st;
+// The ring beside a query tile: K-blocks per stage (a divisor of the row's)
+// and stages.  Every stage costs the MMA thread a wait and a commit, so the
+// largest stages of which three fit, up to 32 KB (2,048 queries x 1e6 rows of
+// 96 dimensions: the seed 51 us with a K-block per stage, 35 with the row's
+// three).  stages = 0: not even four K-blocks fit.
+struct Ring {
+    int group, stages;
+};
+Ring list_ring(int row_bytes, int swb, int epi) {
+    const int kblocks = row_bytes / swb;
+    for (int g = std::min(kblocks, kStageBytes / (TILE * swb)); g >= 1; --g) {
+        if (kblocks % g) continue;
+        int st = kMaxStages;
+        while (st > 0 && list_smem(row_bytes, g * TILE * swb, st, epi) > kMaxSmem) --st;
+        if (st >= 3 && st * g >= 4) return {g, st};
+    }
+    return {1, 0};
 }
 
 template <int SWB, bool F8, int EPI, bool SEED>
@@ -586,15 +656,18 @@ cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
     KernelArgs ka;
     ka.s = s;
     ka.kblocks = s.row_bytes / SWB;
-    ka.stages = list_stages(s.row_bytes, SWB);
+    const Ring ring = list_ring(s.row_bytes, SWB, EPI);
+    if (ring.stages == 0) return cudaErrorInvalidValue;
+    ka.group = ring.group;
+    ka.stages = ring.stages;
     ka.n_wide = SEED ? s.samples : (s.n + WIDE - 1) / WIDE;
-    size_t smem = list_smem(TILE * s.row_bytes, TILE * SWB, ka.stages);
+    size_t smem = list_smem(s.row_bytes, ring.group * TILE * SWB, ring.stages, EPI);
     if (smem < kAloneSmem) smem = kAloneSmem;
     auto kern = tc_list_kernel<SWB, F8, EPI, SEED>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     CUtensorMap map;
-    e = line_map(s, ka.kblocks, &map);
+    e = line_map(s, ka.kblocks, ka.group, &map);
     if (e != cudaSuccess) return e;
     const int64_t qtiles = ((s.m + TILE - 1) / TILE + 1) / 2 * 2;
     kern<<<dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st>>>(ka, map);
@@ -619,10 +692,11 @@ cudaError_t launch_list_any(const ListScan &s, cudaStream_t st) {
 
 }  // namespace
 
-// At least four ring stages beside the query tile, and the database's K-block
-// lines within the tensor map's 32-bit coordinates.
-bool list_fits(int row_bytes, int swb, int64_t n) {
-    return list_stages(row_bytes, swb) >= 4 && (n + 2 * WIDE) * (row_bytes / swb) < (int64_t(1) << 31);
+// Four K-blocks of ring beside the query tile, and the database's lines within the
+// tensor map's 32-bit coordinates.
+bool list_fits(int row_bytes, int swb, int epi, int64_t n) {
+    return list_ring(row_bytes, swb, epi).stages > 0 &&
+           (n / TILE + 2) * (row_bytes / swb) * (TILE * swb / kLine) < (int64_t(1) << 31);
 }
 
 cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches) {
