@@ -424,7 +424,7 @@ int64_t wave_splits(int64_t qctas, int64_t cap, int64_t max_s) {
 
 // How a list scan (tc_list.cu) of kk candidates for m queries runs.
 struct ListPlan {
-    int splits = 0, cap = 0, groups = 0, fine = 0, keys = 0;
+    int splits = 0, cap = 0, groups = 0, per_tile = 0, keys = 0;
     int64_t samples = 0, stride = 0;
     int64_t chunk = 0;  // queries per pass: the lists stay within 1 GiB
 };
@@ -443,8 +443,8 @@ bool list_plan(const ssg_index *idx, int64_t m, int kk, ListPlan *p) {
     if (least > n_full / 4) return false;
     p->samples = std::max<int64_t>(least, n_full / f);
     p->stride = n_full / p->samples;
-    p->fine = ssg::kListSegs * p->samples < 4 * kk;
-    p->groups = int(p->samples * (p->fine ? 8 : ssg::kListSegs));
+    p->per_tile = ssg::kListSegs * p->samples < 4 * kk ? 8 : ssg::kListSegs;
+    p->groups = int(p->samples * p->per_tile);
     const int64_t qtiles = (m + 127) / 128;
     const int64_t pairs = (qtiles + 1) / 2;
     int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(pairs, ssg::device_sm_count() / 2, n_wide);
@@ -459,6 +459,34 @@ bool list_plan(const ssg_index *idx, int64_t m, int kk, ListPlan *p) {
     const size_t per_query = size_t(ssg::kListSegs * splits) * p->cap * 8;
     p->chunk = std::max<int64_t>(256, int64_t((size_t(1) << 30) / per_query) / 256 * 256);
     p->chunk = std::min<int64_t>(p->chunk, (m + 255) / 256 * 256);
+    return true;
+}
+
+// The list scan of allknn in its locality order.  The bound comes from the
+// tiles around each query tile's own group (4,096 rows at least), a minimum
+// per four rows: a cluster has to give kk minima by itself, or the bound is
+// the distance of other clusters and many of their rows pass (100 rows a
+// cluster, 24 candidates: groups of eight let 400 rows through, the scan and
+// merge of 100,003 rows took 19.7 ms; groups of four, and compactions whose
+// bounds the splits share for the clusters that lie elsewhere, 8.2).
+bool list_plan_locality(const ssg_index *idx, int kk, ListPlan *p) {
+    const int64_t n_wide = (idx->n + 255) / 256;
+    p->samples = std::max<int64_t>(16, (kk + 7) / 8);
+    if (kk > (ssg::kListMaxCap - 64) / 2 || 4 * p->samples > n_wide) return false;
+    p->stride = 1;
+    p->per_tile = 64;
+    p->groups = int(p->samples * 64);
+    const int64_t pairs = ((idx->n + 127) / 128 + 1) / 2, cap_pairs = ssg::device_sm_count() / 2;
+    int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(pairs, cap_pairs, n_wide);
+    splits = std::max<int64_t>(1, std::min<int64_t>(splits, n_wide));
+    p->splits = int(splits);
+    p->cap = std::min(ssg::kListMaxCap, (2 * kk + 32 + ssg::kListSlack + 31) / 32 * 32);
+    p->keys = std::max(1024, 4 * kk);
+    const size_t per_query = size_t(ssg::kListSegs * splits) * p->cap * 8 + size_t(p->groups) * 4;
+    // whole waves of query tiles per pass
+    const int64_t wave = cap_pairs * 256;
+    p->chunk = std::max<int64_t>(wave, int64_t((size_t(1) << 30) / per_query) / wave * wave);
+    p->chunk = std::min<int64_t>(p->chunk, (idx->n + 255) / 256 * 256);
     return true;
 }
 
@@ -540,7 +568,7 @@ int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
     s->samples = p.samples;
     s->sample_stride = p.stride;
     s->groups = p.groups;
-    s->fine_groups = p.fine;
+    s->per_tile = p.per_tile;
     s->bound = static_cast<uint32_t *>(idx->qbound.p);
     s->lists = static_cast<uint64_t *>(idx->l_lists.p);
     s->counts = static_cast<int *>(idx->l_counts.p);
@@ -556,6 +584,7 @@ void list_finalize(const ListPlan &p, const ssg::ListScan &s, ssg::FinalizeArgs 
     f->segs = p.splits * ssg::kListSegs;
     f->list_cap = p.cap;
     f->list_keys = p.keys;
+    f->list_bound = s.bound;
     f->kk = s.kk;
 }
 
@@ -569,12 +598,15 @@ int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, const uin
     SSG_RC(list_buffers(idx, plan, &s));
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     const float *gamma = s.gamma;
+    const uint32_t *perm = s.perm;
+    const int *rot = s.rot;
     ScanTimer timer(idx);
     for (int64_t c0 = 0; c0 < m; c0 += plan.chunk) {
         const int64_t mc = std::min<int64_t>(plan.chunk, m - c0);
         s.qt = qtiles + size_t(c0 / 128) * tb;
         s.m = mc;
         s.gamma = gamma ? gamma + c0 : nullptr;
+        s.rot = rot ? rot + c0 / 128 : nullptr;
         SSG_RC(timer.begin());
         SSG_CK(ssg::launch_list_seed(s, idx->stream, &idx->last_launches), "launching the scan's seed");
         SSG_CK(ssg::launch_list_scan(s, idx->stream, &idx->last_launches), "launching the list scan");
@@ -584,12 +616,14 @@ int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, const uin
         f.m = mc;
         f.k_out = k;
         f.exclude_self = exclude_self;
+        // list rows are queries, or places of the locality order
         f.self_base = c0;
-        f.out_ids = d_ids + size_t(c0) * k;
-        f.out_dists = d_dists + size_t(c0) * k;
+        f.query_ids = perm ? perm + c0 : nullptr;
+        f.out_ids = d_ids + (perm ? 0 : size_t(c0) * k);
+        f.out_dists = d_dists + (perm ? 0 : size_t(c0) * k);
         f.n_rows = idx->n;
         f.n_total = idx->n;
-        SSG_CK(finish(c0, f), "launching the merge kernel");
+        SSG_CK(finish(perm ? 0 : c0, f), "launching the merge kernel");
         SSG_RC(timer.collect());
     }
     return SSG_OK;
@@ -1052,16 +1086,25 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     }
     int *flags = static_cast<int *>(idx->flags.p);
     int *flag_count = flags + m;
-    // a batch of queries (allknn scans its locality order, below): the list scan
+    // the list scan; allknn of a large collection in its locality order
     ListPlan lp;
     const bool locality = queries_are_db && idx->locality_param && m == idx->n && idx->n >= kLocalityMinRows;
-    if (!locality && !idx->pair_param && ssg::list_fits(2 * k3, 64, list_epilogue(idx->metric), idx->n) && list_plan(idx, m, plan.rr, &lp)) {
+    if (!idx->pair_param && ssg::list_fits(2 * k3, 64, list_epilogue(idx->metric), idx->n) &&
+        (locality ? list_plan_locality(idx, plan.rr, &lp) : list_plan(idx, m, plan.rr, &lp))) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->ps_db.p);
+        s.alpha = static_cast<const float *>(idx->ps_norm.p);
+        if (locality) {
+            SSG_RC(ensure_plain_locality(idx));
+            qtiles = static_cast<const uint8_t *>(idx->loc_ps_dbq.p);
+            s.dt = static_cast<const uint8_t *>(idx->loc_ps_db.p);
+            s.alpha = static_cast<const float *>(idx->loc_ps_norm.p);
+            s.perm = static_cast<const uint32_t *>(idx->loc_perm.p);
+            s.rot = static_cast<const int *>(idx->loc_rot.p);
+        }
         s.row_bytes = 2 * k3;
         s.swb = 64;
         s.epi = list_epilogue(idx->metric);
-        s.alpha = static_cast<const float *>(idx->ps_norm.p);
         s.n = idx->n;
         s.kk = plan.rr;
         SSG_RC(list_search(idx, s, lp, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
@@ -1573,15 +1616,26 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
     int qt = 0, stages = 0;
     bool long_lists = false;
     idx->last_fallbacks = 0;
-    // a batch of queries (allknn scans its locality order, below) takes the
-    // list scan: the same kk candidates without heaps to fill in every split
+    // the list scan: the same kk candidates without heaps to fill in every
+    // split; allknn of a large collection in its locality order
     ListPlan plan;
-    if (!(queries_are_db && idx->locality_param && !idx->capturing && idx->n >= kLocalityMinRows) &&
-        idx->wide_param && !idx->pair_param && idx->long_param && ssg::list_fits(2 * kp, 64, list_epilogue(idx->metric), idx->n) &&
-        list_plan(idx, m, kk, &plan)) {
+    const bool locality = queries_are_db && idx->locality_param && !idx->capturing && m == idx->n &&
+                          idx->n >= kLocalityMinRows;
+    if (idx->wide_param && !idx->pair_param && idx->long_param &&
+        ssg::list_fits(2 * kp, 64, list_epilogue(idx->metric), idx->n) &&
+        (locality ? list_plan_locality(idx, kk, &plan) : list_plan(idx, m, kk, &plan))) {
         const size_t tb = ssg::tc_tile_bytes(idx->dim);
         const uint8_t *qtiles = static_cast<const uint8_t *>(idx->tc_db.p);
-        if (!queries_are_db) {
+        ssg::ListScan s{};
+        s.dt = qtiles;
+        s.alpha = static_cast<const float *>(idx->tc_norm.p);
+        if (locality) {
+            SSG_RC(ensure_locality(idx));
+            qtiles = s.dt = static_cast<const uint8_t *>(idx->loc_tiles.p);
+            s.alpha = static_cast<const float *>(idx->loc_norm.p);
+            s.perm = static_cast<const uint32_t *>(idx->loc_perm.p);
+            s.rot = static_cast<const int *>(idx->loc_rot.p);
+        } else if (!queries_are_db) {
             const int64_t qt_alloc = ((m + 127) / 128 + 1) / 2 * 2;
             SSG_CK(idx->tc_q.ensure(size_t(qt_alloc) * tb), "allocating BF16 query tiles");
             SSG_CK(ssg::launch_bf16_tiles(static_cast<const float *>(dq), m, idx->dim, qt_alloc,
@@ -1589,12 +1643,9 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
                    "building BF16 query tiles");
             qtiles = static_cast<const uint8_t *>(idx->tc_q.p);
         }
-        ssg::ListScan s{};
-        s.dt = static_cast<const uint8_t *>(idx->tc_db.p);
         s.row_bytes = 2 * kp;
         s.swb = 64;
         s.epi = list_epilogue(idx->metric);
-        s.alpha = static_cast<const float *>(idx->tc_norm.p);
         s.n = idx->n;
         s.kk = kk;
         SSG_RC(list_search(idx, s, plan, qtiles, tb, m, k, exclude_self, d_ids, d_dists,

@@ -81,7 +81,13 @@ struct FinalizeArgs {
     // unsorted keys at cand[(j * segs + s) * list_cap]; kk of them are wanted
     // and together the lists hold the query's kk smallest keys
     const int *counts = nullptr;
+    // the database object that list row j's query is (locality order): its
+    // query row, its own id and its output row; null: j
+    const uint32_t *query_ids = nullptr;
     int list_cap = 0;
+    // the queries' bounds after the scan (ordered distances): keys beyond them
+    // are left out
+    const uint32_t *list_bound = nullptr;
     int list_keys = 0;  // keys per query kept on chip while selecting (more take extra passes)
 };
 cudaError_t launch_finalize(const FinalizeArgs &a, cudaStream_t st, int *launches);
@@ -224,10 +230,16 @@ struct ListScan {
     uint32_t *bound;          // per query (ordered distance; all ones: none), written by the seed
     uint64_t *lists;
     int *counts;
-    // the seed: `samples` wide tiles (256 rows), every sample_stride-th of the
-    // database, all of whole rows; groups = 2 (or 8, fine_groups) minima each
+    // locality order (allknn over a reordered database): the row at position
+    // p of both tile sets has id perm[p]; query tile x (rot's index: x of the
+    // first tile of this scan on) starts at database tile rot[x] and wraps
+    const uint32_t *perm;
+    const int *rot;
+    // the seed: `samples` wide tiles (256 rows) with per_tile = 2, 8 or 64
+    // minima each (groups in all): every sample_stride-th of the database, all
+    // of whole rows, or in a locality order those around rot
     int64_t samples, sample_stride;
-    int groups, fine_groups;
+    int groups, per_tile;
     float *minima;            // m * groups
     int *err;
 };

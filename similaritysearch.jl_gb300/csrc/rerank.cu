@@ -251,7 +251,12 @@ __device__ __forceinline__ void write_row(const FinalizeArgs &f, int64_t j, cons
 }
 
 __device__ __forceinline__ uint32_t self_id(const FinalizeArgs &f, int64_t j) {
-    return uint32_t(f.self_ids ? f.self_ids[j] : j + f.self_base);
+    return f.query_ids ? f.query_ids[j] : uint32_t(f.self_ids ? f.self_ids[j] : j + f.self_base);
+}
+
+// Where query j's row, flag and results are.
+__device__ __forceinline__ int64_t query_row(const FinalizeArgs &f, int64_t j) {
+    return f.query_ids ? int64_t(f.query_ids[j]) : j;
 }
 
 __device__ __forceinline__ uint64_t warp_min64(uint64_t v) {
@@ -287,20 +292,77 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
     const bool live = j < f.m;
     uint64_t *sel = s_sel[warp], *out = s_key[warp];
     if (live) {
-        const int total = f.segs * f.kk;
+        const int64_t jr = query_row(f, j);
+        int total = f.segs * f.kk;
         const uint64_t *src = f.cand + size_t(j) * total;
+        const int *cn = nullptr;
+        if (f.counts) {
+            cn = f.counts + size_t(j) * f.segs;
+            src = f.cand + size_t(j) * f.segs * f.list_cap;
+            total = 0;
+            for (int s = 0; s < f.segs; ++s) total += cn[s];
+        }
+        const uint32_t bound = cn ? f.list_bound[j] : 0xffffffffu;
+        // the query's at-th key, at < total: of its segments, or of its few
+        // lists in turn (empty beyond the bound)
+        auto key_at = [&](int at) {
+            if (!cn) return src[at];
+            int s = 0;
+            for (int c = cn[0]; at >= c; c = cn[s]) { at -= c; ++s; }
+            const uint64_t k = src[size_t(s) * f.list_cap + at];
+            return uint32_t(k >> 32) <= bound ? k : KEY_EMPTY;
+        };
+        // more keys than the registers hold (lists only): those within the
+        // bound gather in the ring's memory, and if they are still too many, a
+        // limit with exactly `need` keys below it is found by counting
         uint64_t key[kWarpKeys];
+        const uint64_t *held = nullptr;
+        if (total > 32 * kWarpKeys) {
+            const int room = RERANK ? kWarpStages * (need + 1) * kRowStride / 2 : 0;
+            uint64_t *scratch = reinterpret_cast<uint64_t *>(smem) + size_t(warp) * room;
+            auto gather = [&](uint64_t below, uint64_t *to, int most) {
+                int base = 0;
+                for (int i0 = 0; i0 < total; i0 += 32) {
+                    const uint64_t k = i0 + lane < total ? key_at(i0 + lane) : KEY_EMPTY;
+                    const uint32_t vote = __ballot_sync(0xffffffffu, k < below);
+                    const int at = base + __popc(vote & ((1u << lane) - 1u));
+                    if (k < below && at < most) to[at] = k;
+                    base += __popc(vote);
+                }
+                __syncwarp();
+                return base;
+            };
+            int have = RERANK ? gather(KEY_EMPTY, scratch, room) : INT_MAX;
+            held = scratch;
+            if (have > 32 * kWarpKeys) {
+                uint64_t p = 0, lim = KEY_EMPTY;
+                const bool on_chip = have <= room;
+                const int all = on_chip ? have : total;
+                for (int b = 63; b >= 0; --b) {
+                    const uint64_t t = p | (1ull << b);
+                    int c = 0;
+                    for (int at = lane; at < all; at += 32) c += (on_chip ? scratch[at] : key_at(at)) < t;
+                    c = __reduce_add_sync(0xffffffffu, c);
+                    if (c == need) { lim = t; break; }
+                    if (c < need) p = t;
+                }
+                have = min(need, gather(lim == KEY_EMPTY ? p + 1 : lim, sel, need));
+                held = sel;
+            }
+            total = have;
+        }
         int cnt = 0;
 #pragma unroll
         for (int i = 0; i < kWarpKeys; ++i) {
             const int at = i * 32 + lane;
-            key[i] = at < total ? src[at] : KEY_EMPTY;
+            key[i] = at >= total ? KEY_EMPTY : held ? held[at] : key_at(at);
             if (RERANK && int64_t(key_id0(key[i])) >= f.n_rows) key[i] = KEY_EMPTY;
             cnt += key[i] != KEY_EMPTY;
         }
         const int nvt = __reduce_add_sync(0xffffffffu, cnt);
+        __syncwarp();
         uint64_t low = KEY_EMPTY;
-        if (RERANK && f.check) {
+        if (RERANK && f.check && !cn) {
             for (int s = lane; s < f.segs; s += 32) low = min(low, src[size_t(s) * f.kk + f.kk - 1]);
             low = warp_min64(low);
         }
@@ -353,7 +415,7 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
             // that row sums |q|^2 for the certificate
             const int rows_s = need + 1;
             float *ring = reinterpret_cast<float *>(smem) + size_t(warp) * kWarpStages * rows_s * kRowStride;
-            const RowSource rs{db, q + size_t(j) * dim, int(dim), vec != 0};
+            const RowSource rs{db, q + size_t(jr) * dim, int(dim), vec != 0};
             const int steps = (int(dim) + kDimStep - 1) / kDimStep;
             float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
             const float s0 = lane == nv ? 0.0f : 1.0f, s1 = lane + 32 == nv ? 0.0f : 1.0f;
@@ -377,7 +439,7 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
                 if (lane + 32 <= nv) a1 = chain_step<METRIC>(a1, buf + (lane + 32) * kRowStride, qr, dims, s1);
                 if (nv == 64 && lane == 0) a2 = chain_step<METRIC>(a2, qr, qr, dims, 0.0f);
             }
-            const float qn = METRIC == COSINE ? q_norm[j] : 0.0f;
+            const float qn = METRIC == COSINE ? q_norm[jr] : 0.0f;
             if (k0 != KEY_EMPTY) k0 = make_key(chain_distance<METRIC>(a0, key_id0(k0), db_norm, qn), key_id0(k0));
             if (k1 != KEY_EMPTY) k1 = make_key(chain_distance<METRIC>(a1, key_id0(k1), db_norm, qn), key_id0(k1));
             if (lane == nv) s_qsq[warp] = a0;
@@ -407,7 +469,7 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
                 if (key_id0(out[i]) == id) self_pos = i;
             self_pos = __reduce_min_sync(0xffffffffu, self_pos);
         }
-        write_row(f, j, out, nv, self_pos, lane, 32);
+        write_row(f, jr, out, nv, self_pos, lane, 32);
         if (RERANK && f.check && lane == 0) {
             const int take = f.k_out + (f.exclude_self ? 1 : 0);
             s_low[warp] = low;
@@ -423,7 +485,7 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
             const int nv = s_nv[threadIdx.x];
             if (int64_t(nv) < f.n_total &&
                 !list_complete<METRIC>(f, dim, nv, s_low[threadIdx.x], s_qsq[threadIdx.x], s_take[threadIdx.x])) {
-                f.flags[jq] = 1;
+                f.flags[query_row(f, jq)] = 1;
                 atomicAdd(f.flag_count, 1);
             }
         }
@@ -448,7 +510,7 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
     __shared__ unsigned long long s_min, s_max, s_low, s_last;
     __shared__ float s_qsq;
     const int tid = threadIdx.x, lane = tid % 32;
-    const int64_t j = blockIdx.x;
+    const int64_t j = blockIdx.x, jr = query_row(f, j);
     const int total = f.segs * f.kk;
     const uint64_t *src = f.cand + size_t(j) * total;
     if (tid == 0) {
@@ -480,13 +542,17 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
         const int *cn = f.counts + size_t(j) * f.segs;
         const uint64_t *lists = f.cand + size_t(j) * f.segs * f.list_cap;
         const int sub = lane % 8;
+        const uint32_t bound = f.list_bound[j];
         auto each_key = [&](auto &&body) {
             for (int s0 = (tid / 32) * 4; s0 < f.segs; s0 += kBlockThreads / 8) {
                 const int sg = s0 + lane / 8;
                 const int c = sg < f.segs ? cn[sg] : 0;
                 const uint64_t *l = lists + size_t(sg) * f.list_cap;
                 const int most = __reduce_max_sync(0xffffffffu, c);
-                for (int i = sub; i < most + sub; i += 8) body(i < c ? l[i] : KEY_EMPTY);
+                for (int i = sub; i < most + sub; i += 8) {
+                    const uint64_t k = i < c ? l[i] : KEY_EMPTY;
+                    body(uint32_t(k >> 32) <= bound ? k : KEY_EMPTY);
+                }
             }
         };
         int sum = 0;
@@ -590,9 +656,9 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
             __syncthreads();
             if (tid == 0 && s_last < s_low) s_low = s_last;
         }
-        const RowSource rs{db, q + size_t(j) * dim, int(dim), vec != 0};
+        const RowSource rs{db, q + size_t(jr) * dim, int(dim), vec != 0};
         const int steps = (int(dim) + kDimStep - 1) / kDimStep;
-        const float qn = METRIC == COSINE ? q_norm[j] : 0.0f;
+        const float qn = METRIC == COSINE ? q_norm[jr] : 0.0f;
         const int rows_s = min(need, kBlockRows) + 1;
         for (int r0 = 0; r0 < nv || r0 == 0; r0 += kBlockRows) {
             const int rows = min(kBlockRows, nv - r0);
@@ -651,11 +717,11 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
             if (key_id0(out[i]) == id) atomicMin(&s_self, i);
         __syncthreads();
     }
-    write_row(f, j, out, nv, s_self, tid, kBlockThreads);
+    write_row(f, jr, out, nv, s_self, tid, kBlockThreads);
     if (RERANK && f.check && tid == 0 && int64_t(nv) < f.n_total) {
         const int take = f.k_out + (f.exclude_self ? 1 : 0);
         if (!list_complete<METRIC>(f, dim, nv, s_low, s_qsq, nv >= take ? key_dist(out[take - 1]) : 0.0f)) {
-            f.flags[j] = 1;
+            f.flags[jr] = 1;
             atomicAdd(f.flag_count, 1);
         }
     }
@@ -668,7 +734,8 @@ cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const floa
     const int total = f.counts ? std::max(f.list_keys, 2 * need) : f.segs * f.kk;
     const bool vec = RERANK && dim % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(db) | reinterpret_cast<uintptr_t>(q)) & 15) == 0;
-    if (!f.counts && total <= 32 * kWarpKeys && need <= kWarpOut) {
+    // (the lists of a locality order's few splits hold little more than need)
+    if ((f.counts ? f.query_ids && f.segs <= 8 : total <= 32 * kWarpKeys) && need <= kWarpOut) {
         const size_t smem = RERANK ? size_t(kWarpsPerBlock) * kWarpStages * (need + 1) * kRowStride * 4 : 0;
         auto kern = finalize_warp_kernel<METRIC, RERANK>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));

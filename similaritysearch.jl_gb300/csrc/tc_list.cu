@@ -70,16 +70,18 @@ struct KernelArgs {
     int group;          // K-blocks per ring stage (a divisor of kblocks)
     int stages;         // ring depth
     int64_t n_wide;     // wide tiles of this pass (the sample's in SEED)
+    int64_t all_wide;   // of the database
 };
 
 // Keeps the kk smallest of each full list (more than `room` entries): the
 // warp takes its lanes' full lists in turn, holds one in registers, finds the
 // kk-th key bit by bit and writes the kept keys back.  Returns the calling
-// lane's new count and sets *top to its largest kept key.  Rare: a bound
-// seeded from the sample leaves the lists far from full unless most of a
-// query's neighbours lie in one split.
+// lane's new count and sets *top to its largest kept key.  Lists hold up to
+// 32 * PER entries.  Rare: a bound seeded from the sample leaves the lists far
+// from full unless most of a query's neighbours lie in one split, or its
+// cluster lies elsewhere in a locality order.
+template <int PER>
 __device__ __noinline__ int compact_lists(uint64_t *list, int nb, int room, int kk, uint64_t *top) {
-    constexpr int PER = kListMaxCap / 32;
     const int lane = threadIdx.x % 32;
     uint32_t todo = __ballot_sync(0xffffffffu, nb > room);
     while (todo) {
@@ -147,30 +149,40 @@ __device__ __forceinline__ float rank_distance(float x, float bits) {
     return EPI == EPI_DOT ? -x : EPI == EPI_HAM ? (bits - x) * 0.5f : x;
 }
 
+// How a scan orders the database: evenly, as stored; or in a locality order
+// (positions with ids, each query tile from its own group on), in one split or
+// in several that share what their compactions find.  (Compiled apart: the
+// locality order's state cost the batch scans 4 to 12 %, the sharing C2's 5.)
+enum { STORED = 0, LOCAL = 1, LOCAL_SHARED = 2 };
+
 // Moves the c raw candidates buffered at shared address buf (slots kBufStride
-// apart: ranking value, id) to the lane's list, as keys.  All 32 lanes call it,
-// with scalars alone and few registers of its own, so the call saves nothing.
-template <int EPI>
-__device__ __noinline__ int drain_raw(uint64_t *list, uint32_t buf, int c, int nb, float bits) {
+// apart: ranking value, position) to the lane's list, as keys; those beyond
+// the largest key a compaction kept are left out.  All 32 lanes call it, with
+// scalars alone and few registers of its own, so the call saves nothing.
+template <int EPI, int ORDER>
+__device__ __noinline__ int drain_raw(uint64_t *list, uint32_t buf, int c, int nb, float bits, uint64_t top,
+                                      const uint32_t *perm) {
     const int cmax = __reduce_max_sync(0xffffffffu, c);
     for (int i = 0; i < cmax; ++i) {
         if (i < c) {
             float v;
-            uint32_t id;
-            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=f"(v), "=r"(id) : "r"(buf + i * kBufStride) : "memory");
-            list[nb] = make_key(rank_distance<EPI>(v, bits), id);
-            ++nb;
+            uint32_t pos;
+            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=f"(v), "=r"(pos) : "r"(buf + i * kBufStride) : "memory");
+            const uint64_t key = make_key(rank_distance<EPI>(v, bits), ORDER != STORED ? perm[pos] : pos);
+            if (ORDER == STORED || key <= top) list[nb++] = key;
         }
     }
     return nb;
 }
 
 // One query row's candidates (one lane).
-template <int EPI>
+template <int EPI, int ORDER>
 struct RowList {
     uint64_t *list;
     uint32_t buf;      // shared address of this lane's raw buffer
     int nb, nbuf, cap, kk;
+    uint64_t top;      // the largest key kept by the last compaction
+    const uint32_t *perm;
     int64_t n;
     bool valid;
     float lim_v;       // a candidate's ranking value: product >= lim_v (raw_rank) or distance <= lim_v
@@ -219,36 +231,58 @@ struct RowList {
     __device__ __forceinline__ static float best(float a, float b) { return raw_rank(EPI) ? fmaxf(a, b) : fminf(a, b); }
     __device__ __forceinline__ bool passes(float x) const { return raw_rank(EPI) ? x >= lim_v : x <= lim_v; }
 
-    // the smallest distance among the chunk's columns (all of them rows)
-    __device__ __forceinline__ float chunk_min(const uint32_t (&r)[32], const float4 *al, const float4 *be) const {
+    // the smallest distance of each four columns of a chunk; +inf where they
+    // are no rows
+    __device__ __forceinline__ void chunk_min(const uint32_t (&r)[32], int64_t id0, const float4 *al, const float4 *be,
+                                              float (&g)[8]) const {
         float dv[32];
         values(r, al, be, dv);
-        const float b = best(best(best8(dv), best8(dv + 8)), best(best8(dv + 16), best8(dv + 24)));
-        return fminf(rank_distance<EPI>(b, bits), INFINITY);  // NaN products: +inf
+        const bool rows = id0 + 32 <= n;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float *v = dv + 4 * i;
+            const float b = raw_rank(EPI) ? fmaxf(fmax3(v[0], v[1], v[2]), v[3]) : fminf(fmin3(v[0], v[1], v[2]), v[3]);
+            g[i] = rows ? fminf(rank_distance<EPI>(b, bits), INFINITY) : INFINITY;  // (a NaN: +inf)
+        }
     }
     __device__ __forceinline__ void drain() {
-        nb = drain_raw<EPI>(list, buf, nbuf, nb, bits);
+        nb = drain_raw<EPI, ORDER>(list, buf, nbuf, nb, bits, ORDER != STORED ? top : KEY_EMPTY, ORDER != STORED ? perm : nullptr);
         nbuf = 0;
     }
     // Between tiles (nothing of an accumulator in registers): makes room for
     // another tile's columns in every list of the warp.
-    __device__ __forceinline__ void make_room() {
+    __device__ __forceinline__ bool make_room() {
         const int room = cap - kTileColumns - kBufCap;
-        if (!__any_sync(0xffffffffu, nb > room)) return;
+        if (!__any_sync(0xffffffffu, nb > room)) return false;
         drain();
-        uint64_t top = 0;
         const bool full = nb > room;
-        nb = compact_lists(list, nb, room, kk, &top);
+        uint64_t t = 0;
+        nb = cap <= 256 ? compact_lists<8>(list, nb, room, kk, &t) : compact_lists<kListMaxCap / 32>(list, nb, room, kk, &t);
         if (full) {
-            // kk keys up to `top` are kept and ids only grow from here: an
-            // equal distance no longer counts
-            const float d = key_dist(top);
-            if (EPI == EPI_HAM) lim_v = fmaxf(lim_v, bits - 2.0f * d + 1.0f);
-            else {
-                const float below = ordered_to_float(float_to_ordered(d) - 1u);
-                lim_v = EPI == EPI_DOT ? fmaxf(lim_v, -below) : fminf(lim_v, below);
-            }
+            // kk keys up to t are kept.  Ids only grow from here where rows come
+            // as stored: an equal distance no longer counts.  Positions of a
+            // locality order have any ids: the drain compares the keys.
+            if (ORDER != STORED) top = t;
+            const float d = key_dist(t);
+            const float e = ORDER != STORED ? d : EPI == EPI_HAM ? d - 0.5f : ordered_to_float(float_to_ordered(d) - 1u);
+            const float v = EPI == EPI_HAM ? bits - 2.0f * e : EPI == EPI_DOT ? -e : e;
+            lim_v = raw_rank(EPI) ? fmaxf(lim_v, v) : fminf(lim_v, v);
         }
+        return true;
+    }
+    // The limit as a bound on the distance, and back: what a compaction found
+    // holds for every list of the query.
+    __device__ __forceinline__ float limit() const {
+        return EPI == EPI_HAM ? (bits - lim_v) * 0.5f : EPI == EPI_DOT ? -lim_v : lim_v;
+    }
+    __device__ __forceinline__ void publish(uint32_t *bound) const {
+        if (valid && top != KEY_EMPTY) bound_lower(bound, limit());
+    }
+    __device__ __forceinline__ void refresh(const uint32_t *bound) {
+        if (!valid) return;
+        const float t = bound_read(bound);
+        const float v = EPI == EPI_HAM ? bits - 2.0f * t : EPI == EPI_DOT ? -t : t;
+        lim_v = raw_rank(EPI) ? fmaxf(lim_v, v) : fminf(lim_v, v);
     }
     // Candidates of a chunk: a vote on the chunk and on each group of 8
     // columns, then branch-free raw appends (the slot is always written, the
@@ -279,7 +313,7 @@ struct RowList {
     }
 };
 
-template <int SWB, bool F8, int EPI, bool SEED>
+template <int SWB, bool F8, int EPI, bool SEED, int ORDER>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     tc_list_kernel(KernelArgs ka, const __grid_constant__ CUtensorMap dmap) {
     constexpr int KBLK = TILE * SWB;   // bytes of a K-block of a tile
@@ -342,7 +376,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int64_t w_lo = int64_t(blockIdx.y) * split_w;
     const int64_t w_hi = w_lo + split_w < ka.n_wide ? w_lo + split_w : ka.n_wide;
     const int W = w_hi > w_lo ? int(w_hi - w_lo) : 0;
-    auto wide_tile = [&](int u) { return SEED ? (w_lo + u) * a.sample_stride : w_lo + u; };
+    // the u-th wide tile: of the whole scan, from the locality rotation on; in
+    // SEED of the evenly spaced sample, or of the tiles around the rotation
+    int64_t first = ORDER != STORED ? int64_t(a.rot[qpair]) / 2 : 0;
+    if (SEED && ORDER != STORED) first = first >= a.samples / 2 ? first - a.samples / 2 : first - a.samples / 2 + ka.all_wide;
+    auto wide_tile = [&](int u) {
+        if (ORDER == STORED) return SEED ? (w_lo + u) * a.sample_stride : w_lo + u;
+        const int64_t p = w_lo + u + first;
+        return p >= ka.all_wide ? p - ka.all_wide : p;
+    };
 
     if (warp == 0) {
         if (lane == 0) {
@@ -428,7 +470,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         const int64_t query = qx * TILE + quarter * 32 + lane;
         const uint32_t release0 = tc::mapa_shared(tc::smem_u32(acc_empty), 0);
         const int seg = int(blockIdx.y) * CS + cs, segs = a.splits * CS;
-        RowList<EPI> T;
+        RowList<EPI, ORDER> T;
         T.valid = query < a.m;
         T.list = SEED ? nullptr : a.lists + (size_t(T.valid ? query : 0) * segs + seg) * a.cap;
         T.nb = 0;
@@ -437,6 +479,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         T.cap = a.cap;
         T.kk = a.kk;
         T.n = a.n;
+        T.top = KEY_EMPTY;
+        T.perm = a.perm;
         T.bits = a.bits;
         T.gamma = (EPI == EPI_AFF && a.gamma && T.valid) ? a.gamma[query] : 1.0f;
         T.set((!SEED && T.valid) ? bound_read(a.bound + query) : INFINITY);
@@ -501,17 +545,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int c = 0; c < LDC; ++c) {
                     const int ch = round * LDC + c;
-                    if constexpr (SEED) gm[ch] = T.chunk_min(r[c], al + ch * 8, al + CH * 8 + ch * 8);
-                    else T.chunk(r[c], row0 + ch * CS * 32, al + ch * 8, al + CH * 8 + ch * 8);
+                    if constexpr (SEED) {
+                        float g[8];
+                        T.chunk_min(r[c], row0 + ch * CS * 32, al + ch * 8, al + CH * 8 + ch * 8, g);
+                        if (ORDER != STORED && T.valid) {
+                            float4 *to = reinterpret_cast<float4 *>(a.minima + size_t(query) * a.groups + (w_lo + u) * 64 +
+                                                                    (cs * CH + ch) * 8);
+                            to[0] = make_float4(g[0], g[1], g[2], g[3]);
+                            to[1] = make_float4(g[4], g[5], g[6], g[7]);
+                        }
+                        gm[ch] = fmin8(g);
+                    } else T.chunk(r[c], row0 + ch * CS * 32, al + ch * 8, al + CH * 8 + ch * 8);
                 }
             }
             if (++b == NACC) { b = 0; ph ^= 1; }
-            if constexpr (SEED) {
+            if constexpr (SEED && ORDER == STORED) {
                 if (T.valid) {
                     float *g = a.minima + size_t(query) * a.groups;
                     const int64_t at = w_lo + u;
-                    if (a.fine_groups) {
-                        // (groups of a wide tile: 8, or one per epilogue warp of a quarter)
+                    if (a.per_tile == 8) {
 #pragma unroll
                         for (int ch = 0; ch < CH; ++ch) g[at * 8 + cs * CH + ch] = gm[ch];
                     } else {
@@ -522,7 +574,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     }
                 }
             }
-            if constexpr (!SEED) T.make_room();
+            if constexpr (!SEED) {
+                const bool tighter = T.make_room();
+                if (ORDER == LOCAL_SHARED) {
+                    if (tighter) T.publish(a.bound + query);
+                    else if ((u & 15) == 15) T.refresh(a.bound + query);
+                }
+            }
             if constexpr (!raw_rank(EPI)) __syncwarp();  // the buffer is refilled a tile later
         }
         if (!raw_rank(EPI)) asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -557,16 +615,26 @@ __global__ void __launch_bounds__(128) seed_bound_kernel(const float *__restrict
         for (int i = 0; i < NV; ++i)
             if (at + i * 32 < groups) f[i] = fminf(f[i], g[at + i * 32]);
     }
-    uint32_t v[NV];
+    uint32_t v[NV], lo = 0xffffffffu, hi = 0;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) v[i] = float_to_ordered(f[i]);
-    uint32_t p = 0;
-    for (int b = 31; b >= 0; --b) {
+    for (int i = 0; i < NV; ++i) {
+        v[i] = float_to_ordered(f[i]);
+        lo = min(lo, v[i]);
+        hi = max(hi, v[i]);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    // the bits above the highest one in which two minima differ are common;
+    // with exactly kk minima below t any value from the kk-th to t - 1 will do
+    const int top = 31 - __clz((lo ^ hi) | 1u);
+    uint32_t p = top >= 31 ? 0u : (lo >> (top + 1)) << (top + 1);
+    for (int b = top; b >= 0; --b) {
         const uint32_t t = p | (1u << b);
         int c = 0;
 #pragma unroll
         for (int i = 0; i < NV; ++i) c += v[i] < t;
         c = __reduce_add_sync(0xffffffffu, c);
+        if (c == kk) { p = t - 1; break; }
         if (c < kk) p = t;
     }
     if (lane == 0) bound[q] = kk <= groups ? p : 0xffffffffu;
@@ -651,7 +719,7 @@ Ring list_ring(int row_bytes, int swb, int epi) {
     return {1, 0};
 }
 
-template <int SWB, bool F8, int EPI, bool SEED>
+template <int SWB, bool F8, int EPI, bool SEED, int ORDER = STORED>
 cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
     KernelArgs ka;
     ka.s = s;
@@ -660,10 +728,11 @@ cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
     if (ring.stages == 0) return cudaErrorInvalidValue;
     ka.group = ring.group;
     ka.stages = ring.stages;
-    ka.n_wide = SEED ? s.samples : (s.n + WIDE - 1) / WIDE;
+    ka.all_wide = (s.n + WIDE - 1) / WIDE;
+    ka.n_wide = SEED ? s.samples : ka.all_wide;
     size_t smem = list_smem(s.row_bytes, ring.group * TILE * SWB, ring.stages, EPI);
     if (smem < kAloneSmem) smem = kAloneSmem;
-    auto kern = tc_list_kernel<SWB, F8, EPI, SEED>;
+    auto kern = tc_list_kernel<SWB, F8, EPI, SEED, ORDER>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     CUtensorMap map;
@@ -672,6 +741,14 @@ cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
     const int64_t qtiles = ((s.m + TILE - 1) / TILE + 1) / 2 * 2;
     kern<<<dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st>>>(ka, map);
     return cudaGetLastError();
+}
+
+// BF16 tiles with 64-byte K-blocks, the form that allknn orders.
+template <int EPI, bool SEED>
+cudaError_t launch_list_order(const ListScan &s, cudaStream_t st) {
+    if (!s.perm) return launch_list_t<64, false, EPI, SEED>(s, st);
+    if (SEED || s.splits == 1) return launch_list_t<64, false, EPI, SEED, LOCAL>(s, st);
+    return launch_list_t<64, false, EPI, SEED, LOCAL_SHARED>(s, st);
 }
 
 template <bool SEED>
@@ -683,9 +760,9 @@ cudaError_t launch_list_any(const ListScan &s, cudaStream_t st) {
     }
     if (s.swb == 128) return s.epi == LIST_AFFINE ? launch_list_t<128, false, EPI_AFF, SEED>(s, st) : cudaErrorInvalidValue;
     switch (s.epi) {
-        case LIST_DOT: return launch_list_t<64, false, EPI_DOT, SEED>(s, st);
-        case LIST_SQ: return launch_list_t<64, false, EPI_SQ, SEED>(s, st);
-        case LIST_COS: return launch_list_t<64, false, EPI_COS, SEED>(s, st);
+        case LIST_DOT: return launch_list_order<EPI_DOT, SEED>(s, st);
+        case LIST_SQ: return launch_list_order<EPI_SQ, SEED>(s, st);
+        case LIST_COS: return launch_list_order<EPI_COS, SEED>(s, st);
         default: return cudaErrorInvalidValue;
     }
 }
@@ -705,7 +782,8 @@ cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches) 
     // about four groups per candidate keep the bound within a fifth of the
     // sample's own kk-th distance in rank
     const unsigned blocks = unsigned((s.m + 3) / 4);
-    if (s.kk <= 64) seed_bound_kernel<8><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
+    if (s.perm) seed_bound_kernel<32><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
+    else if (s.kk <= 64) seed_bound_kernel<8><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
     else if (s.kk <= 160) seed_bound_kernel<20><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
     else seed_bound_kernel<60><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
     if (launches) *launches += 2;

@@ -91,3 +91,33 @@ def test_reduced_keys_do_not_depend_on_splits(ss, prec, dim, m, splits):
                                      splits=s)
         got.append(ss.searchbatch(idx, ss.GenericContext(), ss.MatrixDatabase.from_rows(Q), 20))
     assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("metric,dim,k,splits", [("sql2", 24, 10, 0), ("normcosine", 96, 32, 1), ("cosine", 40, 5, 3)])
+@pytest.mark.parametrize("n,per", [(33_000, 40), (40_961, 700)])
+def test_allknn_locality(ss, metric, dim, k, splits, n, per):
+    """allknn in the locality order (clusters smaller and larger than a pivot's
+    group, so bounds from the neighbourhood miss or hit) equals the oracle on
+    sampled rows and the stored order on all, for the plain method; with
+    over-fetched BF16 candidates both orders give the same arrays."""
+    rng = np.random.default_rng(n + dim)
+    C = rng.standard_normal((n // per, dim), dtype=np.float32)
+    X = C[rng.integers(0, C.shape[0], size=n)] + 0.2 * rng.standard_normal((n, dim), dtype=np.float32)
+    X[500:540] = X[3]  # equal rows
+    if metric == "normcosine":
+        X /= np.linalg.norm(X, axis=1, keepdims=True)
+    dist = {"sql2": ss.Dist.SqL2, "cosine": ss.Dist.Cosine, "normcosine": ss.Dist.NormCosine}[metric]()
+    ctx = ss.GenericContext()
+    idx = ss.GPUExhaustiveSearch(dist, ss.MatrixDatabase.from_rows(X), splits=splits)
+    ids, dists = ss.allknn(idx, ctx, k)
+    rows = np.concatenate([np.arange(490, 545), rng.integers(0, n, size=100)])
+    ri, rd = O.searchbatch(metric, X, X[rows], k)
+    assert np.array_equal(ids.T[rows], ri) and np.array_equal(dists.T[rows], rd)
+    idx.set_param("locality", 0)
+    i2, d2 = ss.allknn(idx, ctx, k)
+    assert np.array_equal(ids, i2) and np.array_equal(dists, d2)
+    idx = ss.GPUExhaustiveSearch(dist, ss.MatrixDatabase.from_rows(X), precision="bf16", overfetch=1.5, splits=splits)
+    a = ss.allknn(idx, ctx, k, exclude_self=True)
+    idx.set_param("locality", 0)
+    b = ss.allknn(idx, ctx, k, exclude_self=True)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
