@@ -110,6 +110,14 @@ struct ssg_index {
     // BF16 threshold-filter path (candidate counts beyond the on-chip heaps):
     // tiles of every smp_r-th database row, filtered lists, counts, bounds
     DevBuf tc_smp, tc_smp_norm, f_out, f_cnt, f_thr, gbound;
+    // pinned host staging: two result words, then the queries and the results of
+    // a host call of up to kPinBytes (pageable copies wait on the host for
+    // every transfer, ~13 us each)
+    void *pin = nullptr, *pin_io = nullptr;
+    size_t io_cap = 0;
+    const void *out_dev = nullptr;  // results to bring along with the status word
+    size_t out_bytes = 0;
+    bool out_done = false;          // they are in the staging
     DevBuf pack_q, pack_out;  // ssg_search_batches staging
     DevBuf qbound;            // per-query bounds shared by a query's split heaps (ScanArgs::qbound)
     // plain GEMM-form scan: k-major tiles of the database (built for gm_rows
@@ -197,6 +205,58 @@ int cuda_fail(ssg_index *idx, cudaError_t e, const char *what) {
         cudaError_t _e = (call);                            \
         if (_e != cudaSuccess) return cuda_fail(idx, _e, what); \
     } while (0)
+
+#define SSG_RC(call)        \
+    do {                    \
+        int _rc = (call);   \
+        if (_rc) return _rc; \
+    } while (0)
+
+// Pinned staging: the result words of a call, and up to kPinBytes each of
+// queries and results (regions of io_cap bytes, grown to a power of two).
+constexpr size_t kPinBytes = size_t(1) << 20;
+int ensure_pin(ssg_index *idx) {
+    if (!idx->pin) SSG_CK(cudaHostAlloc(&idx->pin, 64, cudaHostAllocDefault), "allocating pinned staging");
+    return SSG_OK;
+}
+int ensure_pin_io(ssg_index *idx, size_t bytes) {
+    if (bytes <= idx->io_cap) return SSG_OK;
+    size_t cap = size_t(1) << 15;
+    while (cap < bytes) cap *= 2;
+    if (idx->pin_io) cudaFreeHost(idx->pin_io);
+    idx->pin_io = nullptr;
+    idx->io_cap = 0;
+    SSG_CK(cudaHostAlloc(&idx->pin_io, 2 * cap, cudaHostAllocDefault), "allocating pinned staging");
+    idx->io_cap = cap;
+    return SSG_OK;
+}
+void *pin_in(ssg_index *idx) { return idx->pin_io; }
+void *pin_out(ssg_index *idx) { return static_cast<char *>(idx->pin_io) + idx->io_cap; }
+
+// The status word and the count beside it (uncertified queries), and with
+// them the results of a small host call: one wait for all.
+int read_status(ssg_index *idx, int *status, int *count, const char *what) {
+    SSG_RC(ensure_pin(idx));
+    SSG_CK(cudaMemcpyAsync(idx->pin, idx->status.p, count ? 8 : 4, cudaMemcpyDeviceToHost, idx->stream),
+           "reading the status word");
+    if (idx->out_dev)
+        SSG_CK(cudaMemcpyAsync(pin_out(idx), idx->out_dev, idx->out_bytes, cudaMemcpyDeviceToHost, idx->stream),
+               "copying results");
+    SSG_CK(cudaStreamSynchronize(idx->stream), what);
+    *status = static_cast<const int *>(idx->pin)[0];
+    if (count) *count = static_cast<const int *>(idx->pin)[1];
+    idx->out_done = idx->out_dev != nullptr && *status == 0 && (!count || *count == 0);
+    return SSG_OK;
+}
+
+// The status word, the count of flagged queries and m flags, all cleared:
+// returns the flags (the count is the word before them).
+int clear_flags(ssg_index *idx, int64_t m, int **flags) {
+    SSG_CK(idx->status.ensure(size_t(m + 2) * 4), "allocating query flags");
+    SSG_CK(cudaMemsetAsync(idx->status.p, 0, size_t(m + 2) * 4, idx->stream), "clearing query flags");
+    *flags = static_cast<int *>(idx->status.p) + 2;
+    return SSG_OK;
+}
 
 // Uploads `rows` rows (row stride `ld` elements of `elem`) from host or device
 // memory into dst as contiguous Float32 (or UInt64) rows of `dim`.
@@ -524,12 +584,6 @@ struct ScanTimer {
     }
 };
 
-#define SSG_RC(call)        \
-    do {                    \
-        int _rc = (call);   \
-        if (_rc) return _rc; \
-    } while (0)
-
 // Reduces each query's `segs` sorted candidate segments (kk keys each) by
 // merge passes until one merge block holds them; returns the buffer and the
 // segment count the final merge should read.
@@ -562,7 +616,7 @@ int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
     SSG_CK(idx->l_counts.ensure(size_t(p.chunk) * segs * 4), "allocating list counts");
     SSG_CK(idx->l_minima.ensure(size_t(p.chunk) * p.groups * 4), "allocating the seed's minima");
     SSG_CK(idx->qbound.ensure(size_t(p.chunk) * 4), "allocating query bounds");
-    SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
+    SSG_CK(idx->status.ensure(8), "allocating the status word");
     s->cap = p.cap;
     s->splits = p.splits;
     s->samples = p.samples;
@@ -590,13 +644,15 @@ void list_finalize(const ListPlan &p, const ssg::ListScan &s, ssg::FinalizeArgs 
 
 // Seed, scan and finalize, chunk by chunk of the queries.  s holds the
 // operands (dt, row form, epilogue, n, kk; gamma of the first query), qtiles
-// the query tiles of tb bytes each; finish(c0, f) launches the chunk's
+// the query tiles of tb bytes each; cleared: the status word is zero already;
+// finish(c0, f) launches the chunk's
 // finalize kernel.
 template <typename F>
-int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, const uint8_t *qtiles, size_t tb, int64_t m,
+int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, bool cleared, const uint8_t *qtiles, size_t tb, int64_t m,
                 int k, int exclude_self, uint32_t *d_ids, float *d_dists, F &&finish) {
     SSG_RC(list_buffers(idx, plan, &s));
-    SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
+    if (!cleared)
+        SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     const float *gamma = s.gamma;
     const uint32_t *perm = s.perm;
     const int *rot = s.rot;
@@ -634,9 +690,7 @@ int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, const uin
 int scan_status(ssg_index *idx, const char *what) {
     if (idx->capturing) return SSG_OK;
     int status = 0;
-    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
-           "reading the status word");
-    SSG_CK(cudaStreamSynchronize(idx->stream), "running the scan");
+    SSG_RC(read_status(idx, &status, nullptr, "running the scan"));
     if (status != 0) return fail(idx, SSG_ETIMEOUT, "a bounded wait in the %s scan gave up (code %d)", what, status);
     return SSG_OK;
 }
@@ -679,7 +733,7 @@ int run_hamming_tc(ssg_index *idx, const void *dq, int64_t m, int k, int exclude
     s.bits = float(64 * idx->dim);
     s.n = idx->n;
     s.kk = kk;
-    SSG_RC(list_search(idx, s, plan, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+    SSG_RC(list_search(idx, s, plan, false, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
                        [&](int64_t, ssg::FinalizeArgs &f) {
                            return ssg::launch_finalize(f, idx->stream, &idx->last_launches);
                        }));
@@ -1058,10 +1112,7 @@ void plain_certificate(const ssg_index *idx, int kp, int *flags, int *flag_count
 int plain_finish(ssg_index *idx, const char *what, const float *dq, int64_t m, int k, int exclude_self, int *flags,
                  uint32_t *d_ids, float *d_dists) {
     int status = 0, nflag = 0;
-    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
-           "reading the status word");
-    SSG_CK(cudaMemcpyAsync(&nflag, flags + m, sizeof(int), cudaMemcpyDeviceToHost, idx->stream), "reading flags");
-    SSG_CK(cudaStreamSynchronize(idx->stream), "running the plain method's scan");
+    SSG_RC(read_status(idx, &status, &nflag, "running the plain method's scan"));
     if (status != 0) return fail(idx, SSG_ETIMEOUT, "a bounded wait in the split %s scan gave up (code %d)", what, status);
     idx->last_fallbacks = nflag;
     return run_fallback(idx, dq, m, k, exclude_self, flags, nflag, d_ids, d_dists);
@@ -1072,8 +1123,8 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     const int kk = plan.h, k3 = plan.k3;
     const int kp = ssg::tc_padded_k(idx->dim);
     SSG_RC(ensure_plain_tiles(idx, queries_are_db));
-    SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
-    SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
+    int *flags = nullptr;
+    SSG_RC(clear_flags(idx, m, &flags));
     const size_t tb = ssg::tc_tile_bytes(k3);
     const uint8_t *qtiles = static_cast<const uint8_t *>(idx->ps_dbq.p);
     if (!queries_are_db) {
@@ -1084,8 +1135,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
                "building split query tiles");
         qtiles = static_cast<const uint8_t *>(idx->ps_q.p);
     }
-    int *flags = static_cast<int *>(idx->flags.p);
-    int *flag_count = flags + m;
+    int *flag_count = flags - 1;
     // the list scan; allknn of a large collection in its locality order
     ListPlan lp;
     const bool locality = queries_are_db && idx->locality_param && m == idx->n && idx->n >= kLocalityMinRows;
@@ -1107,7 +1157,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
         s.epi = list_epilogue(idx->metric);
         s.n = idx->n;
         s.kk = plan.rr;
-        SSG_RC(list_search(idx, s, lp, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+        SSG_RC(list_search(idx, s, lp, true, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
                            [&](int64_t c0, ssg::FinalizeArgs &f) {
                                plain_certificate(idx, kp, flags + c0, flag_count, &f);
                                return ssg::launch_finalize_rerank(
@@ -1126,8 +1176,6 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     int64_t chunk = std::max<int64_t>(256, int64_t((size_t(1) << 30) / per_query) / 256 * 256);
     chunk = std::min<int64_t>(chunk, qctas * 128);
     SSG_CK(idx->cand.ensure(per_query * size_t(chunk)), "allocating candidate scratch");
-    SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
-    SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     // allknn in one launch: the database in its locality order (rows grouped
     // by nearest pivot, each query tile starting at its own group), so the
     // heaps hold near neighbours from the first tiles on and few later
@@ -1240,8 +1288,8 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     const int kp = ssg::stream_kbytes(idx->dim, 0) / 2;  // elements per piece
     const int64_t k3 = 3 * int64_t(kp);
     SSG_RC(ensure_plain_stream_tiles(idx, queries_are_db));
-    SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
-    SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
+    int *flags = nullptr;
+    SSG_RC(clear_flags(idx, m, &flags));
     const int64_t qt_alloc = ((m + 127) / 128 + 1) / 2 * 2;  // even: the list scan reads query tiles in pairs
     const size_t tb = 3 * ssg::stream_tile_bytes(idx->dim, 0);
     const uint8_t *qt = static_cast<const uint8_t *>(idx->pss_dbq.p);
@@ -1252,8 +1300,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
                "building split query tiles");
         qt = static_cast<const uint8_t *>(idx->pss_q.p);
     }
-    int *flags = static_cast<int *>(idx->flags.p);
-    int *flag_count = flags + m;
+    int *flag_count = flags - 1;
     // the list scan where a split query tile still fits on chip (to 192 dimensions)
     ListPlan lp;
     const int row_bytes = 3 * ssg::stream_kbytes(idx->dim, 0);
@@ -1267,7 +1314,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
         s.beta = static_cast<const float *>(idx->pss_beta.p);
         s.n = idx->n;
         s.kk = kk;
-        SSG_RC(list_search(idx, s, lp, qt, tb, m, k, exclude_self, d_ids, d_dists,
+        SSG_RC(list_search(idx, s, lp, true, qt, tb, m, k, exclude_self, d_ids, d_dists,
                            [&](int64_t c0, ssg::FinalizeArgs &f) {
                                plain_certificate(idx, kp, flags + c0, flag_count, &f);
                                return ssg::launch_finalize_rerank(
@@ -1286,8 +1333,6 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     int64_t chunk = std::max<int64_t>(128, int64_t((size_t(1) << 30) / per_query) / 128 * 128);
     chunk = std::min<int64_t>(chunk, qtiles * 128);
     SSG_CK(idx->cand.ensure(per_query * size_t(chunk)), "allocating candidate scratch");
-    SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
-    SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     // the K-streaming scan's shared pruning bounds, as for its reduced-precision use
     uint32_t *gbound = nullptr;
     if (kk >= 32 && 2 * splits * cs >= kk) {
@@ -1523,7 +1568,7 @@ int ensure_locality_order(ssg_index *idx, const uint8_t *qtiles, int split) {
     SSG_CK(ssg::launch_tc_norms(idx->metric, x, P, idx->dim, ptiles * 128, static_cast<float *>(pn.p), idx->stream,
                                 &idx->last_launches, pmap),
            "computing pivot norms");
-    SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
+    SSG_CK(idx->status.ensure(8), "allocating the status word");
     DevBuf rank;
     if (idx->loc_chain_param) SSG_RC(pivot_chain(idx, pmap, P, rank));
     // nearest pivot of every row (its keys), then per-row pivot, bucket
@@ -1648,7 +1693,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
         s.epi = list_epilogue(idx->metric);
         s.n = idx->n;
         s.kk = kk;
-        SSG_RC(list_search(idx, s, plan, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+        SSG_RC(list_search(idx, s, plan, false, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
                            [&](int64_t c0, ssg::FinalizeArgs &f) {
                                return ssg::launch_finalize_rerank(
                                    idx->metric, f, static_cast<const float *>(idx->db.p),
@@ -1683,7 +1728,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
     int64_t chunk = std::max<int64_t>(2 * qrows, int64_t((size_t(1) << 30) / per_query) / (2 * qrows) * (2 * qrows));
     chunk = std::min<int64_t>(chunk, (m + qrows - 1) / qrows * qrows);
     SSG_CK(idx->cand.ensure(per_query * size_t(chunk)), "allocating candidate scratch");
-    SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
+    SSG_CK(idx->status.ensure(8), "allocating the status word");
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     const size_t tb = ssg::tc_tile_bytes(idx->dim);
     const uint8_t *qtiles = static_cast<const uint8_t *>(idx->tc_db.p);
@@ -1760,9 +1805,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
     }
     if (idx->capturing) return SSG_OK;  // read after the graph launch
     int status = 0;
-    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
-           "reading the status word");
-    SSG_CK(cudaStreamSynchronize(idx->stream), "running the BF16 search");
+    SSG_RC(read_status(idx, &status, nullptr, "running the BF16 search"));
     if (status != 0)
         return fail(idx, SSG_ETIMEOUT, "a bounded wait in the BF16 scan kernel gave up (code %d)", status);
     return SSG_OK;
@@ -1830,7 +1873,7 @@ int run_knn_tc_filter(ssg_index *idx, const void *dq, const float *dqn, int64_t 
     SSG_CK(idx->cand.ensure(size_t(chunk) * std::max(kk, segs_s * kSampleK) * 8), "allocating candidate scratch");
     SSG_CK(idx->flags.ensure(size_t(m) * 4 + 16), "allocating query flags");
     SSG_CK(cudaMemsetAsync(idx->flags.p, 0, size_t(m) * 4 + 16, idx->stream), "clearing query flags");
-    SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
+    SSG_CK(idx->status.ensure(8), "allocating the status word");
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     int *flags = static_cast<int *>(idx->flags.p);
     int *flag_count = flags + m;
@@ -1957,7 +2000,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
         s.gamma = qgamma;
         s.n = idx->n;
         s.kk = kk;
-        SSG_RC(list_search(idx, s, plan, qt, tb, m, k, exclude_self, d_ids, d_dists,
+        SSG_RC(list_search(idx, s, plan, false, qt, tb, m, k, exclude_self, d_ids, d_dists,
                            [&](int64_t c0, ssg::FinalizeArgs &f) {
                                return ssg::launch_finalize_rerank(
                                    idx->metric, f, static_cast<const float *>(idx->db.p),
@@ -1978,7 +2021,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     int64_t chunk = std::max<int64_t>(128, int64_t((size_t(1) << 30) / per_query) / 128 * 128);
     chunk = std::min<int64_t>(chunk, qtiles * 128);
     SSG_CK(idx->cand.ensure(per_query * size_t(chunk)), "allocating candidate scratch");
-    SSG_CK(idx->status.ensure(sizeof(int)), "allocating the status word");
+    SSG_CK(idx->status.ensure(8), "allocating the status word");
     SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     // shared per-query bounds pay when many splits fill long heaps of the
     // same queries (small batches, long candidate lists): with at least kk / 2
@@ -2022,9 +2065,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     }
     if (idx->capturing) return SSG_OK;  // read after the graph launch
     int status = 0;
-    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
-           "reading the status word");
-    SSG_CK(cudaStreamSynchronize(idx->stream), "running the tensor-core search");
+    SSG_RC(read_status(idx, &status, nullptr, "running the tensor-core search"));
     if (status != 0)
         return fail(idx, SSG_ETIMEOUT, "a bounded wait in the tensor-core scan kernel gave up (code %d)", status);
     return SSG_OK;
@@ -2037,6 +2078,13 @@ int prepare_queries(ssg_index *idx, const void *q, int64_t m, bool src_device, c
         *dq = q;
     } else {
         SSG_CK(idx->qbuf.ensure(qbytes), "allocating query staging");
+        const size_t raw = size_t(m) * idx->dim * elem_size(idx->elem);
+        if (!src_device && raw <= kPinBytes) {
+            // (the previous call has waited for its copies from the staging)
+            SSG_RC(ensure_pin_io(idx, raw));
+            memcpy(pin_in(idx), q, raw);
+            q = pin_in(idx);
+        }
         int rc = upload_rows(idx, idx->qbuf.p, q, m, idx->dim, src_device);
         if (rc) return rc;
         *dq = idx->qbuf.p;
@@ -2237,9 +2285,7 @@ int search_graph(ssg_index *idx, const void *q, int64_t m, int32_t k, uint32_t *
     idx->graph_replays += 1;
     idx->last_graph = 1;
     int status = 0;
-    SSG_CK(cudaMemcpyAsync(&status, idx->status.p, sizeof(int), cudaMemcpyDeviceToHost, idx->stream),
-           "reading the status word");
-    SSG_CK(cudaStreamSynchronize(idx->stream), "running a search graph");
+    SSG_RC(read_status(idx, &status, nullptr, "running a search graph"));
     if (status != 0)
         return fail(idx, SSG_ETIMEOUT, "a bounded wait in the tensor-core scan kernel gave up (code %d)", status);
     return SSG_OK;
@@ -2265,7 +2311,7 @@ int search_common(ssg_index *idx, const void *q, int64_t dim, int64_t m, int32_t
     }
     int rc = search_locked(idx, q, m, k, ids, dists, device);
     if (rc) return rc;
-    return finish_call(idx, !(device && (flags & 1)));
+    return finish_call(idx, !(device && (flags & 1)) && !idx->out_done);
 }
 
 // The body of a search on a locked, validated index with n > 0: query
@@ -2278,10 +2324,13 @@ int search_locked(ssg_index *idx, const void *q, int64_t m, int32_t k, uint32_t 
     if (rc) return rc;
     uint32_t *d_ids = ids;
     float *d_dists = dists;
+    const size_t words = size_t(m) * k;
+    idx->out_dev = nullptr;
+    idx->out_done = false;
     if (!device) {
-        SSG_CK(idx->outbuf.ensure(size_t(m) * k * 8), "allocating result staging");
+        SSG_CK(idx->outbuf.ensure(words * 8), "allocating result staging");
         d_ids = static_cast<uint32_t *>(idx->outbuf.p);
-        d_dists = reinterpret_cast<float *>(static_cast<char *>(idx->outbuf.p) + size_t(m) * k * 4);
+        d_dists = reinterpret_cast<float *>(d_ids + words);
     }
     idx->last_learned = 0;
     if (use_learned(idx)) {
@@ -2291,14 +2340,37 @@ int search_locked(ssg_index *idx, const void *q, int64_t m, int32_t k, uint32_t 
         if (rc) return fail(idx, rc, "learned search: %s", err.c_str());
         idx->last_learned = 1;
     } else {
+        if (!device && words * 8 <= kPinBytes) {
+            // (a growing staging is replaced: the queries in it have to be on
+            // the device by then)
+            if (words * 8 > idx->io_cap) {
+                SSG_CK(cudaStreamSynchronize(idx->stream), "copying queries");
+                SSG_RC(ensure_pin_io(idx, words * 8));
+            }
+            idx->out_dev = idx->outbuf.p;
+            idx->out_bytes = words * 8;
+        }
         rc = run_knn(idx, dq, dqn, m, k, 0, d_ids, d_dists);
+        idx->out_dev = nullptr;
         if (rc) return rc;
     }
-    if (!device) {
-        SSG_CK(cudaMemcpyAsync(ids, d_ids, size_t(m) * k * 4, cudaMemcpyDeviceToHost, idx->stream), "copying ids");
-        SSG_CK(cudaMemcpyAsync(dists, d_dists, size_t(m) * k * 4, cudaMemcpyDeviceToHost, idx->stream),
-               "copying distances");
+    if (device) return SSG_OK;
+    if (words * 8 <= kPinBytes) {
+        if (!idx->out_done) {
+            if (words * 8 > idx->io_cap) {
+                SSG_CK(cudaStreamSynchronize(idx->stream), "running the search");
+                SSG_RC(ensure_pin_io(idx, words * 8));
+            }
+            SSG_CK(cudaMemcpyAsync(pin_out(idx), d_ids, words * 8, cudaMemcpyDeviceToHost, idx->stream),
+                   "copying results");
+            SSG_CK(cudaStreamSynchronize(idx->stream), "running the search");
+        }
+        memcpy(ids, pin_out(idx), words * 4);
+        memcpy(dists, static_cast<const char *>(pin_out(idx)) + words * 4, words * 4);
+        return SSG_OK;
     }
+    SSG_CK(cudaMemcpyAsync(ids, d_ids, words * 4, cudaMemcpyDeviceToHost, idx->stream), "copying ids");
+    SSG_CK(cudaMemcpyAsync(dists, d_dists, words * 4, cudaMemcpyDeviceToHost, idx->stream), "copying distances");
     return SSG_OK;
 }
 
@@ -2883,6 +2955,8 @@ void ssg_destroy(ssg_index *idx) {
                       &idx->pss_dbq, &idx->pss_alpha, &idx->pss_beta, &idx->pss_q, &idx->l_lists, &idx->l_counts,
                       &idx->l_minima, &idx->sk_db, &idx->sk_q})
         b->release();
+    if (idx->pin) cudaFreeHost(idx->pin);
+    if (idx->pin_io) cudaFreeHost(idx->pin_io);
     if (idx->ev0) cudaEventDestroy(idx->ev0);
     if (idx->ev1) cudaEventDestroy(idx->ev1);
     clear_graphs(idx);
