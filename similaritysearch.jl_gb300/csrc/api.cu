@@ -135,9 +135,9 @@ struct ssg_index {
     DevBuf pss_db, pss_dbq, pss_alpha, pss_beta, pss_q;
     int64_t pss_rows = -1, pss_qrows = -1;
     // list scan (tc_list.cu): candidate lists, their counts, the seed's group
-    // minima; +-1 FP8 tiles of the sketches (built for sk_rows rows) and of
-    // the current queries
-    DevBuf l_lists, l_counts, l_minima, sk_db, sk_q;
+    // minima and the queries' bounds; +-1 FP8 tiles of the sketches (built for
+    // sk_rows rows) and of the current queries
+    DevBuf l_buf, sk_db, sk_q;
     int64_t sk_rows = -1;
     int plain_tc_param = 1;
     int last_plain_tc = 0;  // 1: the last plain-method search ran on the tensor cores
@@ -215,7 +215,39 @@ int cuda_fail(ssg_index *idx, cudaError_t e, const char *what) {
 // Pinned staging: the result words of a call, and up to kPinBytes each of
 // queries and results (regions of io_cap bytes, grown to a power of two).
 constexpr size_t kPinBytes = size_t(1) << 20;
+// The result words come from one pinned page per process, 64 bytes an index
+// (pinning memory takes longer than a small search); with more than kPinSlots
+// indexes alive an index pins its own.
+constexpr int kPinSlots = 64;
+struct PinPage {
+    std::mutex mu;
+    char *page = nullptr;
+    uint64_t used = 0;  // a bit per slot
+    void *take() {
+        std::lock_guard<std::mutex> lk(mu);
+        if (!page && cudaHostAlloc(reinterpret_cast<void **>(&page), kPinSlots * 64, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            page = nullptr;
+        }
+        if (!page || used == ~uint64_t(0)) return nullptr;
+        const int s = __builtin_ctzll(~used);
+        used |= uint64_t(1) << s;
+        return page + 64 * s;
+    }
+    bool give(void *p) {
+        std::lock_guard<std::mutex> lk(mu);
+        const char *c = static_cast<const char *>(p);
+        if (!page || c < page || c >= page + kPinSlots * 64) return false;
+        used &= ~(uint64_t(1) << ((c - page) / 64));
+        return true;
+    }
+};
+PinPage &pin_page() {
+    static PinPage *p = new PinPage;  // outlives every index
+    return *p;
+}
 int ensure_pin(ssg_index *idx) {
+    if (!idx->pin) idx->pin = pin_page().take();
     if (!idx->pin) SSG_CK(cudaHostAlloc(&idx->pin, 64, cudaHostAllocDefault), "allocating pinned staging");
     return SSG_OK;
 }
@@ -499,12 +531,15 @@ bool list_plan(const ssg_index *idx, int64_t m, int kk, ListPlan *p) {
     // lets about 1.2 kk f candidates per query through.  With few queries the
     // scan reads memory and hardly appends: a smaller sample.
     const int64_t f = m > 256 ? 8 : 16;
-    const int64_t least = (kk + 1) / 2;  // wide tiles for 4 kk groups of 32 columns
-    if (least > n_full / 4) return false;
+    // four minima per candidate, from groups of 128, 32 or (small databases) 4 rows
+    const int64_t quarter = n_full / 4;
+    p->per_tile = 8 * quarter < 4 * kk ? 64 : 8;
+    const int64_t least = (4 * kk + p->per_tile - 1) / p->per_tile;
+    if (least > quarter) return false;
     p->samples = std::max<int64_t>(least, n_full / f);
-    p->stride = n_full / p->samples;
-    p->per_tile = ssg::kListSegs * p->samples < 4 * kk ? 8 : ssg::kListSegs;
+    if (ssg::kListSegs * p->samples >= 4 * kk) p->per_tile = ssg::kListSegs;
     p->groups = int(p->samples * p->per_tile);
+    p->stride = n_full / p->samples;
     const int64_t qtiles = (m + 127) / 128;
     const int64_t pairs = (qtiles + 1) / 2;
     int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(pairs, ssg::device_sm_count() / 2, n_wide);
@@ -612,10 +647,9 @@ int reduce_segments(ssg_index *idx, const uint64_t *cand, int64_t m, int segs, i
 // Sizes the list scan's buffers for one chunk and points the scan at them.
 int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
     const size_t segs = size_t(p.splits) * ssg::kListSegs;
-    SSG_CK(idx->l_lists.ensure(size_t(p.chunk) * segs * p.cap * 8), "allocating candidate lists");
-    SSG_CK(idx->l_counts.ensure(size_t(p.chunk) * segs * 4), "allocating list counts");
-    SSG_CK(idx->l_minima.ensure(size_t(p.chunk) * p.groups * 4), "allocating the seed's minima");
-    SSG_CK(idx->qbound.ensure(size_t(p.chunk) * 4), "allocating query bounds");
+    // one allocation: lists, minima (16-byte rows), bounds, counts
+    const size_t lists = size_t(p.chunk) * segs * p.cap * 8, minima = size_t(p.chunk) * p.groups * 4;
+    SSG_CK(idx->l_buf.ensure(lists + minima + size_t(p.chunk) * 4 * (1 + segs)), "allocating candidate lists");
     SSG_CK(idx->status.ensure(8), "allocating the status word");
     s->cap = p.cap;
     s->splits = p.splits;
@@ -623,10 +657,10 @@ int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
     s->sample_stride = p.stride;
     s->groups = p.groups;
     s->per_tile = p.per_tile;
-    s->bound = static_cast<uint32_t *>(idx->qbound.p);
-    s->lists = static_cast<uint64_t *>(idx->l_lists.p);
-    s->counts = static_cast<int *>(idx->l_counts.p);
-    s->minima = static_cast<float *>(idx->l_minima.p);
+    s->lists = static_cast<uint64_t *>(idx->l_buf.p);
+    s->minima = reinterpret_cast<float *>(static_cast<char *>(idx->l_buf.p) + lists);
+    s->bound = reinterpret_cast<uint32_t *>(s->minima + size_t(p.chunk) * p.groups);
+    s->counts = reinterpret_cast<int *>(s->bound + p.chunk);
     s->err = static_cast<int *>(idx->status.p);
     return SSG_OK;
 }
@@ -1301,7 +1335,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
         qt = static_cast<const uint8_t *>(idx->pss_q.p);
     }
     int *flag_count = flags - 1;
-    // the list scan where a split query tile still fits on chip (to 192 dimensions)
+    // the list scan where the database is large enough for its seed
     ListPlan lp;
     const int row_bytes = 3 * ssg::stream_kbytes(idx->dim, 0);
     if (ssg::list_fits(row_bytes, 128, ssg::LIST_AFFINE, idx->n) && list_plan(idx, m, kk, &lp)) {
@@ -1446,7 +1480,7 @@ int run_knn(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, 
             // sketches are scanned as they are
             const int rc = run_hamming_tc(idx, dq, m, k, exclude_self, d_ids, d_dists, queries_are_db, kk, plan);
             if (rc != SSG_ENOMEM) return rc;
-            for (DevBuf *b : {&idx->sk_db, &idx->sk_q, &idx->l_lists, &idx->l_minima}) b->release();
+            for (DevBuf *b : {&idx->sk_db, &idx->sk_q, &idx->l_buf}) b->release();
             idx->sk_rows = -1;
         }
     }
@@ -1983,9 +2017,8 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
         qt = static_cast<const uint8_t *>(idx->st_q.p);
         qgamma = qs;
     }
-    // the list scan where a query tile fits on chip (FP8 to 1,280 dimensions,
-    // BF16 to 640) and the database is large enough for its seed; the same kk
-    // candidates
+    // the list scan where the database is large enough for its seed: the same
+    // kk candidates
     ListPlan plan;
     const int row_bytes = ssg::stream_kbytes(idx->dim, fp8);
     if (ssg::list_fits(row_bytes, 128, ssg::LIST_AFFINE, idx->n) && list_plan(idx, m, kk, &plan)) {
@@ -2223,7 +2256,7 @@ std::vector<uint64_t> graph_key(const ssg_index *idx, int64_t m, int k) {
     for (const DevBuf *b : {&idx->db, &idx->db_norm, &idx->tc_db, &idx->tc_norm, &idx->tc_q, &idx->st_db,
                             &idx->st_scale, &idx->st_alpha, &idx->st_beta, &idx->st_q, &idx->st_qscale, &idx->cand,
                             &idx->red[0], &idx->red[1], &idx->status, &idx->gbound, &idx->qnorm, &idx->pack_q,
-                            &idx->pack_out, &idx->qbound, &idx->l_lists, &idx->l_counts, &idx->l_minima})
+                            &idx->pack_out, &idx->qbound, &idx->l_buf})
         key.push_back(uint64_t(reinterpret_cast<uintptr_t>(b->p)));
     return key;
 }
@@ -2952,10 +2985,9 @@ void ssg_destroy(ssg_index *idx) {
                       &idx->fb_cand, &idx->fb_qn, &idx->tc_smp, &idx->tc_smp_norm, &idx->f_out, &idx->f_cnt,
                       &idx->f_thr, &idx->gbound, &idx->pack_q, &idx->pack_out, &idx->gm_db, &idx->gm_q,
                       &idx->ps_db, &idx->ps_dbq, &idx->ps_norm, &idx->ps_q, &idx->qbound, &idx->pss_db,
-                      &idx->pss_dbq, &idx->pss_alpha, &idx->pss_beta, &idx->pss_q, &idx->l_lists, &idx->l_counts,
-                      &idx->l_minima, &idx->sk_db, &idx->sk_q})
+                      &idx->pss_dbq, &idx->pss_alpha, &idx->pss_beta, &idx->pss_q, &idx->l_buf, &idx->sk_db, &idx->sk_q})
         b->release();
-    if (idx->pin) cudaFreeHost(idx->pin);
+    if (idx->pin && !pin_page().give(idx->pin)) cudaFreeHost(idx->pin);
     if (idx->pin_io) cudaFreeHost(idx->pin_io);
     if (idx->ev0) cudaEventDestroy(idx->ev0);
     if (idx->ev1) cudaEventDestroy(idx->ev1);

@@ -295,53 +295,67 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
         const int64_t jr = query_row(f, j);
         int total = f.segs * f.kk;
         const uint64_t *src = f.cand + size_t(j) * total;
-        const int *cn = nullptr;
-        if (f.counts) {
-            cn = f.counts + size_t(j) * f.segs;
-            src = f.cand + size_t(j) * f.segs * f.list_cap;
-            total = 0;
-            for (int s = 0; s < f.segs; ++s) total += cn[s];
-        }
-        const uint32_t bound = cn ? f.list_bound[j] : 0xffffffffu;
-        // the query's at-th key, at < total: of its segments, or of its few
-        // lists in turn (empty beyond the bound)
-        auto key_at = [&](int at) {
-            if (!cn) return src[at];
-            int s = 0;
-            for (int c = cn[0]; at >= c; c = cn[s]) { at -= c; ++s; }
-            const uint64_t k = src[size_t(s) * f.list_cap + at];
-            return uint32_t(k >> 32) <= bound ? k : KEY_EMPTY;
-        };
-        // more keys than the registers hold (lists only): those within the
-        // bound gather in the ring's memory, and if they are still too many, a
-        // limit with exactly `need` keys below it is found by counting
         uint64_t key[kWarpKeys];
         const uint64_t *held = nullptr;
-        if (total > 32 * kWarpKeys) {
-            const int room = RERANK ? kWarpStages * (need + 1) * kRowStride / 2 : 0;
+        if (f.counts) {
+            // lists: the keys within the bound gather in the ring's memory
+            // (each lane copies whole lists, its places from a running sum);
+            // where they are more than the registers hold, a limit with
+            // exactly `need` keys below it is found by counting
+            const int *cn = f.counts + size_t(j) * f.segs;
+            const uint64_t *lists = f.cand + size_t(j) * f.segs * f.list_cap;
+            const uint32_t bound = f.list_bound[j];
+            const int room = kWarpStages * (need + 1) * kRowStride / 2;
             uint64_t *scratch = reinterpret_cast<uint64_t *>(smem) + size_t(warp) * room;
+            // body(key) for every key within the bound, by whole warps: lists
+            // in rounds of 32, one per lane, or all lanes along one where
+            // there are few
+            auto each_key = [&](auto &&body) {
+                if (f.segs >= 8) {
+                    for (int s0 = 0; s0 < f.segs; s0 += 32) {
+                        const int c = s0 + lane < f.segs ? cn[s0 + lane] : 0;
+                        const uint64_t *l = lists + size_t(s0 + lane) * f.list_cap;
+                        const int most = __reduce_max_sync(0xffffffffu, c);
+                        for (int i = 0; i < most; ++i) {
+                            const uint64_t k = i < c ? l[i] : KEY_EMPTY;
+                            body(uint32_t(k >> 32) <= bound ? k : KEY_EMPTY);
+                        }
+                    }
+                } else {
+                    for (int s = 0; s < f.segs; ++s) {
+                        const int c = cn[s];
+                        const uint64_t *l = lists + size_t(s) * f.list_cap;
+                        for (int i0 = 0; i0 < c; i0 += 32) {
+                            const uint64_t k = i0 + lane < c ? l[i0 + lane] : KEY_EMPTY;
+                            body(uint32_t(k >> 32) <= bound ? k : KEY_EMPTY);
+                        }
+                    }
+                }
+            };
             auto gather = [&](uint64_t below, uint64_t *to, int most) {
                 int base = 0;
-                for (int i0 = 0; i0 < total; i0 += 32) {
-                    const uint64_t k = i0 + lane < total ? key_at(i0 + lane) : KEY_EMPTY;
+                each_key([&](uint64_t k) {
                     const uint32_t vote = __ballot_sync(0xffffffffu, k < below);
                     const int at = base + __popc(vote & ((1u << lane) - 1u));
                     if (k < below && at < most) to[at] = k;
                     base += __popc(vote);
-                }
+                });
                 __syncwarp();
                 return base;
             };
-            int have = RERANK ? gather(KEY_EMPTY, scratch, room) : INT_MAX;
+            int have = gather(KEY_EMPTY, scratch, room);
             held = scratch;
             if (have > 32 * kWarpKeys) {
                 uint64_t p = 0, lim = KEY_EMPTY;
                 const bool on_chip = have <= room;
-                const int all = on_chip ? have : total;
                 for (int b = 63; b >= 0; --b) {
                     const uint64_t t = p | (1ull << b);
                     int c = 0;
-                    for (int at = lane; at < all; at += 32) c += (on_chip ? scratch[at] : key_at(at)) < t;
+                    if (on_chip) {
+                        for (int at = lane; at < have; at += 32) c += scratch[at] < t;
+                    } else {
+                        each_key([&](uint64_t k) { c += k < t; });
+                    }
                     c = __reduce_add_sync(0xffffffffu, c);
                     if (c == need) { lim = t; break; }
                     if (c < need) p = t;
@@ -355,14 +369,14 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
 #pragma unroll
         for (int i = 0; i < kWarpKeys; ++i) {
             const int at = i * 32 + lane;
-            key[i] = at >= total ? KEY_EMPTY : held ? held[at] : key_at(at);
+            key[i] = at >= total ? KEY_EMPTY : held ? held[at] : src[at];
             if (RERANK && int64_t(key_id0(key[i])) >= f.n_rows) key[i] = KEY_EMPTY;
             cnt += key[i] != KEY_EMPTY;
         }
         const int nvt = __reduce_add_sync(0xffffffffu, cnt);
         __syncwarp();
         uint64_t low = KEY_EMPTY;
-        if (RERANK && f.check && !cn) {
+        if (RERANK && f.check && !f.counts) {
             for (int s = lane; s < f.segs; s += 32) low = min(low, src[size_t(s) * f.kk + f.kk - 1]);
             low = warp_min64(low);
         }
@@ -734,9 +748,14 @@ cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const floa
     const int total = f.counts ? std::max(f.list_keys, 2 * need) : f.segs * f.kk;
     const bool vec = RERANK && dim % 4 == 0 &&
                      ((reinterpret_cast<uintptr_t>(db) | reinterpret_cast<uintptr_t>(q)) & 15) == 0;
-    // (the lists of a locality order's few splits hold little more than need)
-    if ((f.counts ? f.query_ids && f.segs <= 8 : total <= 32 * kWarpKeys) && need <= kWarpOut) {
-        const size_t smem = RERANK ? size_t(kWarpsPerBlock) * kWarpStages * (need + 1) * kRowStride * 4 : 0;
+    // (lists: a block is done sooner with few queries, and with more rows to
+    // gather than lanes: 777 queries x 45 rows of 300 dimensions 30 us against
+    // 38 in warps, 1,000 x 18 of 128 27.5 against 23.6; in a locality order the
+    // warps share rows, 38,912 x 23 of 100 744 against 600)
+    if ((f.counts ? f.m >= 256 && (f.query_ids || (need <= 32 && f.list_keys <= 1024)) : total <= 32 * kWarpKeys) &&
+        need <= kWarpOut) {
+        const size_t smem =
+            RERANK || f.counts ? size_t(kWarpsPerBlock) * kWarpStages * (need + 1) * kRowStride * 4 : 0;
         auto kern = finalize_warp_kernel<METRIC, RERANK>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;

@@ -313,9 +313,12 @@ struct RowList {
     }
 };
 
-template <int SWB, bool F8, int EPI, bool SEED, int ORDER>
+// QSTREAM: the query tile does not fit on chip; its K-blocks come through the
+// ring beside the database's (64 bytes per clock and SM at the full MMA rate,
+// half of what 128 x 128 tiles take).
+template <int SWB, bool F8, int EPI, bool SEED, int ORDER, bool QSTREAM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
-    tc_list_kernel(KernelArgs ka, const __grid_constant__ CUtensorMap dmap) {
+    tc_list_kernel(KernelArgs ka, const __grid_constant__ CUtensorMap dmap, const __grid_constant__ CUtensorMap qmap) {
     constexpr int KBLK = TILE * SWB;   // bytes of a K-block of a tile
     constexpr int KSTEPS = SWB / 32;   // MMAs per K-block (32 bytes of K each)
     const ListScan &a = ka.s;
@@ -324,9 +327,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int kblocks = ka.kblocks, stages = ka.stages, group = ka.group;
     const int groups_per_tile = kblocks / group;
     const size_t tile_bytes = size_t(kblocks) * KBLK;
-    const uint32_t stage_bytes = uint32_t(group) * KBLK;
+    const uint32_t part_bytes = uint32_t(group) * KBLK;  // of one operand
+    const uint32_t stage_bytes = (QSTREAM ? 2 : 1) * part_bytes;
     uint8_t *sA = smem;
-    uint8_t *sB = sA + tile_bytes;
+    uint8_t *sB = sA + (QSTREAM ? 0 : tile_bytes);  // stages: database part, then the query part
     // per epilogue warp, two buffers of its 64 columns' coefficients
     float4 *coef = reinterpret_cast<float4 *>(sB + size_t(stages) * stage_bytes);
     uint64_t *bufs = reinterpret_cast<uint64_t *>(coef + (raw_rank(EPI) ? 0 : kCoefBytes / 16));  // raw candidates
@@ -391,19 +395,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             // producer: this CTA's query tile, then its tile's part of
             // every K-block group; both halves of a stage complete on the
             // even CTA's full[s]
-            tc::mbar_arrive_expect_tx(a_full, uint32_t(tile_bytes));
-            for (int kb = 0; kb < kblocks; ++kb)
-                tc::bulk_g2s(sA + size_t(kb) * KBLK, a.qt + size_t(qx) * tile_bytes + size_t(kb) * KBLK, KBLK, a_full);
+            if constexpr (!QSTREAM) {
+                tc::mbar_arrive_expect_tx(a_full, uint32_t(tile_bytes));
+                for (int kb = 0; kb < kblocks; ++kb)
+                    tc::bulk_g2s(sA + size_t(kb) * KBLK, a.qt + size_t(qx) * tile_bytes + size_t(kb) * KBLK, KBLK,
+                                 a_full);
+            }
             const uint32_t full0 = tc::mapa_shared(tc::smem_u32(full), 0);
             int s = 0, issued = 0;
             uint32_t ph = 1;
             bool ok = true;
             for (int u = 0; ok && u < W; ++u) {
                 int line = (int(wide_tile(u)) * 2 + int(rank)) * kblocks * (KBLK / kLine);
+                int qline = int(qx) * kblocks * (KBLK / kLine);
                 for (int g = 0; g < groups_per_tile; ++g, line += group * (KBLK / kLine)) {
                     if (!tc::mbar_wait(&empty[s], ph, a.err, 21)) { ok = false; break; }
                     if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
-                    tc::tma_load_2d_pair(sB + size_t(s) * stage_bytes, &dmap, 0, line, full0 + uint32_t(s * 8));
+                    uint8_t *dst = sB + size_t(s) * stage_bytes;
+                    tc::tma_load_2d_pair(dst, &dmap, 0, line, full0 + uint32_t(s * 8));
+                    if constexpr (QSTREAM) {
+                        tc::tma_load_2d_pair(dst + part_bytes, &qmap, 0, qline, full0 + uint32_t(s * 8));
+                        qline += group * (KBLK / kLine);
+                    }
                     issued = issued < stages ? issued + 1 : stages;
                     if (++s == stages) { s = 0; ph ^= 1; }
                 }
@@ -411,7 +424,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             // wait (bounded) until every copy of this pair has landed (the
             // even CTA's barriers count both halves; the final cluster
             // barrier keeps the odd CTA alive until then)
-            tc::mbar_wait(a_full, 0, a.err, 22);
+            if (!QSTREAM) tc::mbar_wait(a_full, 0, a.err, 22);
             if (rank == 0) {
                 // the last `issued` stages, newest first: a stage's landing
                 // phase is the opposite of the one its emptiness was waited for
@@ -424,11 +437,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     } else if (warp == 1) {
         if (lane == 0 && rank == 1) {
             // the odd CTA tells the even CTA that its query tile landed
-            if (tc::mbar_wait(a_full, 0, a.err, 28)) tc::mbar_arrive_cluster(tc::mapa_shared(tc::smem_u32(pa_full), peer));
+            if (!QSTREAM && tc::mbar_wait(a_full, 0, a.err, 28)) tc::mbar_arrive_cluster(tc::mapa_shared(tc::smem_u32(pa_full), peer));
         } else if (lane == 0) {
             // the even CTA issues the pair's MMAs
             constexpr uint32_t idesc = F8 ? tc::idesc_e4m3_f32(2 * TILE, WIDE) : tc::idesc_bf16_f32(2 * TILE, WIDE);
-            bool ok = tc::mbar_wait(a_full, 0, a.err, 23) && tc::mbar_wait(pa_full, 0, a.err, 23);
+            bool ok = QSTREAM || (tc::mbar_wait(a_full, 0, a.err, 23) && tc::mbar_wait(pa_full, 0, a.err, 23));
             // descriptors address 16-byte units
             const uint64_t a_desc = tc::smem_desc(tc::smem_u32(sA), SWB);
             const uint64_t b_desc = tc::smem_desc(tc::smem_u32(sB), SWB);
@@ -443,6 +456,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     if (!tc::mbar_wait(&full[s], ph, a.err, 24)) { ok = false; break; }
                     tc::tc_fence_after();
                     uint64_t bd = b_desc + uint64_t((uint32_t(s) * stage_bytes) >> 4);
+                    if (QSTREAM) ad = bd + uint64_t(part_bytes >> 4);
                     for (int kb = 0; kb < group; ++kb) {
 #pragma unroll
                         for (int k = 0; k < KSTEPS; ++k) {
@@ -548,7 +562,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     if constexpr (SEED) {
                         float g[8];
                         T.chunk_min(r[c], row0 + ch * CS * 32, al + ch * 8, al + CH * 8 + ch * 8, g);
-                        if (ORDER != STORED && T.valid) {
+                        if ((ORDER != STORED || a.per_tile == 64) && T.valid) {
                             float4 *to = reinterpret_cast<float4 *>(a.minima + size_t(query) * a.groups + (w_lo + u) * 64 +
                                                                     (cs * CH + ch) * 8);
                             to[0] = make_float4(g[0], g[1], g[2], g[3]);
@@ -560,7 +574,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             }
             if (++b == NACC) { b = 0; ph ^= 1; }
             if constexpr (SEED && ORDER == STORED) {
-                if (T.valid) {
+                if (T.valid && a.per_tile != 64) {
                     float *g = a.minima + size_t(query) * a.groups;
                     const int64_t at = w_lo + u;
                     if (a.per_tile == 8) {
@@ -670,7 +684,7 @@ __global__ void sketch_tile_kernel(const uint64_t *__restrict__ x, int64_t rows,
 // The database tiles as lines of 2 KB (256 eight-byte elements; the bytes are
 // already swizzled, so a box is copied verbatim): a box is one tile's part of
 // a ring stage, a whole row's K-blocks where they fit.
-cudaError_t line_map(const ListScan &s, int kblocks, int group, CUtensorMap *map) {
+cudaError_t line_map(const ListScan &s, const uint8_t *base, int64_t rows, int kblocks, int group, CUtensorMap *map) {
     using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -683,64 +697,80 @@ cudaError_t line_map(const ListScan &s, int kblocks, int group, CUtensorMap *map
         if (q != cudaDriverEntryPointSuccess || !fn) return cudaErrorNotSupported;
         encode = reinterpret_cast<EncodeFn>(fn);
     }
-    if (reinterpret_cast<uintptr_t>(s.dt) % 16 != 0) return cudaErrorInvalidValue;
-    const int64_t tiles = (s.n + WIDE - 1) / WIDE * 2;
+    if (reinterpret_cast<uintptr_t>(base) % 16 != 0) return cudaErrorInvalidValue;
+    const int64_t tiles = (rows + WIDE - 1) / WIDE * 2;
     const cuuint64_t dims[2] = {cuuint64_t(kLine / 8), cuuint64_t(tiles) * kblocks * (TILE * s.swb / kLine)};
     const cuuint64_t strides[1] = {cuuint64_t(kLine)};
     const cuuint32_t box[2] = {cuuint32_t(kLine / 8), cuuint32_t(group * (TILE * s.swb / kLine))};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<uint8_t *>(s.dt), dims, strides, box,
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<uint8_t *>(base), dims, strides, box,
                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-size_t list_smem(int row_bytes, int stage_bytes, int stages, int epi) {
-    return 1024 + size_t(TILE) * row_bytes + size_t(stages) * stage_bytes + (raw_rank(epi) ? 0 : kCoefBytes) + kBufBytes +
+size_t list_smem(int query_bytes, int stage_bytes, int stages, int epi) {
+    return 1024 + size_t(query_bytes) + size_t(stages) * stage_bytes + (raw_rank(epi) ? 0 : kCoefBytes) + kBufBytes +
            (2 + 2 * kMaxStages + 2 * NACC + 1) * 8 + 16;
 }
 
-// The ring beside a query tile: K-blocks per stage (a divisor of the row's)
-// and stages.  Every stage costs the MMA thread a wait and a commit, so the
-// largest stages of which three fit, up to 32 KB (2,048 queries x 1e6 rows of
-// 96 dimensions: the seed 51 us with a K-block per stage, 35 with the row's
-// three).  stages = 0: not even four K-blocks fit.
+// The ring: K-blocks per stage (a divisor of the row's) and stages, beside a
+// resident query tile or with its K-blocks in the stages.  Every stage costs
+// the MMA thread a wait and a commit, so the largest stages of which three
+// fit, up to 32 KB (2,048 queries x 1e6 rows of 96 dimensions: the seed 51 us
+// with a K-block per stage, 35 with the row's three).  stages = 0: not even
+// four K-blocks fit.
 struct Ring {
     int group, stages;
+    bool qstream;
+    size_t smem;
 };
 Ring list_ring(int row_bytes, int swb, int epi) {
     const int kblocks = row_bytes / swb;
-    for (int g = std::min(kblocks, kStageBytes / (TILE * swb)); g >= 1; --g) {
-        if (kblocks % g) continue;
-        int st = kMaxStages;
-        while (st > 0 && list_smem(row_bytes, g * TILE * swb, st, epi) > kMaxSmem) --st;
-        if (st >= 3 && st * g >= 4) return {g, st};
+    for (int qstream = 0; qstream < 2; ++qstream) {
+        const int query_bytes = qstream ? 0 : TILE * row_bytes, parts = qstream ? 2 : 1;
+        for (int g = std::min(kblocks, kStageBytes / (TILE * swb)); g >= 1; --g) {
+            if (kblocks % g) continue;
+            const int stage = parts * g * TILE * swb;
+            int st = kMaxStages;
+            while (st > 0 && list_smem(query_bytes, stage, st, epi) > kMaxSmem) --st;
+            if (st >= 3 && st * g >= 4) return {g, st, qstream != 0, list_smem(query_bytes, stage, st, epi)};
+        }
     }
-    return {1, 0};
+    return {1, 0, false, 0};
 }
 
-template <int SWB, bool F8, int EPI, bool SEED, int ORDER = STORED>
-cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
+template <int SWB, bool F8, int EPI, bool SEED, int ORDER, bool QSTREAM>
+cudaError_t launch_list_q(const ListScan &s, const Ring &ring, cudaStream_t st) {
     KernelArgs ka;
     ka.s = s;
     ka.kblocks = s.row_bytes / SWB;
-    const Ring ring = list_ring(s.row_bytes, SWB, EPI);
-    if (ring.stages == 0) return cudaErrorInvalidValue;
     ka.group = ring.group;
     ka.stages = ring.stages;
     ka.all_wide = (s.n + WIDE - 1) / WIDE;
     ka.n_wide = SEED ? s.samples : ka.all_wide;
-    size_t smem = list_smem(s.row_bytes, ring.group * TILE * SWB, ring.stages, EPI);
-    if (smem < kAloneSmem) smem = kAloneSmem;
-    auto kern = tc_list_kernel<SWB, F8, EPI, SEED, ORDER>;
+    const size_t smem = std::max(ring.smem, kAloneSmem);
+    auto kern = tc_list_kernel<SWB, F8, EPI, SEED, ORDER, QSTREAM>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
-    CUtensorMap map;
-    e = line_map(s, ka.kblocks, ka.group, &map);
+    CUtensorMap dmap, qmap;
+    e = line_map(s, s.dt, s.n, ka.kblocks, ka.group, &dmap);
+    if (e == cudaSuccess) e = line_map(s, s.qt, s.m, ka.kblocks, ka.group, &qmap);
     if (e != cudaSuccess) return e;
     const int64_t qtiles = ((s.m + TILE - 1) / TILE + 1) / 2 * 2;
-    kern<<<dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st>>>(ka, map);
+    kern<<<dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st>>>(ka, dmap, qmap);
     return cudaGetLastError();
+}
+
+template <int SWB, bool F8, int EPI, bool SEED, int ORDER = STORED>
+cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
+    const Ring ring = list_ring(s.row_bytes, SWB, EPI);
+    if (ring.stages == 0) return cudaErrorInvalidValue;
+    if constexpr (EPI == EPI_AFF) {
+        if (ring.qstream) return launch_list_q<SWB, F8, EPI, SEED, ORDER, true>(s, ring, st);
+    }
+    if (ring.qstream) return cudaErrorInvalidValue;
+    return launch_list_q<SWB, F8, EPI, SEED, ORDER, false>(s, ring, st);
 }
 
 // BF16 tiles with 64-byte K-blocks, the form that allknn orders.
@@ -772,7 +802,8 @@ cudaError_t launch_list_any(const ListScan &s, cudaStream_t st) {
 // Four K-blocks of ring beside the query tile, and the database's lines within the
 // tensor map's 32-bit coordinates.
 bool list_fits(int row_bytes, int swb, int epi, int64_t n) {
-    return list_ring(row_bytes, swb, epi).stages > 0 &&
+    const Ring ring = list_ring(row_bytes, swb, epi);
+    return ring.stages > 0 && (!ring.qstream || epi == LIST_AFFINE) &&
            (n / TILE + 2) * (row_bytes / swb) * (TILE * swb / kLine) < (int64_t(1) << 31);
 }
 
@@ -782,7 +813,7 @@ cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches) 
     // about four groups per candidate keep the bound within a fifth of the
     // sample's own kk-th distance in rank
     const unsigned blocks = unsigned((s.m + 3) / 4);
-    if (s.perm) seed_bound_kernel<32><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
+    if (s.per_tile == 64 && s.kk <= 256) seed_bound_kernel<32><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
     else if (s.kk <= 64) seed_bound_kernel<8><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
     else if (s.kk <= 160) seed_bound_kernel<20><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
     else seed_bound_kernel<60><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
