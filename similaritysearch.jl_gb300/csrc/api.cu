@@ -135,7 +135,7 @@ struct ssg_index {
     DevBuf pss_db, pss_dbq, pss_alpha, pss_beta, pss_q;
     int64_t pss_rows = -1, pss_qrows = -1;
     // list scan (tc_list.cu): candidate lists, their counts, the seed's group
-    // minima and the queries' bounds; +-1 FP8 tiles of the sketches (built for
+    // minima and the queries' bounds; +-1 FP4 tiles of the sketches (built for
     // sk_rows rows) and of the current queries
     DevBuf l_buf, sk_db, sk_q;
     int64_t sk_rows = -1;
@@ -525,7 +525,9 @@ struct ListPlan {
 // (four groups of columns per candidate from at most a quarter of the
 // database), or lists longer than a list's room.
 bool list_plan(const ssg_index *idx, int64_t m, int kk, ListPlan *p) {
-    const int64_t n_full = idx->n / 256, n_wide = (idx->n + 255) / 256;
+    // rows of a wide tile
+    const int64_t wide = idx->metric == SSG_METRIC_HAMMING ? 2 * ssg::sketch_tile_rows(false) : 256;
+    const int64_t n_full = idx->n / wide, n_wide = (idx->n + wide - 1) / wide;
     if (kk > (ssg::kListMaxCap - 64) / 2 || n_full < 8) return false;
     // The sample costs its share of a scan, and a bound from one row in f
     // lets about 1.2 kk f candidates per query through.  With few queries the
@@ -734,35 +736,33 @@ int list_epilogue(int metric) {
     return is_sq_metric(metric) ? ssg::LIST_SQ : metric == SSG_METRIC_COSINE ? ssg::LIST_COS : ssg::LIST_DOT;
 }
 
-// Hamming on the tensor cores: sketches as +-1 FP8 rows, products exact in
+// Hamming on the tensor cores: sketches as +-1 FP4 rows, products exact in
 // FP32 (at most 2,048 terms of +-1), distance = (bits - product) / 2, so the
 // keys are the ones hamming_kernel makes.
 int run_hamming_tc(ssg_index *idx, const void *dq, int64_t m, int k, int exclude_self, uint32_t *d_ids,
-                   float *d_dists, bool queries_are_db, int kk, const ListPlan &plan) {
+                   float *d_dists, int kk, const ListPlan &plan) {
     const int row_bytes = ssg::sketch_row_bytes(idx->dim);
-    const size_t tb = size_t(128) * row_bytes;
-    const int64_t tiles = (ssg::tc_tiles(idx->n) + 1) / 2 * 2;
+    const int rows = ssg::sketch_tile_rows(false);
+    const int64_t tiles = (idx->n + 2 * rows - 1) / (2 * rows) * 2;
     if (idx->sk_rows != idx->n) {
-        SSG_CK(idx->sk_db.ensure(size_t(tiles) * tb), "allocating sketch tiles");
-        SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(idx->db.p), idx->n, idx->dim, tiles,
+        SSG_CK(idx->sk_db.ensure(size_t(tiles) * rows * row_bytes), "allocating sketch tiles");
+        SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(idx->db.p), idx->n, idx->dim, false, tiles,
                                         static_cast<uint8_t *>(idx->sk_db.p), idx->stream, &idx->last_launches),
                "building sketch tiles");
         idx->sk_rows = idx->n;
     }
-    const uint8_t *qtiles = static_cast<const uint8_t *>(idx->sk_db.p);
-    if (!queries_are_db) {
-        const int64_t qt = (ssg::tc_tiles(m) + 1) / 2 * 2;
-        SSG_CK(idx->sk_q.ensure(size_t(qt) * tb), "allocating query sketch tiles");
-        SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(dq), m, idx->dim, qt,
-                                        static_cast<uint8_t *>(idx->sk_q.p), idx->stream, &idx->last_launches),
-               "building query sketch tiles");
-        qtiles = static_cast<const uint8_t *>(idx->sk_q.p);
-    }
+    // (allknn's queries too: the database's tiles have fewer rows)
+    const size_t tb = size_t(128) * row_bytes;
+    const int64_t qt = (ssg::tc_tiles(m) + 1) / 2 * 2;
+    SSG_CK(idx->sk_q.ensure(size_t(qt) * tb), "allocating query sketch tiles");
+    SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(dq), m, idx->dim, true, qt,
+                                    static_cast<uint8_t *>(idx->sk_q.p), idx->stream, &idx->last_launches),
+           "building query sketch tiles");
+    const uint8_t *qtiles = static_cast<const uint8_t *>(idx->sk_q.p);
     ssg::ListScan s{};
     s.dt = static_cast<const uint8_t *>(idx->sk_db.p);
     s.row_bytes = row_bytes;
     s.swb = 128;
-    s.fp8 = 1;
     s.epi = ssg::LIST_HAMMING;
     s.bits = float(64 * idx->dim);
     s.n = idx->n;
@@ -1476,9 +1476,9 @@ int run_knn(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, 
         const int kk = int(std::min<int64_t>(int64_t(k) + (exclude_self ? 1 : 0), idx->n));
         ListPlan plan;
         if (ssg::list_fits(ssg::sketch_row_bytes(idx->dim), 128, ssg::LIST_HAMMING, idx->n) && list_plan(idx, m, kk, &plan)) {
-            // the tiles take 8 times the sketches: without the memory the
+            // the tiles take 4 times the sketches: without the memory the
             // sketches are scanned as they are
-            const int rc = run_hamming_tc(idx, dq, m, k, exclude_self, d_ids, d_dists, queries_are_db, kk, plan);
+            const int rc = run_hamming_tc(idx, dq, m, k, exclude_self, d_ids, d_dists, kk, plan);
             if (rc != SSG_ENOMEM) return rc;
             for (DevBuf *b : {&idx->sk_db, &idx->sk_q, &idx->l_buf}) b->release();
             idx->sk_rows = -1;

@@ -220,6 +220,7 @@ constexpr int kListSegs = 2;       // lists of a query per split
 struct ListScan {
     const uint8_t *qt, *dt;   // operand tiles (an even number of each)
     int row_bytes, swb, fp8;  // bytes per padded row, per K-block row (64 / 128), FP8 or BF16
+                              // (HAMMING: sketch tiles, 240 rows to a wide tile)
     int epi;                  // LIST_*
     const float *alpha;       // per padded row: |x|^2 (SQ), 1 / |x| (COS), alpha (AFFINE)
     const float *beta;        // AFFINE
@@ -246,9 +247,11 @@ struct ListScan {
 bool list_fits(int row_bytes, int swb, int epi, int64_t n);
 cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches);
 cudaError_t launch_list_scan(const ListScan &s, cudaStream_t st, int *launches);
-// Sketches as +-1 FP8 rows (128-byte K-blocks).
+// Sketches as +-1 FP4 rows (128-byte K-blocks), in tiles of sketch_tile_rows
+// rows: as queries, or as the database (an even number of tiles of each).
 int sketch_row_bytes(int64_t words);
-cudaError_t launch_sketch_tiles(const uint64_t *x, int64_t rows, int64_t words, int64_t tiles, uint8_t *out,
+int sketch_tile_rows(bool queries);
+cudaError_t launch_sketch_tiles(const uint64_t *x, int64_t rows, int64_t words, bool queries, int64_t tiles, uint8_t *out,
                                 cudaStream_t st, int *launches);
 
 // ---- plain FP32 GEMM-form scan (gemm_f32.cu) ----

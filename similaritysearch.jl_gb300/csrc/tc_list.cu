@@ -4,7 +4,7 @@
 // One scan for every operand form whose 128-query tile fits on chip beside a
 // ring of database K-blocks: BF16 and two-piece BF16 rows (64-byte K-blocks,
 // tc_bf16.cu), FP8 and wide BF16 rows (128-byte K-blocks, tc_stream.cu), and
-// bit sketches as +-1 FP8 rows (Hamming distance = (bits - dot) / 2, exact).
+// bit sketches as +-1 FP4 rows (Hamming distance = (bits - dot) / 2, exact).
 //
 // Why lists and a seeded bound.  A search over S splits fills 2 S heaps per
 // query, each from scratch: kk (1 + ln(rows / kk)) insertions per heap, and
@@ -42,18 +42,17 @@ namespace ssg {
 
 namespace {
 
-constexpr int TILE = 128;      // query rows per CTA, database rows per tile
-constexpr int WIDE = 2 * TILE;  // database rows per MMA: a tile of each CTA
-constexpr int NACC = 2;         // accumulators of 256 columns: all 512 TMEM columns
+constexpr int TILE = 128;  // query rows per CTA
+constexpr int NACC = 2;    // accumulators, of a wide tile's columns each
 constexpr int CS = kListSegs;   // epilogue warps per TMEM lane quarter, a list each
 constexpr int kThreads = 64 + CS * TILE;
 constexpr int kStageBytes = 32 * 1024;  // most of a ring stage
-constexpr int kLine = 2048;             // bytes of a tensor-map line
+constexpr int kLine = 1024;             // bytes of a tensor-map line
 constexpr int kMaxStages = 16;
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kAloneSmem = 120 * 1024;  // all 512 TMEM columns: alone on the SM
 constexpr int kCoefBytes = 4 * CS * 2 * (8 / CS) * 256;  // per warp two buffers of its columns' coefficients
-constexpr int kTileColumns = WIDE / CS;    // columns of a tile that one list can take
+constexpr int kTileColumns = 256 / CS;     // columns of a wide tile that one list can take
 constexpr int kBufCap = 12;                // raw candidates buffered per lane
 constexpr int kBufStride = CS * TILE * 8;  // bytes between a lane's buffer slots
 constexpr int kBufBytes = kBufCap * kBufStride;
@@ -149,6 +148,14 @@ __device__ __forceinline__ float rank_distance(float x, float bits) {
     return EPI == EPI_DOT ? -x : EPI == EPI_HAM ? (bits - x) * 0.5f : x;
 }
 
+// Operand kinds.  Sketches are +-1 in FP4 (e2m1, kind::mxf4 with every scale
+// factor 1): half the bytes and MMAs of FP8.  The scale factors take 32 TMEM
+// columns, so FP4's accumulators have 240 columns and its database tiles 120
+// rows; the others have 256 and 128.
+enum { BF16 = 0, FP8 = 1, FP4 = 2 };
+__host__ __device__ constexpr int db_rows(int kind) { return kind == FP4 ? 120 : 128; }
+constexpr uint32_t kScaleColumns = 480;  // TMEM column of A's scale factors (B's 16 on)
+
 // How a scan orders the database: evenly, as stored; or in a locality order
 // (positions with ids, each query tile from its own group on), in one split or
 // in several that share what their compactions find.  (Compiled apart: the
@@ -233,16 +240,17 @@ struct RowList {
 
     // the smallest distance of each four columns of a chunk; +inf where they
     // are no rows
-    __device__ __forceinline__ void chunk_min(const uint32_t (&r)[32], int64_t id0, const float4 *al, const float4 *be,
-                                              float (&g)[8]) const {
+    // (cols: the chunk's columns that are the tile's)
+    __device__ __forceinline__ void chunk_min(const uint32_t (&r)[32], int64_t id0, int cols, const float4 *al,
+                                              const float4 *be, float (&g)[8]) const {
         float dv[32];
         values(r, al, be, dv);
-        const bool rows = id0 + 32 <= n;
+        const bool rows = id0 + cols <= n;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const float *v = dv + 4 * i;
             const float b = raw_rank(EPI) ? fmaxf(fmax3(v[0], v[1], v[2]), v[3]) : fminf(fmin3(v[0], v[1], v[2]), v[3]);
-            g[i] = rows ? fminf(rank_distance<EPI>(b, bits), INFINITY) : INFINITY;  // (a NaN: +inf)
+            g[i] = rows && 4 * i < cols ? fminf(rank_distance<EPI>(b, bits), INFINITY) : INFINITY;  // (a NaN: +inf)
         }
     }
     __device__ __forceinline__ void drain() {
@@ -291,13 +299,14 @@ struct RowList {
     // MMAs: 2,048 queries x 1e6 rows x 96 dimensions took 691 us with the
     // keys appended at the sites, 497 through a function (its calls spilled
     // the accumulator's registers), 356 so.
-    __device__ __forceinline__ void chunk(const uint32_t (&r)[32], int64_t id0, const float4 *al, const float4 *be) {
+    __device__ __forceinline__ void chunk(const uint32_t (&r)[32], int64_t id0, int cols, const float4 *al,
+                                          const float4 *be) {
         float dv[32], g[4];
         values(r, al, be, dv);
 #pragma unroll
         for (int i = 0; i < 4; ++i) g[i] = best8(dv + 8 * i);
         if (!__any_sync(0xffffffffu, passes(best(best(g[0], g[1]), best(g[2], g[3]))))) return;
-        const int lim = !valid ? 0 : id0 + 32 <= n ? 32 : int(n - id0);  // columns that are rows
+        const int lim = !valid ? 0 : id0 + cols <= n ? cols : int(n - id0);  // columns that are rows
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             if (!__any_sync(0xffffffffu, passes(g[i]))) continue;
@@ -316,10 +325,13 @@ struct RowList {
 // QSTREAM: the query tile does not fit on chip; its K-blocks come through the
 // ring beside the database's (64 bytes per clock and SM at the full MMA rate,
 // half of what 128 x 128 tiles take).
-template <int SWB, bool F8, int EPI, bool SEED, int ORDER, bool QSTREAM>
+template <int SWB, int KIND, int EPI, bool SEED, int ORDER, bool QSTREAM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     tc_list_kernel(KernelArgs ka, const __grid_constant__ CUtensorMap dmap, const __grid_constant__ CUtensorMap qmap) {
-    constexpr int KBLK = TILE * SWB;   // bytes of a K-block of a tile
+    constexpr int HROWS = db_rows(KIND);  // database rows per tile
+    constexpr int WIDE = 2 * HROWS;       // and per MMA: a tile of each CTA
+    constexpr int KBLK = TILE * SWB;      // bytes of a K-block of a query tile
+    constexpr int DBLK = HROWS * SWB;     // and of a database tile
     constexpr int KSTEPS = SWB / 32;   // MMAs per K-block (32 bytes of K each)
     const ListScan &a = ka.s;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -327,8 +339,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int kblocks = ka.kblocks, stages = ka.stages, group = ka.group;
     const int groups_per_tile = kblocks / group;
     const size_t tile_bytes = size_t(kblocks) * KBLK;
-    const uint32_t part_bytes = uint32_t(group) * KBLK;  // of one operand
-    const uint32_t stage_bytes = (QSTREAM ? 2 : 1) * part_bytes;
+    const uint32_t part_bytes = uint32_t(group) * DBLK;
+    const uint32_t stage_bytes = (QSTREAM ? 2 : 1) * part_bytes;  // (QSTREAM: KBLK = DBLK)
     uint8_t *sA = smem;
     uint8_t *sB = sA + (QSTREAM ? 0 : tile_bytes);  // stages: database part, then the query part
     // per epilogue warp, two buffers of its 64 columns' coefficients
@@ -371,9 +383,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     if (warp == 1) tc::tmem_alloc_pair<512>(tmem_slot);
     tc::tc_fence_before();
     __syncthreads();
-    tc::cluster_sync();  // both CTAs' barriers exist before any cross-CTA arrive
     tc::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if constexpr (KIND == FP4) {
+        // every scale factor is 1 (UE8M0 127), so their layout does not matter
+        if (warp >= 2 && warp < 6) {
+            tc::tmem_st_32x32b_x32(tmem_base + (uint32_t(warp % 4 * 32) << 16) + kScaleColumns, 0x7f7f7f7fu);
+            tc::tmem_wait_st();
+        }
+        tc::tc_fence_before();
+        __syncthreads();
+    }
+    tc::cluster_sync();  // both CTAs' barriers (and scale factors) exist before any cross-CTA arrive
+    tc::tc_fence_after();
 
     // this split's wide tiles (places in the sample when SEED)
     const int64_t split_w = (ka.n_wide + a.splits - 1) / a.splits;
@@ -406,9 +428,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             uint32_t ph = 1;
             bool ok = true;
             for (int u = 0; ok && u < W; ++u) {
-                int line = (int(wide_tile(u)) * 2 + int(rank)) * kblocks * (KBLK / kLine);
+                int line = (int(wide_tile(u)) * 2 + int(rank)) * kblocks * (DBLK / kLine);
                 int qline = int(qx) * kblocks * (KBLK / kLine);
-                for (int g = 0; g < groups_per_tile; ++g, line += group * (KBLK / kLine)) {
+                for (int g = 0; g < groups_per_tile; ++g, line += group * (DBLK / kLine)) {
                     if (!tc::mbar_wait(&empty[s], ph, a.err, 21)) { ok = false; break; }
                     if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
                     uint8_t *dst = sB + size_t(s) * stage_bytes;
@@ -440,7 +462,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             if (!QSTREAM && tc::mbar_wait(a_full, 0, a.err, 28)) tc::mbar_arrive_cluster(tc::mapa_shared(tc::smem_u32(pa_full), peer));
         } else if (lane == 0) {
             // the even CTA issues the pair's MMAs
-            constexpr uint32_t idesc = F8 ? tc::idesc_e4m3_f32(2 * TILE, WIDE) : tc::idesc_bf16_f32(2 * TILE, WIDE);
+            constexpr uint32_t idesc = KIND == FP4   ? tc::idesc_mxf4_f32(2 * TILE, WIDE)
+                                       : KIND == FP8 ? tc::idesc_e4m3_f32(2 * TILE, WIDE)
+                                                     : tc::idesc_bf16_f32(2 * TILE, WIDE);
             bool ok = QSTREAM || (tc::mbar_wait(a_full, 0, a.err, 23) && tc::mbar_wait(pa_full, 0, a.err, 23));
             // descriptors address 16-byte units
             const uint64_t a_desc = tc::smem_desc(tc::smem_u32(sA), SWB);
@@ -460,12 +484,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     for (int kb = 0; kb < group; ++kb) {
 #pragma unroll
                         for (int k = 0; k < KSTEPS; ++k) {
-                            if (F8) tc::mma_f8_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, k ? 1u : acc);
+                            if (KIND == FP4)
+                                tc::mma_mxf4_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, tmem_base + kScaleColumns,
+                                                  tmem_base + kScaleColumns + 16, k ? 1u : acc);
+                            else if (KIND == FP8) tc::mma_f8_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, k ? 1u : acc);
                             else tc::mma_f16_pair(d_tmem, ad + 2 * k, bd + 2 * k, idesc, k ? 1u : acc);
                         }
                         acc = 1;
                         ad += KBLK >> 4;
-                        bd += KBLK >> 4;
+                        bd += DBLK >> 4;
                     }
                     tc::mma_commit_both(&empty[s]);
                     if (++s == stages) { s = 0; ph ^= 1; }
@@ -540,8 +567,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             for (int round = 0; round < CH / LDC; ++round) {
                 __syncwarp();
 #pragma unroll
-                for (int c = 0; c < LDC; ++c)
-                    tc::tmem_ld_32x32b_x32_async(tbase + uint32_t((round * LDC + c) * CS * 32), r[c]);
+                for (int c = 0; c < LDC; ++c) {
+                    const uint32_t from = tbase + uint32_t((round * LDC + c) * CS * 32);
+                    // (FP4's wide tile ends after 16 columns of the last chunk)
+                    if (KIND == FP4 && round * LDC + c == CH - 1 && cs == CS - 1) tc::tmem_ld_32x32b_x16_async(from, r[c]);
+                    else tc::tmem_ld_32x32b_x32_async(from, r[c]);
+                }
                 if constexpr (!raw_rank(EPI)) {
                     if (round == 0) {
                         if (u + 1 < W) fetch(u + 1, (u + 1) & 1);
@@ -559,9 +590,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 #pragma unroll
                 for (int c = 0; c < LDC; ++c) {
                     const int ch = round * LDC + c;
+                    const int col0 = (cs + ch * CS) * 32;
+                    const int cols = WIDE == 256 || col0 + 32 <= WIDE ? 32 : WIDE - col0;
                     if constexpr (SEED) {
                         float g[8];
-                        T.chunk_min(r[c], row0 + ch * CS * 32, al + ch * 8, al + CH * 8 + ch * 8, g);
+                        T.chunk_min(r[c], row0 + ch * CS * 32, cols, al + ch * 8, al + CH * 8 + ch * 8, g);
                         if ((ORDER != STORED || a.per_tile == 64) && T.valid) {
                             float4 *to = reinterpret_cast<float4 *>(a.minima + size_t(query) * a.groups + (w_lo + u) * 64 +
                                                                     (cs * CH + ch) * 8);
@@ -569,7 +602,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                             to[1] = make_float4(g[4], g[5], g[6], g[7]);
                         }
                         gm[ch] = fmin8(g);
-                    } else T.chunk(r[c], row0 + ch * CS * 32, al + ch * 8, al + CH * 8 + ch * 8);
+                    } else T.chunk(r[c], row0 + ch * CS * 32, cols, al + ch * 8, al + CH * 8 + ch * 8);
                 }
             }
             if (++b == NACC) { b = 0; ph ^= 1; }
@@ -654,37 +687,40 @@ __global__ void __launch_bounds__(128) seed_bound_kernel(const float *__restrict
     if (lane == 0) bound[q] = kk <= groups ? p : 0xffffffffu;
 }
 
-// Sketches -> +-1 FP8 (e4m3) tiles in the 128-byte K-block layout: bit 0 is
-// +1, bit 1 is -1, words past the sketch and rows past the end are zeros.
-// Thread = 16 bits = one 16-byte chunk.
-__global__ void sketch_tile_kernel(const uint64_t *__restrict__ x, int64_t rows, int words, int kblocks, int64_t tiles,
-                                   uint8_t *__restrict__ out) {
-    const int chunks = kblocks * 8;  // 16-bit chunks per padded row
-    const int64_t total = tiles * TILE * chunks;
+// Sketches -> +-1 FP4 (e2m1) tiles of tile_rows rows in the 128-byte K-block
+// layout: bit 0 is +1 (2), bit 1 is -1 (10), words past the sketch and rows past
+// the end are zeros.  Thread = 32 bits = one 16-byte chunk.
+__global__ void sketch_tile_kernel(const uint64_t *__restrict__ x, int64_t rows, int words, int kblocks, int tile_rows,
+                                   int64_t tiles, uint8_t *__restrict__ out) {
+    const int chunks = kblocks * 8;  // 32-bit chunks per padded row
+    const int64_t total = tiles * tile_rows * chunks;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
         const int ch = int(i % chunks);
         const int64_t row = i / chunks;
         uint32_t w[4] = {0, 0, 0, 0};
-        if (row < rows && ch < words * 4) {
-            const uint32_t bits = uint32_t(x[row * words + ch / 4] >> ((ch % 4) * 16)) & 0xffffu;
+        if (row < rows && ch < words * 2) {
+            const uint32_t bits = uint32_t(x[row * words + ch / 2] >> ((ch % 2) * 32));
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                // four bits spread to the bytes' sign bits
-                const uint32_t nib = (bits >> (4 * k)) & 0xfu;
-                w[k] = (((nib * 0x00204081u) & 0x01010101u) << 7) | 0x38383838u;
+                // eight bits spread to the nibbles' sign bits
+                uint32_t b = (bits >> (8 * k)) & 0xffu;
+                b = (b | (b << 12)) & 0x000f000fu;
+                b = (b | (b << 6)) & 0x03030303u;
+                b = (b | (b << 3)) & 0x11111111u;
+                w[k] = (b << 3) | 0x22222222u;
             }
         }
-        const int64_t tile = row / TILE;
-        const uint32_t off = tc::swizzled_offset(uint32_t(row % TILE), uint32_t((ch % 8) * 16), 128);
-        uint8_t *dst = out + (size_t(tile) * kblocks + ch / 8) * (TILE * 128) + off;
+        const int64_t tile = row / tile_rows;
+        const uint32_t off = tc::swizzled_offset(uint32_t(row % tile_rows), uint32_t((ch % 8) * 16), 128);
+        uint8_t *dst = out + (size_t(tile) * kblocks + ch / 8) * (tile_rows * 128) + off;
         *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
-// The database tiles as lines of 2 KB (256 eight-byte elements; the bytes are
+// The database tiles as lines of 1 KB (128 eight-byte elements; the bytes are
 // already swizzled, so a box is copied verbatim): a box is one tile's part of
 // a ring stage, a whole row's K-blocks where they fit.
-cudaError_t line_map(const ListScan &s, const uint8_t *base, int64_t rows, int kblocks, int group, CUtensorMap *map) {
+cudaError_t line_map(const uint8_t *base, int64_t bytes, int64_t box_bytes, CUtensorMap *map) {
     using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -698,10 +734,9 @@ cudaError_t line_map(const ListScan &s, const uint8_t *base, int64_t rows, int k
         encode = reinterpret_cast<EncodeFn>(fn);
     }
     if (reinterpret_cast<uintptr_t>(base) % 16 != 0) return cudaErrorInvalidValue;
-    const int64_t tiles = (rows + WIDE - 1) / WIDE * 2;
-    const cuuint64_t dims[2] = {cuuint64_t(kLine / 8), cuuint64_t(tiles) * kblocks * (TILE * s.swb / kLine)};
+    const cuuint64_t dims[2] = {cuuint64_t(kLine / 8), cuuint64_t(bytes / kLine)};
     const cuuint64_t strides[1] = {cuuint64_t(kLine)};
-    const cuuint32_t box[2] = {cuuint32_t(kLine / 8), cuuint32_t(group * (TILE * s.swb / kLine))};
+    const cuuint32_t box[2] = {cuuint32_t(kLine / 8), cuuint32_t(box_bytes / kLine)};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<uint8_t *>(base), dims, strides, box,
                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -727,11 +762,12 @@ struct Ring {
 };
 Ring list_ring(int row_bytes, int swb, int epi) {
     const int kblocks = row_bytes / swb;
+    const int rows = db_rows(epi == EPI_HAM ? FP4 : BF16);
     for (int qstream = 0; qstream < 2; ++qstream) {
         const int query_bytes = qstream ? 0 : TILE * row_bytes, parts = qstream ? 2 : 1;
         for (int g = std::min(kblocks, kStageBytes / (TILE * swb)); g >= 1; --g) {
             if (kblocks % g) continue;
-            const int stage = parts * g * TILE * swb;
+            const int stage = parts * g * rows * swb;
             int st = kMaxStages;
             while (st > 0 && list_smem(query_bytes, stage, st, epi) > kMaxSmem) --st;
             if (st >= 3 && st * g >= 4) return {g, st, qstream != 0, list_smem(query_bytes, stage, st, epi)};
@@ -740,55 +776,56 @@ Ring list_ring(int row_bytes, int swb, int epi) {
     return {1, 0, false, 0};
 }
 
-template <int SWB, bool F8, int EPI, bool SEED, int ORDER, bool QSTREAM>
+template <int SWB, int KIND, int EPI, bool SEED, int ORDER, bool QSTREAM>
 cudaError_t launch_list_q(const ListScan &s, const Ring &ring, cudaStream_t st) {
     KernelArgs ka;
     ka.s = s;
     ka.kblocks = s.row_bytes / SWB;
     ka.group = ring.group;
     ka.stages = ring.stages;
-    ka.all_wide = (s.n + WIDE - 1) / WIDE;
+    constexpr int rows = db_rows(KIND);
+    ka.all_wide = (s.n + 2 * rows - 1) / (2 * rows);
     ka.n_wide = SEED ? s.samples : ka.all_wide;
     const size_t smem = std::max(ring.smem, kAloneSmem);
-    auto kern = tc_list_kernel<SWB, F8, EPI, SEED, ORDER, QSTREAM>;
+    auto kern = tc_list_kernel<SWB, KIND, EPI, SEED, ORDER, QSTREAM>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     CUtensorMap dmap, qmap;
-    e = line_map(s, s.dt, s.n, ka.kblocks, ka.group, &dmap);
-    if (e == cudaSuccess) e = line_map(s, s.qt, s.m, ka.kblocks, ka.group, &qmap);
-    if (e != cudaSuccess) return e;
     const int64_t qtiles = ((s.m + TILE - 1) / TILE + 1) / 2 * 2;
+    e = line_map(s.dt, ka.all_wide * 2 * rows * s.row_bytes, int64_t(ka.group) * rows * SWB, &dmap);
+    if (e == cudaSuccess) e = line_map(s.qt, qtiles * TILE * s.row_bytes, int64_t(ka.group) * TILE * SWB, &qmap);
+    if (e != cudaSuccess) return e;
     kern<<<dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st>>>(ka, dmap, qmap);
     return cudaGetLastError();
 }
 
-template <int SWB, bool F8, int EPI, bool SEED, int ORDER = STORED>
+template <int SWB, int KIND, int EPI, bool SEED, int ORDER = STORED>
 cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
     const Ring ring = list_ring(s.row_bytes, SWB, EPI);
     if (ring.stages == 0) return cudaErrorInvalidValue;
     if constexpr (EPI == EPI_AFF) {
-        if (ring.qstream) return launch_list_q<SWB, F8, EPI, SEED, ORDER, true>(s, ring, st);
+        if (ring.qstream) return launch_list_q<SWB, KIND, EPI, SEED, ORDER, true>(s, ring, st);
     }
     if (ring.qstream) return cudaErrorInvalidValue;
-    return launch_list_q<SWB, F8, EPI, SEED, ORDER, false>(s, ring, st);
+    return launch_list_q<SWB, KIND, EPI, SEED, ORDER, false>(s, ring, st);
 }
 
 // BF16 tiles with 64-byte K-blocks, the form that allknn orders.
 template <int EPI, bool SEED>
 cudaError_t launch_list_order(const ListScan &s, cudaStream_t st) {
-    if (!s.perm) return launch_list_t<64, false, EPI, SEED>(s, st);
-    if (SEED || s.splits == 1) return launch_list_t<64, false, EPI, SEED, LOCAL>(s, st);
-    return launch_list_t<64, false, EPI, SEED, LOCAL_SHARED>(s, st);
+    if (!s.perm) return launch_list_t<64, BF16, EPI, SEED>(s, st);
+    if (SEED || s.splits == 1) return launch_list_t<64, BF16, EPI, SEED, LOCAL>(s, st);
+    return launch_list_t<64, BF16, EPI, SEED, LOCAL_SHARED>(s, st);
 }
 
 template <bool SEED>
 cudaError_t launch_list_any(const ListScan &s, cudaStream_t st) {
-    if (s.swb == 128 && s.fp8) {
-        if (s.epi == LIST_HAMMING) return launch_list_t<128, true, EPI_HAM, SEED>(s, st);
-        if (s.epi == LIST_AFFINE) return launch_list_t<128, true, EPI_AFF, SEED>(s, st);
-        return cudaErrorInvalidValue;
+    if (s.epi == LIST_HAMMING)
+        return s.swb == 128 ? launch_list_t<128, FP4, EPI_HAM, SEED>(s, st) : cudaErrorInvalidValue;
+    if (s.swb == 128) {
+        if (s.epi != LIST_AFFINE) return cudaErrorInvalidValue;
+        return s.fp8 ? launch_list_t<128, FP8, EPI_AFF, SEED>(s, st) : launch_list_t<128, BF16, EPI_AFF, SEED>(s, st);
     }
-    if (s.swb == 128) return s.epi == LIST_AFFINE ? launch_list_t<128, false, EPI_AFF, SEED>(s, st) : cudaErrorInvalidValue;
     switch (s.epi) {
         case LIST_DOT: return launch_list_order<EPI_DOT, SEED>(s, st);
         case LIST_SQ: return launch_list_order<EPI_SQ, SEED>(s, st);
@@ -804,7 +841,7 @@ cudaError_t launch_list_any(const ListScan &s, cudaStream_t st) {
 bool list_fits(int row_bytes, int swb, int epi, int64_t n) {
     const Ring ring = list_ring(row_bytes, swb, epi);
     return ring.stages > 0 && (!ring.qstream || epi == LIST_AFFINE) &&
-           (n / TILE + 2) * (row_bytes / swb) * (TILE * swb / kLine) < (int64_t(1) << 31);
+           (n + 512) * row_bytes / kLine < (int64_t(1) << 31);
 }
 
 cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches) {
@@ -826,15 +863,17 @@ cudaError_t launch_list_scan(const ListScan &s, cudaStream_t st, int *launches) 
     return launch_list_any<false>(s, st);
 }
 
-int sketch_row_bytes(int64_t words) { return int((words + 1) / 2 * 128); }
+int sketch_row_bytes(int64_t words) { return int((words + 3) / 4 * 128); }
+int sketch_tile_rows(bool queries) { return queries ? TILE : db_rows(FP4); }
 
-cudaError_t launch_sketch_tiles(const uint64_t *x, int64_t rows, int64_t words, int64_t tiles, uint8_t *out,
+cudaError_t launch_sketch_tiles(const uint64_t *x, int64_t rows, int64_t words, bool queries, int64_t tiles, uint8_t *out,
                                 cudaStream_t st, int *launches) {
-    const int kblocks = sketch_row_bytes(words) / 128;
-    const int64_t total = tiles * TILE * kblocks * 8;
+    const int kblocks = sketch_row_bytes(words) / 128, tile_rows = sketch_tile_rows(queries);
+    const int64_t total = tiles * tile_rows * kblocks * 8;
     const int64_t blocks = std::min<int64_t>((total + 255) / 256, 152 * 64);
     if (launches) *launches += 1;
-    sketch_tile_kernel<<<unsigned(std::max<int64_t>(1, blocks)), 256, 0, st>>>(x, rows, int(words), kblocks, tiles, out);
+    sketch_tile_kernel<<<unsigned(std::max<int64_t>(1, blocks)), 256, 0, st>>>(x, rows, int(words), kblocks, tile_rows,
+                                                                               tiles, out);
     return cudaGetLastError();
 }
 

@@ -173,6 +173,19 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32_async(uint32_t taddr, uint32_
         : "memory");
 }
 
+// The same for 16 columns (r[16..31] are zeroed).
+__device__ __forceinline__ void tmem_ld_32x32b_x16_async(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+#pragma unroll
+    for (int i = 16; i < 32; ++i) r[i] = 0;
+}
+
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // Shared-memory matrix descriptor (tcgen05 format) for a K-major operand
@@ -205,6 +218,16 @@ __host__ __device__ constexpr uint32_t idesc_e4m3_f32(int M, int N) {
     return (1u << 4)                      // D format: F32
            | (uint32_t(N >> 3) << 17)     // N >> 3
            | (uint32_t(M >> 4) << 24);    // M >> 4
+}
+
+// Instruction descriptor: kind::mxf4 with E2M1 A/B (format code 1), UE8M0
+// scale factors (data id 0 of both), FP32 accumulator, K = 64, shape M x N.
+__host__ __device__ constexpr uint32_t idesc_mxf4_f32(int M, int N) {
+    return (1u << 7)                      // A format: E2M1
+           | (1u << 10)                   // B format: E2M1
+           | (uint32_t(N >> 3) << 17)     // N >> 3
+           | (1u << 23)                   // scale factors: UE8M0
+           | (uint32_t(M >> 7) << 27);    // M >> 7
 }
 
 // Byte offset of the 16-byte chunk holding (row r, byte b) inside a K-block
@@ -323,6 +346,30 @@ __device__ __forceinline__ void mma_f8_pair(uint32_t d_tmem, uint64_t a_desc, ui
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+
+// The same for kind::mxf4: packed FP4 (e2m1) operands, K = 64, a scale factor
+// per 32 elements from TMEM (UE8M0).
+__device__ __forceinline__ void mma_mxf4_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                              uint32_t scale_a, uint32_t scale_b, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.scale_vec::2X [%0], %1, %2, %3, [%5], [%6], p;\n\t}" ::"r"(
+            d_tmem),
+        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(scale_a), "r"(scale_b)
+        : "memory");
+}
+
+// Writes v to 32 consecutive columns of this warp's 32 TMEM lanes.
+__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, uint32_t v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
+        "%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr),
+        "r"(v)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // Arrives once on the mbarrier at this offset in both CTAs of the pair when
 // the pair MMAs this thread issued so far have completed.
