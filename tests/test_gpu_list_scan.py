@@ -94,7 +94,7 @@ def test_reduced_keys_do_not_depend_on_splits(ss, prec, dim, m, splits):
 
 
 @pytest.mark.parametrize("metric,dim,k,splits", [("sql2", 24, 10, 0), ("normcosine", 96, 32, 1), ("cosine", 40, 5, 3)])
-@pytest.mark.parametrize("n,per", [(33_000, 40), (40_961, 700)])
+@pytest.mark.parametrize("n,per", [(66_000, 40), (70_033, 700)])
 def test_allknn_locality(ss, metric, dim, k, splits, n, per):
     """allknn in the locality order (clusters smaller and larger than a pivot's
     group, so bounds from the neighbourhood miss or hit) equals the oracle on
