@@ -38,7 +38,7 @@ namespace {
 constexpr int BM = 128;          // rows per tile (TMEM lanes)
 constexpr int BK = 64;           // K elements per K-block: one 128-byte BF16 row
 constexpr int SWB = 128;         // swizzle bytes
-constexpr int GT = 128;          // threads per CTA (4 warps: one TMEM lane quarter each)
+constexpr int GT = 256;          // threads per CTA (two warps per TMEM lane quarter)
 
 template <int BN, bool EXACT>
 struct GemmSmem {
@@ -65,44 +65,47 @@ struct Staged {
     float v[CPT][8];
 };
 
-template <int R>
-__device__ __forceinline__ void load_operand(Staged<R> &t, const float *__restrict__ X, int64_t ld, int kmajor, int r0,
-                                             int rlim, int k0, int klim, bool vec4) {
+template <int R, bool KMAJOR>
+__device__ __forceinline__ void load_operand(Staged<R> &t, const float *__restrict__ X, int64_t ld, int r0, int rlim,
+                                             int k0, int klim, bool vec4) {
+    if (r0 + R <= rlim && k0 + BK <= klim && (vec4 || !KMAJOR)) {
+        // a whole tile: nothing to test per element
+#pragma unroll
+        for (int i = 0; i < Staged<R>::CPT; ++i) {
+            const int c = int(threadIdx.x) + i * GT;
+            float *v = t.v[i];
+            if (KMAJOR) {
+                const float *p = X + int64_t(r0 + c / (BK / 8)) * ld + k0 + c % (BK / 8) * 8;
+                const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
+                const float4 b = __ldg(reinterpret_cast<const float4 *>(p + 4));
+                v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+            } else {
+                const float *p = X + int64_t(k0 + c / R * 8) * ld + r0 + c % R;  // consecutive threads: consecutive rows
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = __ldg(p + j * ld);
+            }
+        }
+        return;
+    }
 #pragma unroll
     for (int i = 0; i < Staged<R>::CPT; ++i) {
         const int c = int(threadIdx.x) + i * GT;
-        int r, kc;
-        if (kmajor) { r = c / (BK / 8); kc = c % (BK / 8); }
-        else { kc = c / R; r = c % R; }  // consecutive threads: consecutive rows (coalesced)
+        const int r = KMAJOR ? c / (BK / 8) : c % R, kc = KMAJOR ? c % (BK / 8) : c / R;
         const int gr = r0 + r, gk = k0 + kc * 8;
         float *v = t.v[i];
-        if (gr < rlim && kmajor && vec4 && gk + 8 <= klim) {
-            const float *p = X + int64_t(gr) * ld + gk;
-            const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-            const float4 b = __ldg(reinterpret_cast<const float4 *>(p + 4));
-            v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-        } else if (gr < rlim && kmajor) {
-            const float *p = X + int64_t(gr) * ld + gk;
+        const float *p = KMAJOR ? X + int64_t(gr) * ld + gk : X + int64_t(gk) * ld + gr;
+        const int64_t step = KMAJOR ? 1 : ld;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = gk + j < klim ? __ldg(p + j) : 0.0f;
-        } else if (gr < rlim) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = gk + j < klim ? __ldg(X + int64_t(gk + j) * ld + gr) : 0.0f;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = 0.0f;
-        }
+        for (int j = 0; j < 8; ++j) v[j] = gr < rlim && gk + j < klim ? __ldg(p + j * step) : 0.0f;
     }
 }
 
-template <int R, bool EXACT>
-__device__ __forceinline__ void store_operand(const Staged<R> &t, int kmajor, uint8_t *hi, int piece) {
+template <int R, bool KMAJOR, bool EXACT>
+__device__ __forceinline__ void store_operand(const Staged<R> &t, uint8_t *hi, int piece) {
 #pragma unroll
     for (int i = 0; i < Staged<R>::CPT; ++i) {
         const int c = int(threadIdx.x) + i * GT;
-        int r, kc;
-        if (kmajor) { r = c / (BK / 8); kc = c % (BK / 8); }
-        else { kc = c / R; r = c % R; }
+        const int r = KMAJOR ? c / (BK / 8) : c % R, kc = KMAJOR ? c % (BK / 8) : c / R;
         const float *v = t.v[i];
         __align__(16) __nv_bfloat16 h[8];
         __align__(16) __nv_bfloat16 md[8];
@@ -125,8 +128,8 @@ __device__ __forceinline__ void store_operand(const Staged<R> &t, int kmajor, ui
     }
 }
 
-template <int BN, bool EXACT>
-__global__ void __launch_bounds__(GT, 1) mlp_gemm_kernel(MlpGemm g, int vec_a, int vec_b) {
+template <int BN, bool EXACT, bool AK, bool BKM>
+__global__ void __launch_bounds__(GT, EXACT ? 1 : 2) mlp_gemm_kernel(MlpGemm g, int vec_a, int vec_b) {
     using S = GemmSmem<BN, EXACT>;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -167,10 +170,10 @@ __global__ void __launch_bounds__(GT, 1) mlp_gemm_kernel(MlpGemm g, int vec_a, i
         {
             Staged<BM> ta;
             Staged<BN> tb;
-            load_operand<BM>(ta, g.A, g.lda, g.a_kmajor, m0, g.M, k0, kend, vec_a != 0);
-            load_operand<BN>(tb, g.B, g.ldb, g.b_kmajor, n0, g.N, k0, kend, vec_b != 0);
-            store_operand<BM, EXACT>(ta, g.a_kmajor, a_hi, S::a_bytes);
-            store_operand<BN, EXACT>(tb, g.b_kmajor, b_hi, S::b_bytes);
+            load_operand<BM, AK>(ta, g.A, g.lda, m0, g.M, k0, kend, vec_a != 0);
+            load_operand<BN, BKM>(tb, g.B, g.ldb, n0, g.N, k0, kend, vec_b != 0);
+            store_operand<BM, AK, EXACT>(ta, a_hi, S::a_bytes);
+            store_operand<BN, BKM, EXACT>(tb, b_hi, S::b_bytes);
         }
         fence_proxy_async();  // generic-proxy stores -> visible to the tensor core
         __syncthreads();
@@ -209,12 +212,39 @@ __global__ void __launch_bounds__(GT, 1) mlp_gemm_kernel(MlpGemm g, int vec_a, i
     // columns of one row; the bias, ReLU, mask and column sums are applied in
     // that pass, where each lane owns one column.
     float *tile = reinterpret_cast<float *>(smem) + warp * (32 * 33);
+    const int quarter = warp % 4, row0 = m0 + quarter * 32;
+    const bool plain = !g.bias && !g.relu && !g.mask && !g.colsum;
     float *C = g.C + size_t(blockIdx.z) * size_t(g.M) * size_t(g.ldc);
-    for (int c = 0; c < BN / 32; ++c) {
+    for (int c = warp / 4; c < BN / 32; c += GT / 128) {
+        const int n = n0 + c * 32 + lane;
+        const bool nvalid = n < g.N;
+        const float b = (g.bias && nvalid) ? g.bias[n] : 0.0f;
+        if (plain && row0 + 32 <= g.M && n0 + c * 32 + 32 <= g.N && nkb > 0 && ok) {
+            // a whole block of a split product: nothing but the turn
+            float v[32];
+            __syncwarp();
+            tc::tmem_ld_32x32b_x32(tmem + (uint32_t(quarter * 32) << 16) + uint32_t(c * 32), v);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = v[j];
+            __syncwarp();
+            float *dst = C + int64_t(row0) * g.ldc + n;
+#pragma unroll
+            for (int r = 0; r < 32; ++r) dst[r * g.ldc] = tile[r * 33 + lane];
+            __syncwarp();
+            continue;
+        }
+        // the mask values first (independent loads in flight together, over
+        // the accumulator's way through shared memory)
+        float mk[32];
+#pragma unroll
+        for (int r = 0; r < 32; ++r) {
+            const int row = row0 + r;
+            mk[r] = (g.mask && nvalid && row < g.M) ? __ldg(g.mask + int64_t(row) * g.ldc + n) : 1.0f;
+        }
         float v[32];
         if (nkb > 0 && ok) {
             __syncwarp();
-            tc::tmem_ld_32x32b_x32(tmem + (uint32_t(warp * 32) << 16) + uint32_t(c * 32), v);
+            tc::tmem_ld_32x32b_x32(tmem + (uint32_t(quarter * 32) << 16) + uint32_t(c * 32), v);
         } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = 0.0f;
@@ -222,20 +252,10 @@ __global__ void __launch_bounds__(GT, 1) mlp_gemm_kernel(MlpGemm g, int vec_a, i
 #pragma unroll
         for (int j = 0; j < 32; ++j) tile[lane * 33 + j] = v[j];  // row = lane
         __syncwarp();
-        const int n = n0 + c * 32 + lane;
-        const bool nvalid = n < g.N;
-        const float b = (g.bias && nvalid) ? g.bias[n] : 0.0f;
-        // the mask values first (independent loads in flight together)
-        float mk[32];
-#pragma unroll
-        for (int r = 0; r < 32; ++r) {
-            const int row = m0 + warp * 32 + r;
-            mk[r] = (g.mask && nvalid && row < g.M) ? __ldg(g.mask + int64_t(row) * g.ldc + n) : 1.0f;
-        }
         float csum = 0.0f;
 #pragma unroll
         for (int r = 0; r < 32; ++r) {
-            const int row = m0 + warp * 32 + r;
+            const int row = row0 + r;
             const bool valid = nvalid && row < g.M;
             float x = tile[r * 33 + lane] + b;
             if (g.relu) x = fmaxf(x, 0.0f);
@@ -245,7 +265,7 @@ __global__ void __launch_bounds__(GT, 1) mlp_gemm_kernel(MlpGemm g, int vec_a, i
                 csum += x;
             }
         }
-        if (g.colsum) red[warp * BN + c * 32 + lane] = csum;
+        if (g.colsum) red[quarter * BN + c * 32 + lane] = csum;
         __syncwarp();
     }
     if (g.colsum) {
@@ -262,15 +282,25 @@ __global__ void __launch_bounds__(GT, 1) mlp_gemm_kernel(MlpGemm g, int vec_a, i
     }
 }
 
-template <int BN, bool EXACT>
-cudaError_t launch_gemm_t(const MlpGemm &g, int vec_a, int vec_b, cudaStream_t st) {
+template <int BN, bool EXACT, bool AK, bool BKM>
+cudaError_t launch_gemm_k(const MlpGemm &g, int vec_a, int vec_b, cudaStream_t st) {
     const size_t smem = GemmSmem<BN, EXACT>::total;
-    auto kern = mlp_gemm_kernel<BN, EXACT>;
+    auto kern = mlp_gemm_kernel<BN, EXACT, AK, BKM>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     dim3 grid(unsigned((g.M + BM - 1) / BM), unsigned((g.N + BN - 1) / BN), unsigned(g.splits));
     kern<<<grid, GT, smem, st>>>(g, vec_a, vec_b);
     return cudaGetLastError();
+}
+
+// The layouts of the three products: forward (both K-major), the hidden
+// gradient (B transposed), the weight gradients (both transposed).
+template <int BN, bool EXACT>
+cudaError_t launch_gemm_t(const MlpGemm &g, int vec_a, int vec_b, cudaStream_t st) {
+    if (g.a_kmajor && g.b_kmajor) return launch_gemm_k<BN, EXACT, true, true>(g, vec_a, vec_b, st);
+    if (g.a_kmajor) return launch_gemm_k<BN, EXACT, true, false>(g, vec_a, vec_b, st);
+    if (!g.b_kmajor) return launch_gemm_k<BN, EXACT, false, false>(g, vec_a, vec_b, st);
+    return cudaErrorInvalidValue;
 }
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -445,7 +475,11 @@ cudaError_t mlp_gemm(const MlpGemm &g, cudaStream_t st, int *launches) {
     const int vec_a = g.a_kmajor && g.lda % 4 == 0 && aligned16(g.A);
     const int vec_b = g.b_kmajor && g.ldb % 4 == 0 && aligned16(g.B);
     if (launches) *launches += 1;
-    if (g.N <= 64) return g.exact ? launch_gemm_t<64, true>(g, vec_a, vec_b, st) : launch_gemm_t<64, false>(g, vec_a, vec_b, st);
+    int bn = g.N <= 64 ? 64 : 128;
+    const int mt = mlp_gemm_mtiles(g.M);
+    while (bn > 32 && mt * ((g.N + bn - 1) / bn) * g.splits < device_sm_count()) bn /= 2;
+    if (bn == 32) return g.exact ? launch_gemm_t<32, true>(g, vec_a, vec_b, st) : launch_gemm_t<32, false>(g, vec_a, vec_b, st);
+    if (bn == 64) return g.exact ? launch_gemm_t<64, true>(g, vec_a, vec_b, st) : launch_gemm_t<64, false>(g, vec_a, vec_b, st);
     return g.exact ? launch_gemm_t<128, true>(g, vec_a, vec_b, st) : launch_gemm_t<128, false>(g, vec_a, vec_b, st);
 }
 

@@ -14,71 +14,6 @@
 
 namespace ssg {
 
-namespace {
-
-template <int METRIC>
-__global__ void rerank_kernel(const void *db, const float *xn, int64_t dim, const void *q,
-                              const float *qn, int len, int P, uint32_t *ids, float *dists) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint64_t *s = reinterpret_cast<uint64_t *>(smem);
-    __shared__ int valid;
-    const int64_t j = blockIdx.x;
-    uint32_t *rid = ids + j * len;
-    float *rd = dists + j * len;
-    if (threadIdx.x == 0) {
-        int v = 0;
-        while (v < len && rid[v] != 0) ++v;
-        valid = v;
-    }
-    __syncthreads();
-    const int nv = valid;
-    for (int i = threadIdx.x; i < P; i += blockDim.x) {
-        if (i < nv) {
-            const uint32_t id = rid[i];
-            const float d = exact_pair<METRIC>(db, int64_t(id) - 1, dim, q, j, xn, qn);
-            s[i] = make_key(d, id - 1);
-        } else {
-            s[i] = KEY_EMPTY;
-        }
-    }
-    block_bitonic_sort(s, P);
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-        rid[i] = key_id0(s[i]) + 1;
-        rd[i] = key_dist(s[i]);
-    }
-}
-
-}  // namespace
-
-cudaError_t launch_rerank(int metric, const void *db, const float *db_norm, int64_t dim,
-                          const void *q, const float *q_norm, int64_t m, int len,
-                          uint32_t *ids, float *dists, cudaStream_t st, int *launches) {
-    if (m <= 0 || len <= 0) return cudaSuccess;
-    const int P = next_pow2(len);
-    const size_t smem = size_t(P) * 8;
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
-    if (launches) *launches += 1;
-#define SSG_RR(MET)                                                                               \
-    case MET: {                                                                                   \
-        cudaError_t e = cudaFuncSetAttribute(rerank_kernel<MET>,                                  \
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)); \
-        if (e != cudaSuccess) return e;                                                           \
-        rerank_kernel<MET><<<unsigned(m), 128, smem, st>>>(db, db_norm, dim, q, q_norm, len, P,   \
-                                                           ids, dists);                            \
-        return cudaGetLastError();                                                                \
-    }
-    switch (metric) {
-        SSG_RR(SQL2)
-        SSG_RR(L2)
-        SSG_RR(NORMCOSINE)
-        SSG_RR(COSINE)
-        SSG_RR(IP)
-        SSG_RR(HAMMING)
-        default: return cudaErrorInvalidValue;
-    }
-#undef SSG_RR
-}
-
 // ---------------------------------------------------------------------------
 // Finalize: select a query's best keys among its candidate segments, re-rank
 // them with the exact FP32 distance (RERANK) and write the k best in
@@ -112,6 +47,17 @@ constexpr int kWarpStages = 3;
 constexpr int kBlockThreads = 256;
 constexpr int kBlockRows = 128;            // candidates staged together in the block shape
 constexpr int kBlockStages = 4;
+
+// Length of a candidate row: the ids before its first 0 (by a block).
+__device__ __forceinline__ int valid_prefix(const uint32_t *rid, int len) {
+    __shared__ int valid;
+    if (threadIdx.x == 0) valid = len;
+    __syncthreads();
+    for (int i = threadIdx.x; i < len; i += blockDim.x)
+        if (rid[i] == 0) atomicMin(&valid, i);
+    __syncthreads();
+    return valid;
+}
 
 struct RowSource {
     const float *db, *q;  // database rows, this query's row
@@ -506,6 +452,48 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
     }
 }
 
+// Exact keys out[i] of the rows key_id0(sel[i]), i < nv, by a block: up to
+// kBlockRows rows at a time stream through the ring (rows_s of kRowStride
+// floats per stage: the rows and, behind them, the query), one thread per row
+// and chain.  *q_sq (not null): the query's own squares.  Ends with a barrier.
+template <int METRIC>
+__device__ __forceinline__ void block_distances(const RowSource &rs, const uint64_t *sel, int nv, uint64_t *out,
+                                                float *ring, int rows_s, const float *db_norm, float qn, float *q_sq) {
+    const int tid = threadIdx.x;
+    const int steps = (rs.dim + kDimStep - 1) / kDimStep;
+    for (int r0 = 0; r0 < nv || r0 == 0; r0 += kBlockRows) {
+        const int rows = min(kBlockRows, nv - r0);
+        float acc = 0.0f;
+        const float qs = tid == rows ? 0.0f : 1.0f;
+#pragma unroll
+        for (int p = 0; p < kBlockStages - 1; ++p) {
+            if (p < steps)
+                stage_rows(rs, sel + r0, rows, p * kDimStep, ring + size_t(p) * rows_s * kRowStride, tid,
+                           kBlockThreads);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+        for (int c = 0; c < steps; ++c) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kBlockStages - 2) : "memory");
+            __syncthreads();
+            const int nx = c + kBlockStages - 1;
+            if (nx < steps)
+                stage_rows(rs, sel + r0, rows, nx * kDimStep, ring + size_t(nx % kBlockStages) * rows_s * kRowStride,
+                           tid, kBlockThreads);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            const float *buf = ring + size_t(c % kBlockStages) * rows_s * kRowStride;
+            if (tid <= rows)
+                acc = chain_step<METRIC>(acc, buf + tid * kRowStride, buf + rows * kRowStride,
+                                         min(kDimStep, rs.dim - c * kDimStep), qs);
+        }
+        if (tid < rows) {
+            const uint32_t id0 = key_id0(sel[r0 + tid]);
+            out[r0 + tid] = make_key(chain_distance<METRIC>(acc, id0, db_norm, qn), id0);
+        }
+        if (r0 == 0 && tid == rows && q_sq) *q_sq = acc;  // the query's row: |q|^2
+        __syncthreads();  // the ring is refilled
+    }
+}
+
 // A block per query.  cap: room for keys in shared memory (every key of the
 // query's segments; of lists with more than that, only keys below a limit
 // found by counting are taken); sel_cap: room for the selected ones (0: they take the keys' place,
@@ -671,40 +659,8 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
             if (tid == 0 && s_last < s_low) s_low = s_last;
         }
         const RowSource rs{db, q + size_t(jr) * dim, int(dim), vec != 0};
-        const int steps = (int(dim) + kDimStep - 1) / kDimStep;
-        const float qn = METRIC == COSINE ? q_norm[jr] : 0.0f;
-        const int rows_s = min(need, kBlockRows) + 1;
-        for (int r0 = 0; r0 < nv || r0 == 0; r0 += kBlockRows) {
-            const int rows = min(kBlockRows, nv - r0);
-            float acc = 0.0f;
-            const float qs = tid == rows ? 0.0f : 1.0f;
-#pragma unroll
-            for (int p = 0; p < kBlockStages - 1; ++p) {
-                if (p < steps)
-                    stage_rows(rs, sel + r0, rows, p * kDimStep, ring + size_t(p) * rows_s * kRowStride, tid,
-                               kBlockThreads);
-                asm volatile("cp.async.commit_group;" ::: "memory");
-            }
-            for (int c = 0; c < steps; ++c) {
-                asm volatile("cp.async.wait_group %0;" ::"n"(kBlockStages - 2) : "memory");
-                __syncthreads();
-                const int nx = c + kBlockStages - 1;
-                if (nx < steps)
-                    stage_rows(rs, sel + r0, rows, nx * kDimStep,
-                               ring + size_t(nx % kBlockStages) * rows_s * kRowStride, tid, kBlockThreads);
-                asm volatile("cp.async.commit_group;" ::: "memory");
-                const float *buf = ring + size_t(c % kBlockStages) * rows_s * kRowStride;
-                if (tid <= rows)
-                    acc = chain_step<METRIC>(acc, buf + tid * kRowStride, buf + rows * kRowStride,
-                                             min(kDimStep, int(dim) - c * kDimStep), qs);
-            }
-            if (tid < rows) {
-                const uint32_t id0 = key_id0(sel[r0 + tid]);
-                out[r0 + tid] = make_key(chain_distance<METRIC>(acc, id0, db_norm, qn), id0);
-            }
-            if (r0 == 0 && tid == rows) s_qsq = acc;  // the query's row: |q|^2
-            __syncthreads();  // the ring is refilled
-        }
+        block_distances<METRIC>(rs, sel, nv, out, ring, min(need, kBlockRows) + 1, db_norm,
+                                METRIC == COSINE ? q_norm[jr] : 0.0f, &s_qsq);
         uint64_t *t = sel;
         sel = out;
         out = t;
@@ -799,6 +755,95 @@ cudaError_t launch_finalize_rerank(int metric, const FinalizeArgs &f, const floa
         case NORMCOSINE: return launch_finalize_t<NORMCOSINE, true>(f, db, db_norm, dim, q, q_norm, rr, st);
         case COSINE: return launch_finalize_t<COSINE, true>(f, db, db_norm, dim, q, q_norm, rr, st);
         case IP: return launch_finalize_t<IP, true>(f, db, db_norm, dim, q, q_norm, rr, st);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+namespace {
+
+// Sketches are two words or so long: a thread per candidate.
+__global__ void rerank_sketches_kernel(const void *db, int64_t dim, const void *q, int len, int P, uint32_t *ids,
+                                       float *dists) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint64_t *s = reinterpret_cast<uint64_t *>(smem);
+    const int64_t j = blockIdx.x;
+    uint32_t *rid = ids + j * len;
+    float *rd = dists + j * len;
+    const int nv = valid_prefix(rid, len);
+    for (int i = threadIdx.x; i < P; i += blockDim.x) {
+        s[i] = KEY_EMPTY;
+        if (i < nv) s[i] = make_key(exact_pair<HAMMING>(db, int64_t(rid[i]) - 1, dim, q, j, nullptr, nullptr), rid[i] - 1);
+    }
+    block_bitonic_sort(s, P);
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+        rid[i] = key_id0(s[i]) + 1;
+        rd[i] = key_dist(s[i]);
+    }
+}
+
+// Rows of floats: staged through shared memory as the finalize's are, not
+// read by the thread that walks the chain (32 lanes on 32 rows used one
+// sector in 32 loads).  What bounds it: the gather of m * len rows.
+template <int METRIC>
+__global__ void __launch_bounds__(kBlockThreads)
+rerank_rows_kernel(const float *__restrict__ db, const float *__restrict__ db_norm, int64_t dim,
+                   const float *__restrict__ q, const float *__restrict__ q_norm, int len, int P, uint32_t *ids,
+                   float *dists, int vec) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    uint64_t *s = reinterpret_cast<uint64_t *>(smem);
+    float *ring = reinterpret_cast<float *>(s + P);
+    const int64_t j = blockIdx.x;
+    uint32_t *rid = ids + j * len;
+    float *rd = dists + j * len;
+    const int nv = valid_prefix(rid, len);
+    if (nv == 0) return;
+    for (int i = threadIdx.x; i < P; i += blockDim.x) s[i] = i < nv ? uint64_t(rid[i] - 1) : KEY_EMPTY;
+    __syncthreads();
+    const RowSource rs{db, q + size_t(j) * dim, int(dim), vec != 0};
+    block_distances<METRIC>(rs, s, nv, s, ring, min(len, kBlockRows) + 1, db_norm, METRIC == COSINE ? q_norm[j] : 0.0f,
+                            nullptr);
+    block_bitonic_sort(s, P);
+    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
+        rid[i] = key_id0(s[i]) + 1;
+        rd[i] = key_dist(s[i]);
+    }
+}
+
+template <int METRIC>
+cudaError_t launch_rerank_rows(const float *db, const float *db_norm, int64_t dim, const float *q, const float *q_norm,
+                               int64_t m, int len, int P, uint32_t *ids, float *dists, cudaStream_t st) {
+    const bool vec = dim % 4 == 0 && ((reinterpret_cast<uintptr_t>(db) | reinterpret_cast<uintptr_t>(q)) & 15) == 0;
+    const size_t smem = size_t(P) * 8 + size_t(kBlockStages) * (std::min(len, kBlockRows) + 1) * kRowStride * 4;
+    auto kern = rerank_rows_kernel<METRIC>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e != cudaSuccess) return e;
+    kern<<<unsigned(m), kBlockThreads, smem, st>>>(db, db_norm, dim, q, q_norm, len, P, ids, dists, vec);
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t launch_rerank(int metric, const void *db, const float *db_norm, int64_t dim,
+                          const void *q, const float *q_norm, int64_t m, int len,
+                          uint32_t *ids, float *dists, cudaStream_t st, int *launches) {
+    if (m <= 0 || len <= 0) return cudaSuccess;
+    const int P = std::max(2, next_pow2(len));  // even: the ring behind the keys is 16-byte aligned
+    if (size_t(P) * 8 > 200 * 1024) return cudaErrorInvalidValue;  // (+ 74 KB of the ring: P is at most 16,384)
+    if (launches) *launches += 1;
+    if (metric == HAMMING) {
+        const int smem = P * 8;
+        cudaError_t e = cudaFuncSetAttribute(rerank_sketches_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        rerank_sketches_kernel<<<unsigned(m), 128, smem, st>>>(db, dim, q, len, P, ids, dists);
+        return cudaGetLastError();
+    }
+    const float *x = static_cast<const float *>(db), *y = static_cast<const float *>(q);
+    switch (metric) {
+        case SQL2: return launch_rerank_rows<SQL2>(x, db_norm, dim, y, q_norm, m, len, P, ids, dists, st);
+        case L2: return launch_rerank_rows<L2>(x, db_norm, dim, y, q_norm, m, len, P, ids, dists, st);
+        case NORMCOSINE: return launch_rerank_rows<NORMCOSINE>(x, db_norm, dim, y, q_norm, m, len, P, ids, dists, st);
+        case COSINE: return launch_rerank_rows<COSINE>(x, db_norm, dim, y, q_norm, m, len, P, ids, dists, st);
+        case IP: return launch_rerank_rows<IP>(x, db_norm, dim, y, q_norm, m, len, P, ids, dists, st);
         default: return cudaErrorInvalidValue;
     }
 }
