@@ -248,4 +248,81 @@ inline int next_pow2(int64_t v) {
     return p;
 }
 
+// |x|^2 of one row per lane by the sequential chain (index order, one fma
+// each).  A warp calls it together, `row` null where a lane has none; `vec`:
+// every row is 16-byte aligned and dim % 4 == 0.  What bounds it is the
+// latency of the rows' way in: a lane that reads its own row waits for a
+// sector 32 lanes apart at every few dimensions (777 rows of 300: 20 us), so
+// 32 dimensions of all 32 rows stream through `ring` (kNormRing floats,
+// 16-byte aligned) by coalesced copies, three steps in flight.
+constexpr int kNormStages = 4;
+constexpr int kNormStride = 36;
+constexpr int kNormRing = kNormStages * 32 * kNormStride;
+
+__device__ __forceinline__ float warp_row_squares(const float *row, int64_t dim, float *ring, bool vec) {
+    const int lane = threadIdx.x % 32;
+    const int64_t steps = (dim + 31) / 32;
+    auto stage = [&](int64_t c) {
+        float *buf = ring + int(c % kNormStages) * 32 * kNormStride;
+        const int64_t c0 = c * 32;
+        if (vec) {
+            const int sub = lane % 8 * 4;
+#pragma unroll
+            for (int r0 = 0; r0 < 32; r0 += 4) {
+                const int r = r0 + lane / 8;
+                const float *src = reinterpret_cast<const float *>(
+                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(row), r));
+                if (src && c0 + sub < dim) {
+                    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(buf + r * kNormStride + sub));
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + c0 + sub) : "memory");
+                }
+            }
+        } else {
+            for (int r = 0; r < 32; ++r) {
+                const float *src = reinterpret_cast<const float *>(
+                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(row), r));
+                if (src && c0 + lane < dim) {
+                    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(buf + r * kNormStride + lane));
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src + c0 + lane) : "memory");
+                }
+            }
+        }
+    };
+#pragma unroll
+    for (int p = 0; p < kNormStages - 1; ++p) {
+        if (p < steps) stage(p);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    float s = 0.0f;
+    for (int64_t c = 0; c < steps; ++c) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kNormStages - 2) : "memory");
+        __syncwarp();  // every lane's copies of step c; every lane done with step c - 1
+        if (c + kNormStages - 1 < steps) stage(c + kNormStages - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (!row) continue;
+        const float *x = ring + int(c % kNormStages) * 32 * kNormStride + lane * kNormStride;
+        const int n = dim - c * 32 < 32 ? int(dim - c * 32) : 32;
+        if (n == 32) {
+#pragma unroll
+            for (int e = 0; e < 32; e += 4) {
+                const float4 a = *reinterpret_cast<const float4 *>(x + e);
+                s = fmaf(a.x, a.x, s);
+                s = fmaf(a.y, a.y, s);
+                s = fmaf(a.z, a.z, s);
+                s = fmaf(a.w, a.w, s);
+            }
+        } else {
+            for (int e = 0; e < n; ++e) s = fmaf(x[e], x[e], s);
+        }
+    }
+    return s;
+}
+
+// One row per thread of a block of kNormThreads.
+constexpr int kNormThreads = 64;
+
+__device__ __forceinline__ bool rows_vec16(const float *x, int64_t dim) {
+    return dim % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+}
+
 }  // namespace ssg

@@ -235,12 +235,10 @@ namespace {
 
 __global__ void row_norms_kernel(const float *__restrict__ x, int64_t rows, int64_t dim,
                                  float *__restrict__ out) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= rows) return;
-    const float *r = x + i * dim;
-    float s = 0.0f;
-    for (int64_t c = 0; c < dim; ++c) s = fmaf(r[c], r[c], s);
-    out[i] = sqrtf(s);
+    __shared__ __align__(16) float ring[kNormThreads / 32][kNormRing];
+    const int64_t i = int64_t(blockIdx.x) * kNormThreads + threadIdx.x;
+    const float s = warp_row_squares(i < rows ? x + i * dim : nullptr, dim, ring[threadIdx.x / 32], rows_vec16(x, dim));
+    if (i < rows) out[i] = sqrtf(s);
 }
 
 template <typename T>
@@ -258,13 +256,10 @@ __global__ void cast_kernel(const T *__restrict__ src, int64_t count, float *__r
 
 __global__ void row_sq_norms_kernel(const float *__restrict__ x, int64_t rows, int64_t dim,
                                     float *__restrict__ out, float *__restrict__ max_out) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    float s = 0.0f;
-    if (i < rows) {
-        const float *r = x + i * dim;
-        for (int64_t c = 0; c < dim; ++c) s = fmaf(r[c], r[c], s);
-        out[i] = s;
-    }
+    __shared__ __align__(16) float ring[kNormThreads / 32][kNormRing];
+    const int64_t i = int64_t(blockIdx.x) * kNormThreads + threadIdx.x;
+    float s = warp_row_squares(i < rows ? x + i * dim : nullptr, dim, ring[threadIdx.x / 32], rows_vec16(x, dim));
+    if (i < rows) out[i] = s;
     // block max, then one atomic per block (non-negative floats order as ints)
     for (int o = 16; o > 0; o >>= 1) s = fmaxf(s, __shfl_xor_sync(0xffffffffu, s, o));
     if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int *>(max_out), __float_as_int(s));
@@ -298,7 +293,7 @@ cudaError_t launch_row_sq_norms(const float *x, int64_t rows, int64_t dim, float
                                 cudaStream_t st, int *launches) {
     if (rows <= 0) return cudaSuccess;
     if (launches) *launches += 1;
-    row_sq_norms_kernel<<<unsigned((rows + 255) / 256), 256, 0, st>>>(x, rows, dim, out, max_out);
+    row_sq_norms_kernel<<<unsigned((rows + kNormThreads - 1) / kNormThreads), kNormThreads, 0, st>>>(x, rows, dim, out, max_out);
     return cudaGetLastError();
 }
 
@@ -367,7 +362,7 @@ cudaError_t launch_row_norms(const float *x, int64_t rows, int64_t dim, float *o
                              cudaStream_t st, int *launches) {
     if (rows <= 0) return cudaSuccess;
     if (launches) *launches += 1;
-    row_norms_kernel<<<unsigned((rows + 255) / 256), 256, 0, st>>>(x, rows, dim, out);
+    row_norms_kernel<<<unsigned((rows + kNormThreads - 1) / kNormThreads), kNormThreads, 0, st>>>(x, rows, dim, out);
     return cudaGetLastError();
 }
 

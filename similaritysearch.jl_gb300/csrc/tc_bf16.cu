@@ -131,14 +131,11 @@ __global__ void bf16_tile_kernel(const float *__restrict__ x, int64_t rows, int 
 // Per padded row: |x|^2 (MC_SQ) or 1/|x| (MC_COS), 0 for padding rows.
 __global__ void tc_norm_kernel(const float *__restrict__ x, int64_t rows, int dim, int64_t padded, int mc,
                                const uint32_t *__restrict__ map, float *__restrict__ out) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= padded) return;
-    float s = 0.0f;
-    if (i < rows) {
-        const float *r = x + (map ? int64_t(map[i]) : i) * dim;
-        for (int c = 0; c < dim; ++c) s = fmaf(r[c], r[c], s);
-    }
-    out[i] = (mc == MC_COS) ? (s > 0.0f ? 1.0f / sqrtf(s) : 0.0f) : s;
+    __shared__ __align__(16) float ring[kNormThreads / 32][kNormRing];
+    const int64_t i = int64_t(blockIdx.x) * kNormThreads + threadIdx.x;
+    const float *row = i < rows ? x + (map ? int64_t(map[i]) : i) * dim : nullptr;
+    const float s = warp_row_squares(row, dim, ring[threadIdx.x / 32], rows_vec16(x, dim));
+    if (i < padded) out[i] = (mc == MC_COS) ? (s > 0.0f ? 1.0f / sqrtf(s) : 0.0f) : s;
 }
 
 // ---------------------------------------------------------------------------
@@ -1276,7 +1273,7 @@ cudaError_t launch_tc_norms(int metric, const float *x, int64_t rows, int64_t di
                             cudaStream_t st, int *launches, const uint32_t *map) {
     const int mc = metric_class(metric);
     if (launches) *launches += 1;
-    tc_norm_kernel<<<unsigned((padded + 255) / 256), 256, 0, st>>>(x, rows, int(dim), padded, mc, map, out);
+    tc_norm_kernel<<<unsigned((padded + kNormThreads - 1) / kNormThreads), kNormThreads, 0, st>>>(x, rows, int(dim), padded, mc, map, out);
     return cudaGetLastError();
 }
 

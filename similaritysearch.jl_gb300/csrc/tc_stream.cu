@@ -115,15 +115,14 @@ __global__ void stream_tile_kernel(const float *__restrict__ x, int64_t rows, in
 __global__ void stream_coef_kernel(const float *__restrict__ x, int64_t rows, int dim, int64_t padded, int metric,
                                    const float *__restrict__ scale, float *__restrict__ alpha,
                                    float *__restrict__ beta) {
-    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    __shared__ __align__(16) float ring[kNormThreads / 32][kNormRing];
+    const int64_t i = int64_t(blockIdx.x) * kNormThreads + threadIdx.x;
+    float sq = 0.0f;
+    if (metric == SQL2 || metric == L2 || metric == COSINE)
+        sq = warp_row_squares(i < rows ? x + i * dim : nullptr, dim, ring[threadIdx.x / 32], rows_vec16(x, dim));
     if (i >= padded) return;
     if (i >= rows) { alpha[i] = 0.0f; beta[i] = 0.0f; return; }
     const float s = scale ? scale[i] : 1.0f;
-    float sq = 0.0f;
-    if (metric == SQL2 || metric == L2 || metric == COSINE) {
-        const float *r = x + i * dim;
-        for (int c = 0; c < dim; ++c) sq = fmaf(r[c], r[c], sq);
-    }
     if (metric == SQL2 || metric == L2) { alpha[i] = -2.0f * s; beta[i] = sq; }
     else if (metric == COSINE) { alpha[i] = sq > 0.0f ? -s / sqrtf(sq) : 0.0f; beta[i] = 0.0f; }
     else { alpha[i] = -s; beta[i] = 0.0f; }
@@ -509,7 +508,7 @@ cudaError_t launch_stream_tiles(const float *x, int64_t rows, int64_t dim, int f
 cudaError_t launch_stream_coefs(int metric, const float *x, int64_t rows, int64_t dim, int64_t padded,
                                 const float *scale, float *alpha, float *beta, cudaStream_t st, int *launches) {
     if (launches) *launches += 1;
-    stream_coef_kernel<<<unsigned((padded + 255) / 256), 256, 0, st>>>(x, rows, int(dim), padded, metric, scale,
+    stream_coef_kernel<<<unsigned((padded + kNormThreads - 1) / kNormThreads), kNormThreads, 0, st>>>(x, rows, int(dim), padded, metric, scale,
                                                                        alpha, beta);
     return cudaGetLastError();
 }

@@ -1,6 +1,7 @@
-"""rerank! at the edges of its staging (128 rows and 32 dimensions at a time,
-16-byte copies or not), against the oracle's sequential run: ids and distances
-identical; and the network's products at every tile width, against FP64."""
+"""Row kernels at the edges of their staging (32 dimensions at a time, 16-byte
+copies or not): rerank! and the row norms against the oracle's sequential run,
+ids and distances identical, and the network's products at every tile width
+against FP64."""
 import numpy as np
 import pytest
 
@@ -62,3 +63,17 @@ def test_product_tile_widths(ss, d, H, E, B):
     for i, (g, r) in enumerate(zip(grads, want)):
         scale = max(np.abs(r).max(), np.abs(want[2]).max() if i == 3 else 0.0)
         assert np.abs(g - r).max() <= 1e-4 * scale
+
+
+@pytest.mark.parametrize("rows,dim", [(1, 1), (31, 3), (32, 31), (33, 32), (64, 33), (65, 64), (200, 130)])
+def test_row_norms(ss, rows, dim):
+    """Cosine divides by the norms of both sides: a norm off in its last bit shows."""
+    rng = np.random.default_rng(rows + dim)
+    X = rng.standard_normal((rows, dim), dtype=np.float32)
+    Q = rng.standard_normal((rows, dim), dtype=np.float32)
+    k = min(rows, 5)
+    idx = ss.GPUExhaustiveSearch(ss.Dist.Cosine(), ss.MatrixDatabase.from_rows(X), exact_scan=1)
+    ids, dists = ss.searchbatch(idx, ss.GenericContext(), ss.MatrixDatabase.from_rows(Q), k)
+    ri, rd = O.searchbatch("cosine", X, Q, k)
+    assert np.array_equal(ids.T, ri)
+    assert np.array_equal(dists.T, rd)
