@@ -89,6 +89,9 @@ struct FinalizeArgs {
     // are left out
     const uint32_t *list_bound = nullptr;
     int list_keys = 0;  // keys per query kept on chip while selecting (more take extra passes)
+    // set by the launcher: sqrt(max_x_sq), and the relative error t of the
+    // certificate (FP64 square roots that every block would repeat)
+    double x_max = 0.0, err_t = 0.0;
 };
 cudaError_t launch_finalize(const FinalizeArgs &a, cudaStream_t st, int *launches);
 

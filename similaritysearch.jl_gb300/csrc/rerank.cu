@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 
 namespace ssg {
 
@@ -22,8 +23,8 @@ namespace ssg {
 // What bounds it: for many queries the gather of the candidates' rows (C2:
 // 1e6 queries x 50 rows x 384 bytes = 19.2 GB); for few queries the latency
 // of one block.  So nothing here sorts the candidates: the `need` smallest of
-// a query's unique 64-bit keys are selected by bisection on the key's bits
-// (one compare and count per key and step), the rows of the selected
+// a query's unique 64-bit keys are selected by their bits (bisection in a
+// warp, 8 bits at a time by histogram in a block), the rows of the selected
 // candidates stream through shared memory 32 dimensions at a time (coalesced
 // cp.async copies, three or four steps in flight), one thread then walks each
 // candidate's sequential fma chain, and the order is found by counting the
@@ -34,7 +35,12 @@ namespace ssg {
 // keys 71 us (with the query norms' own launch) -> 26 us, one query of 5,472
 // keys 171 -> 21 us, 4,096 queries x 125 rows of 768 dimensions 1,229 ->
 // 391 us, C2's 1e6 queries x 50 rows of 96 10.2 -> 6.5 ms (3.0 TB/s of
-// gathered rows).
+// gathered rows).  The block shape gathers lists in one flat pass and selects
+// by an 8-bit histogram; while it walked list after list and counted bit by
+// bit, those two took most of it (64 queries of 152 lists: 16,000 and 37,000
+// cycles): hamming, 64 queries x 1,550 keys 34 -> 20 us, 777 queries x 400
+// keys, 44 rows of 300 30 -> 21 us, 20,000 x 1,060 keys, 115 rows of 768
+// 2,640 -> 1,850 us.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -47,6 +53,9 @@ constexpr int kWarpStages = 3;
 constexpr int kBlockThreads = 256;
 constexpr int kBlockRows = 128;            // candidates staged together in the block shape
 constexpr int kBlockStages = 4;
+constexpr int kBlockStagesFew = 8;         // few queries: nothing else hides the rows' latency
+constexpr int kFlatSegs = 512;             // lists per query whose keys a block gathers in one pass
+constexpr int kMinSel = kFlatSegs / 4;     // sel and out together hold an int per list
 
 // Length of a candidate row: the ids before its first 0 (by a block).
 __device__ __forceinline__ int valid_prefix(const uint32_t *rid, int len) {
@@ -153,20 +162,16 @@ __device__ __forceinline__ float chain_distance(float acc, uint32_t id0, const f
 // row needs no check (the caller's business); one shorter than `take`
 // cannot be certified.  low: a_low's key, KEY_EMPTY if there is none.
 template <int METRIC>
-__device__ bool list_complete(const FinalizeArgs &f, int64_t dim, int nv, uint64_t low, float q_sq, float d_take) {
+__device__ bool list_complete(const FinalizeArgs &f, int nv, uint64_t low, double qs, double q_abs, float d_take) {
     const int take = f.k_out + (f.exclude_self ? 1 : 0);
     if (nv < take || low == KEY_EMPTY) return false;
-    const double qs = double(q_sq);
-    const double xm = sqrt(double(f.max_x_sq));
+    const double xm = f.x_max;
     double dtake = double(d_take);
     if (METRIC == L2) dtake = dtake * dtake * (1.0 + 9.5367431640625e-7);
     double c, E;
     if (f.check == 1) {
-        double r = xm + sqrt(qs);
-        if (dtake >= 0.0) {
-            const double t = sqrt(double(dim + 2) * 5.9604644775390625e-8);
-            r = fmin(xm, ((1.0 + t) * sqrt(qs) + sqrt(dtake)) / (1.0 - t)) + sqrt(qs);
-        }
+        double r = xm + q_abs;
+        if (dtake >= 0.0) r = fmin(xm, ((1.0 + f.err_t) * q_abs + sqrt(dtake)) / (1.0 - f.err_t)) + q_abs;
         c = qs;
         E = double(f.err_scale) * r * r;
     } else if (f.check == 3) {
@@ -174,9 +179,9 @@ __device__ bool list_complete(const FinalizeArgs &f, int64_t dim, int nv, uint64
         E = double(f.err_scale);
     } else {
         c = METRIC == NORMCOSINE ? 1.0 : 0.0;
-        E = double(f.err_scale) * xm * sqrt(qs) + 2.384185791015625e-7;
+        E = double(f.err_scale) * xm * q_abs + 2.384185791015625e-7;
     }
-    const double a_low = f.check == 3 ? double(key_dist(low)) / sqrt(qs) : double(key_dist(low));
+    const double a_low = f.check == 3 ? double(key_dist(low)) / q_abs : double(key_dist(low));
     return a_low + c - E > dtake;
 }
 
@@ -444,7 +449,8 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
         if (threadIdx.x < kWarpsPerBlock && jq < f.m) {
             const int nv = s_nv[threadIdx.x];
             if (int64_t(nv) < f.n_total &&
-                !list_complete<METRIC>(f, dim, nv, s_low[threadIdx.x], s_qsq[threadIdx.x], s_take[threadIdx.x])) {
+                !list_complete<METRIC>(f, nv, s_low[threadIdx.x], double(s_qsq[threadIdx.x]),
+                                       sqrt(double(s_qsq[threadIdx.x])), s_take[threadIdx.x])) {
                 f.flags[query_row(f, jq)] = 1;
                 atomicAdd(f.flag_count, 1);
             }
@@ -456,7 +462,7 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
 // kBlockRows rows at a time stream through the ring (rows_s of kRowStride
 // floats per stage: the rows and, behind them, the query), one thread per row
 // and chain.  *q_sq (not null): the query's own squares.  Ends with a barrier.
-template <int METRIC>
+template <int METRIC, int STAGES>
 __device__ __forceinline__ void block_distances(const RowSource &rs, const uint64_t *sel, int nv, uint64_t *out,
                                                 float *ring, int rows_s, const float *db_norm, float qn, float *q_sq) {
     const int tid = threadIdx.x;
@@ -466,21 +472,21 @@ __device__ __forceinline__ void block_distances(const RowSource &rs, const uint6
         float acc = 0.0f;
         const float qs = tid == rows ? 0.0f : 1.0f;
 #pragma unroll
-        for (int p = 0; p < kBlockStages - 1; ++p) {
+        for (int p = 0; p < STAGES - 1; ++p) {
             if (p < steps)
                 stage_rows(rs, sel + r0, rows, p * kDimStep, ring + size_t(p) * rows_s * kRowStride, tid,
                            kBlockThreads);
             asm volatile("cp.async.commit_group;" ::: "memory");
         }
         for (int c = 0; c < steps; ++c) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(kBlockStages - 2) : "memory");
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
             __syncthreads();
-            const int nx = c + kBlockStages - 1;
+            const int nx = c + STAGES - 1;
             if (nx < steps)
-                stage_rows(rs, sel + r0, rows, nx * kDimStep, ring + size_t(nx % kBlockStages) * rows_s * kRowStride,
+                stage_rows(rs, sel + r0, rows, nx * kDimStep, ring + size_t(nx % STAGES) * rows_s * kRowStride,
                            tid, kBlockThreads);
             asm volatile("cp.async.commit_group;" ::: "memory");
-            const float *buf = ring + size_t(c % kBlockStages) * rows_s * kRowStride;
+            const float *buf = ring + size_t(c % STAGES) * rows_s * kRowStride;
             if (tid <= rows)
                 acc = chain_step<METRIC>(acc, buf + tid * kRowStride, buf + rows * kRowStride,
                                          min(kDimStep, rs.dim - c * kDimStep), qs);
@@ -498,7 +504,7 @@ __device__ __forceinline__ void block_distances(const RowSource &rs, const uint6
 // query's segments; of lists with more than that, only keys below a limit
 // found by counting are taken); sel_cap: room for the selected ones (0: they take the keys' place,
 // when nothing is left out).
-template <int METRIC, bool RERANK>
+template <int METRIC, bool RERANK, int STAGES>
 __global__ void __launch_bounds__(kBlockThreads)
 finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float *__restrict__ db_norm, int64_t dim,
                       const float *__restrict__ q, const float *__restrict__ q_norm, int need, int cap, int sel_cap,
@@ -508,7 +514,11 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
     uint64_t *sel = sel_cap ? keys + cap : keys;
     uint64_t *out = sel_cap ? sel + sel_cap : keys + cap;  // as long as sel
     float *ring = reinterpret_cast<float *>(out + (sel_cap ? sel_cap : cap));
-    __shared__ int s_cnt[3], s_n, s_self;
+    // where each list's keys start, then the selection's histogram, in the
+    // room of the selected keys (sel_cap >= kMinSel or nothing is selected)
+    int *s_pre = reinterpret_cast<int *>(sel);
+    __shared__ int s_cnt[3], s_n, s_self, s_digit, s_under, s_in;
+    __shared__ int s_warp[kBlockThreads / 32];
     __shared__ unsigned long long s_min, s_max, s_low, s_last;
     __shared__ float s_qsq;
     const int tid = threadIdx.x, lane = tid % 32;
@@ -523,7 +533,9 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
         s_self = INT_MAX;
     }
     __syncthreads();
-    // the query's keys, empty slots left out
+    // the query's keys, empty slots left out (or, gathered in one pass, left
+    // empty in place: `slots` of them)
+    int slots = -1;
     uint64_t mn = KEY_EMPTY, mx = 0;
     auto push = [&](uint64_t key) {  // by whole warps
         if (RERANK && int64_t(key_id0(key)) >= f.n_rows) key = KEY_EMPTY;
@@ -557,18 +569,44 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
                 }
             }
         };
-        int sum = 0;
-        for (int s = tid; s < f.segs; s += kBlockThreads) sum += cn[s];
-        sum = __reduce_add_sync(0xffffffffu, sum);
-        if (lane == 0 && sum) atomicAdd(&s_cnt[0], sum);
-        __syncthreads();
-        const int all = s_cnt[0];
+        // two lists per thread: where each one's keys start among all
+        int all;
+        const bool flat = f.segs <= kFlatSegs && sel_cap;
+        if (flat) {
+            const int s2 = 2 * tid;
+            const int c0 = s2 < f.segs ? cn[s2] : 0, c1 = s2 + 1 < f.segs ? cn[s2 + 1] : 0;
+            int incl = c0 + c1;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) s_warp[tid / 32] = incl;
+            __syncthreads();
+            int before = 0;
+            all = 0;
+#pragma unroll
+            for (int w = 0; w < kBlockThreads / 32; ++w) {
+                before += w < tid / 32 ? s_warp[w] : 0;
+                all += s_warp[w];
+            }
+            s_pre[s2] = before + incl - c0 - c1;
+            s_pre[s2 + 1] = before + incl - c1;
+            __syncthreads();
+        } else {
+            int sum = 0;
+            for (int s = tid; s < f.segs; s += kBlockThreads) sum += cn[s];
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            if (lane == 0 && sum) atomicAdd(&s_cnt[0], sum);
+            __syncthreads();
+            all = s_cnt[0];
+            __syncthreads();
+            if (tid == 0) s_cnt[0] = 0;
+        }
         uint64_t lim = KEY_EMPTY;
         if (all > cap) {
             // more keys than fit: a limit with at least `need` and at most
             // cap keys below it (keys are unique, so one exists)
-            __syncthreads();
-            if (tid == 0) s_cnt[0] = 0;
             __syncthreads();
             uint64_t p = 0;
             int it = 0;
@@ -587,11 +625,32 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
             __syncthreads();
             if (tid < 3) s_cnt[tid] = 0;
             __syncthreads();
-        } else {
-            __syncthreads();
-            if (tid == 0) s_cnt[0] = 0;
         }
-        each_key([&](uint64_t key) { push(key < lim ? key : KEY_EMPTY); });
+        if (flat && all <= cap) {
+            // one pass over all keys side by side (a group of lanes walking
+            // lists in turn waits for a count, then for keys, list after list)
+            slots = all;
+            int have = 0;
+#pragma unroll 4
+            for (int i = tid; i < all; i += kBlockThreads) {
+                int sg = 0;
+#pragma unroll
+                for (int step = kFlatSegs / 2; step > 0; step >>= 1)
+                    if (sg + step < f.segs && s_pre[sg + step] <= i) sg += step;
+                uint64_t key = lists[size_t(sg) * f.list_cap + (i - s_pre[sg])];
+                if (uint32_t(key >> 32) > bound || (RERANK && int64_t(key_id0(key)) >= f.n_rows)) key = KEY_EMPTY;
+                keys[i] = key;
+                if (key != KEY_EMPTY) {
+                    ++have;
+                    mn = min(mn, key);
+                    mx = max(mx, key);
+                }
+            }
+            have = __reduce_add_sync(0xffffffffu, have);
+            if (lane == 0 && have) atomicAdd(&s_n, have);
+        } else {
+            each_key([&](uint64_t key) { push(key < lim ? key : KEY_EMPTY); });
+        }
     } else {
         for (int i0 = 0; i0 < total; i0 += kBlockThreads) push(i0 + tid < total ? src[i0 + tid] : KEY_EMPTY);
     }
@@ -610,32 +669,69 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
     __syncthreads();
     const int nvt = min(s_n, cap);
     const int nv = min(need, nvt);
-    if (nvt > need) {
-        const uint64_t lo = s_min, hi = s_max;
-        const int top = 63 - __clzll(lo ^ hi);
-        uint64_t p = top >= 63 ? 0ull : (lo >> (top + 1)) << (top + 1), below = KEY_EMPTY;
-        bool done = false;
-        int it = 0;
-        for (int b = top; b >= 0; --b, ++it) {
-            const uint64_t t = p | (1ull << b);
-            int c = 0;
-            for (int i = tid; i < nvt; i += kBlockThreads) c += keys[i] < t;
-            c = __reduce_add_sync(0xffffffffu, c);
-            int *slot = &s_cnt[it % 3];
-            if (lane == 0 && c) atomicAdd(slot, c);
-            __syncthreads();
-            c = *slot;
-            if (tid == 0) s_cnt[(it + 2) % 3] = 0;  // read by all before the last barrier, written after the next
-            if (c == need) { below = t; done = true; break; }
-            if (c < need) p = t;
+    const bool holes = slots >= 0;  // (then sel is apart from keys)
+    if (!holes) slots = nvt;
+    if (nvt > need || holes) {
+        // the keys below `below` are the `need` smallest: the digit (8 bits
+        // from the first one that differs) that the need-th falls into, by a
+        // histogram, until a digit's end meets the count (a compare and count
+        // per bit took 900 to 1,150 cycles for each of 6 to 40 bits)
+        uint64_t below = KEY_EMPTY;
+        if (nvt > need) {
+            const uint64_t lo = s_min, hi = s_max;
+            int bits = 64 - __clzll(lo ^ hi), rem = need;
+            uint64_t p = bits >= 64 ? 0ull : lo >> bits;
+            for (;;) {
+                const int w = min(8, bits), shift = bits - w;
+                s_pre[tid] = 0;
+                __syncthreads();
+                for (int i = tid; i < slots; i += kBlockThreads) {
+                    const uint64_t key = keys[i];
+                    if (key != KEY_EMPTY && (bits >= 64 || key >> bits == p))
+                        atomicAdd(&s_pre[int(key >> shift) & ((1 << w) - 1)], 1);
+                }
+                __syncthreads();
+                if (tid < 32) {
+                    int c[8], sum = 0;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) sum += c[e] = s_pre[8 * tid + e];
+                    int incl = sum;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                        if (lane >= o) incl += v;
+                    }
+                    int under = incl - sum;
+                    if (under < rem && rem <= incl) {
+                        bool found = false;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            if (!found && rem <= under + c[e]) {
+                                found = true;
+                                s_digit = 8 * tid + e;
+                                s_under = under;
+                                s_in = c[e];
+                            }
+                            under += c[e];
+                        }
+                    }
+                }
+                __syncthreads();
+                p = (p << w) | uint64_t(s_digit);
+                rem -= s_under;
+                bits = shift;
+                if (s_in == rem || bits == 0) {
+                    below = (p + 1) << bits;
+                    if (below == 0) below = KEY_EMPTY;
+                    break;
+                }
+            }
         }
-        if (!done) below = p + 1;
-        __syncthreads();
         if (tid == 0) s_n = 0;
         __syncthreads();
-        for (int i0 = 0; i0 < nvt; i0 += kBlockThreads) {
+        for (int i0 = 0; i0 < slots; i0 += kBlockThreads) {
             const int i = i0 + tid;
-            const uint64_t key = i < nvt ? keys[i] : KEY_EMPTY;
+            const uint64_t key = i < slots ? keys[i] : KEY_EMPTY;
             const bool take = key < below;
             const uint32_t vote = __ballot_sync(0xffffffffu, take);
             int base = 0;
@@ -659,12 +755,14 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
             if (tid == 0 && s_last < s_low) s_low = s_last;
         }
         const RowSource rs{db, q + size_t(jr) * dim, int(dim), vec != 0};
-        block_distances<METRIC>(rs, sel, nv, out, ring, min(need, kBlockRows) + 1, db_norm,
+        block_distances<METRIC, STAGES>(rs, sel, nv, out, ring, min(need, kBlockRows) + 1, db_norm,
                                 METRIC == COSINE ? q_norm[jr] : 0.0f, &s_qsq);
         uint64_t *t = sel;
         sel = out;
         out = t;
     }
+    double q_abs = 0.0;
+    if (RERANK && f.check && tid == 0) q_abs = sqrt(double(s_qsq));  // beside the placing
     // place by counting the smaller keys; long lists by a bitonic sort
     if (nv <= 512) {
         for (int i = tid; i < nv; i += kBlockThreads) {
@@ -690,7 +788,7 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
     write_row(f, jr, out, nv, s_self, tid, kBlockThreads);
     if (RERANK && f.check && tid == 0 && int64_t(nv) < f.n_total) {
         const int take = f.k_out + (f.exclude_self ? 1 : 0);
-        if (!list_complete<METRIC>(f, dim, nv, s_low, s_qsq, nv >= take ? key_dist(out[take - 1]) : 0.0f)) {
+        if (!list_complete<METRIC>(f, nv, s_low, double(s_qsq), q_abs, nv >= take ? key_dist(out[take - 1]) : 0.0f)) {
             f.flags[jr] = 1;
             atomicAdd(f.flag_count, 1);
         }
@@ -720,14 +818,21 @@ cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const floa
         return cudaGetLastError();
     }
     // the sorted order of more than 512 selected keys takes a power of two
-    const int out_cap = need <= 512 ? (need + 1) / 2 * 2 : next_pow2(need);  // even: the ring behind is 16-byte aligned
     const bool in_place = total <= need;
+    int out_cap = need <= 512 ? (need + 1) / 2 * 2 : next_pow2(need);  // even: the ring behind is 16-byte aligned
+    if (!in_place) out_cap = std::max(out_cap, kMinSel);
     const int cap = in_place ? std::max((total + 1) / 2 * 2, out_cap) : (total + 1) / 2 * 2;
     const size_t keys = in_place ? 2 * size_t(cap) : size_t(cap) + 2 * size_t(out_cap);
-    const size_t ring = RERANK ? size_t(kBlockStages) * (std::min(need, kBlockRows) + 1) * kRowStride * 4 : 0;
-    const size_t smem = keys * 8 + ring;
+    const size_t stage = RERANK ? size_t(std::min(need, kBlockRows) + 1) * kRowStride * 4 : 0;
+    size_t smem = keys * 8 + kBlockStages * stage;
     if (smem > 226 * 1024) return cudaErrorInvalidValue;
-    auto kern = finalize_block_kernel<METRIC, RERANK>;
+    auto kern = finalize_block_kernel<METRIC, RERANK, kBlockStages>;
+    // at most a block per SM: more steps of the rows in flight (at more, the
+    // other blocks of an SM hide the rows' latency and room is what counts)
+    if (RERANK && f.m <= device_sm_count() && keys * 8 + kBlockStagesFew * stage <= 226 * 1024) {
+        smem = keys * 8 + kBlockStagesFew * stage;
+        kern = finalize_block_kernel<METRIC, RERANK, kBlockStagesFew>;
+    }
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     kern<<<unsigned(f.m), kBlockThreads, smem, st>>>(f, db, db_norm, dim, q, q_norm, need, cap,
@@ -743,12 +848,15 @@ cudaError_t launch_finalize(const FinalizeArgs &f, cudaStream_t st, int *launche
     return launch_finalize_t<SQL2, false>(f, nullptr, nullptr, 0, nullptr, nullptr, need, st);
 }
 
-cudaError_t launch_finalize_rerank(int metric, const FinalizeArgs &f, const float *db, const float *db_norm,
+cudaError_t launch_finalize_rerank(int metric, const FinalizeArgs &args, const float *db, const float *db_norm,
                                    int64_t dim, const float *q, const float *q_norm, cudaStream_t st,
                                    int *launches) {
+    FinalizeArgs f = args;
     const int rr = f.rerank ? f.rerank : f.kk;
     if (rr > (f.counts ? f.kk : f.segs * f.kk)) return cudaErrorInvalidValue;
     if (launches) *launches += 1;
+    f.x_max = std::sqrt(double(f.max_x_sq));
+    f.err_t = std::sqrt(double(dim + 2) * 5.9604644775390625e-8);
     switch (metric) {
         case SQL2: return launch_finalize_t<SQL2, true>(f, db, db_norm, dim, q, q_norm, rr, st);
         case L2: return launch_finalize_t<L2, true>(f, db, db_norm, dim, q, q_norm, rr, st);
@@ -800,7 +908,7 @@ rerank_rows_kernel(const float *__restrict__ db, const float *__restrict__ db_no
     for (int i = threadIdx.x; i < P; i += blockDim.x) s[i] = i < nv ? uint64_t(rid[i] - 1) : KEY_EMPTY;
     __syncthreads();
     const RowSource rs{db, q + size_t(j) * dim, int(dim), vec != 0};
-    block_distances<METRIC>(rs, s, nv, s, ring, min(len, kBlockRows) + 1, db_norm, METRIC == COSINE ? q_norm[j] : 0.0f,
+    block_distances<METRIC, kBlockStages>(rs, s, nv, s, ring, min(len, kBlockRows) + 1, db_norm, METRIC == COSINE ? q_norm[j] : 0.0f,
                             nullptr);
     block_bitonic_sort(s, P);
     for (int i = threadIdx.x; i < nv; i += blockDim.x) {

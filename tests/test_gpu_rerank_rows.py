@@ -77,3 +77,16 @@ def test_row_norms(ss, rows, dim):
     ri, rd = O.searchbatch("cosine", X, Q, k)
     assert np.array_equal(ids.T, ri)
     assert np.array_equal(dists.T, rd)
+
+
+@pytest.mark.parametrize("m,k,splits", [(3, 10, 300), (3, 10, 256), (200, 60, 257)])
+def test_many_lists(ss, m, k, splits):
+    """More than 512 candidate lists per query are walked, fewer gathered flat."""
+    rng = np.random.default_rng(m + splits)
+    X = rng.standard_normal((80_000, 8), dtype=np.float32)
+    Q = rng.standard_normal((m, 8), dtype=np.float32)
+    idx = ss.GPUExhaustiveSearch(ss.Dist.SqL2(), ss.MatrixDatabase.from_rows(X), splits=splits)
+    ids, dists = ss.searchbatch(idx, ss.GenericContext(), ss.MatrixDatabase.from_rows(Q), k)
+    ri, rd = O.searchbatch("sql2", X, Q, k)
+    assert np.array_equal(ids.T, ri)
+    assert np.array_equal(dists.T, rd)
