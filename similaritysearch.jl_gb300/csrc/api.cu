@@ -290,6 +290,14 @@ int clear_flags(ssg_index *idx, int64_t m, int **flags) {
     return SSG_OK;
 }
 
+// The status word alone, ahead of the query tiles: a copy or a memset between
+// two kernels keeps the second from starting early.
+int clear_status(ssg_index *idx) {
+    SSG_CK(idx->status.ensure(8), "allocating the status word");
+    SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
+    return SSG_OK;
+}
+
 // Uploads `rows` rows (row stride `ld` elements of `elem`) from host or device
 // memory into dst as contiguous Float32 (or UInt64) rows of `dim`.
 int upload_rows(ssg_index *idx, void *dst, const void *src, int64_t rows, int64_t ld, bool src_device) {
@@ -652,7 +660,6 @@ int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
     // one allocation: lists, minima (16-byte rows), bounds, counts
     const size_t lists = size_t(p.chunk) * segs * p.cap * 8, minima = size_t(p.chunk) * p.groups * 4;
     SSG_CK(idx->l_buf.ensure(lists + minima + size_t(p.chunk) * 4 * (1 + segs)), "allocating candidate lists");
-    SSG_CK(idx->status.ensure(8), "allocating the status word");
     s->cap = p.cap;
     s->splits = p.splits;
     s->samples = p.samples;
@@ -680,15 +687,12 @@ void list_finalize(const ListPlan &p, const ssg::ListScan &s, ssg::FinalizeArgs 
 
 // Seed, scan and finalize, chunk by chunk of the queries.  s holds the
 // operands (dt, row form, epilogue, n, kk; gamma of the first query), qtiles
-// the query tiles of tb bytes each; cleared: the status word is zero already;
-// finish(c0, f) launches the chunk's
-// finalize kernel.
+// the query tiles of tb bytes each; the status word is zero already;
+// finish(c0, f) launches the chunk's finalize kernel.
 template <typename F>
-int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, bool cleared, const uint8_t *qtiles, size_t tb, int64_t m,
+int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, const uint8_t *qtiles, size_t tb, int64_t m,
                 int k, int exclude_self, uint32_t *d_ids, float *d_dists, F &&finish) {
     SSG_RC(list_buffers(idx, plan, &s));
-    if (!cleared)
-        SSG_CK(cudaMemsetAsync(idx->status.p, 0, sizeof(int), idx->stream), "clearing the status word");
     const float *gamma = s.gamma;
     const uint32_t *perm = s.perm;
     const int *rot = s.rot;
@@ -754,6 +758,7 @@ int run_hamming_tc(ssg_index *idx, const void *dq, int64_t m, int k, int exclude
     // (allknn's queries too: the database's tiles have fewer rows)
     const size_t tb = size_t(128) * row_bytes;
     const int64_t qt = (ssg::tc_tiles(m) + 1) / 2 * 2;
+    SSG_RC(clear_status(idx));
     SSG_CK(idx->sk_q.ensure(size_t(qt) * tb), "allocating query sketch tiles");
     SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(dq), m, idx->dim, true, qt,
                                     static_cast<uint8_t *>(idx->sk_q.p), idx->stream, &idx->last_launches),
@@ -767,7 +772,7 @@ int run_hamming_tc(ssg_index *idx, const void *dq, int64_t m, int k, int exclude
     s.bits = float(64 * idx->dim);
     s.n = idx->n;
     s.kk = kk;
-    SSG_RC(list_search(idx, s, plan, false, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+    SSG_RC(list_search(idx, s, plan, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
                        [&](int64_t, ssg::FinalizeArgs &f) {
                            return ssg::launch_finalize(f, idx->stream, &idx->last_launches);
                        }));
@@ -1195,7 +1200,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
         s.epi = list_epilogue(idx->metric);
         s.n = idx->n;
         s.kk = plan.rr;
-        SSG_RC(list_search(idx, s, lp, true, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+        SSG_RC(list_search(idx, s, lp, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
                            [&](int64_t c0, ssg::FinalizeArgs &f) {
                                plain_certificate(idx, kp, flags + c0, flag_count, &f);
                                return ssg::launch_finalize_rerank(
@@ -1352,7 +1357,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
         s.beta = static_cast<const float *>(idx->pss_beta.p);
         s.n = idx->n;
         s.kk = kk;
-        SSG_RC(list_search(idx, s, lp, true, qt, tb, m, k, exclude_self, d_ids, d_dists,
+        SSG_RC(list_search(idx, s, lp, qt, tb, m, k, exclude_self, d_ids, d_dists,
                            [&](int64_t c0, ssg::FinalizeArgs &f) {
                                plain_certificate(idx, kp, flags + c0, flag_count, &f);
                                return ssg::launch_finalize_rerank(
@@ -1707,6 +1712,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
     if (idx->wide_param && !idx->pair_param && idx->long_param &&
         ssg::list_fits(2 * kp, 64, list_epilogue(idx->metric), idx->n) &&
         (locality ? list_plan_locality(idx, kk, &plan) : list_plan(idx, m, kk, &plan))) {
+        SSG_RC(clear_status(idx));
         const size_t tb = ssg::tc_tile_bytes(idx->dim);
         const uint8_t *qtiles = static_cast<const uint8_t *>(idx->tc_db.p);
         ssg::ListScan s{};
@@ -1731,7 +1737,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
         s.epi = list_epilogue(idx->metric);
         s.n = idx->n;
         s.kk = kk;
-        SSG_RC(list_search(idx, s, plan, false, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
+        SSG_RC(list_search(idx, s, plan, qtiles, tb, m, k, exclude_self, d_ids, d_dists,
                            [&](int64_t c0, ssg::FinalizeArgs &f) {
                                return ssg::launch_finalize_rerank(
                                    idx->metric, f, static_cast<const float *>(idx->db.p),
@@ -2008,6 +2014,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     const size_t tb = ssg::stream_tile_bytes(idx->dim, fp8);
     const uint8_t *qt = static_cast<const uint8_t *>(idx->st_db.p);
     const float *qgamma = fp8 ? static_cast<const float *>(idx->st_scale.p) : nullptr;
+    SSG_RC(clear_status(idx));
     if (!queries_are_db) {
         SSG_CK(idx->st_q.ensure(size_t(qt_alloc) * tb), "allocating query tiles");
         float *qs = nullptr;
@@ -2037,7 +2044,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
         s.gamma = qgamma;
         s.n = idx->n;
         s.kk = kk;
-        SSG_RC(list_search(idx, s, plan, false, qt, tb, m, k, exclude_self, d_ids, d_dists,
+        SSG_RC(list_search(idx, s, plan, qt, tb, m, k, exclude_self, d_ids, d_dists,
                            [&](int64_t c0, ssg::FinalizeArgs &f) {
                                return ssg::launch_finalize_rerank(
                                    idx->metric, f, static_cast<const float *>(idx->db.p),

@@ -248,6 +248,31 @@ inline int next_pow2(int64_t v) {
     return p;
 }
 
+// The kernels of a search follow one another within microseconds, so they are
+// launched early: a kernel's blocks start while the one before drains, set up
+// their shared memory, TMEM and barriers, and griddep_wait() holds them until
+// every kernel before is complete and its writes are visible.  Every thread
+// of such a kernel waits before its first access to global memory (and so
+// completes after all that came before); griddep_launch() lets the next
+// kernel's blocks in as soon as there is room.
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 // |x|^2 of one row per lane by the sequential chain (index order, one fma
 // each).  A warp calls it together, `row` null where a lane has none; `vec`:
 // every row is 16-byte aligned and dim % 4 == 0.  What bounds it is the

@@ -242,6 +242,7 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
     const int64_t j = int64_t(blockIdx.x) * kWarpsPerBlock + warp;
     const bool live = j < f.m;
     uint64_t *sel = s_sel[warp], *out = s_key[warp];
+    griddep_wait();
     if (live) {
         const int64_t jr = query_row(f, j);
         int total = f.segs * f.kk;
@@ -522,6 +523,7 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
     __shared__ unsigned long long s_min, s_max, s_low, s_last;
     __shared__ float s_qsq;
     const int tid = threadIdx.x, lane = tid % 32;
+    griddep_wait();
     const int64_t j = blockIdx.x, jr = query_row(f, j);
     const int total = f.segs * f.kk;
     const uint64_t *src = f.cand + size_t(j) * total;
@@ -814,8 +816,8 @@ cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const floa
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
         const unsigned blocks = unsigned((f.m + kWarpsPerBlock - 1) / kWarpsPerBlock);
-        kern<<<blocks, 32 * kWarpsPerBlock, smem, st>>>(f, db, db_norm, dim, q, q_norm, need, vec ? 1 : 0);
-        return cudaGetLastError();
+        return launch_early(kern, dim3(blocks), 32 * kWarpsPerBlock, smem, st, f, db, db_norm, dim, q, q_norm, need,
+                            vec ? 1 : 0);
     }
     // the sorted order of more than 512 selected keys takes a power of two
     const bool in_place = total <= need;
@@ -835,9 +837,8 @@ cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const floa
     }
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
-    kern<<<unsigned(f.m), kBlockThreads, smem, st>>>(f, db, db_norm, dim, q, q_norm, need, cap,
-                                                     in_place ? 0 : out_cap, vec ? 1 : 0);
-    return cudaGetLastError();
+    return launch_early(kern, dim3(unsigned(f.m)), kBlockThreads, smem, st, f, db, db_norm, dim, q, q_norm, need, cap,
+                        in_place ? 0 : out_cap, vec ? 1 : 0);
 }
 
 }  // namespace

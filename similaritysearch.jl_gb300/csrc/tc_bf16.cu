@@ -99,6 +99,7 @@ int metric_class(int metric) {
 // terms first (while the accumulator, and so its rounding, is small).
 __global__ void bf16_tile_kernel(const float *__restrict__ x, int64_t rows, int dim, int kp, int split, int64_t tiles,
                                  const uint32_t *__restrict__ map, uint8_t *__restrict__ out) {
+    griddep_launch();
     const int kout = split ? 3 * kp : kp;
     const int chunks_per_row = kout / 8;
     const int64_t total = tiles * TILE * chunks_per_row;

@@ -366,6 +366,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     for (int w = 0; w < 8; ++w)
         if (qpair * TILE + w * 32 < a.m) live += CS;
 
+    // (not the scan's: finalize blocks held on its SMs cost 45 us of 2,680)
+    if (SEED) griddep_launch();
     if (threadIdx.x == 0) {
         tc::mbar_init(a_full, 1);
         tc::mbar_init(pa_full, 1);
@@ -395,6 +397,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         __syncthreads();
     }
     tc::cluster_sync();  // both CTAs' barriers (and scale factors) exist before any cross-CTA arrive
+    griddep_wait();
     tc::tc_fence_after();
 
     // this split's wide tiles (places in the sample when SEED)
@@ -650,6 +653,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 template <int NV>
 __global__ void __launch_bounds__(128) seed_bound_kernel(const float *__restrict__ minima, int64_t m, int groups, int kk,
                                                          uint32_t *__restrict__ bound) {
+    griddep_launch();
+    griddep_wait();
     const int64_t q = int64_t(blockIdx.x) * 4 + threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     if (q >= m) return;
@@ -692,6 +697,7 @@ __global__ void __launch_bounds__(128) seed_bound_kernel(const float *__restrict
 // the end are zeros.  Thread = 32 bits = one 16-byte chunk.
 __global__ void sketch_tile_kernel(const uint64_t *__restrict__ x, int64_t rows, int words, int kblocks, int tile_rows,
                                    int64_t tiles, uint8_t *__restrict__ out) {
+    griddep_launch();
     const int chunks = kblocks * 8;  // 32-bit chunks per padded row
     const int64_t total = tiles * tile_rows * chunks;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
@@ -795,8 +801,7 @@ cudaError_t launch_list_q(const ListScan &s, const Ring &ring, cudaStream_t st) 
     e = line_map(s.dt, ka.all_wide * 2 * rows * s.row_bytes, int64_t(ka.group) * rows * SWB, &dmap);
     if (e == cudaSuccess) e = line_map(s.qt, qtiles * TILE * s.row_bytes, int64_t(ka.group) * TILE * SWB, &qmap);
     if (e != cudaSuccess) return e;
-    kern<<<dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st>>>(ka, dmap, qmap);
-    return cudaGetLastError();
+    return launch_early(kern, dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st, ka, dmap, qmap);
 }
 
 template <int SWB, int KIND, int EPI, bool SEED, int ORDER = STORED>
@@ -850,12 +855,12 @@ cudaError_t launch_list_seed(const ListScan &s, cudaStream_t st, int *launches) 
     // about four groups per candidate keep the bound within a fifth of the
     // sample's own kk-th distance in rank
     const unsigned blocks = unsigned((s.m + 3) / 4);
-    if (s.per_tile == 64 && s.kk <= 256) seed_bound_kernel<32><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
-    else if (s.kk <= 64) seed_bound_kernel<8><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
-    else if (s.kk <= 160) seed_bound_kernel<20><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
-    else seed_bound_kernel<60><<<blocks, 128, 0, st>>>(s.minima, s.m, s.groups, s.kk, s.bound);
+    auto bound = s.per_tile == 64 && s.kk <= 256 ? seed_bound_kernel<32>
+                 : s.kk <= 64                    ? seed_bound_kernel<8>
+                 : s.kk <= 160                   ? seed_bound_kernel<20>
+                                                 : seed_bound_kernel<60>;
     if (launches) *launches += 2;
-    return cudaGetLastError();
+    return launch_early(bound, dim3(blocks), 128, 0, st, s.minima, s.m, s.groups, s.kk, s.bound);
 }
 
 cudaError_t launch_list_scan(const ListScan &s, cudaStream_t st, int *launches) {

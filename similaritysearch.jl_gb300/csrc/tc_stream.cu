@@ -56,6 +56,7 @@ __host__ __device__ constexpr int st_threads() { return 64 + TILE * CS; }
 // hi = bf16(x) and lo = bf16(x - hi) (see tc_bf16.cu, bf16_tile_kernel).
 __global__ void stream_tile_kernel(const float *__restrict__ x, int64_t rows, int dim, int kbytes, int fp8,
                                    int split, int64_t tiles, uint8_t *__restrict__ out, float *__restrict__ scale) {
+    griddep_launch();
     const int lane = threadIdx.x % 32;
     const int64_t wid = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
     const int64_t nw = int64_t(gridDim.x) * blockDim.x / 32;
