@@ -740,6 +740,12 @@ int list_epilogue(int metric) {
     return is_sq_metric(metric) ? ssg::LIST_SQ : metric == SSG_METRIC_COSINE ? ssg::LIST_COS : ssg::LIST_DOT;
 }
 
+// The 128-byte K-block tiles': scale and offset of every row, or the one of
+// them that the metric has (BF16 rows have no scale).
+int list_epilogue_stream(int metric, bool fp8) {
+    return !is_sq_metric(metric) ? ssg::LIST_SCALE : fp8 ? ssg::LIST_AFFINE : ssg::LIST_SQ;
+}
+
 // Hamming on the tensor cores: sketches as +-1 FP4 rows, products exact in
 // FP32 (at most 2,048 terms of +-1), distance = (bits - product) / 2, so the
 // keys are the ones hamming_kernel makes.
@@ -1347,13 +1353,14 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     // the list scan where the database is large enough for its seed
     ListPlan lp;
     const int row_bytes = 3 * ssg::stream_kbytes(idx->dim, 0);
-    if (ssg::list_fits(row_bytes, 128, ssg::LIST_AFFINE, idx->n) && list_plan(idx, m, kk, &lp)) {
+    const int epi = list_epilogue_stream(idx->metric, false);
+    if (ssg::list_fits(row_bytes, 128, epi, idx->n) && list_plan(idx, m, kk, &lp)) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->pss_db.p);
         s.row_bytes = row_bytes;
         s.swb = 128;
-        s.epi = ssg::LIST_AFFINE;
-        s.alpha = static_cast<const float *>(idx->pss_alpha.p);
+        s.epi = epi;
+        s.alpha = static_cast<const float *>(epi == ssg::LIST_SQ ? idx->pss_beta.p : idx->pss_alpha.p);
         s.beta = static_cast<const float *>(idx->pss_beta.p);
         s.n = idx->n;
         s.kk = kk;
@@ -2032,14 +2039,15 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     // kk candidates
     ListPlan plan;
     const int row_bytes = ssg::stream_kbytes(idx->dim, fp8);
-    if (ssg::list_fits(row_bytes, 128, ssg::LIST_AFFINE, idx->n) && list_plan(idx, m, kk, &plan)) {
+    const int epi = list_epilogue_stream(idx->metric, fp8);
+    if (ssg::list_fits(row_bytes, 128, epi, idx->n) && list_plan(idx, m, kk, &plan)) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->st_db.p);
         s.row_bytes = row_bytes;
         s.swb = 128;
         s.fp8 = fp8;
-        s.epi = ssg::LIST_AFFINE;
-        s.alpha = static_cast<const float *>(idx->st_alpha.p);
+        s.epi = epi;
+        s.alpha = static_cast<const float *>(epi == ssg::LIST_SQ ? idx->st_beta.p : idx->st_alpha.p);
         s.beta = static_cast<const float *>(idx->st_beta.p);
         s.gamma = qgamma;
         s.n = idx->n;

@@ -213,7 +213,7 @@ cudaError_t launch_stream_scan(const uint8_t *q_tiles, const uint8_t *d_tiles, c
                                int *launches, int *segs_per_split);
 
 // ---- resident-query scan with candidate lists (tc_list.cu) ----
-enum { LIST_DOT = 0, LIST_SQ = 1, LIST_COS = 2, LIST_AFFINE = 3, LIST_HAMMING = 4 };
+enum { LIST_DOT = 0, LIST_SQ = 1, LIST_COS = 2, LIST_AFFINE = 3, LIST_HAMMING = 4, LIST_SCALE = 5 };
 constexpr int kListMaxCap = 1024;  // entries of one list at most
 constexpr int kListSlack = 160;    // entries beyond kk that every list has room for at least
 constexpr int kListSegs = 2;       // lists of a query per split
@@ -225,7 +225,7 @@ struct ListScan {
     int row_bytes, swb, fp8;  // bytes per padded row, per K-block row (64 / 128), FP8 or BF16
                               // (HAMMING: sketch tiles, 240 rows to a wide tile)
     int epi;                  // LIST_*
-    const float *alpha;       // per padded row: |x|^2 (SQ), 1 / |x| (COS), alpha (AFFINE)
+    const float *alpha;       // per padded row: |x|^2 (SQ), 1 / |x| (COS), alpha (AFFINE, SCALE)
     const float *beta;        // AFFINE
     const float *gamma;       // AFFINE: per query, null: 1
     float bits;               // HAMMING: bits per sketch

@@ -51,17 +51,24 @@ constexpr int kLine = 1024;             // bytes of a tensor-map line
 constexpr int kMaxStages = 16;
 constexpr size_t kMaxSmem = 227 * 1024;
 constexpr size_t kAloneSmem = 120 * 1024;  // all 512 TMEM columns: alone on the SM
-constexpr int kCoefBytes = 4 * CS * 2 * (8 / CS) * 256;  // per warp two buffers of its columns' coefficients
+constexpr int kCoefBytes = 4 * CS * 2 * (8 / CS) * 128;  // per warp two buffers of a float for each of its columns
 constexpr int kTileColumns = 256 / CS;     // columns of a wide tile that one list can take
 constexpr int kBufCap = 12;                // raw candidates buffered per lane
 constexpr int kBufStride = CS * TILE * 8;  // bytes between a lane's buffer slots
 constexpr int kBufBytes = kBufCap * kBufStride;
 
-enum { EPI_DOT = LIST_DOT, EPI_SQ = LIST_SQ, EPI_COS = LIST_COS, EPI_AFF = LIST_AFFINE, EPI_HAM = LIST_HAMMING };
+enum { EPI_DOT = LIST_DOT, EPI_SQ = LIST_SQ, EPI_COS = LIST_COS, EPI_AFF = LIST_AFFINE, EPI_HAM = LIST_HAMMING,
+       EPI_SCALE = LIST_SCALE };
 
 // EPI_DOT and EPI_HAM rank by the raw product, largest first; the distance is
 // made from it only for a candidate.
 __host__ __device__ constexpr bool raw_rank(int epi) { return epi == EPI_DOT || epi == EPI_HAM; }
+// Floats per database row that the epilogue reads.  Every warp reads them for
+// all its columns, as broadcasts of 16 bytes that cost the shared-memory pipe
+// as much as 512 bytes of operands: with both factors of AFF for metrics whose
+// offset is 0 that was two thirds of what the MMAs' own reads leave (4,096
+// queries x 2e6 FP8 rows of 768: 5.42 ms against 5.14 with one).
+__host__ __device__ constexpr int coefs(int epi) { return raw_rank(epi) ? 0 : epi == EPI_AFF ? 2 : 1; }
 
 struct KernelArgs {
     ListScan s;
@@ -194,7 +201,7 @@ struct RowList {
     bool valid;
     float lim_v;       // a candidate's ranking value: product >= lim_v (raw_rank) or distance <= lim_v
     float bits;        // EPI_HAM: bits per sketch
-    float gamma;       // EPI_AFF: the query's scale
+    float gamma;       // EPI_AFF, EPI_SCALE: the query's scale
 
     // the limit for a bound t on the distance; a row that is no query's lets nothing through
     __device__ __forceinline__ void set(float t) {
@@ -225,7 +232,7 @@ struct RowList {
                     dv[4 * j + 2] = -v2 * a.z;
                     dv[4 * j + 3] = -v3 * a.w;
                 } else {
-                    const float4 b = be[j];
+                    const float4 b = EPI == EPI_AFF ? be[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     dv[4 * j] = fmaf(v0 * gamma, a.x, b.x);
                     dv[4 * j + 1] = fmaf(v1 * gamma, a.y, b.y);
                     dv[4 * j + 2] = fmaf(v2 * gamma, a.z, b.z);
@@ -345,7 +352,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     uint8_t *sB = sA + (QSTREAM ? 0 : tile_bytes);  // stages: database part, then the query part
     // per epilogue warp, two buffers of its 64 columns' coefficients
     float4 *coef = reinterpret_cast<float4 *>(sB + size_t(stages) * stage_bytes);
-    uint64_t *bufs = reinterpret_cast<uint64_t *>(coef + (raw_rank(EPI) ? 0 : kCoefBytes / 16));  // raw candidates
+    uint64_t *bufs = reinterpret_cast<uint64_t *>(coef + coefs(EPI) * kCoefBytes / 16);  // raw candidates
     uint64_t *bars = bufs + (SEED ? 0 : kBufBytes / 8);
     uint64_t *a_full = bars;                  // this CTA's query tile landed
     uint64_t *pa_full = a_full + 1;           // (even CTA) the odd CTA's query tile landed
@@ -526,20 +533,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         T.top = KEY_EMPTY;
         T.perm = a.perm;
         T.bits = a.bits;
-        T.gamma = (EPI == EPI_AFF && a.gamma && T.valid) ? a.gamma[query] : 1.0f;
+        T.gamma = ((EPI == EPI_AFF || EPI == EPI_SCALE) && a.gamma && T.valid) ? a.gamma[query] : 1.0f;
         T.set((!SEED && T.valid) ? bound_read(a.bound + query) : INFINITY);
         const bool warp_live = qx * TILE + quarter * 32 < a.m;
         // this warp's columns of a wide tile: the 32-column chunks cs, cs + CS, ...;
         // their coefficients are copied a tile ahead
         constexpr int CH = 8 / CS;
-        float4 *mine = coef + (warp - 2) * CH * 32;
+        float4 *mine = coef + (warp - 2) * coefs(EPI) * CH * 16;
         auto fetch = [&](int u, int buf) {
             if constexpr (!raw_rank(EPI)) {
                 constexpr int PER = CH * 8;  // 16-byte pieces of alpha, and of beta
-                for (int p = lane; p < (EPI == EPI_AFF ? 2 : 1) * PER; p += 32) {
+                for (int p = lane; p < coefs(EPI) * PER; p += 32) {
                     const float *src = (p < PER ? a.alpha : a.beta) + wide_tile(u) * WIDE +
                                        (cs + CS * (p % PER / 8)) * 32 + (p % 8) * 4;
-                    const uint32_t d = tc::smem_u32(mine + buf * 2 * PER + p);
+                    const uint32_t d = tc::smem_u32(mine + buf * coefs(EPI) * PER + p);
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
@@ -563,7 +570,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             constexpr int LDC = raw_rank(EPI) ? 4 : 2;
             const uint32_t tbase = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(b * WIDE + cs * 32);
             const int64_t row0 = wide_tile(u) * WIDE + cs * 32;
-            const float4 *al = mine + (u & 1) * (CH * 16);  // alpha, then beta
+            const float4 *al = mine + (u & 1) * (coefs(EPI) * CH * 8);  // alpha, then beta
             uint32_t r[LDC][32];
             float gm[CH];
 #pragma unroll
@@ -751,7 +758,7 @@ cudaError_t line_map(const uint8_t *base, int64_t bytes, int64_t box_bytes, CUte
 }
 
 size_t list_smem(int query_bytes, int stage_bytes, int stages, int epi) {
-    return 1024 + size_t(query_bytes) + size_t(stages) * stage_bytes + (raw_rank(epi) ? 0 : kCoefBytes) + kBufBytes +
+    return 1024 + size_t(query_bytes) + size_t(stages) * stage_bytes + coefs(epi) * kCoefBytes + kBufBytes +
            (2 + 2 * kMaxStages + 2 * NACC + 1) * 8 + 16;
 }
 
@@ -808,7 +815,7 @@ template <int SWB, int KIND, int EPI, bool SEED, int ORDER = STORED>
 cudaError_t launch_list_t(const ListScan &s, cudaStream_t st) {
     const Ring ring = list_ring(s.row_bytes, SWB, EPI);
     if (ring.stages == 0) return cudaErrorInvalidValue;
-    if constexpr (EPI == EPI_AFF) {
+    if constexpr (SWB == 128 && KIND != FP4) {
         if (ring.qstream) return launch_list_q<SWB, KIND, EPI, SEED, ORDER, true>(s, ring, st);
     }
     if (ring.qstream) return cudaErrorInvalidValue;
@@ -828,8 +835,11 @@ cudaError_t launch_list_any(const ListScan &s, cudaStream_t st) {
     if (s.epi == LIST_HAMMING)
         return s.swb == 128 ? launch_list_t<128, FP4, EPI_HAM, SEED>(s, st) : cudaErrorInvalidValue;
     if (s.swb == 128) {
-        if (s.epi != LIST_AFFINE) return cudaErrorInvalidValue;
-        return s.fp8 ? launch_list_t<128, FP8, EPI_AFF, SEED>(s, st) : launch_list_t<128, BF16, EPI_AFF, SEED>(s, st);
+        if (s.epi == LIST_SCALE)
+            return s.fp8 ? launch_list_t<128, FP8, EPI_SCALE, SEED>(s, st) : launch_list_t<128, BF16, EPI_SCALE, SEED>(s, st);
+        if (s.epi == LIST_AFFINE && s.fp8) return launch_list_t<128, FP8, EPI_AFF, SEED>(s, st);
+        if (s.epi == LIST_SQ && !s.fp8) return launch_list_t<128, BF16, EPI_SQ, SEED>(s, st);
+        return cudaErrorInvalidValue;
     }
     switch (s.epi) {
         case LIST_DOT: return launch_list_order<EPI_DOT, SEED>(s, st);
@@ -845,7 +855,7 @@ cudaError_t launch_list_any(const ListScan &s, cudaStream_t st) {
 // tensor map's 32-bit coordinates.
 bool list_fits(int row_bytes, int swb, int epi, int64_t n) {
     const Ring ring = list_ring(row_bytes, swb, epi);
-    return ring.stages > 0 && (!ring.qstream || epi == LIST_AFFINE) &&
+    return ring.stages > 0 && (!ring.qstream || (swb == 128 && epi != LIST_HAMMING)) &&
            (n + 512) * row_bytes / kLine < (int64_t(1) << 31);
 }
 

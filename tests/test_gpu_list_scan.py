@@ -121,3 +121,31 @@ def test_allknn_locality(ss, metric, dim, k, splits, n, per):
     idx.set_param("locality", 0)
     b = ss.allknn(idx, ctx, k, exclude_self=True)
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("metric", ["sql2", "l2", "ip", "cosine", "normcosine"])
+@pytest.mark.parametrize("prec,dim", [("fp32", 300), ("fp32", 701), ("bf16", 640), ("fp8", 130)])
+def test_wide_row_epilogues(ss, metric, prec, dim):
+    """Scale, offset or both per row, the query tile resident or streamed: plain
+    results are the oracle's; of reduced keys, every row is a candidate of one
+    search and what is far behind the k-th of another."""
+    rng = np.random.default_rng(dim)
+    X, q = clustered(24_600, dim, rng)
+    Q = (q + 0.2 * rng.standard_normal((5, dim))).astype(np.float32)
+    if metric == "normcosine":
+        X /= np.linalg.norm(X, axis=1, keepdims=True)
+        Q /= np.linalg.norm(Q, axis=1, keepdims=True)
+    dist = {"sql2": ss.Dist.SqL2, "cosine": ss.Dist.Cosine, "normcosine": ss.Dist.NormCosine, "l2": ss.Dist.L2,
+            "ip": ss.Dist.InnerProduct}[metric]()
+    kw = {} if prec == "fp32" else {"precision": prec, "overfetch": 30.0}
+    idx = ss.GPUExhaustiveSearch(dist, ss.MatrixDatabase.from_rows(X), **kw)
+    ids, dists = ss.searchbatch(idx, ss.GenericContext(), ss.MatrixDatabase.from_rows(Q), 10)
+    ri, rd = O.searchbatch(metric, X, Q, 10)
+    if prec == "fp32":
+        assert np.array_equal(ids.T, ri)
+        assert np.array_equal(dists.T, rd)
+    else:
+        assert np.mean([len(set(a) & set(b)) for a, b in zip(ids.T, ri)]) >= 9.5
+        for j in range(5):  # exact distances of what was found
+            pos = {i: d for i, d in zip(ri[j], rd[j])}
+            assert all(pos.get(i, d) == d for i, d in zip(ids.T[j], dists.T[j]))
