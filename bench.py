@@ -62,11 +62,6 @@ N_DB = 1_000_000
 DIM = 96
 K = 32
 OVERFETCH_LADDER = (1.25, 1.5, 1.75)
-# DRAM bytes (read + write) of one headline scan launch at n = 1e6 and
-# over-fetch 1.5, from the one-pass ncu capture summarised in
-# profiles/tc_wide_bf16_allknn.md
-HEADLINE_SCAN_TRAFFIC = 56.662e9 + 0.815e9
-HEADLINE_TRAFFIC_OVERFETCH = 1.5
 
 METRIC = "queries/s @ recall@10>=0.99 (allknn NormCosine n=1e6 d=96 k=32 excl. self)"
 DATA = ("synthetic: seeded 1000-cluster Gaussian mixture (centres N(0,1), sigma U[0.1,0.5]), "
@@ -418,10 +413,6 @@ def allknn_mode(cx, X, mode, overfetch, steps, warmup, **params):
     q_per_launch = n * steps / max(1, main_launches)
     roof = (plain_tc_roofline(q_per_launch * n, d, avg) if plain_tc
             else roofline_flops(mode, 2.0 * q_per_launch * n * d, avg))
-    if mode == "bf16" and n == 1_000_000 and d == 96 and main_launches == steps and overfetch == HEADLINE_TRAFFIC_OVERFETCH:
-        roof["traffic"] = HEADLINE_SCAN_TRAFFIC
-        roof["traffic_note"] = ("dram__bytes_read.sum + dram__bytes_write.sum of one launch at over-fetch %.2f, "
-                                "one ncu capture (profiles/tc_wide_bf16_allknn.md)" % HEADLINE_TRAFFIC_OVERFETCH)
     return {"ms_per_step": ms, "qps": cx.world * n / (ms / 1e3), "launches": launches, "roofline": roof,
             "clocks": clocks, "ids": ids_host, "dists": dists_host, "fallbacks": fallbacks, "plain_tc": plain_tc}
 
@@ -637,7 +628,8 @@ def search_entry(cx, name, X, Q, k, mode, steps, warmup, desc, roof_fn, parity_l
     L.ssg_destroy(h)
     del Qd, ids_d, dists_d
     avg = main_ms / max(1, main_launches)
-    roof = plain_tc_roofline(m * n, d, avg) if plain_tc else roof_fn(avg)
+    # (a timed launch is a chunk's scan with its seed; most calls are one chunk)
+    roof = plain_tc_roofline(m * n * steps / max(1, main_launches), d, avg) if plain_tc else roof_fn(avg)
     # end to end: create from pinned host memory + search from host + results to host
     Xp, Qp = cx.pinned(X), cx.pinned(Q)
     oi = torch.empty((m, k), dtype=torch.int32).pin_memory()
@@ -716,19 +708,16 @@ def suite_c3(cx, args):
         def roof(ms, m=m):
             # one pass over the sketches + the queries + the results (bytes per call)
             r = roofline_bytes(8.0 * words * n + 8.0 * words * m + 8.0 * k * m, ms)
-            # the binding roof at these m: 64-bit XOR + POPC issue, 16 32-bit
-            # POPC per clock per SM = 8 words per clock per SM (nominal, at
-            # the measured maximum SM clock; no measured INT peak exists)
-            words_peak = 152 * 8 * peaks().get("sm_max_mhz", 2070.0) * 1e6
-            r["popcount_words_per_s"] = n * m * words / (ms / 1e3)
-            r["popcount_peak_words_per_s"] = words_peak
-            r["popcount_frac"] = r["popcount_words_per_s"] / words_peak
+            # the scan multiplies +-1 rows in FP4 (two operations per bit);
+            # no measured FP4 peak exists, the nominal dense one is 13.5 PFLOP/s
+            r["tensor_tflops"] = 2.0 * n * m * 64 * words / (ms / 1e3) / 1e12
+            r["bytes_note"] = "the FP4 rows that the scan reads are 4 times the sketches"
             return r
 
         out[tag] = search_entry(cx, "hamming", X, Qm, k, "fp32", max(args.steps, 10 if m > 64 else 50),
                                 args.warmup, desc, roof, cpu_budget=6.0)
-    out["note"] = ("the binding roof is the XOR + POPC issue rate down to m ~ 6 queries (16 m popcounts per "
-                   "128-byte row against the HBM rate), so the HBM fraction stays small by construction at m = 64")
+    out["note"] = ("tensor-bound at m = 10,000; at m = 64 the FP4 rows (4 times the sketches) at the HBM rate "
+                   "take most of the scan")
     return out
 
 
@@ -871,7 +860,7 @@ def suite_c4(cx, args, data):
         # HBM bytes one scan of the stream reads per batch (FP8 rows + the
         # two epilogue coefficients per row) plus its queries and results
         bytes_total = float(scans) * n * (d + 8) + tq * d * 4 + float((sizes * ks).sum()) * 8
-        roof = roofline_bytes(bytes_total / max(1, scans), scan_ms / max(1, scans), kernel="tc_stream_kernel")
+        roof = roofline_bytes(bytes_total / max(1, scans), scan_ms / max(1, scans), kernel="tc_list_kernel")
         roof["note"] = ("HBM bytes per scan launch (n x (d + 8) FP8 row bytes + queries + results), averaged over "
                         "the stream's launches; large batches are tensor-bound instead")
         out[name] = {

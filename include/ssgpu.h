@@ -146,21 +146,22 @@ int ssg_rerank(ssg_index *idx, const void *host_q, int64_t m, int32_t len,
 /* Tunables: "overfetch" (candidates per k in BF16/FP8 modes), "splits"
  * (database splits per query tile, 0 = auto), "margin" (extra candidates of
  * the plain GEMM-form scan, 0 = auto), "exact_scan" (1 = plain method through
- * the direct difference-form scan only), "plain" (1 = plain FP32 method on a
+ * the direct difference-form scan, Hamming through the XOR + POPC scan, only), "plain" (1 = plain FP32 method on a
  * BF16/FP8 index, e.g. to calibrate "overfetch" against it), "profile"
  * (1 = time the scan kernel with events), "graphs" (0 = no CUDA-graph replay
- * in ssg_search_batches), "wide" (0 = BF16 scans in 128 x 128 tiles instead
- * of 128 x 256), "pair" (1 = BF16 / split scans on CTA pairs with M = 256
- * MMAs), "long_lists" (0 = BF16 candidate lists too long for two heaps per
- * query go through the threshold filter instead of CTA pairs with one heap
- * per query; same candidates), "locality" (0 = BF16 allknn scans in id order
- * instead of the pivot-grouped order; results are identical either way),
+ * in ssg_search_batches), "wide", "pair" and "long_lists" (heap
+ * scans of BF16 / split tiles instead of the candidate-list scan, same
+ * results: wide 0 = in 128 x 128 tiles, pair 1 = on CTA pairs with one or two
+ * heaps per query, long_lists 0 = in 128 x 256 tiles, lists too long for two
+ * heaps per query through the threshold filter), "locality" (0 = allknn of
+ * 65,536 objects and more scans in id order instead of the pivot-grouped
+ * order; results are identical either way),
  * "locality_rows" (database rows per pivot of that order, 64..65536, default
  * 128), "locality_chain" (0 = the pivots' groups in pivot order instead of a
  * greedy nearest-pivot chain; results identical), "plain_tc"
  * (0 = keep the plain method on the CUDA cores; by default the float
- * metrics over at least 4096 objects run it on the tensor cores: a two-piece BF16 scan -- query tiles resident for
- * dim <= 128, both operands streamed along K beyond -- whose candidates are
+ * metrics over at least 4096 objects run it on the tensor cores: a two-piece
+ * BF16 scan whose candidates are
  * re-scored in exact FP32 and certified complete, uncertified queries
  * recomputed by the exact scan; results identical either way).  Unknown
  * keys return SSG_EINVAL. */

@@ -7,6 +7,11 @@
 // (distance, id) keys -- and therefore ids, distances and their order -- are
 // bit-exact with the reference.
 //
+// Sketches are scanned on the tensor cores (tc_list.cu, +-1 rows in FP4) where
+// that scan applies; this one serves databases too small for its seed, k
+// beyond its 480 candidates, "exact_scan", and a device without room for the
+// FP4 rows (4 times the sketches).
+//
 // Block = QPB threads, one query per thread; the query's words live in
 // registers (zero-padded to WMAX words).  Database sketches stream through
 // shared memory in tiles of TN rows, copied 16 bytes at a time (cp.async;

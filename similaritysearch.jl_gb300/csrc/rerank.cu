@@ -892,7 +892,8 @@ __global__ void rerank_sketches_kernel(const void *db, int64_t dim, const void *
 
 // Rows of floats: staged through shared memory as the finalize's are, not
 // read by the thread that walks the chain (32 lanes on 32 rows used one
-// sector in 32 loads).  What bounds it: the gather of m * len rows.
+// sector in 32 loads).  What bounds it: the gather of m * len rows (1,000 x
+// 512 rows of 768: 1,298 -> 317 us, 5 TB/s).
 template <int METRIC>
 __global__ void __launch_bounds__(kBlockThreads)
 rerank_rows_kernel(const float *__restrict__ db, const float *__restrict__ db_norm, int64_t dim,

@@ -6,7 +6,7 @@
 // accumulators in TMEM), turned into an approximate distance in the epilogue
 // and pushed into a per-query bounded top-k of kk = overfetch * k candidates.
 // The distance matrix never reaches HBM.  The candidates are then re-ranked
-// with the exact FP32 difference-form distance (finalize_rerank_kernel), so
+// with the exact FP32 difference-form distance (rerank.cu), so
 // the reported distances are the plain method's and the ids are exact
 // whenever the true neighbours survive the BF16 over-fetch.
 //
@@ -16,10 +16,13 @@
 // copy (cp.async.bulk) of a tile lands in shared memory ready for the MMA --
 // no tensor map and no reformatting on chip.
 //
-// Two scans share this layout: tc_wide_kernel (heap mode, 128 x 256 MMAs
-// over a ring of database K-blocks; the default) and tc_scan_kernel (128 x
-// 128 tiles: the threshold filter, the "wide" = 0 setting and the locality
-// order's pivot scan).  allknn may scan the database in a locality order
+// The scan of this layout is tc_list.cu's (candidate lists under a seeded
+// bound).  The heap scans here serve what it does not take: databases too
+// small for its seed (fewer than 2,048 rows, or than four groups per
+// candidate), more than 480 candidates per query, and the parameters that
+// ask for them: tc_wide_kernel (128 x 256 MMAs over a ring of database
+// K-blocks), tc_pair_kernel (CTA pairs) and tc_scan_kernel (128 x 128 tiles:
+// the threshold filter, "wide" = 0 and the locality order's pivot scan).  allknn may scan the database in a locality order
 // (rows grouped by nearest pivot; see launch_locality_order).
 //
 // CTA roles (one 128-row query tile, 320 threads):

@@ -48,7 +48,8 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
 // A failed try sleeps until the phase completes or kSuspendNs have passed:
 // without the hint it returns after a short system limit, and the polling
 // warps take issue slots and shared-memory cycles from the MMA thread (FP8
-// scan of 10,000 queries x 2e6 sketches: 12.6 ms without, 10.4 with).
+// scan of 10,000 queries x 2e6 sketches: 12.6 ms without, 10.4 with; the MMA
+// thread's own waits polled: FP4 7.26 -> 8.49 ms, the epilogue's too 9.82).
 constexpr uint32_t kSuspendNs = 20000;
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
@@ -285,16 +286,6 @@ __device__ __forceinline__ void tma_load_2d_pair(void *dst_smem, const void *tma
         "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
         " [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst_smem)),
         "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster), "r"(x), "r"(y)
-        : "memory");
-}
-
-// The same for a 3D tensor map, coordinates {x, y, z}.
-__device__ __forceinline__ void tma_load_3d_pair(void *dst_smem, const void *tmap, int x, int y, int z,
-                                                 uint32_t bar_cluster) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-        " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst_smem)),
-        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster), "r"(x), "r"(y), "r"(z)
         : "memory");
 }
 

@@ -12,7 +12,11 @@
 //      Cosine:          alpha = -s_x / |x|,        beta = 0
 //      SqL2, L2:        alpha = -2 s_x,            beta = |x|^2
 // which ranks like the exact metric.  kk = overfetch * k candidates per query
-// survive into the exact FP32 rerank (finalize_rerank_kernel).
+// survive into the exact FP32 rerank (rerank.cu).
+//
+// The scan of this layout is tc_list.cu's (candidate lists under a seeded
+// bound, on CTA pairs); the heap scan here serves databases too small for its
+// seed and candidate lists beyond its 480.
 //
 // Layout in HBM: tiles of 128 rows; each tile is a sequence of K-blocks of
 // 128 bytes per row (64 BF16 or 128 FP8 elements) with the 128-byte swizzle
