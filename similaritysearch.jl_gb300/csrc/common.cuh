@@ -255,6 +255,9 @@ inline int next_pow2(int64_t v) {
 // of such a kernel waits before its first access to global memory (and so
 // completes after all that came before); griddep_launch() lets the next
 // kernel's blocks in as soon as there is room.
+// What a kernel of the same chain wrote is read by plain or L2 loads: one
+// through __ldg or a const __restrict__ parameter may be moved ahead of the
+// wait, as of memory that does not change while the kernel runs.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

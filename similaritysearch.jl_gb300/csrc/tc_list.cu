@@ -373,8 +373,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     for (int w = 0; w < 8; ++w)
         if (qpair * TILE + w * 32 < a.m) live += CS;
 
-    // (not the scan's: finalize blocks held on its SMs cost 45 us of 2,680)
-    if (SEED) griddep_launch();
     if (threadIdx.x == 0) {
         tc::mbar_init(a_full, 1);
         tc::mbar_init(pa_full, 1);
@@ -394,6 +392,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // behind this block's allocation: no later kernel's block can take the
+    // TMEM first and then wait for this one.  (Not the scan's: finalize blocks
+    // held on its SMs cost 45 us of 2,680.)
+    if (SEED) griddep_launch();
     if constexpr (KIND == FP4) {
         // every scale factor is 1 (UE8M0 127), so their layout does not matter
         if (warp >= 2 && warp < 6) {
@@ -658,8 +660,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 // A warp per query; groups beyond 32 * NV are joined (their minimum is still
 // a row's distance), the kk-th value is found bit by bit from registers.
 template <int NV>
-__global__ void __launch_bounds__(128) seed_bound_kernel(const float *__restrict__ minima, int64_t m, int groups, int kk,
-                                                         uint32_t *__restrict__ bound) {
+__global__ void __launch_bounds__(128) seed_bound_kernel(const float *minima, int64_t m, int groups, int kk,
+                                                         uint32_t *bound) {
     griddep_launch();
     griddep_wait();
     const int64_t q = int64_t(blockIdx.x) * 4 + threadIdx.x / 32;
@@ -668,11 +670,11 @@ __global__ void __launch_bounds__(128) seed_bound_kernel(const float *__restrict
     const float *g = minima + size_t(q) * groups;
     float f[NV];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) f[i] = i * 32 + lane < groups ? g[i * 32 + lane] : INFINITY;
+    for (int i = 0; i < NV; ++i) f[i] = i * 32 + lane < groups ? __ldcg(g + i * 32 + lane) : INFINITY;
     for (int at = NV * 32 + lane; at < groups; at += NV * 32) {
 #pragma unroll
         for (int i = 0; i < NV; ++i)
-            if (at + i * 32 < groups) f[i] = fminf(f[i], g[at + i * 32]);
+            if (at + i * 32 < groups) f[i] = fminf(f[i], __ldcg(g + at + i * 32));
     }
     uint32_t v[NV], lo = 0xffffffffu, hi = 0;
 #pragma unroll
