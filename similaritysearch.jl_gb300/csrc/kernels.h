@@ -343,7 +343,7 @@ cudaError_t mlp_sum_parts(const float *G, int parts, int64_t count, float *out, 
 cudaError_t mlp_adam4(float *const W[4], const float *const G[4], const int parts[4], float *const M[4],
                       float *const V[4], const int64_t count[4], float lr, int step, cudaStream_t st, int *launches);
 // X = [S[idx[off..]]; S[idx[T + off..]]; S[idx[2T + off..]]] (bb rows each)
-cudaError_t mlp_gather3(const float *S, const int64_t *idx, int64_t T, int64_t off, int bb, int d, float *X,
+cudaError_t mlp_gather3(const float *S, const int64_t *idx, int64_t T, int64_t off, int bb, int d, float *X, float *stat,
                         cudaStream_t st, int *launches);
 
 // What the learned code needs of an index.

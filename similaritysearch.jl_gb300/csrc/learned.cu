@@ -419,8 +419,7 @@ int learned_train(const IndexView &v, const TrainArgs &t, LearnedModel **out, st
                 float *const am[4] = {mW1, mb1, mW2, mb2};
                 float *const av[4] = {vW1, vb1, vW2, vb2};
                 const int64_t ac[4] = {int64_t(H) * d, H, int64_t(E) * H, E};
-                bool ok = cu.ok(mlp_gather3(S, d_trip, T, off, bb, int(d), X, v.stream, v.launches), "gathering a batch") &&
-                          cu.ok(cudaMemsetAsync(stat, 0, 8, v.stream), "loss") &&
+                bool ok = cu.ok(mlp_gather3(S, d_trip, T, off, bb, int(d), X, stat, v.stream, v.launches), "gathering a batch") &&
                           cu.ok(mlp_gemm(f1, v.stream, v.launches), "fwd") &&
                           cu.ok(mlp_reduce_parts(P, sf1, rows, int(H), m->b1, 1, Hh, v.stream, v.launches), "fwd") &&
                           cu.ok(mlp_gemm(f2, v.stream, v.launches), "fwd") &&

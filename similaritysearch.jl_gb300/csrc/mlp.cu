@@ -26,6 +26,7 @@
 // (the dropped ones are below 2^-24 relative).  The gradient check runs the
 // same kernels in this mode against an FP64 oracle, at FP32-class accuracy;
 // training and embedding use plain BF16 operands.
+#include "common.cuh"
 #include "kernels.h"
 #include "tc_ptx.cuh"
 
@@ -68,7 +69,7 @@ struct Staged {
 };
 
 template <int R, bool KMAJOR>
-__device__ __forceinline__ void load_operand(Staged<R> &t, const float *__restrict__ X, int64_t ld, int r0, int rlim,
+__device__ __forceinline__ void load_operand(Staged<R> &t, const float *X, int64_t ld, int r0, int rlim,
                                              int k0, int klim, bool vec4) {
     if (r0 + R <= rlim && k0 + BK <= klim && (vec4 || !KMAJOR)) {
         // a whole tile: nothing to test per element
@@ -78,13 +79,13 @@ __device__ __forceinline__ void load_operand(Staged<R> &t, const float *__restri
             float *v = t.v[i];
             if (KMAJOR) {
                 const float *p = X + int64_t(r0 + c / (BK / 8)) * ld + k0 + c % (BK / 8) * 8;
-                const float4 a = __ldg(reinterpret_cast<const float4 *>(p));
-                const float4 b = __ldg(reinterpret_cast<const float4 *>(p + 4));
+                const float4 a = *reinterpret_cast<const float4 *>(p);
+                const float4 b = *reinterpret_cast<const float4 *>(p + 4);
                 v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
             } else {
                 const float *p = X + int64_t(k0 + c / R * 8) * ld + r0 + c % R;  // consecutive threads: consecutive rows
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = __ldg(p + j * ld);
+                for (int j = 0; j < 8; ++j) v[j] = p[j * ld];
             }
         }
         return;
@@ -98,7 +99,7 @@ __device__ __forceinline__ void load_operand(Staged<R> &t, const float *__restri
         const float *p = KMAJOR ? X + int64_t(gr) * ld + gk : X + int64_t(gk) * ld + gr;
         const int64_t step = KMAJOR ? 1 : ld;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = gr < rlim && gk + j < klim ? __ldg(p + j * step) : 0.0f;
+        for (int j = 0; j < 8; ++j) v[j] = gr < rlim && gk + j < klim ? p[j * step] : 0.0f;
     }
 }
 
@@ -155,6 +156,8 @@ __global__ void __launch_bounds__(GT, EXACT ? 1 : 2) mlp_gemm_kernel(MlpGemm g, 
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    griddep_launch();  // (its TMEM is its own by now)
+    griddep_wait();
     constexpr uint32_t idesc = tc::idesc_bf16_f32(BM, BN);
 
     bool ok = true;
@@ -241,7 +244,7 @@ __global__ void __launch_bounds__(GT, EXACT ? 1 : 2) mlp_gemm_kernel(MlpGemm g, 
 #pragma unroll
         for (int r = 0; r < 32; ++r) {
             const int row = row0 + r;
-            mk[r] = (g.mask && nvalid && row < g.M) ? __ldg(g.mask + int64_t(row) * g.ldc + n) : 1.0f;
+            mk[r] = (g.mask && nvalid && row < g.M) ? g.mask[int64_t(row) * g.ldc + n] : 1.0f;
         }
         float v[32];
         if (nkb > 0 && ok) {
@@ -291,8 +294,7 @@ cudaError_t launch_gemm_k(const MlpGemm &g, int vec_a, int vec_b, cudaStream_t s
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e != cudaSuccess) return e;
     dim3 grid(unsigned((g.M + BM - 1) / BM), unsigned((g.N + BN - 1) / BN), unsigned(g.splits));
-    kern<<<grid, GT, smem, st>>>(g, vec_a, vec_b);
-    return cudaGetLastError();
+    return launch_early(kern, grid, GT, smem, st, g, vec_a, vec_b);
 }
 
 // The layouts of the three products: forward (both K-major), the hidden
@@ -312,8 +314,9 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 // Triplet loss on Z = [anchors; positives; negatives] (3B rows of E):
 // l = max(0, |a-p|^2 - |a-n|^2 + margin), mean over the batch; writes dL/dZ.
 // One warp per triplet, lanes over the embedding's coordinates.
-__global__ void triplet_kernel(const float *__restrict__ Z, int B, int E, float margin, float *__restrict__ dZ,
-                               float *__restrict__ loss_sum, int *__restrict__ active) {
+__global__ void triplet_kernel(const float *Z, int B, int E, float margin, float *dZ, float *loss_sum, int *active) {
+    griddep_wait();
+    griddep_launch();
     const int b = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32);
     const int lane = threadIdx.x % 32;
     if (b >= B) return;
@@ -351,8 +354,9 @@ __global__ void triplet_kernel(const float *__restrict__ Z, int B, int E, float 
 // C[m][n] = sum over p of P[p][m][n] (in order) + bias[n], ReLU: the
 // epilogue of the split-K forward products.  Block = 32 columns x 8 rows,
 // each thread four rows 8 apart.
-__global__ void reduce_parts_kernel(const float *__restrict__ P, int parts, int M, int N, const float *__restrict__ bias,
-                                    int relu, float *__restrict__ C) {
+__global__ void reduce_parts_kernel(const float *P, int parts, int M, int N, const float *bias, int relu, float *C) {
+    griddep_wait();
+    griddep_launch();
     const int n = blockIdx.y * 32 + threadIdx.x;
     if (n >= N) return;
     const int64_t stride = int64_t(M) * N;
@@ -373,7 +377,9 @@ __global__ void reduce_parts_kernel(const float *__restrict__ P, int parts, int 
 
 // Column sums of G (rows x N) in `parts` row ranges: out[p * N + n].  Block
 // (32 columns x 8 row lanes); the 8 lanes are combined in a fixed order.
-__global__ void colsum_parts_kernel(const float *__restrict__ G, int rows, int N, int parts, float *__restrict__ out) {
+__global__ void colsum_parts_kernel(const float *G, int rows, int N, int parts, float *out) {
+    griddep_wait();
+    griddep_launch();
     __shared__ float s[8][33];
     const int n = blockIdx.x * 32 + threadIdx.x;
     const int p = blockIdx.y;
@@ -400,11 +406,18 @@ __global__ void sum_parts_kernel(const float *__restrict__ G, int parts, int64_t
     }
 }
 
+// A training step is a chain of a dozen small kernels, each launched early
+// (common.cuh; 196 steps, embedding and search 45.7 -> 38.7 ms): read by plain
+// loads what another of them wrote.
+//
 // X rows [part * bb, part * bb + bb) = S rows idx[part * T + off + i]: the
 // anchors, positives and negatives of one batch in one launch, one block per
 // row (16-byte copies when the rows allow them).
 __global__ void gather3_kernel(const float *__restrict__ S, const int64_t *__restrict__ idx, int64_t T, int64_t off,
-                               int bb, int d, float *__restrict__ X) {
+                               int bb, int d, float *X, float *stat) {
+    griddep_wait();
+    griddep_launch();
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2) stat[threadIdx.x] = 0.0f;  // the step's loss and count
     const int part = blockIdx.y;
     const int i = blockIdx.x;
     const float *src = S + idx[part * T + off + i] * d;
@@ -429,11 +442,13 @@ struct AdamGroups {
 };
 
 __global__ void adam_groups_kernel(AdamGroups a, float lr, float b1, float b2, float eps, float c1, float c2) {
+    griddep_wait();
+    griddep_launch();
     const int g = blockIdx.y;
-    float *__restrict__ W = a.W[g];
-    const float *__restrict__ G = a.G[g];
-    float *__restrict__ Mo = a.M[g];
-    float *__restrict__ Vo = a.V[g];
+    float *W = a.W[g];
+    const float *G = a.G[g];
+    float *Mo = a.M[g];
+    float *Vo = a.V[g];
     const int64_t count = a.count[g];
     const int parts = a.parts[g];
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += int64_t(gridDim.x) * blockDim.x) {
@@ -465,9 +480,8 @@ cudaError_t mlp_reduce_parts(const float *P, int parts, int M, int N, const floa
                              cudaStream_t st, int *launches) {
     if (M <= 0 || N <= 0) return cudaSuccess;
     if (launches) *launches += 1;
-    reduce_parts_kernel<<<dim3(unsigned((M + 31) / 32), unsigned((N + 31) / 32)), dim3(32, 8), 0, st>>>(
-        P, parts, M, N, bias, relu, C);
-    return cudaGetLastError();
+    return launch_early(reduce_parts_kernel, dim3(unsigned((M + 31) / 32), unsigned((N + 31) / 32)), dim3(32, 8), 0, st,
+                        P, parts, M, N, bias, relu, C);
 }
 
 cudaError_t mlp_gemm(const MlpGemm &g, cudaStream_t st, int *launches) {
@@ -494,14 +508,13 @@ cudaError_t mlp_gemm(const MlpGemm &g, cudaStream_t st, int *launches) {
 cudaError_t mlp_triplet(const float *Z, int B, int E, float margin, float *dZ, float *loss_sum, int *active,
                         cudaStream_t st, int *launches) {
     if (launches) *launches += 1;
-    triplet_kernel<<<unsigned((B + 7) / 8), 256, 0, st>>>(Z, B, E, margin, dZ, loss_sum, active);
-    return cudaGetLastError();
+    return launch_early(triplet_kernel, dim3(unsigned((B + 7) / 8)), 256, 0, st, Z, B, E, margin, dZ, loss_sum, active);
 }
 
 cudaError_t mlp_colsum_parts(const float *G, int rows, int N, int parts, float *out, cudaStream_t st, int *launches) {
     if (launches) *launches += 1;
-    colsum_parts_kernel<<<dim3(unsigned((N + 31) / 32), unsigned(parts)), dim3(32, 8), 0, st>>>(G, rows, N, parts, out);
-    return cudaGetLastError();
+    return launch_early(colsum_parts_kernel, dim3(unsigned((N + 31) / 32), unsigned(parts)), dim3(32, 8), 0, st, G, rows, N,
+                        parts, out);
 }
 
 cudaError_t mlp_sum_parts(const float *G, int parts, int64_t count, float *out, cudaStream_t st, int *launches) {
@@ -513,12 +526,12 @@ cudaError_t mlp_sum_parts(const float *G, int parts, int64_t count, float *out, 
 }
 
 cudaError_t mlp_gather3(const float *S, const int64_t *idx, int64_t T, int64_t off, int bb, int d, float *X,
-                        cudaStream_t st, int *launches) {
+                        float *stat, cudaStream_t st, int *launches) {
     if (bb <= 0) return cudaSuccess;
     if (launches) *launches += 1;
     const int threads = d >= 512 ? 192 : 64;
-    gather3_kernel<<<dim3(unsigned(bb), 3), threads, 0, st>>>(S, idx, T, off, bb, d, X);
-    return cudaGetLastError();
+    return launch_early(gather3_kernel, dim3(unsigned(bb), 3), dim3(unsigned(threads)), 0, st, S, idx, T, off, bb, d, X,
+                        stat);
 }
 
 cudaError_t mlp_adam4(float *const W[4], const float *const G[4], const int parts[4], float *const M[4],
@@ -534,8 +547,7 @@ cudaError_t mlp_adam4(float *const W[4], const float *const G[4], const int part
     int64_t blocks = (most + 255) / 256;
     if (blocks > 1024) blocks = 1024;
     if (launches) *launches += 1;
-    adam_groups_kernel<<<dim3(unsigned(blocks), 4), 256, 0, st>>>(a, lr, b1, b2, 1e-8f, c1, c2);
-    return cudaGetLastError();
+    return launch_early(adam_groups_kernel, dim3(unsigned(blocks), 4), 256, 0, st, a, lr, b1, b2, 1e-8f, c1, c2);
 }
 
 }  // namespace ssg
