@@ -531,16 +531,23 @@ struct ListPlan {
 
 // False when the scan does not apply: too few whole wide tiles for a bound
 // (four groups of columns per candidate from at most a quarter of the
-// database), or lists longer than a list's room.
-bool list_plan(const ssg_index *idx, int64_t m, int kk, ListPlan *p) {
+// database), or lists longer than a list's room.  streamed: rows in 128-byte
+// K-blocks.
+bool list_plan(const ssg_index *idx, int64_t m, int kk, bool streamed, ListPlan *p) {
     // rows of a wide tile
     const int64_t wide = idx->metric == SSG_METRIC_HAMMING ? 2 * ssg::sketch_tile_rows(false) : 256;
     const int64_t n_full = idx->n / wide, n_wide = (idx->n + wide - 1) / wide;
     if (kk > (ssg::kListMaxCap - 64) / 2 || n_full < 8) return false;
     // The sample costs its share of a scan, and a bound from one row in f
-    // lets about 1.2 kk f candidates per query through.  With few queries the
-    // scan reads memory and hardly appends: a smaller sample.
-    const int64_t f = m > 256 ? 8 : 16;
+    // lets about 1.2 kk f candidates per query through.  Where the scan waits
+    // for its epilogue (sketches, rows in 64-byte K-blocks) a sixth: 10,000
+    // queries x 2e6 sketches 6.87 ms (an eighth 7.26, a quarter 6.85), 2,048 x
+    // 1e6 BF16 rows of 96 460 us (476, 460), 1,000 x 1e5 split rows of 128 164
+    // (178, 164).  Long rows' MMAs hide more of the appends: an eighth, 4,096 x
+    // 2e6 FP8 rows of 768 4.71 ms (a sixth 4.84, a twelfth 4.77).  With few
+    // queries the scan reads memory and hardly appends: a twelfth, 64 queries
+    // x 2e6 sketches 254 us (a sixteenth 262, an eighth 259).
+    const int64_t f = m <= 256 ? 12 : streamed ? 8 : 6;
     // four minima per candidate, from groups of 128, 32 or (small databases) 4 rows
     const int64_t quarter = n_full / 4;
     p->per_tile = 8 * quarter < 4 * kk ? 64 : 8;
@@ -1189,7 +1196,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     ListPlan lp;
     const bool locality = queries_are_db && idx->locality_param && m == idx->n && idx->n >= kLocalityMinRows;
     if (!idx->pair_param && ssg::list_fits(2 * k3, 64, list_epilogue(idx->metric), idx->n) &&
-        (locality ? list_plan_locality(idx, plan.rr, &lp) : list_plan(idx, m, plan.rr, &lp))) {
+        (locality ? list_plan_locality(idx, plan.rr, &lp) : list_plan(idx, m, plan.rr, false, &lp))) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->ps_db.p);
         s.alpha = static_cast<const float *>(idx->ps_norm.p);
@@ -1354,7 +1361,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     ListPlan lp;
     const int row_bytes = 3 * ssg::stream_kbytes(idx->dim, 0);
     const int epi = list_epilogue_stream(idx->metric, false);
-    if (ssg::list_fits(row_bytes, 128, epi, idx->n) && list_plan(idx, m, kk, &lp)) {
+    if (ssg::list_fits(row_bytes, 128, epi, idx->n) && list_plan(idx, m, kk, true, &lp)) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->pss_db.p);
         s.row_bytes = row_bytes;
@@ -1491,7 +1498,7 @@ int run_knn(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, 
         // 18.8 ms).
         const int kk = int(std::min<int64_t>(int64_t(k) + (exclude_self ? 1 : 0), idx->n));
         ListPlan plan;
-        if (ssg::list_fits(ssg::sketch_row_bytes(idx->dim), 128, ssg::LIST_HAMMING, idx->n) && list_plan(idx, m, kk, &plan)) {
+        if (ssg::list_fits(ssg::sketch_row_bytes(idx->dim), 128, ssg::LIST_HAMMING, idx->n) && list_plan(idx, m, kk, false, &plan)) {
             // the tiles take 4 times the sketches: without the memory the
             // sketches are scanned as they are
             const int rc = run_hamming_tc(idx, dq, m, k, exclude_self, d_ids, d_dists, kk, plan);
@@ -1718,7 +1725,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
                           idx->n >= kLocalityMinRows;
     if (idx->wide_param && !idx->pair_param && idx->long_param &&
         ssg::list_fits(2 * kp, 64, list_epilogue(idx->metric), idx->n) &&
-        (locality ? list_plan_locality(idx, kk, &plan) : list_plan(idx, m, kk, &plan))) {
+        (locality ? list_plan_locality(idx, kk, &plan) : list_plan(idx, m, kk, false, &plan))) {
         SSG_RC(clear_status(idx));
         const size_t tb = ssg::tc_tile_bytes(idx->dim);
         const uint8_t *qtiles = static_cast<const uint8_t *>(idx->tc_db.p);
@@ -2040,7 +2047,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     ListPlan plan;
     const int row_bytes = ssg::stream_kbytes(idx->dim, fp8);
     const int epi = list_epilogue_stream(idx->metric, fp8);
-    if (ssg::list_fits(row_bytes, 128, epi, idx->n) && list_plan(idx, m, kk, &plan)) {
+    if (ssg::list_fits(row_bytes, 128, epi, idx->n) && list_plan(idx, m, kk, true, &plan)) {
         ssg::ListScan s{};
         s.dt = static_cast<const uint8_t *>(idx->st_db.p);
         s.row_bytes = row_bytes;
