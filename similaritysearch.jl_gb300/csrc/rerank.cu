@@ -7,6 +7,7 @@
 // orders the reference can produce and makes the output deterministic.
 #include "common.cuh"
 #include "exact.cuh"
+#include "finalize_shape.h"
 #include "kernels.h"
 
 #include <algorithm>
@@ -44,12 +45,8 @@ namespace ssg {
 // ---------------------------------------------------------------------------
 namespace {
 
-constexpr int kDimStep = 32;               // dimensions staged per step
-constexpr int kRowStride = kDimStep + 4;   // floats: 16-byte rows, float4 reads of 8 lanes on distinct banks
-constexpr int kWarpKeys = 8;               // keys per lane in the warp shape (256 in all)
 constexpr int kWarpOut = 64;               // candidates re-ranked per query in the warp shape
 constexpr int kWarpsPerBlock = 4;
-constexpr int kWarpStages = 3;
 constexpr int kBlockThreads = 256;
 constexpr int kBlockRows = 128;            // candidates staged together in the block shape
 constexpr int kBlockStages = 4;
@@ -257,7 +254,7 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
             const int *cn = f.counts + size_t(j) * f.segs;
             const uint64_t *lists = f.cand + size_t(j) * f.segs * f.list_cap;
             const uint32_t bound = f.list_bound[j];
-            const int room = kWarpStages * (need + 1) * kRowStride / 2;
+            const int room = warp_room(need);  // at least what the registers hold
             uint64_t *scratch = reinterpret_cast<uint64_t *>(smem) + size_t(warp) * room;
             // body(key) for every key within the bound, by whole warps: lists
             // in rounds of 32, one per lane, or all lanes along one where
@@ -380,7 +377,7 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
             // the query's row is staged behind the candidates; the lane of
             // that row sums |q|^2 for the certificate
             const int rows_s = need + 1;
-            float *ring = reinterpret_cast<float *>(smem) + size_t(warp) * kWarpStages * rows_s * kRowStride;
+            float *ring = reinterpret_cast<float *>(smem) + size_t(warp) * 2 * warp_room(need);
             const RowSource rs{db, q + size_t(jr) * dim, int(dim), vec != 0};
             const int steps = (int(dim) + kDimStep - 1) / kDimStep;
             float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
@@ -811,7 +808,7 @@ cudaError_t launch_finalize_t(const FinalizeArgs &f, const float *db, const floa
     if ((f.counts ? f.m >= 256 && (f.query_ids || (need <= 32 && f.list_keys <= 1024)) : total <= 32 * kWarpKeys) &&
         need <= kWarpOut) {
         const size_t smem =
-            RERANK || f.counts ? size_t(kWarpsPerBlock) * kWarpStages * (need + 1) * kRowStride * 4 : 0;
+            RERANK || f.counts ? size_t(kWarpsPerBlock) * warp_room(need) * 8 : 0;
         auto kern = finalize_warp_kernel<METRIC, RERANK>;
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
         if (e != cudaSuccess) return e;
