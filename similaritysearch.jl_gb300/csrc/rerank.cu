@@ -515,7 +515,7 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
     // where each list's keys start, then the selection's histogram, in the
     // room of the selected keys (sel_cap >= kMinSel or nothing is selected)
     int *s_pre = reinterpret_cast<int *>(sel);
-    __shared__ int s_cnt[3], s_n, s_self, s_digit, s_under, s_in;
+    __shared__ int s_cnt[3], s_n, s_picked, s_self, s_digit, s_under, s_in;
     __shared__ int s_warp[kBlockThreads / 32];
     __shared__ unsigned long long s_min, s_max, s_low, s_last;
     __shared__ float s_qsq;
@@ -525,7 +525,7 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
     const int total = f.segs * f.kk;
     const uint64_t *src = f.cand + size_t(j) * total;
     if (tid == 0) {
-        s_n = 0;
+        s_n = s_picked = 0;
         s_cnt[0] = s_cnt[1] = s_cnt[2] = 0;
         s_min = s_low = KEY_EMPTY;
         s_max = s_last = 0;
@@ -726,15 +726,14 @@ finalize_block_kernel(FinalizeArgs f, const float *__restrict__ db, const float 
                 }
             }
         }
-        if (tid == 0) s_n = 0;
-        __syncthreads();
+        // (a count of its own: slower warps may still be reading s_n)
         for (int i0 = 0; i0 < slots; i0 += kBlockThreads) {
             const int i = i0 + tid;
             const uint64_t key = i < slots ? keys[i] : KEY_EMPTY;
             const bool take = key < below;
             const uint32_t vote = __ballot_sync(0xffffffffu, take);
             int base = 0;
-            if (lane == 0 && vote) base = atomicAdd(&s_n, __popc(vote));
+            if (lane == 0 && vote) base = atomicAdd(&s_picked, __popc(vote));
             base = __shfl_sync(0xffffffffu, base, 0);
             const int at = base + __popc(vote & ((1u << lane) - 1u));
             if (take && at < need) sel[at] = key;

@@ -1,5 +1,6 @@
 """Few neighbours wanted of many that pass the bound: the finalize's warp shape
-with 1 to 3 results and up to a few hundred keys within the bound."""
+with 1 to 3 results and up to a few hundred keys within the bound, and exactly
+as many keys as are wanted in its block shape."""
 import numpy as np
 import pytest
 
@@ -97,3 +98,34 @@ def test_locality_close_rows(ss, exclude_self, k, prec):
         rows = np.concatenate([np.arange(490, 745), rng.integers(0, n, size=60)])
         ri, rd = O.searchbatch("sql2", X, X[rows], k)
         assert np.array_equal(a[0].T[rows], ri) and np.array_equal(a[1].T[rows], rd)
+
+
+@pytest.mark.parametrize("k", [1, 5, 40, 150])
+@pytest.mark.parametrize("m", [1, 40, 300])
+@pytest.mark.parametrize("splits", [0, 1])
+def test_exactly_as_many_keys(ss, k, m, splits):
+    """The k nearest sketches of every query lie in k groups of the seed's
+    sample, so the bound is the k-th distance and exactly k keys are within it."""
+    rng = np.random.default_rng(k + m)
+    tiles, words = 87, 4
+    X = rng.integers(0, 2**64 - 1, size=(tiles * 240, words), dtype=np.uint64, endpoint=True)
+    base = rng.integers(0, 2**64 - 1, size=words, dtype=np.uint64, endpoint=True)
+    # the sample's tiles and their groups' first rows
+    per = 64 if 8 * (tiles // 4) < 4 * k else 8
+    samples = max(-(-4 * k // per), tiles // (12 if m <= 256 else 6))
+    if 2 * samples >= 4 * k:
+        per = 2
+    first = {2: [0, 32], 8: range(0, 240, 32), 64: range(0, 240, 4)}[per]
+    places = [t * (tiles // samples) * 240 + c for t in range(samples) for c in first]
+    assert len(places) >= k
+    for i, p in enumerate(rng.permutation(places[:k])):
+        X[p] = base
+        X[p, i % 4] ^= np.uint64((1 << (1 + i % 30)) - 1)  # 1 to 30 bits off; random sketches are 90 and more
+    Q = np.tile(base, (m, 1))
+    ri, rd = O.searchbatch("hamming", X, Q[:1], k)
+    assert rd.max() <= 30
+    idx = ss.GPUExhaustiveSearch(ss.Dist.Bits.Hamming(), ss.MatrixDatabase.from_rows(X), splits=splits)
+    for _ in range(20):
+        ids, dists = ss.searchbatch(idx, ss.GenericContext(), ss.MatrixDatabase.from_rows(Q), k)
+        assert np.array_equal(ids.T, np.repeat(ri, m, axis=0))
+        assert np.array_equal(dists.T, np.repeat(rd, m, axis=0))
