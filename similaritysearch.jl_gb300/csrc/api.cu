@@ -10,6 +10,7 @@
 #include "ssgpu.h"
 #include "common.cuh"
 #include "kernels.h"
+#include "list_plan.h"
 #include "chain.h"
 
 #include <cuda_runtime.h>
@@ -502,106 +503,29 @@ int create_common(int metric, int elem, int64_t dim, int64_t n, const void *src,
     return SSG_OK;
 }
 
+// How a list scan of kk candidates for m queries of this index runs (list_plan.h).
+ssg::ListCall list_call(const ssg_index *idx, int64_t m, int kk, bool streamed) {
+    ssg::ListCall c;
+    c.n = idx->n;
+    c.m = m;
+    c.kk = kk;
+    // rows of a wide tile
+    c.wide = idx->metric == SSG_METRIC_HAMMING ? 2 * ssg::sketch_tile_rows(false) : 256;
+    c.streamed = streamed;
+    c.splits = idx->splits_param;
+    c.pairs = ssg::device_sm_count() / 2;
+    return c;
+}
+bool list_plan(const ssg_index *idx, int64_t m, int kk, bool streamed, ssg::ListPlan *p) {
+    return ssg::list_plan(list_call(idx, m, kk, streamed), p);
+}
+bool list_plan_locality(const ssg_index *idx, int kk, ssg::ListPlan *p) {
+    return ssg::list_plan_locality(list_call(idx, idx->n, kk, false), p);
+}
+
 // Picks the number of database splits per query tile: enough blocks to fill
 // the GPU several times over, while every split stays long enough to amortise
 // its heap and the merge stays within one block's shared memory.
-// Database splits per query tile for a kernel with `cap` resident CTAs on the
-// device: qctas * s CTAs run in ceil(qctas * s / cap) waves, each CTA scanning
-// 1/s of the database, so the scan takes ~ waves(s) / s.  Minimise that, with
-// a 1% charge per extra split for the wider merge, over s <= max_s.
-int64_t wave_splits(int64_t qctas, int64_t cap, int64_t max_s) {
-    qctas = std::max<int64_t>(1, qctas);
-    const int64_t hi = std::max<int64_t>(1, std::min<int64_t>(max_s, 4 * ((cap + qctas - 1) / qctas)));
-    int64_t best = 1;
-    double best_cost = 1e300;
-    for (int64_t sp = 1; sp <= hi; ++sp) {
-        const double waves = double((qctas * sp + cap - 1) / cap);
-        const double cost = waves / double(sp) * (1.0 + 0.01 * double(sp - 1));
-        if (cost < best_cost * (1.0 - 1e-9)) { best_cost = cost; best = sp; }
-    }
-    return best;
-}
-
-// How a list scan (tc_list.cu) of kk candidates for m queries runs.
-struct ListPlan {
-    int splits = 0, cap = 0, groups = 0, per_tile = 0, keys = 0;
-    int64_t samples = 0, stride = 0;
-    int64_t chunk = 0;  // queries per pass: the lists stay within 1 GiB
-};
-
-// False when the scan does not apply: too few whole wide tiles for a bound
-// (four groups of columns per candidate from at most a quarter of the
-// database), or lists longer than a list's room.  streamed: rows in 128-byte
-// K-blocks.
-bool list_plan(const ssg_index *idx, int64_t m, int kk, bool streamed, ListPlan *p) {
-    // rows of a wide tile
-    const int64_t wide = idx->metric == SSG_METRIC_HAMMING ? 2 * ssg::sketch_tile_rows(false) : 256;
-    const int64_t n_full = idx->n / wide, n_wide = (idx->n + wide - 1) / wide;
-    if (kk > (ssg::kListMaxCap - 64) / 2 || n_full < 8) return false;
-    // The sample costs its share of a scan, and a bound from one row in f
-    // lets about 1.2 kk f candidates per query through.  Where the scan waits
-    // for its epilogue (sketches, rows in 64-byte K-blocks) a sixth: 10,000
-    // queries x 2e6 sketches 6.87 ms (an eighth 7.26, a quarter 6.85), 2,048 x
-    // 1e6 BF16 rows of 96 460 us (476, 460), 1,000 x 1e5 split rows of 128 164
-    // (178, 164).  Long rows' MMAs hide more of the appends: an eighth, 4,096 x
-    // 2e6 FP8 rows of 768 4.71 ms (a sixth 4.84, a twelfth 4.77).  With few
-    // queries the scan reads memory and hardly appends: a twelfth, 64 queries
-    // x 2e6 sketches 254 us (a sixteenth 262, an eighth 259).
-    const int64_t f = m <= 256 ? 12 : streamed ? 8 : 6;
-    // four minima per candidate, from groups of 128, 32 or (small databases) 4 rows
-    const int64_t quarter = n_full / 4;
-    p->per_tile = 8 * quarter < 4 * kk ? 64 : 8;
-    const int64_t least = (4 * kk + p->per_tile - 1) / p->per_tile;
-    if (least > quarter) return false;
-    p->samples = std::max<int64_t>(least, n_full / f);
-    if (ssg::kListSegs * p->samples >= 4 * kk) p->per_tile = ssg::kListSegs;
-    p->groups = int(p->samples * p->per_tile);
-    p->stride = n_full / p->samples;
-    const int64_t qtiles = (m + 127) / 128;
-    const int64_t pairs = (qtiles + 1) / 2;
-    int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(pairs, ssg::device_sm_count() / 2, n_wide);
-    splits = std::max<int64_t>(1, std::min<int64_t>(splits, n_wide));
-    p->splits = int(splits);
-    const int64_t expect = int64_t(1.25 * kk * double(n_wide) / double(p->samples)) + kk;
-    const int64_t cap = std::max<int64_t>(std::max(2 * kk, kk + 192) + ssg::kListSlack, 4 * expect / (ssg::kListSegs * splits) + 64);
-    p->cap = int(std::min<int64_t>(ssg::kListMaxCap, (cap + 31) / 32 * 32));
-    int64_t keys = 1024;
-    while (keys < 2 * expect && keys < 8192) keys *= 2;
-    p->keys = int(keys);
-    const size_t per_query = size_t(ssg::kListSegs * splits) * p->cap * 8;
-    p->chunk = std::max<int64_t>(256, int64_t((size_t(1) << 30) / per_query) / 256 * 256);
-    p->chunk = std::min<int64_t>(p->chunk, (m + 255) / 256 * 256);
-    return true;
-}
-
-// The list scan of allknn in its locality order.  The bound comes from the
-// tiles around each query tile's own group (4,096 rows at least), a minimum
-// per four rows: a cluster has to give kk minima by itself, or the bound is
-// the distance of other clusters and many of their rows pass (100 rows a
-// cluster, 24 candidates: groups of eight let 400 rows through, the scan and
-// merge of 100,003 rows took 19.7 ms; groups of four, and compactions whose
-// bounds the splits share for the clusters that lie elsewhere, 8.2).
-bool list_plan_locality(const ssg_index *idx, int kk, ListPlan *p) {
-    const int64_t n_wide = (idx->n + 255) / 256;
-    p->samples = std::max<int64_t>(16, (kk + 7) / 8);
-    if (kk > (ssg::kListMaxCap - 64) / 2 || 4 * p->samples > n_wide) return false;
-    p->stride = 1;
-    p->per_tile = 64;
-    p->groups = int(p->samples * 64);
-    const int64_t pairs = ((idx->n + 127) / 128 + 1) / 2, cap_pairs = ssg::device_sm_count() / 2;
-    int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(pairs, cap_pairs, n_wide);
-    splits = std::max<int64_t>(1, std::min<int64_t>(splits, n_wide));
-    p->splits = int(splits);
-    p->cap = std::min(ssg::kListMaxCap, (2 * kk + 32 + ssg::kListSlack + 31) / 32 * 32);
-    p->keys = std::max(1024, 4 * kk);
-    const size_t per_query = size_t(ssg::kListSegs * splits) * p->cap * 8 + size_t(p->groups) * 4;
-    // whole waves of query tiles per pass
-    const int64_t wave = cap_pairs * 256;
-    p->chunk = std::max<int64_t>(wave, int64_t((size_t(1) << 30) / per_query) / wave * wave);
-    p->chunk = std::min<int64_t>(p->chunk, (idx->n + 255) / 256 * 256);
-    return true;
-}
-
 int choose_splits(ssg_index *idx, int64_t m, int kk, int qpb) {
     if (idx->splits_param > 0) return idx->splits_param;
     const int64_t qtiles = (m + qpb - 1) / qpb;
@@ -662,11 +586,11 @@ int reduce_segments(ssg_index *idx, const uint64_t *cand, int64_t m, int segs, i
 }
 
 // Sizes the list scan's buffers for one chunk and points the scan at them.
-int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
+int list_buffers(ssg_index *idx, const ssg::ListPlan &p, ssg::ListScan *s) {
     const size_t segs = size_t(p.splits) * ssg::kListSegs;
     // one allocation: lists, minima (16-byte rows), bounds, counts
-    const size_t lists = size_t(p.chunk) * segs * p.cap * 8, minima = size_t(p.chunk) * p.groups * 4;
-    SSG_CK(idx->l_buf.ensure(lists + minima + size_t(p.chunk) * 4 * (1 + segs)), "allocating candidate lists");
+    const size_t lists = size_t(p.chunk) * segs * p.cap * 8;
+    SSG_CK(idx->l_buf.ensure(size_t(p.chunk) * ssg::list_query_bytes(p)), "allocating candidate lists");
     s->cap = p.cap;
     s->splits = p.splits;
     s->samples = p.samples;
@@ -682,7 +606,7 @@ int list_buffers(ssg_index *idx, const ListPlan &p, ssg::ListScan *s) {
 }
 
 // The finalize side of a chunk's lists.
-void list_finalize(const ListPlan &p, const ssg::ListScan &s, ssg::FinalizeArgs *f) {
+void list_finalize(const ssg::ListPlan &p, const ssg::ListScan &s, ssg::FinalizeArgs *f) {
     f->cand = s.lists;
     f->counts = s.counts;
     f->segs = p.splits * ssg::kListSegs;
@@ -697,7 +621,7 @@ void list_finalize(const ListPlan &p, const ssg::ListScan &s, ssg::FinalizeArgs 
 // the query tiles of tb bytes each; the status word is zero already;
 // finish(c0, f) launches the chunk's finalize kernel.
 template <typename F>
-int list_search(ssg_index *idx, ssg::ListScan s, const ListPlan &plan, const uint8_t *qtiles, size_t tb, int64_t m,
+int list_search(ssg_index *idx, ssg::ListScan s, const ssg::ListPlan &plan, const uint8_t *qtiles, size_t tb, int64_t m,
                 int k, int exclude_self, uint32_t *d_ids, float *d_dists, F &&finish) {
     SSG_RC(list_buffers(idx, plan, &s));
     const float *gamma = s.gamma;
@@ -757,7 +681,7 @@ int list_epilogue_stream(int metric, bool fp8) {
 // FP32 (at most 2,048 terms of +-1), distance = (bits - product) / 2, so the
 // keys are the ones hamming_kernel makes.
 int run_hamming_tc(ssg_index *idx, const void *dq, int64_t m, int k, int exclude_self, uint32_t *d_ids,
-                   float *d_dists, int kk, const ListPlan &plan) {
+                   float *d_dists, int kk, const ssg::ListPlan &plan) {
     const int row_bytes = ssg::sketch_row_bytes(idx->dim);
     const int rows = ssg::sketch_tile_rows(false);
     const int64_t tiles = (idx->n + 2 * rows - 1) / (2 * rows) * 2;
@@ -879,7 +803,7 @@ int run_gemm(ssg_index *idx, const float *dq, const float *dqn, int64_t m, int k
     const int64_t qtiles = (m + 127) / 128;
     int64_t splits = idx->splits_param > 0
                          ? idx->splits_param
-                         : wave_splits(qtiles, int64_t(ssg::gemm_ctas_per_sm(kk)) * ssg::device_sm_count(),
+                         : ssg::wave_splits(qtiles, int64_t(ssg::gemm_ctas_per_sm(kk)) * ssg::device_sm_count(),
                                        std::max<int64_t>(1, idx->n / 512));
     splits = std::min<int64_t>(splits, std::max<int64_t>(1, idx->n / 512));
     splits = std::max<int64_t>(1, splits);
@@ -1193,7 +1117,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     }
     int *flag_count = flags - 1;
     // the list scan; allknn of a large collection in its locality order
-    ListPlan lp;
+    ssg::ListPlan lp;
     const bool locality = queries_are_db && idx->locality_param && m == idx->n && idx->n >= kLocalityMinRows;
     if (!idx->pair_param && ssg::list_fits(2 * k3, 64, list_epilogue(idx->metric), idx->n) &&
         (locality ? list_plan_locality(idx, plan.rr, &lp) : list_plan(idx, m, plan.rr, false, &lp))) {
@@ -1225,7 +1149,7 @@ int run_plain_tc(ssg_index *idx, const float *dq, const float *dqn, int64_t m, i
     }
     const int64_t qctas = (m + 127) / 128;
     const int64_t n_tiles = ssg::tc_tiles(idx->n);
-    int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(qctas, ssg::device_sm_count(), n_tiles);
+    int64_t splits = idx->splits_param > 0 ? idx->splits_param : ssg::wave_splits(qctas, ssg::device_sm_count(), n_tiles);
     splits = std::max<int64_t>(1, std::min<int64_t>(splits, n_tiles));
     const int segs = int(splits) * ssg::tc_segments_per_split(1);
     const size_t per_query = size_t(segs) * kk * 8;
@@ -1358,7 +1282,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     }
     int *flag_count = flags - 1;
     // the list scan where the database is large enough for its seed
-    ListPlan lp;
+    ssg::ListPlan lp;
     const int row_bytes = 3 * ssg::stream_kbytes(idx->dim, 0);
     const int epi = list_epilogue_stream(idx->metric, false);
     if (ssg::list_fits(row_bytes, 128, epi, idx->n) && list_plan(idx, m, kk, true, &lp)) {
@@ -1383,7 +1307,7 @@ int run_plain_stream(ssg_index *idx, const float *dq, const float *dqn, int64_t 
     }
     const int64_t qtiles = (m + 127) / 128;
     const int64_t n_tiles = ssg::tc_tiles(idx->n);
-    int64_t splits = idx->splits_param > 0 ? idx->splits_param : wave_splits(qtiles, ssg::device_sm_count(), n_tiles);
+    int64_t splits = idx->splits_param > 0 ? idx->splits_param : ssg::wave_splits(qtiles, ssg::device_sm_count(), n_tiles);
     splits = std::max<int64_t>(1, std::min<int64_t>(splits, n_tiles));
     const int segs = int(splits) * cs;
     const size_t per_query = size_t(segs) * kk * 8;
@@ -1497,7 +1421,7 @@ int run_knn(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, 
         // bits: one query 409 against 1,631 us, 1,024 queries 1.45 against
         // 18.8 ms).
         const int kk = int(std::min<int64_t>(int64_t(k) + (exclude_self ? 1 : 0), idx->n));
-        ListPlan plan;
+        ssg::ListPlan plan;
         if (ssg::list_fits(ssg::sketch_row_bytes(idx->dim), 128, ssg::LIST_HAMMING, idx->n) && list_plan(idx, m, kk, false, &plan)) {
             // the tiles take 4 times the sketches: without the memory the
             // sketches are scanned as they are
@@ -1720,7 +1644,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
     idx->last_fallbacks = 0;
     // the list scan: the same kk candidates without heaps to fill in every
     // split; allknn of a large collection in its locality order
-    ListPlan plan;
+    ssg::ListPlan plan;
     const bool locality = queries_are_db && idx->locality_param && !idx->capturing && m == idx->n &&
                           idx->n >= kLocalityMinRows;
     if (idx->wide_param && !idx->pair_param && idx->long_param &&
@@ -1777,7 +1701,7 @@ int run_knn_tc(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int 
     const int64_t qctas = (m + qrows - 1) / qrows;
     const int64_t n_tiles = ssg::tc_tiles(idx->n);
     int64_t splits = idx->splits_param > 0 ? idx->splits_param
-                                           : wave_splits(qctas, ssg::device_sm_count(), n_tiles);
+                                           : ssg::wave_splits(qctas, ssg::device_sm_count(), n_tiles);
     splits = std::min<int64_t>(splits, n_tiles);
     splits = std::max<int64_t>(1, splits);
     // chunk the queries (a multiple of the CTA's query rows) to bound scratch
@@ -1970,7 +1894,7 @@ int run_knn_tc_filter(ssg_index *idx, const void *dq, const float *dqn, int64_t 
         }
         SSG_CK(cudaMemsetAsync(fcnt, 0, size_t(mc) * 4, idx->stream), "clearing filter counts");
         const int64_t splits = idx->splits_param > 0 ? std::min<int64_t>(idx->splits_param, n_tiles)
-                                                     : wave_splits(qct, ssg::device_sm_count(), n_tiles);
+                                                     : ssg::wave_splits(qct, ssg::device_sm_count(), n_tiles);
         SSG_RC(timer.begin());
         SSG_CK(ssg::launch_tc_filter(idx->metric, qc_tiles, static_cast<const uint8_t *>(idx->tc_db.p),
                                      static_cast<const float *>(idx->tc_norm.p), n, mc, idx->dim, int(splits), thr,
@@ -2044,7 +1968,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     }
     // the list scan where the database is large enough for its seed: the same
     // kk candidates
-    ListPlan plan;
+    ssg::ListPlan plan;
     const int row_bytes = ssg::stream_kbytes(idx->dim, fp8);
     const int epi = list_epilogue_stream(idx->metric, fp8);
     if (ssg::list_fits(row_bytes, 128, epi, idx->n) && list_plan(idx, m, kk, true, &plan)) {
@@ -2072,7 +1996,7 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
     const int64_t qtiles = (m + 127) / 128;
     const int64_t n_tiles = ssg::tc_tiles(idx->n);
     int64_t splits = idx->splits_param > 0 ? idx->splits_param
-                                           : wave_splits(qtiles, ssg::device_sm_count(), n_tiles);
+                                           : ssg::wave_splits(qtiles, ssg::device_sm_count(), n_tiles);
     splits = std::min<int64_t>(splits, n_tiles);
     splits = std::max<int64_t>(1, splits);
     const int segs = int(splits) * cs;

@@ -1,5 +1,7 @@
 // kernels.h -- host-side launchers of the device kernels (internal to libssgpu).
 #pragma once
+#include "list_plan.h"
+
 #include <cstdint>
 #include <string>
 #include <cuda_runtime.h>
@@ -212,11 +214,8 @@ cudaError_t launch_stream_scan(const uint8_t *q_tiles, const uint8_t *d_tiles, c
                                int heap_rows, uint32_t *gbound, uint64_t *cand, int *err, cudaStream_t st,
                                int *launches, int *segs_per_split);
 
-// ---- resident-query scan with candidate lists (tc_list.cu) ----
+// ---- resident-query scan with candidate lists (tc_list.cu; sizes: list_plan.h) ----
 enum { LIST_DOT = 0, LIST_SQ = 1, LIST_COS = 2, LIST_AFFINE = 3, LIST_HAMMING = 4, LIST_SCALE = 5 };
-constexpr int kListMaxCap = 1024;  // entries of one list at most
-constexpr int kListSlack = 160;    // entries beyond kk that every list has room for at least
-constexpr int kListSegs = 2;       // lists of a query per split
 // One scan of n database rows for m queries: (q, seg) of kListSegs * splits
 // segments leaves counts[q * segs + seg] unsorted keys at
 // lists[(q * segs + seg) * cap]; together they hold the query's kk smallest.

@@ -1,0 +1,106 @@
+"""CPU tests of the list scan's plan (csrc/list_plan.h): what a pass allocates
+over the whole range of rows, queries and candidates, and that its sample and
+chunks are what the kernels take."""
+import itertools
+import os
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "similaritysearch.jl_gb300", "csrc")
+BUDGET = 1 << 30
+FIELDS = ["ok", "splits", "cap", "groups", "per_tile", "keys", "samples", "stride", "chunk", "alone", "query_bytes"]
+
+DRIVER = r"""
+#include "list_plan.h"
+#include <cstdio>
+int main() {
+    long long n, m, wide, splits, pairs;
+    int kk, streamed, locality;
+    while (std::scanf("%lld %lld %d %lld %d %lld %lld %d", &n, &m, &kk, &wide, &streamed, &splits, &pairs, &locality) == 8) {
+        ssg::ListCall c;
+        c.n = n; c.m = m; c.kk = kk; c.wide = wide; c.streamed = streamed; c.splits = splits; c.pairs = pairs;
+        ssg::ListPlan p;
+        const bool ok = locality ? ssg::list_plan_locality(c, &p) : ssg::list_plan(c, &p);
+        std::printf("%d %d %d %d %d %d %lld %lld %lld %lld %lld\n", int(ok), p.splits, p.cap, p.groups, p.per_tile, p.keys,
+                    (long long)p.samples, (long long)p.stride, (long long)p.chunk,
+                    (long long)ssg::wave_splits((m + 255) / 256, pairs, (n + wide - 1) / wide), (long long)ssg::list_query_bytes(p));
+    }
+    return 0;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def plans(tmp_path_factory):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("g++ not found")
+    d = tmp_path_factory.mktemp("plan")
+    src = d / "plan.cpp"
+    src.write_text(DRIVER)
+    exe = d / "plan"
+    subprocess.run([gxx, "-std=c++17", "-O1", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+
+    def run(calls):
+        text = "\n".join(" ".join(str(int(v)) for v in c) for c in calls) + "\n"
+        out = subprocess.run([str(exe)], input=text, capture_output=True, text=True, check=True).stdout
+        return [dict(zip(FIELDS, map(int, line.split()))) for line in out.splitlines()]
+
+    return run
+
+
+def pass_bytes(p):
+    """Lists (8 bytes an entry), minima, bounds and counts of a chunk, as the scan addresses them."""
+    segs = 2 * p["splits"]
+    return p["chunk"] * (segs * p["cap"] * 8 + p["groups"] * 4 + 4 + segs * 4)
+
+
+N = [2048, 5000, 30_011, 100_000, 1_000_003, 2_000_000, 10_000_000, 100_000_000, 1_000_000_000, 2**32 - 2]
+M = [1, 64, 256, 257, 1000, 10_000, 100_000, 1_000_000]
+KK = [1, 3, 10, 64, 65, 160, 161, 480]
+
+
+def test_pass_stays_within_its_budget(plans):
+    calls = [(n, m, kk, wide, st, 0, 76, 0) for n, m, kk, (wide, st) in itertools.product(
+        N, M, KK, [(256, 0), (256, 1), (240, 0)])]
+    calls += [(n, n, kk, 256, 0, 0, 76, 0) for n in N for kk in KK]  # allknn in id order
+    taken = 0
+    for c, p in zip(calls, plans(calls)):
+        n, m, kk, wide = c[:4]
+        if not p["ok"]:
+            assert n // wide // 4 * 64 < 4 * kk or n // wide < 8
+            continue
+        taken += 1
+        assert pass_bytes(p) == p["chunk"] * p["query_bytes"] <= BUDGET
+        assert p["chunk"] % 256 == 0 and 256 <= p["chunk"] <= -(-m // 256) * 256
+        # the bound: enough minima, from whole tiles
+        assert p["groups"] == p["samples"] * p["per_tile"] >= 4 * kk
+        assert p["per_tile"] in (2, 8, 64)
+        assert p["samples"] * p["stride"] <= n // wide and p["stride"] >= 1
+        # the lists: kk stay after a compaction, beside a tile's columns and a buffer
+        assert 1 <= p["splits"] <= -(-n // wide)
+        assert p["cap"] % 32 == 0 and p["cap"] <= 1024 and p["cap"] - 128 - 12 >= kk
+        # one pass wherever it fits, split as for all queries
+        if p["chunk"] >= m:
+            assert p["splits"] == p["alone"]
+    assert taken > 500
+
+
+def test_small_chunks_fill_the_device(plans):
+    """A chunk bounded by the minima is split until its CTA pairs fill the 76."""
+    calls = [(n, m, kk, 256, 0, 0, 76, 0) for n in (10_000_000, 30_000_000, 100_000_000, 1_000_000_000)
+             for m in (20_000, 100_000, 1_000_000) for kk in (10, 100)]
+    for p in plans(calls):
+        pairs = p["chunk"] // 256 * p["splits"]
+        waves = -(-pairs // 76)
+        assert pairs / (76 * waves) > 0.85
+
+
+def test_locality_pass_stays_within_its_budget(plans):
+    calls = [(n, n, kk, 256, 0, 0, 76, 1) for n in N if n >= 65_536 for kk in KK]
+    for c, p in zip(calls, plans(calls)):
+        if p["ok"]:
+            assert pass_bytes(p) <= BUDGET
+            assert p["groups"] >= 4 * c[2]
