@@ -97,7 +97,11 @@ inline bool list_plan(const ListCall &c, ListPlan *p) {
     };
     // all queries in one pass where their lists and minima fit the budget
     const int64_t tiles = (c.m + 255) / 256;
-    const size_t one = split(c.splits > 0 ? c.splits : wave_splits(tiles, c.pairs, n_wide));
+    size_t one = split(c.splits > 0 ? c.splits : wave_splits(tiles, c.pairs, n_wide));
+    // splits that were asked for yield to the budget (every split of a query
+    // takes two lists, whatever kk is; the results do not depend on them)
+    if (c.splits > 0)
+        for (int64_t s = p->splits; one > kListBudget && s > 1;) one = split(--s);
     int64_t chunk = tiles;
     if (size_t(tiles) * one > kListBudget) {
         if (c.splits > 0) {

@@ -104,3 +104,16 @@ def test_locality_pass_stays_within_its_budget(plans):
         if p["ok"]:
             assert pass_bytes(p) <= BUDGET
             assert p["groups"] >= 4 * c[2]
+
+
+@pytest.mark.parametrize("locality", [0, 1])
+def test_splits_asked_for_yield_to_the_budget(plans, locality):
+    calls = [(n, n if locality else m, kk, 256, 0, splits, 76, locality) for n in (100_000, 2_000_000, 1_000_000_000)
+             for m in (1, 300) for kk in (10, 200) for splits in (1, 3, 17, 300, 5000, 65_535)]
+    for c, p in zip(calls, plans(calls)):
+        if not p["ok"]:
+            continue
+        assert pass_bytes(p) <= BUDGET
+        assert 1 <= p["splits"] <= c[5]
+        if not locality and c[5] <= 300 and c[0] < 1_000_000_000:
+            assert p["splits"] == min(c[5], -(-c[0] // 256))
