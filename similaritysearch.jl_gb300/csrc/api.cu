@@ -2206,8 +2206,12 @@ std::vector<uint64_t> graph_key(const ssg_index *idx, int64_t m, int k) {
     for (const DevBuf *b : {&idx->db, &idx->db_norm, &idx->tc_db, &idx->tc_norm, &idx->tc_q, &idx->st_db,
                             &idx->st_scale, &idx->st_alpha, &idx->st_beta, &idx->st_q, &idx->st_qscale, &idx->cand,
                             &idx->red[0], &idx->red[1], &idx->status, &idx->gbound, &idx->qnorm, &idx->pack_q,
-                            &idx->pack_out, &idx->qbound, &idx->l_buf})
+                            &idx->pack_out, &idx->qbound, &idx->l_buf}) {
+        // (the size too: after an allocation that failed, or a release, a
+        // smaller buffer can come to lie where a graph's larger one was)
         key.push_back(uint64_t(reinterpret_cast<uintptr_t>(b->p)));
+        key.push_back(uint64_t(b->bytes));
+    }
     return key;
 }
 
