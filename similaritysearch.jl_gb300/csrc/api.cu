@@ -1361,10 +1361,12 @@ int run_knn_stream(ssg_index *idx, const void *dq, const float *dqn, int64_t m, 
                    uint32_t *d_ids, float *d_dists, bool queries_are_db);
 
 // Frees the plain method's split tiles (and their locality-ordered copies).
+// The plain method's tensor-core forms, with the list scan's workspace: what a
+// device that ran out of memory gets back before the CUDA-core form answers.
 void release_plain_tiles(ssg_index *idx) {
     for (DevBuf *b : {&idx->ps_db, &idx->ps_dbq, &idx->ps_norm, &idx->ps_q, &idx->pss_db, &idx->pss_dbq,
                       &idx->pss_alpha, &idx->pss_beta, &idx->pss_q, &idx->loc_ps_db, &idx->loc_ps_dbq,
-                      &idx->loc_ps_norm})
+                      &idx->loc_ps_norm, &idx->l_buf})
         b->release();
     idx->ps_rows = idx->ps_qrows = idx->pss_rows = idx->pss_qrows = idx->loc_ps_n = -1;
 }
