@@ -171,7 +171,8 @@ int ssg_set_param(ssg_index *idx, const char *key, double value);
  * "kernel_launches" (kernels launched by the last call), "fallbacks" (queries
  * the last plain call recomputed with the exact scan), "last_plain_tc"
  * (1 when the last plain call ran on the tensor cores), "max_x_sq",
- * "device_bytes". */
+ * "device_bytes" (device memory held by the index: data, operand tiles and
+ * workspaces, a learned model apart). */
 int ssg_get_param(ssg_index *idx, const char *key, double *value);
 
 /* Runs the index's work on `stream` (a cudaStream_t) instead of its own. */

@@ -186,6 +186,20 @@ struct ssg_index {
 
 namespace {
 
+// f(buffer) for every device buffer of an index (not a learned model's).
+template <typename F>
+void each_buffer(ssg_index *i, F &&f) {
+    for (DevBuf *b : {&i->db, &i->db_norm, &i->qbuf, &i->qnorm, &i->qraw, &i->cand, &i->gheap, &i->outbuf, &i->stage,
+                      &i->tc_db, &i->tc_norm, &i->tc_q, &i->status, &i->loc_perm, &i->loc_rot, &i->loc_tiles,
+                      &i->loc_norm, &i->loc_ps_db, &i->loc_ps_dbq, &i->loc_ps_norm, &i->st_db, &i->st_scale,
+                      &i->st_alpha, &i->st_beta, &i->st_q, &i->st_qscale, &i->red[0], &i->red[1], &i->sq_norm,
+                      &i->sq_max, &i->flags, &i->fb_list, &i->fb_q, &i->fb_out, &i->fb_cand, &i->fb_qn, &i->tc_smp,
+                      &i->tc_smp_norm, &i->f_out, &i->f_cnt, &i->f_thr, &i->gbound, &i->pack_q, &i->pack_out, &i->gm_db,
+                      &i->gm_q, &i->ps_db, &i->ps_dbq, &i->ps_norm, &i->ps_q, &i->qbound, &i->pss_db, &i->pss_dbq,
+                      &i->pss_alpha, &i->pss_beta, &i->pss_q, &i->l_buf, &i->sk_db, &i->sk_q})
+        f(*b);
+}
+
 int fail(ssg_index *idx, int code, const char *fmt, ...) {
     char *dst = idx ? idx->err : g_err;
     va_list ap;
@@ -2714,11 +2728,11 @@ int ssg_get_param(ssg_index *idx, const char *key, double *value) {
     else if (k == "learned_used") *value = idx->last_learned;
     else if (k == "fallbacks") *value = idx->last_fallbacks;
     else if (k == "max_x_sq") *value = idx->max_x_sq;
-    else if (k == "device_bytes")
-        *value = double(idx->db.bytes + idx->db_norm.bytes + idx->qbuf.bytes + idx->qnorm.bytes + idx->cand.bytes +
-                        idx->gheap.bytes + idx->outbuf.bytes + idx->stage.bytes + idx->tc_db.bytes +
-                        idx->tc_norm.bytes + idx->tc_q.bytes);
-    else {
+    else if (k == "device_bytes") {
+        size_t bytes = 0;
+        each_buffer(idx, [&](DevBuf &b) { bytes += b.bytes; });
+        *value = double(bytes);
+    } else {
         bool found = false;
         const double v = ssg::learned_get(idx->learned, key, &found);
         if (!found) return fail(idx, SSG_EINVAL, "unknown parameter '%s'", key);
@@ -2916,33 +2930,9 @@ void ssg_destroy(ssg_index *idx) {
     if (!idx) return;
     cudaSetDevice(idx->device);
     if (idx->stream) cudaStreamSynchronize(idx->stream);
-    idx->db.release();
-    idx->db_norm.release();
-    idx->qbuf.release();
-    idx->qnorm.release();
-    idx->qraw.release();
-    idx->cand.release();
-    idx->gheap.release();
-    idx->outbuf.release();
-    idx->stage.release();
-    idx->tc_db.release();
-    idx->tc_norm.release();
-    idx->tc_q.release();
-    idx->status.release();
-    for (DevBuf *b : {&idx->loc_perm, &idx->loc_rot, &idx->loc_tiles, &idx->loc_norm, &idx->loc_ps_db,
-                      &idx->loc_ps_dbq, &idx->loc_ps_norm})
-        b->release();
+    each_buffer(idx, [](DevBuf &b) { b.release(); });
     ssg::learned_free(idx->learned);
     idx->learned = nullptr;
-    for (DevBuf *b : {&idx->st_db, &idx->st_scale, &idx->st_alpha, &idx->st_beta, &idx->st_q, &idx->st_qscale,
-                      &idx->red[0], &idx->red[1]})
-        b->release();
-    for (DevBuf *b : {&idx->sq_norm, &idx->sq_max, &idx->flags, &idx->fb_list, &idx->fb_q, &idx->fb_out,
-                      &idx->fb_cand, &idx->fb_qn, &idx->tc_smp, &idx->tc_smp_norm, &idx->f_out, &idx->f_cnt,
-                      &idx->f_thr, &idx->gbound, &idx->pack_q, &idx->pack_out, &idx->gm_db, &idx->gm_q,
-                      &idx->ps_db, &idx->ps_dbq, &idx->ps_norm, &idx->ps_q, &idx->qbound, &idx->pss_db,
-                      &idx->pss_dbq, &idx->pss_alpha, &idx->pss_beta, &idx->pss_q, &idx->l_buf, &idx->sk_db, &idx->sk_q})
-        b->release();
     if (idx->pin && !pin_page().give(idx->pin)) cudaFreeHost(idx->pin);
     if (idx->pin_io) cudaFreeHost(idx->pin_io);
     if (idx->ev0) cudaEventDestroy(idx->ev0);

@@ -28,3 +28,15 @@ def test_bf16_in_chunks(ss):
     for s in (slice(0, 50_000), slice(50_000, 100_000), slice(100_000, None)):
         b = ss.searchbatch(idx, ctx, ss.MatrixDatabase.from_rows(Q[s]), 3)
         assert np.array_equal(a[0][:, s], b[0]) and np.array_equal(a[1][:, s], b[1])
+
+
+def test_device_bytes_count_tiles_and_lists(ss):
+    rng = np.random.default_rng(5)
+    B = rng.integers(0, 2**64 - 1, size=(50_000, 4), dtype=np.uint64, endpoint=True)
+    F = rng.standard_normal((50_000, 64), dtype=np.float32)
+    ctx = ss.GenericContext()
+    for dist, X, forms in ((ss.Dist.Bits.Hamming(), B, 50_000 * 128), (ss.Dist.SqL2(), F, 50_000 * 3 * 64 * 2)):
+        idx = ss.GPUExhaustiveSearch(dist, ss.MatrixDatabase.from_rows(X))
+        ss.searchbatch(idx, ctx, ss.MatrixDatabase.from_rows(X[:300]), 10)
+        # the rows as given, as FP4 or split BF16 tiles, and 300 x 10 candidates at least
+        assert idx.get_param("device_bytes") >= X.nbytes + forms + 300 * 10 * 8
