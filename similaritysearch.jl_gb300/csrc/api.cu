@@ -140,6 +140,7 @@ struct ssg_index {
     // sk_rows rows) and of the current queries
     DevBuf l_buf, sk_db, sk_q;
     int64_t sk_rows = -1;
+    size_t sk_cap = 0;  // bytes of sk_db that are tiles'; behind them the first search's workspace
     int plain_tc_param = 1;
     int last_plain_tc = 0;  // 1: the last plain-method search ran on the tensor cores
     int64_t smp_r = 0, smp_n = -1, smp_rows = 0;
@@ -599,22 +600,34 @@ int reduce_segments(ssg_index *idx, const uint64_t *cand, int64_t m, int segs, i
     return SSG_OK;
 }
 
-// Sizes the list scan's buffers for one chunk and points the scan at them.
-int list_buffers(ssg_index *idx, const ssg::ListPlan &p, ssg::ListScan *s) {
+// Queries of an m-query call that a pass holds lists for.  Rows that only pad
+// a query tile are never touched, so a small call takes what its own queries
+// need (by powers of two, so that calls of all sizes soon find it there): one
+// query over 100,000 rows 0.4 MB, not the 110 MB of a pair of tiles.
+size_t list_rows(const ssg::ListPlan &p, int64_t m) {
+    return size_t(std::min<int64_t>(p.chunk, ssg::next_pow2(std::min<int64_t>(m, p.chunk))));
+}
+
+// Sizes the list scan's buffers for an m-query call and points the scan at them.
+int list_buffers(ssg_index *idx, const ssg::ListPlan &p, int64_t m, ssg::ListScan *s) {
+    const size_t rows = list_rows(p, m), need = rows * ssg::list_query_bytes(p);
     const size_t segs = size_t(p.splits) * ssg::kListSegs;
     // one allocation: lists, minima (16-byte rows), bounds, counts
-    const size_t lists = size_t(p.chunk) * segs * p.cap * 8;
-    SSG_CK(idx->l_buf.ensure(size_t(p.chunk) * ssg::list_query_bytes(p)), "allocating candidate lists");
+    char *base = static_cast<char *>(idx->sk_db.p) + idx->sk_cap;
+    if (idx->sk_db.bytes - idx->sk_cap < need) {
+        SSG_CK(idx->l_buf.ensure(need), "allocating candidate lists");
+        base = static_cast<char *>(idx->l_buf.p);
+    }
     s->cap = p.cap;
     s->splits = p.splits;
     s->samples = p.samples;
     s->sample_stride = p.stride;
     s->groups = p.groups;
     s->per_tile = p.per_tile;
-    s->lists = static_cast<uint64_t *>(idx->l_buf.p);
-    s->minima = reinterpret_cast<float *>(static_cast<char *>(idx->l_buf.p) + lists);
-    s->bound = reinterpret_cast<uint32_t *>(s->minima + size_t(p.chunk) * p.groups);
-    s->counts = reinterpret_cast<int *>(s->bound + p.chunk);
+    s->lists = reinterpret_cast<uint64_t *>(base);
+    s->minima = reinterpret_cast<float *>(base + rows * segs * p.cap * 8);
+    s->bound = reinterpret_cast<uint32_t *>(s->minima + rows * p.groups);
+    s->counts = reinterpret_cast<int *>(s->bound + rows);
     s->err = static_cast<int *>(idx->status.p);
     return SSG_OK;
 }
@@ -637,7 +650,7 @@ void list_finalize(const ssg::ListPlan &p, const ssg::ListScan &s, ssg::Finalize
 template <typename F>
 int list_search(ssg_index *idx, ssg::ListScan s, const ssg::ListPlan &plan, const uint8_t *qtiles, size_t tb, int64_t m,
                 int k, int exclude_self, uint32_t *d_ids, float *d_dists, F &&finish) {
-    SSG_RC(list_buffers(idx, plan, &s));
+    SSG_RC(list_buffers(idx, plan, m, &s));
     const float *gamma = s.gamma;
     const uint32_t *perm = s.perm;
     const int *rot = s.rot;
@@ -700,7 +713,16 @@ int run_hamming_tc(ssg_index *idx, const void *dq, int64_t m, int k, int exclude
     const int rows = ssg::sketch_tile_rows(false);
     const int64_t tiles = (idx->n + 2 * rows - 1) / (2 * rows) * 2;
     if (idx->sk_rows != idx->n) {
-        SSG_CK(idx->sk_db.ensure(size_t(tiles) * rows * row_bytes), "allocating sketch tiles");
+        const size_t tile_bytes = size_t(tiles) * rows * row_bytes;
+        if (idx->sk_cap < tile_bytes) {
+            // in one allocation with this call's workspace where none is held
+            // yet: an allocation takes 55 us of an index's first search,
+            // whatever its size
+            const size_t ws = idx->l_buf.bytes ? 0 : list_rows(plan, m) * ssg::list_query_bytes(plan);
+            idx->sk_cap = 0;
+            SSG_CK(idx->sk_db.ensure(tile_bytes + ws), "allocating sketch tiles");
+            idx->sk_cap = tile_bytes;
+        }
         SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(idx->db.p), idx->n, idx->dim, false, tiles,
                                         static_cast<uint8_t *>(idx->sk_db.p), idx->stream, &idx->last_launches),
                "building sketch tiles");
@@ -1445,6 +1467,7 @@ int run_knn(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, 
             if (rc != SSG_ENOMEM) return rc;
             for (DevBuf *b : {&idx->sk_db, &idx->sk_q, &idx->l_buf}) b->release();
             idx->sk_rows = -1;
+            idx->sk_cap = 0;
         }
     }
     return run_exact_scan(idx, dq, dqn, m, k, exclude_self, nullptr, d_ids, d_dists, idx->cand);

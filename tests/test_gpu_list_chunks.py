@@ -40,3 +40,30 @@ def test_device_bytes_count_tiles_and_lists(ss):
         ss.searchbatch(idx, ctx, ss.MatrixDatabase.from_rows(X[:300]), 10)
         # the rows as given, as FP4 or split BF16 tiles, and 300 x 10 candidates at least
         assert idx.get_param("device_bytes") >= X.nbytes + forms + 300 * 10 * 8
+
+
+@pytest.mark.parametrize("kind", ["sketches", "fp32", "bf16", "fp8"])
+def test_workspace_is_the_calls_own(ss, kind):
+    """One query holds no lists for the rows that pad its tile, and calls of
+    growing and shrinking sizes find theirs."""
+    from oracle import oracle as O
+    rng = np.random.default_rng(6)
+    ctx = ss.GenericContext()
+    if kind == "sketches":
+        X = rng.integers(0, 2**64 - 1, size=(20_000, 4), dtype=np.uint64, endpoint=True)
+        dist, kw, forms = ss.Dist.Bits.Hamming(), {}, 20_160 * 128
+    else:
+        X = rng.standard_normal((20_000, 48), dtype=np.float32)
+        # operand tiles: at most six bytes an element, padded to 128
+        dist, kw, forms = ss.Dist.SqL2(), {} if kind == "fp32" else {"precision": kind, "overfetch": 4.0}, 20_224 * 128 * 6
+    idx = ss.GPUExhaustiveSearch(dist, ss.MatrixDatabase.from_rows(X), **kw)
+    order = rng.permutation(20_000)
+    for call, m in enumerate((1, 3, 40, 1, 300, 7, 700)):
+        ids, dists = ss.searchbatch(idx, ctx, ss.MatrixDatabase.from_rows(X[order[:m]]), 5)
+        if call == 0:
+            assert idx.get_param("device_bytes") < X.nbytes + forms + (1 << 20)
+        if kind in ("sketches", "fp32"):
+            ri, rd = O.searchbatch("hamming" if kind == "sketches" else "sql2", X, X[order[:m]], 5)
+            assert np.array_equal(ids.T, ri) and np.array_equal(dists.T, rd)
+        else:
+            assert np.array_equal(ids[0], order[:m] + 1)  # each its own nearest
