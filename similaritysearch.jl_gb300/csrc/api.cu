@@ -713,15 +713,22 @@ int run_hamming_tc(ssg_index *idx, const void *dq, int64_t m, int k, int exclude
     const int rows = ssg::sketch_tile_rows(false);
     const int64_t tiles = (idx->n + 2 * rows - 1) / (2 * rows) * 2;
     if (idx->sk_rows != idx->n) {
-        const size_t tile_bytes = size_t(tiles) * rows * row_bytes;
+        const size_t tile = size_t(rows) * row_bytes, tile_bytes = size_t(tiles) * tile;
         if (idx->sk_cap < tile_bytes) {
-            // in one allocation with this call's workspace where none is held
-            // yet: an allocation takes 55 us of an index's first search,
+            // for the rows that the database has room for, so that appends
+            // seldom allocate, and with this call's workspace where none is
+            // held yet: an allocation takes 55 us of an index's first search,
             // whatever its size
+            const size_t room = size_t((idx->cap + 2 * rows - 1) / (2 * rows) * 2) * tile;
             const size_t ws = idx->l_buf.bytes ? 0 : list_rows(plan, m) * ssg::list_query_bytes(plan);
             idx->sk_cap = 0;
-            SSG_CK(idx->sk_db.ensure(tile_bytes + ws), "allocating sketch tiles");
-            idx->sk_cap = tile_bytes;
+            if (idx->sk_db.ensure(room + ws) == cudaSuccess) {
+                idx->sk_cap = room;
+            } else {
+                cudaGetLastError();
+                SSG_CK(idx->sk_db.ensure(tile_bytes), "allocating sketch tiles");
+                idx->sk_cap = tile_bytes;
+            }
         }
         SSG_CK(ssg::launch_sketch_tiles(static_cast<const uint64_t *>(idx->db.p), idx->n, idx->dim, false, tiles,
                                         static_cast<uint8_t *>(idx->sk_db.p), idx->stream, &idx->last_launches),

@@ -67,3 +67,26 @@ def test_workspace_is_the_calls_own(ss, kind):
             assert np.array_equal(ids.T, ri) and np.array_equal(dists.T, rd)
         else:
             assert np.array_equal(ids[0], order[:m] + 1)  # each its own nearest
+
+
+def test_appends_find_their_tiles(ss):
+    """Tiles of an index of sketches are allocated for the rows that the
+    database has room for: appends within it allocate nothing, and every
+    search sees the rows appended before it."""
+    from oracle import oracle as O
+    rng = np.random.default_rng(8)
+    X = rng.integers(0, 2**64 - 1, size=(52_000, 3), dtype=np.uint64, endpoint=True)
+    idx = ss.GPUExhaustiveSearch(ss.Dist.Bits.Hamming(), ss.MatrixDatabase.from_rows(X[:30_000]))
+    ctx = ss.GenericContext()
+    n, held = 30_000, []
+    for step in (0, 1, 239, 240, 700, 1, 20_000):
+        if step:
+            ss.append_items_b(idx, ctx, ss.MatrixDatabase.from_rows(X[n:n + step]))
+            n += step
+        Q = X[[0, n - 1, n // 2]]
+        ids, dists = ss.searchbatch(idx, ctx, ss.MatrixDatabase.from_rows(Q), 4)
+        ri, rd = O.searchbatch("hamming", X[:n], Q, 4)
+        assert np.array_equal(ids.T, ri) and np.array_equal(dists.T, rd)
+        held.append(idx.get_param("device_bytes"))
+    # the first append makes room for 45,000 rows, the last one for more
+    assert len(set(held[1:6])) == 1
