@@ -887,7 +887,7 @@ cudaError_t launch_sketch_tiles(const uint64_t *x, int64_t rows, int64_t words, 
                                 cudaStream_t st, int *launches) {
     const int kblocks = sketch_row_bytes(words) / 128, tile_rows = sketch_tile_rows(queries);
     const int64_t total = tiles * tile_rows * kblocks * 8;
-    const int64_t blocks = std::min<int64_t>((total + 255) / 256, 152 * 64);
+    const int64_t blocks = std::min<int64_t>((total + 255) / 256, int64_t(device_sm_count()) * 64);
     if (launches) *launches += 1;
     sketch_tile_kernel<<<unsigned(std::max<int64_t>(1, blocks)), 256, 0, st>>>(x, rows, int(words), kblocks, tile_rows,
                                                                                tiles, out);
