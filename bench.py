@@ -546,12 +546,11 @@ def gpu_arm(args):
     four_k = None
     if mode == "bf16" and cx.world == 1 and not args.no_plain:
         # the configuration as written: FP32 rerank of the top 4k candidates
-        # (over-fetch 4 x (k+1) = 132 per object: beyond two heaps per object,
-        # so CTA pairs keep one heap per object)
+        # (over-fetch 4 x (k+1) = 132 per object)
         four_k = allknn_mode(cx, X, "bf16", 4.0, 3, 1)
         modes["bf16_4k"] = {"value": four_k["qps"], "ms_per_step": four_k["ms_per_step"], "overfetch": 4.0,
                             "steps": 3, "warmup": 1, "roofline": four_k["roofline"],
-                            "note": "rerank of the top 4k = 132 candidates per object; the scan keeps them in one heap per object on CTA pairs"}
+                            "note": "rerank of the top 4k = 132 candidates per object; the list scan keeps them in candidate lists"}
     suite = None
     if cx.world == 1 and args.suite != "none":
         suite = run_suite(cx, args)
@@ -711,12 +710,12 @@ def suite_c3(cx, args):
             # the scan multiplies +-1 rows in FP4 (two operations per bit);
             # no measured FP4 peak exists, the nominal dense one is 13.5 PFLOP/s
             r["tensor_tflops"] = 2.0 * n * m * 64 * words / (ms / 1e3) / 1e12
-            r["bytes_note"] = "the FP4 rows that the scan reads are 4 times the sketches"
+            r["bytes_note"] = "the FP4 rows that the scan reads are 4 times these 16-word sketches"
             return r
 
         out[tag] = search_entry(cx, "hamming", X, Qm, k, "fp32", max(args.steps, 10 if m > 64 else 50),
                                 args.warmup, desc, roof, cpu_budget=6.0)
-    out["note"] = ("tensor-bound at m = 10,000; at m = 64 the FP4 rows (4 times the sketches) at the HBM rate "
+    out["note"] = ("tensor-bound at m = 10,000; at m = 64 the FP4 rows (4 times these sketches) at the HBM rate "
                    "take most of the scan")
     return out
 

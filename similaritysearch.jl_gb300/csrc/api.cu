@@ -1460,16 +1460,18 @@ int run_knn(ssg_index *idx, const void *dq, const float *dqn, int64_t m, int k, 
     }
     if (idx->metric == SSG_METRIC_HAMMING && !idx->exact_scan_param) {
         // On the tensor cores wherever the seed has its groups: measured
-        // against the POPC scan for 1 to 1,024 queries x 1 to 16 words x
-        // 8,192 to 2e6 sketches it is the faster one throughout (8,192
-        // sketches of 64 bits, one query: 85 against 95 us; 2e6 of 1,024
-        // bits: one query 409 against 1,631 us, 1,024 queries 1.45 against
-        // 18.8 ms).
+        // against the POPC scan for 1 to 2,000 queries x 1 to 32 words x
+        // 2,048 to 2e7 sketches, k = 1 to 100, repeated searches are the
+        // faster ones throughout (k = 10: 2,048 sketches of 64 bits, one query
+        // 59 against 81 us; 2e6 of 64 bits, 256 queries 412 against 653; 2e6
+        // of 1,024 bits, one query 212 against 1,786 us, 2,000 queries 1.2
+        // against 27.7 ms).  An index's first search builds the tiles: slower
+        // by up to 50 us for 20,000 to 50,000 sketches of up to four words.
         const int kk = int(std::min<int64_t>(int64_t(k) + (exclude_self ? 1 : 0), idx->n));
         ssg::ListPlan plan;
         if (ssg::list_fits(ssg::sketch_row_bytes(idx->dim), 128, ssg::LIST_HAMMING, idx->n) && list_plan(idx, m, kk, false, &plan)) {
-            // the tiles take 4 times the sketches: without the memory the
-            // sketches are scanned as they are
+            // the tiles take 128 bytes for every four words of a sketch: without
+            // the memory the sketches are scanned as they are
             const int rc = run_hamming_tc(idx, dq, m, k, exclude_self, d_ids, d_dists, kk, plan);
             if (rc != SSG_ENOMEM) return rc;
             for (DevBuf *b : {&idx->sk_db, &idx->sk_q, &idx->l_buf}) b->release();

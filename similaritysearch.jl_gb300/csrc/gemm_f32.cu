@@ -17,7 +17,7 @@
 //     the row and dropped).  That GEMM form differs from the reference's
 //     difference form sum (x_i - q_i)^2 (src/dist/vecs.jl:93-102) by
 //     rounding, so kk = k + margin candidates are kept and re-scored exactly
-//     in finalize_rerank_kernel, which checks that the margin provably covers
+//     in the finalize kernels (rerank.cu), which checks that the margin provably covers
 //     the exact top k and flags the query for the exact direct scan otherwise.
 #include "common.cuh"
 #include "kernels.h"

@@ -10,7 +10,8 @@
 // Sketches are scanned on the tensor cores (tc_list.cu, +-1 rows in FP4) where
 // that scan applies; this one serves databases too small for its seed, k
 // beyond its 480 candidates, "exact_scan", and a device without room for the
-// FP4 rows (4 times the sketches).
+// FP4 rows (128 bytes for every four words: 4 times the sketches, 16 times
+// those of one word).
 //
 // Block = QPB threads, one query per thread; the query's words live in
 // registers (zero-padded to WMAX words).  Database sketches stream through
