@@ -222,6 +222,46 @@ __device__ __forceinline__ uint64_t warp_max64(uint64_t v) {
     return v;
 }
 
+// Keeps the `need` smallest of the `have` > need unique keys in a warp's scratch
+// (in its first places) and returns a limit that they, and no others, are
+// below: found bit by bit by counting.
+__device__ __noinline__ uint64_t keep_smallest(uint64_t *s, int have, int need) {
+    const int lane = threadIdx.x % 32;
+    __syncwarp();
+    uint64_t all = ~0ull, any = 0;
+    for (int i = lane; i < have; i += 32) {
+        all &= s[i];
+        any |= s[i];
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        all &= __shfl_xor_sync(0xffffffffu, all, o);
+        any |= __shfl_xor_sync(0xffffffffu, any, o);
+    }
+    // bits above the highest one in which two keys differ are common
+    const int hi = 63 - __clzll(all ^ any);
+    uint64_t p = hi >= 63 ? 0ull : (all >> (hi + 1)) << (hi + 1), below = KEY_EMPTY;
+    bool done = false;
+    for (int b = hi; b >= 0; --b) {
+        const uint64_t t = p | (1ull << b);
+        int c = 0;
+        for (int i = lane; i < have; i += 32) c += s[i] < t;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c == need) { below = t; done = true; break; }
+        if (c < need) p = t;
+    }
+    if (!done) below = p + 1;
+    int base = 0;
+    for (int i0 = 0; i0 < have; i0 += 32) {
+        const uint64_t k = i0 + lane < have ? s[i0 + lane] : KEY_EMPTY;
+        const uint32_t vote = __ballot_sync(0xffffffffu, k < below);
+        __syncwarp();  // the places written lie at or before those read
+        if (k < below) s[base + __popc(vote & ((1u << lane) - 1u))] = k;
+        base += __popc(vote);
+        __syncwarp();
+    }
+    return below;
+}
+
 // A warp per query: its segs * kk <= 32 * kWarpKeys keys in registers.
 template <int METRIC, bool RERANK>
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
@@ -247,70 +287,63 @@ finalize_warp_kernel(FinalizeArgs f, const float *__restrict__ db, const float *
         uint64_t key[kWarpKeys];
         const uint64_t *held = nullptr;
         if (f.counts) {
-            // lists: the keys within the bound gather in the ring's memory
-            // (each lane copies whole lists, its places from a running sum);
-            // where they are more than the registers hold, a limit with
-            // exactly `need` keys below it is found by counting
+            // lists: the keys within the bound gather in the ring's memory;
+            // where they are more than it holds, the `need` smallest so far
+            // stay and later keys have to be below them
             const int *cn = f.counts + size_t(j) * f.segs;
             const uint64_t *lists = f.cand + size_t(j) * f.segs * f.list_cap;
             const uint32_t bound = f.list_bound[j];
             const int room = warp_room(need);  // at least what the registers hold
             uint64_t *scratch = reinterpret_cast<uint64_t *>(smem) + size_t(warp) * room;
-            // body(key) for every key within the bound, by whole warps: lists
-            // in rounds of 32, one per lane, or all lanes along one where
-            // there are few
-            auto each_key = [&](auto &&body) {
-                if (f.segs >= 8) {
-                    for (int s0 = 0; s0 < f.segs; s0 += 32) {
-                        const int c = s0 + lane < f.segs ? cn[s0 + lane] : 0;
-                        const uint64_t *l = lists + size_t(s0 + lane) * f.list_cap;
-                        const int most = __reduce_max_sync(0xffffffffu, c);
-                        for (int i = 0; i < most; ++i) {
-                            const uint64_t k = i < c ? l[i] : KEY_EMPTY;
-                            body(uint32_t(k >> 32) <= bound ? k : KEY_EMPTY);
-                        }
+            uint64_t below = KEY_EMPTY;
+            int have = 0;
+            auto push = [&](uint64_t k) {
+                if (uint32_t(k >> 32) > bound) k = KEY_EMPTY;
+                uint32_t vote = __ballot_sync(0xffffffffu, k < below);
+                if (have + __popc(vote) > room) {
+                    below = keep_smallest(scratch, have, need);
+                    have = need;
+                    vote = __ballot_sync(0xffffffffu, k < below);
+                }
+                if (k < below) scratch[have + __popc(vote & ((1u << lane) - 1u))] = k;
+                have += __popc(vote);
+            };
+            if (f.segs >= 8) {
+                // the keys of 32 lists side by side (a lane along each list
+                // waits for one load after another where a cluster fills a
+                // few of them)
+                for (int s0 = 0; s0 < f.segs; s0 += 32) {
+                    const int c = s0 + lane < f.segs ? cn[s0 + lane] : 0;
+                    int first = c;
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int v = __shfl_up_sync(0xffffffffu, first, o);
+                        if (lane >= o) first += v;
                     }
-                } else {
-                    for (int s = 0; s < f.segs; ++s) {
-                        const int c = cn[s];
-                        const uint64_t *l = lists + size_t(s) * f.list_cap;
-                        for (int i0 = 0; i0 < c; i0 += 32) {
-                            const uint64_t k = i0 + lane < c ? l[i0 + lane] : KEY_EMPTY;
-                            body(uint32_t(k >> 32) <= bound ? k : KEY_EMPTY);
-                        }
+                    const int all = __shfl_sync(0xffffffffu, first, 31);
+                    first -= c;
+                    for (int i0 = 0; i0 < all; i0 += 32) {
+                        const int i = i0 + lane;
+                        int l = 0;
+#pragma unroll
+                        for (int step = 16; step > 0; step >>= 1)
+                            if (__shfl_sync(0xffffffffu, first, l + step) <= i) l += step;
+                        const int at = i - __shfl_sync(0xffffffffu, first, l);
+                        push(i < all ? lists[size_t(s0 + l) * f.list_cap + at] : KEY_EMPTY);
                     }
                 }
-            };
-            auto gather = [&](uint64_t below, uint64_t *to, int most) {
-                int base = 0;
-                each_key([&](uint64_t k) {
-                    const uint32_t vote = __ballot_sync(0xffffffffu, k < below);
-                    const int at = base + __popc(vote & ((1u << lane) - 1u));
-                    if (k < below && at < most) to[at] = k;
-                    base += __popc(vote);
-                });
-                __syncwarp();
-                return base;
-            };
-            int have = gather(KEY_EMPTY, scratch, room);
+            } else {
+                for (int s = 0; s < f.segs; ++s) {
+                    const int c = cn[s];
+                    const uint64_t *l = lists + size_t(s) * f.list_cap;
+                    for (int i0 = 0; i0 < c; i0 += 32) push(i0 + lane < c ? l[i0 + lane] : KEY_EMPTY);
+                }
+            }
+            __syncwarp();
             held = scratch;
             if (have > 32 * kWarpKeys) {
-                uint64_t p = 0, lim = KEY_EMPTY;
-                const bool on_chip = have <= room;
-                for (int b = 63; b >= 0; --b) {
-                    const uint64_t t = p | (1ull << b);
-                    int c = 0;
-                    if (on_chip) {
-                        for (int at = lane; at < have; at += 32) c += scratch[at] < t;
-                    } else {
-                        each_key([&](uint64_t k) { c += k < t; });
-                    }
-                    c = __reduce_add_sync(0xffffffffu, c);
-                    if (c == need) { lim = t; break; }
-                    if (c < need) p = t;
-                }
-                have = min(need, gather(lim == KEY_EMPTY ? p + 1 : lim, sel, need));
-                held = sel;
+                keep_smallest(scratch, have, need);
+                have = need;
             }
             total = have;
         }
