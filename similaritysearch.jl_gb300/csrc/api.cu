@@ -621,7 +621,6 @@ int list_buffers(ssg_index *idx, const ssg::ListPlan &p, int64_t m, ssg::ListSca
     s->cap = p.cap;
     s->splits = p.splits;
     s->samples = p.samples;
-    s->sample_stride = p.stride;
     s->groups = p.groups;
     s->per_tile = p.per_tile;
     s->lists = reinterpret_cast<uint64_t *>(base);

@@ -239,9 +239,9 @@ struct ListScan {
     const uint32_t *perm;
     const int *rot;
     // the seed: `samples` wide tiles (256 rows) with per_tile = 2, 8 or 64
-    // minima each (groups in all): every sample_stride-th of the database, all
-    // of whole rows, or in a locality order those around rot
-    int64_t samples, sample_stride;
+    // minima each (groups in all): of rows from all over the database
+    // (SampleRows), or in a locality order those around rot
+    int64_t samples;
     int groups, per_tile;
     float *minima;            // m * groups
     int *err;

@@ -12,8 +12,8 @@
 // the MMAs (2,048 queries x 1e6 rows x 96 dimensions: 6,400 cycles per
 // 128 x 256 tile against 1,940 in allknn, whose order fills the heaps in the
 // first tiles).  Long heaps also take the shared memory that the resident
-// query tile needs.  Here a first pass over an evenly spaced sample of the
-// database (SEED) keeps only the smallest distance of each group of columns;
+// query tile needs.  Here a first pass over a sample of rows from all over the
+// database (SEED, SampleRows) keeps only the smallest distance of each group of columns;
 // the kk-th smallest of a query's group minima is a bound with at least kk
 // rows at or below it.  The scan then appends what lies at or below that
 // bound (about 1.2 kk rows / sample rows per query) to a list in global
@@ -77,6 +77,7 @@ struct KernelArgs {
     int stages;         // ring depth
     int64_t n_wide;     // wide tiles of this pass (the sample's in SEED)
     int64_t all_wide;   // of the database
+    SampleRows sample;  // SEED: the sampled rows
 };
 
 // Keeps the kk smallest of each full list (more than `room` entries): the
@@ -415,11 +416,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     const int64_t w_hi = w_lo + split_w < ka.n_wide ? w_lo + split_w : ka.n_wide;
     const int W = w_hi > w_lo ? int(w_hi - w_lo) : 0;
     // the u-th wide tile: of the whole scan, from the locality rotation on; in
-    // SEED of the evenly spaced sample, or of the tiles around the rotation
+    // SEED of the tiles around the rotation (the sample of a stored order is
+    // put together from atoms)
     int64_t first = ORDER != STORED ? int64_t(a.rot[qpair]) / 2 : 0;
     if (SEED && ORDER != STORED) first = first >= a.samples / 2 ? first - a.samples / 2 : first - a.samples / 2 + ka.all_wide;
+    constexpr bool SPREAD = SEED && ORDER == STORED;  // sampled rows from all over the database
+    constexpr int ATOMS = HROWS / 8;
     auto wide_tile = [&](int u) {
-        if (ORDER == STORED) return SEED ? (w_lo + u) * a.sample_stride : w_lo + u;
+        if (ORDER == STORED) return w_lo + u;
         const int64_t p = w_lo + u + first;
         return p >= ka.all_wide ? p - ka.all_wide : p;
     };
@@ -441,12 +445,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             bool ok = true;
             for (int u = 0; ok && u < W; ++u) {
                 int line = (int(wide_tile(u)) * 2 + int(rank)) * kblocks * (DBLK / kLine);
+                int64_t tile0 = 0;
+                int atom = 0;
+                if (SPREAD) sample_unit(ka.sample, ATOMS, 2 * (w_lo + u) + int(rank), &tile0, &atom);
                 int qline = int(qx) * kblocks * (KBLK / kLine);
                 for (int g = 0; g < groups_per_tile; ++g, line += group * (DBLK / kLine)) {
                     if (!tc::mbar_wait(&empty[s], ph, a.err, 21)) { ok = false; break; }
                     if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], 2 * stage_bytes);
                     uint8_t *dst = sB + size_t(s) * stage_bytes;
-                    tc::tma_load_2d_pair(dst, &dmap, 0, line, full0 + uint32_t(s * 8));
+                    if constexpr (SPREAD) {
+                        for (int kb = 0; kb < group; ++kb)
+                            tc::tma_load_5d_pair(dst + kb * DBLK, &dmap, 0, atom, g * group + kb, int(tile0), 0,
+                                                 full0 + uint32_t(s * 8));
+                    } else {
+                        tc::tma_load_2d_pair(dst, &dmap, 0, line, full0 + uint32_t(s * 8));
+                    }
                     if constexpr (QSTREAM) {
                         tc::tma_load_2d_pair(dst + part_bytes, &qmap, 0, qline, full0 + uint32_t(s * 8));
                         qline += group * (KBLK / kLine);
@@ -546,8 +559,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             if constexpr (!raw_rank(EPI)) {
                 constexpr int PER = CH * 8;  // 16-byte pieces of alpha, and of beta
                 for (int p = lane; p < coefs(EPI) * PER; p += 32) {
-                    const float *src = (p < PER ? a.alpha : a.beta) + wide_tile(u) * WIDE +
-                                       (cs + CS * (p % PER / 8)) * 32 + (p % 8) * 4;
+                    const int col = (cs + CS * (p % PER / 8)) * 32 + (p % 8) * 4;
+                    int64_t row = wide_tile(u) * WIDE + col;
+                    if constexpr (SPREAD) {
+                        int64_t tile0;
+                        int atom;
+                        sample_unit(ka.sample, ATOMS, 2 * (w_lo + u) + col / HROWS, &tile0, &atom);
+                        row = sample_row(ka.sample, HROWS, tile0, atom, col % HROWS);
+                    }
+                    const float *src = (p < PER ? a.alpha : a.beta) + row;
                     const uint32_t d = tc::smem_u32(mine + buf * coefs(EPI) * PER + p);
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
                 }
@@ -571,7 +591,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             // 11.8 ms against 10.4.)
             constexpr int LDC = raw_rank(EPI) ? 4 : 2;
             const uint32_t tbase = tmem_base + (uint32_t(quarter * 32) << 16) + uint32_t(b * WIDE + cs * 32);
-            const int64_t row0 = wide_tile(u) * WIDE + cs * 32;
+            const int64_t row0 = (SPREAD ? 0 : wide_tile(u) * WIDE) + cs * 32;  // (all sampled places are rows)
             const float4 *al = mine + (u & 1) * (coefs(EPI) * CH * 8);  // alpha, then beta
             uint32_t r[LDC][32];
             float gm[CH];
@@ -735,7 +755,9 @@ __global__ void sketch_tile_kernel(const uint64_t *__restrict__ x, int64_t rows,
 // The database tiles as lines of 1 KB (128 eight-byte elements; the bytes are
 // already swizzled, so a box is copied verbatim): a box is one tile's part of
 // a ring stage, a whole row's K-blocks where they fit.
-cudaError_t line_map(const uint8_t *base, int64_t bytes, int64_t box_bytes, CUtensorMap *map) {
+// (rank 5: the seed's sample, an atom of 8 rows at a time)
+cudaError_t encode_map(const uint8_t *base, int rank, const cuuint64_t *dims, const cuuint64_t *strides,
+                       const cuuint32_t *box, CUtensorMap *map) {
     using EncodeFn = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -749,14 +771,27 @@ cudaError_t line_map(const uint8_t *base, int64_t bytes, int64_t box_bytes, CUte
         encode = reinterpret_cast<EncodeFn>(fn);
     }
     if (reinterpret_cast<uintptr_t>(base) % 16 != 0) return cudaErrorInvalidValue;
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, cuuint32_t(rank), const_cast<uint8_t *>(base), dims,
+                              strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+cudaError_t line_map(const uint8_t *base, int64_t bytes, int64_t box_bytes, CUtensorMap *map) {
     const cuuint64_t dims[2] = {cuuint64_t(kLine / 8), cuuint64_t(bytes / kLine)};
     const cuuint64_t strides[1] = {cuuint64_t(kLine)};
     const cuuint32_t box[2] = {cuuint32_t(kLine / 8), cuuint32_t(box_bytes / kLine)};
-    const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<uint8_t *>(base), dims, strides, box,
-                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+    return encode_map(base, 2, dims, strides, box, map);
+}
+
+// The sample: a box is a K-block of one unit (SampleRows), an atom of 8 rows
+// from each of its tiles; coordinates (0, line of atoms, K-block, first tile, 0).
+cudaError_t sample_map(const uint8_t *base, int tile_rows, int swb, int kblocks, int64_t q, CUtensorMap *map) {
+    const cuuint64_t atoms = cuuint64_t(tile_rows / 8), atom = cuuint64_t(8 * swb), block = atoms * atom;
+    const cuuint64_t dims[5] = {atom / 8, atoms, cuuint64_t(kblocks), cuuint64_t(q), atoms};
+    const cuuint64_t strides[4] = {atom, block, cuuint64_t(kblocks) * block, cuuint64_t(q) * cuuint64_t(kblocks) * block};
+    const cuuint32_t box[5] = {cuuint32_t(atom / 8), 1, 1, 1, cuuint32_t(atoms)};
+    return encode_map(base, 5, dims, strides, box, map);
 }
 
 size_t list_smem(int query_bytes, int stage_bytes, int stages, int epi) {
@@ -807,7 +842,12 @@ cudaError_t launch_list_q(const ListScan &s, const Ring &ring, cudaStream_t st) 
     if (e != cudaSuccess) return e;
     CUtensorMap dmap, qmap;
     const int64_t qtiles = ((s.m + TILE - 1) / TILE + 1) / 2 * 2;
-    e = line_map(s.dt, ka.all_wide * 2 * rows * s.row_bytes, int64_t(ka.group) * rows * SWB, &dmap);
+    if (SEED && ORDER == STORED) {
+        ka.sample = sample_rows(s.n, rows, s.samples);
+        e = sample_map(s.dt, rows, SWB, ka.kblocks, ka.sample.q, &dmap);
+    } else {
+        e = line_map(s.dt, ka.all_wide * 2 * rows * s.row_bytes, int64_t(ka.group) * rows * SWB, &dmap);
+    }
     if (e == cudaSuccess) e = line_map(s.qt, qtiles * TILE * s.row_bytes, int64_t(ka.group) * TILE * SWB, &qmap);
     if (e != cudaSuccess) return e;
     return launch_early(kern, dim3(unsigned(qtiles), unsigned(s.splits)), kThreads, smem, st, ka, dmap, qmap);

@@ -289,6 +289,16 @@ __device__ __forceinline__ void tma_load_2d_pair(void *dst_smem, const void *tma
         : "memory");
 }
 
+// The same for a 5D map.
+__device__ __forceinline__ void tma_load_5d_pair(void *dst_smem, const void *tmap, int c0, int c1, int c2, int c3, int c4,
+                                                 uint32_t bar_cluster) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(smem_u32(dst_smem)),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(bar_cluster), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4)
+        : "memory");
+}
+
 // Every thread of both CTAs of the cluster.
 __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

@@ -116,7 +116,13 @@ def test_exactly_as_many_keys(ss, k, m, splits):
     if 2 * samples >= 4 * k:
         per = 2
     first = {2: [0, 32], 8: range(0, 240, 32), 64: range(0, 240, 4)}[per]
-    places = [t * (tiles // samples) * 240 + c for t in range(samples) for c in first]
+    q = 2 * tiles // 15  # tiles between a unit's 15 atoms of 8 rows
+
+    def row(v, c):  # place c of the sample's v-th unit of 120 rows
+        e = v * 15 * q // (2 * samples)
+        return (e // 15 + c // 8 * q) * 120 + e % 15 * 8 + c % 8
+
+    places = [row(2 * t + c // 120, c % 120) for t in range(samples) for c in first]
     assert len(places) >= k
     for i, p in enumerate(rng.permutation(places[:k])):
         X[p] = base

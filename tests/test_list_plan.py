@@ -10,7 +10,7 @@ import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "similaritysearch.jl_gb300", "csrc")
 BUDGET = 1 << 30
-FIELDS = ["ok", "splits", "cap", "groups", "per_tile", "keys", "samples", "stride", "chunk", "alone", "query_bytes"]
+FIELDS = ["ok", "splits", "cap", "groups", "per_tile", "keys", "samples", "chunk", "alone", "query_bytes"]
 
 DRIVER = r"""
 #include "list_plan.h"
@@ -23,8 +23,8 @@ int main() {
         c.n = n; c.m = m; c.kk = kk; c.wide = wide; c.streamed = streamed; c.splits = splits; c.pairs = pairs;
         ssg::ListPlan p;
         const bool ok = locality ? ssg::list_plan_locality(c, &p) : ssg::list_plan(c, &p);
-        std::printf("%d %d %d %d %d %d %lld %lld %lld %lld %lld\n", int(ok), p.splits, p.cap, p.groups, p.per_tile, p.keys,
-                    (long long)p.samples, (long long)p.stride, (long long)p.chunk,
+        std::printf("%d %d %d %d %d %d %lld %lld %lld %lld\n", int(ok), p.splits, p.cap, p.groups, p.per_tile, p.keys,
+                    (long long)p.samples, (long long)p.chunk,
                     (long long)ssg::wave_splits((m + 255) / 256, pairs, (n + wide - 1) / wide), (long long)ssg::list_query_bytes(p));
     }
     return 0;
@@ -78,7 +78,7 @@ def test_pass_stays_within_its_budget(plans):
         # the bound: enough minima, from whole tiles
         assert p["groups"] == p["samples"] * p["per_tile"] >= 4 * kk
         assert p["per_tile"] in (2, 8, 64)
-        assert p["samples"] * p["stride"] <= n // wide and p["stride"] >= 1
+        assert 4 * p["samples"] <= n // wide
         # the lists: kk stay after a compaction, beside a tile's columns and a buffer
         assert 1 <= p["splits"] <= -(-n // wide)
         assert p["cap"] % 32 == 0 and p["cap"] <= 1024 and p["cap"] - 128 - 12 >= kk
@@ -117,3 +117,62 @@ def test_splits_asked_for_yield_to_the_budget(plans, locality):
         assert 1 <= p["splits"] <= c[5]
         if not locality and c[5] <= 300 and c[0] < 1_000_000_000:
             assert p["splits"] == min(c[5], -(-c[0] // 256))
+
+
+SAMPLE_DRIVER = r"""
+#include "list_plan.h"
+#include <cstdio>
+#include <vector>
+// Every sampled place is a row of its own, of a whole tile; prints the largest
+// run of rows without a sampled one among the tiles sampled from, and their number.
+int main() {
+    long long n, samples;
+    int tile_rows;
+    while (std::scanf("%lld %d %lld", &n, &tile_rows, &samples) == 3) {
+        const int atoms = tile_rows / 8;
+        const ssg::SampleRows s = ssg::sample_rows(n, tile_rows, samples);
+        std::vector<bool> seen(static_cast<size_t>(n));
+        bool ok = true;
+        for (long long v = 0; v < 2 * samples; ++v) {
+            int64_t tile;
+            int line;
+            ssg::sample_unit(s, atoms, v, &tile, &line);
+            ok = ok && tile >= 0 && tile < s.q && line >= 0 && line < atoms;
+            for (int c = 0; ok && c < tile_rows; ++c) {
+                const int64_t row = ssg::sample_row(s, tile_rows, tile, line, c);
+                ok = row >= 0 && row < n / tile_rows * tile_rows && !seen[size_t(row)];
+                if (ok) seen[size_t(row)] = true;
+            }
+        }
+        const long long reach = s.q * atoms * tile_rows;
+        long long gap = 0, run = 0;
+        for (long long i = 0; i < reach; ++i) {
+            run = seen[size_t(i)] ? 0 : run + 1;
+            gap = run > gap ? run : gap;
+        }
+        std::printf("%d %lld %lld\n", int(ok), gap, reach);
+    }
+    return 0;
+}
+"""
+
+
+def test_sample_is_distinct_rows_from_everywhere(plans, tmp_path):
+    src = tmp_path / "sample.cpp"
+    src.write_text(SAMPLE_DRIVER)
+    exe = tmp_path / "sample"
+    subprocess.run([shutil.which("g++"), "-std=c++17", "-O1", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    sizes = [2048, 2100, 3839, 4095, 4096, 5000, 24_600, 30_011, 100_000, 777_777]
+    calls = [(n, m, kk, wide, st, 0, 76, 0) for n in sizes for m in (1, 1000) for kk in (1, 10, 100)
+             for wide, st in ((256, 0), (256, 1), (240, 0))]
+    text, asked = "", []
+    for c, p in zip(calls, plans(calls)):
+        if p["ok"]:
+            asked.append((c[0], c[3] // 2, p["samples"]))
+            text += "%d %d %d\n" % asked[-1]
+    out = subprocess.run([str(exe)], input=text, capture_output=True, text=True, check=True).stdout.split("\n")
+    for (n, tile_rows, samples), line in zip(asked, out):
+        ok, gap, reach = map(int, line.split())
+        assert ok == 1
+        assert reach > n - tile_rows * (tile_rows // 8) - tile_rows  # less than a span of tiles is left out
+        assert gap <= 2 * (reach // (2 * samples * 8 * (tile_rows // 8))) * 8 + 16  # evenly spread
