@@ -217,6 +217,40 @@ static __device__ __noinline__ uint64_t heap_drain_raw(uint64_t *h, const uint64
     return top;
 }
 
+// A limit that exactly `need` of a warp's more than `need` unique keys (PER per
+// lane, KEY_EMPTY is none) are below, found by counting, bit by bit from the
+// top; bits in which no two keys differ are taken over (Hamming distances
+// differ in few).
+template <int PER>
+__device__ __forceinline__ uint64_t warp_limit(const uint64_t (&key)[PER], int need) {
+    uint64_t all = ~0ull, any = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        if (key[i] != KEY_EMPTY) {
+            all &= key[i];
+            any |= key[i];
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        all &= __shfl_xor_sync(0xffffffffu, all, o);
+        any |= __shfl_xor_sync(0xffffffffu, any, o);
+    }
+    // p: the bits decided so far, those below taken as in `all`
+    uint64_t p = all, diff = all ^ any;
+    while (diff) {
+        const uint64_t bit = 1ull << (63 - __clzll(diff));
+        diff ^= bit;
+        const uint64_t t = (p | bit) & ~(bit - 1);
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < PER; ++i) c += key[i] < t;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c == need) return t;
+        if (c < need) p |= bit;
+    }
+    return p + 1;
+}
+
 // Bitonic sort of P (a power of two) keys in shared memory by the whole block.
 __device__ __forceinline__ void block_bitonic_sort(uint64_t *s, int P) {
     for (int size = 2; size <= P; size <<= 1) {

@@ -84,9 +84,12 @@ struct KernelArgs {
 // warp takes its lanes' full lists in turn, holds one in registers, finds the
 // kk-th key bit by bit and writes the kept keys back.  Returns the calling
 // lane's new count and sets *top to its largest kept key.  Lists hold up to
-// 32 * PER entries.  Rare: a bound seeded from the sample leaves the lists far
-// from full unless most of a query's neighbours lie in one split, or its
-// cluster lies elsewhere in a locality order.
+// 32 * PER entries.  A bound seeded from the sample leaves the lists far from
+// full unless most of a query's neighbours lie in one split, or its cluster
+// lies elsewhere in a locality order; of clusters and duplicates stored side by
+// side every query of a tile comes here at once, so registers for lists of 384
+// entries have a variant of their own (1,000 queries x 1e5 sketches of two
+// words in clusters of 1,000: 348 us, 218 with it and warp_limit).
 template <int PER>
 __device__ __noinline__ int compact_lists(uint64_t *list, int nb, int room, int kk, uint64_t *top) {
     const int lane = threadIdx.x % 32;
@@ -99,31 +102,9 @@ __device__ __noinline__ int compact_lists(uint64_t *list, int nb, int room, int 
         const int cnt = __shfl_sync(0xffffffffu, nb, who);
         __syncwarp();
         uint64_t key[PER];
-        uint64_t all = ~0ull, any = 0;
 #pragma unroll
-        for (int i = 0; i < PER; ++i) {
-            const int at = i * 32 + lane;
-            key[i] = at < cnt ? l[at] : KEY_EMPTY;
-            if (at < cnt) { all &= key[i]; any |= key[i]; }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            all &= __shfl_xor_sync(0xffffffffu, all, o);
-            any |= __shfl_xor_sync(0xffffffffu, any, o);
-        }
-        // bits above the highest one in which two keys differ are common
-        const int hi = 63 - __clzll((all ^ any) | 1ull);
-        uint64_t p = hi >= 63 ? 0ull : (all >> (hi + 1)) << (hi + 1), below = KEY_EMPTY;
-        bool done = false;
-        for (int b = hi; b >= 0; --b) {
-            const uint64_t t = p | (1ull << b);
-            int c = 0;
-#pragma unroll
-            for (int i = 0; i < PER; ++i) c += key[i] < t;
-            c = __reduce_add_sync(0xffffffffu, c);
-            if (c == kk) { below = t; done = true; break; }
-            if (c < kk) p = t;
-        }
-        if (!done) below = p + 1;
+        for (int i = 0; i < PER; ++i) key[i] = i * 32 + lane < cnt ? l[i * 32 + lane] : KEY_EMPTY;
+        const uint64_t below = warp_limit<PER>(key, kk);
         int base = 0;
         uint64_t mx = 0;
 #pragma unroll
@@ -273,7 +254,7 @@ struct RowList {
         drain();
         const bool full = nb > room;
         uint64_t t = 0;
-        nb = cap <= 256 ? compact_lists<8>(list, nb, room, kk, &t) : compact_lists<kListMaxCap / 32>(list, nb, room, kk, &t);
+        nb = cap <= 384 ? compact_lists<12>(list, nb, room, kk, &t) : compact_lists<kListMaxCap / 32>(list, nb, room, kk, &t);
         if (full) {
             // kk keys up to t are kept.  Ids only grow from here where rows come
             // as stored: an equal distance no longer counts.  Positions of a
