@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <numeric>
 
 #ifdef __CUDACC__
 #define SSG_PLAN_HD __host__ __device__
@@ -48,18 +49,37 @@ inline int64_t wave_splits(int64_t qctas, int64_t cap, int64_t max_s) {
 // clusters, and the bound is then the distance of many others (2,048 queries x
 // 1e6 BF16 rows of 96 stored in clusters of 100, k = 10: 1,659 us, in units
 // 1,017; allknn of 40,000 split rows of 64, likewise: 4.9 ms and 2.3).
+// A group of columns whose minimum the seed keeps is the rows at two of the
+// eight places of their atoms, of atoms far apart: alike rows count as several,
+// and not as the one that is nearest, though they lie together.  So wide tiles
+// are visited a golden section of the sample apart, one's two units half of it
+// (groups of whole chunks of columns: allknn of 37,705 rows of 11, Cosine, in
+// clusters of 37, k = 11, 3,491 us, so 1,140; of 24,481 BF16 rows of 22 in
+// clusters of 139 923 and 423; rows in random order the same).
 struct SampleRows {
     int64_t q = 0;      // tiles between the atoms of a unit
     uint64_t step = 0;  // units per sampled unit, 32 fractional bits
+    int samples = 1, stride = 1;  // wide tiles; wide tile w's first unit is w * stride mod samples
 };
 inline SampleRows sample_rows(int64_t n, int tile_rows, int64_t samples) {
     const int atoms = tile_rows / 8;
     SampleRows s;
     s.q = n / tile_rows / atoms;
     s.step = (uint64_t(s.q * atoms) << 32) / uint64_t(2 * samples);
+    s.samples = int(samples);
+    s.stride = std::max(1, int(0.618034 * double(samples)));
+    while (std::gcd(s.stride, s.samples) != 1) ++s.stride;
     return s;
 }
-// The v-th of the sample's units (two to a wide tile): its first tile and its line of atoms.
+// The first of the two units of wide tile w; the other one is s.samples further on.
+SSG_PLAN_HD inline int sample_first(const SampleRows &s, int64_t w) {
+    return int(uint64_t(w) * uint64_t(s.stride) % uint64_t(s.samples));
+}
+SSG_PLAN_HD inline int sample_next(const SampleRows &s, int v) {
+    v += s.stride;
+    return v >= s.samples ? v - s.samples : v;
+}
+// The v-th of the sample's units: its first tile and its line of atoms.
 SSG_PLAN_HD inline void sample_unit(const SampleRows &s, int atoms, int64_t v, int64_t *tile, int *line) {
     const int64_t e = int64_t((uint64_t(v) * s.step) >> 32);
     *tile = e / atoms;
@@ -112,12 +132,10 @@ inline bool list_plan(const ListCall &c, ListPlan *p) {
     const int64_t f = c.m <= 256 ? 12 : c.streamed ? 8 : 6;
     // four minima per candidate, from groups of 128, 32 or (small databases) 4 rows
     const int64_t quarter = n_full / 4;
-    p->per_tile = 8 * quarter < 4 * kk ? 64 : 8;
-    const int64_t least = (4 * kk + p->per_tile - 1) / p->per_tile;
+    const int most = 8 * quarter < 4 * kk ? 64 : 8;
+    const int64_t least = (4 * kk + most - 1) / most;
     if (least > quarter) return false;
     p->samples = std::max<int64_t>(least, std::min<int64_t>(n_full / f, kListMaxGroups / kListSegs));
-    if (kListSegs * p->samples >= 4 * kk) p->per_tile = kListSegs;
-    p->groups = int(p->samples * p->per_tile);
     const int64_t expect = int64_t(1.25 * kk * double(n_wide) / double(p->samples)) + kk;
     int64_t keys = 1024;
     while (keys < 2 * expect && keys < 8192) keys *= 2;
@@ -125,6 +143,10 @@ inline bool list_plan(const ListCall &c, ListPlan *p) {
     auto split = [&](int64_t splits) {
         splits = std::max<int64_t>(1, std::min<int64_t>(splits, n_wide));
         p->splits = int(splits);
+        // (groups of 128 take four wide tiles of a split to keep the places of
+        // an atom apart)
+        p->per_tile = kListSegs * p->samples >= 4 * kk && p->samples >= 4 * splits ? kListSegs : most;
+        p->groups = int(p->samples * p->per_tile);
         const int64_t cap = std::max<int64_t>(std::max(2 * kk, kk + 192) + kListSlack, 4 * expect / (kListSegs * splits) + 64);
         p->cap = int(std::min<int64_t>(kListMaxCap, (cap + 31) / 32 * 32));
         return 256 * list_query_bytes(*p);  // of a pair of query tiles

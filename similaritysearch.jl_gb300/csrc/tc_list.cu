@@ -227,20 +227,26 @@ struct RowList {
     __device__ __forceinline__ static float best(float a, float b) { return raw_rank(EPI) ? fmaxf(a, b) : fminf(a, b); }
     __device__ __forceinline__ bool passes(float x) const { return raw_rank(EPI) ? x >= lim_v : x <= lim_v; }
 
-    // the smallest distance of each four columns of a chunk; +inf where they
-    // are no rows
+    // The best ranking value at each of P places of a chunk's atoms of 8 rows
+    // (columns p, p + P, ...), with those before it.
     // (cols: the chunk's columns that are the tile's)
-    __device__ __forceinline__ void chunk_min(const uint32_t (&r)[32], int64_t id0, int cols, const float4 *al,
-                                              const float4 *be, float (&g)[8]) const {
+    template <int P>
+    __device__ __forceinline__ void places(const uint32_t (&r)[32], int cols, const float4 *al, const float4 *be,
+                                           float (&g)[P]) const {
         float dv[32];
         values(r, al, be, dv);
-        const bool rows = id0 + cols <= n;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float *v = dv + 4 * i;
-            const float b = raw_rank(EPI) ? fmaxf(fmax3(v[0], v[1], v[2]), v[3]) : fminf(fmin3(v[0], v[1], v[2]), v[3]);
-            g[i] = rows && 4 * i < cols ? fminf(rank_distance<EPI>(b, bits), INFINITY) : INFINITY;  // (a NaN: +inf)
+        for (int j = 0; j < 32; j += 2 * P) {
+            if (j >= 16 && cols != 32) break;
+#pragma unroll
+            for (int i = 0; i < P; ++i)
+                g[i] = raw_rank(EPI) ? fmax3(g[i], dv[j + i], dv[j + P + i]) : fmin3(g[i], dv[j + i], dv[j + P + i]);
         }
+    }
+    template <int P>
+    __device__ __forceinline__ static void no_places(float (&g)[P]) {
+#pragma unroll
+        for (int i = 0; i < P; ++i) g[i] = raw_rank(EPI) ? -INFINITY : INFINITY;
     }
     __device__ __forceinline__ void drain() {
         nb = drain_raw<EPI, ORDER>(list, buf, nbuf, nb, bits, ORDER != STORED ? top : KEY_EMPTY, ORDER != STORED ? perm : nullptr);
@@ -424,11 +430,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             int s = 0, issued = 0;
             uint32_t ph = 1;
             bool ok = true;
+            int unit = SPREAD ? sample_first(ka.sample, w_lo) : 0;
             for (int u = 0; ok && u < W; ++u) {
                 int line = (int(wide_tile(u)) * 2 + int(rank)) * kblocks * (DBLK / kLine);
                 int64_t tile0 = 0;
                 int atom = 0;
-                if (SPREAD) sample_unit(ka.sample, ATOMS, 2 * (w_lo + u) + int(rank), &tile0, &atom);
+                if (SPREAD) {
+                    sample_unit(ka.sample, ATOMS, unit + int(rank) * ka.sample.samples, &tile0, &atom);
+                    unit = sample_next(ka.sample, unit);
+                }
                 int qline = int(qx) * kblocks * (KBLK / kLine);
                 for (int g = 0; g < groups_per_tile; ++g, line += group * (DBLK / kLine)) {
                     if (!tc::mbar_wait(&empty[s], ph, a.err, 21)) { ok = false; break; }
@@ -536,6 +546,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         // their coefficients are copied a tile ahead
         constexpr int CH = 8 / CS;
         float4 *mine = coef + (warp - 2) * coefs(EPI) * CH * 16;
+        int unit = SPREAD ? sample_first(ka.sample, w_lo) : 0;
         auto fetch = [&](int u, int buf) {
             if constexpr (!raw_rank(EPI)) {
                 constexpr int PER = CH * 8;  // 16-byte pieces of alpha, and of beta
@@ -545,17 +556,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     if constexpr (SPREAD) {
                         int64_t tile0;
                         int atom;
-                        sample_unit(ka.sample, ATOMS, 2 * (w_lo + u) + col / HROWS, &tile0, &atom);
+                        sample_unit(ka.sample, ATOMS, unit + col / HROWS * ka.sample.samples, &tile0, &atom);
                         row = sample_row(ka.sample, HROWS, tile0, atom, col % HROWS);
                     }
                     const float *src = (p < PER ? a.alpha : a.beta) + row;
                     const uint32_t d = tc::smem_u32(mine + buf * coefs(EPI) * PER + p);
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
                 }
+                if (SPREAD) unit = sample_next(ka.sample, unit);
                 asm volatile("cp.async.commit_group;" ::: "memory");
             }
         };
         if (warp_live && W > 0) fetch(0, 0);
+        float place[4];  // SEED: the best ranking value at each second place of the sampled atoms
+        T.no_places(place);
         int b = 0;
         uint32_t ph = 0;
         for (int u = 0; warp_live && u < W; ++u) {
@@ -575,7 +589,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
             const int64_t row0 = (SPREAD ? 0 : wide_tile(u) * WIDE) + cs * 32;  // (all sampled places are rows)
             const float4 *al = mine + (u & 1) * (coefs(EPI) * CH * 8);  // alpha, then beta
             uint32_t r[LDC][32];
-            float gm[CH];
 #pragma unroll
             for (int round = 0; round < CH / LDC; ++round) {
                 __syncwarp();
@@ -606,32 +619,49 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                     const int col0 = (cs + ch * CS) * 32;
                     const int cols = WIDE == 256 || col0 + 32 <= WIDE ? 32 : WIDE - col0;
                     if constexpr (SEED) {
-                        float g[8];
-                        T.chunk_min(r[c], row0 + ch * CS * 32, cols, al + ch * 8, al + CH * 8 + ch * 8, g);
-                        if ((ORDER != STORED || a.per_tile == 64) && T.valid) {
+                        if (SPREAD && a.per_tile != 64) {
+                            T.places(r[c], cols, al + ch * 8, al + CH * 8 + ch * 8, place);
+                        } else if (T.valid) {
+                            float g[8];
+                            T.no_places(g);
+                            T.places(r[c], cols, al + ch * 8, al + CH * 8 + ch * 8, g);
+                            // (a locality order's last tile has columns that are no rows)
+                            const bool rows = SPREAD || row0 + ch * CS * 32 + cols <= a.n;
+#pragma unroll
+                            for (int i = 0; i < 8; ++i)
+                                g[i] = rows ? fminf(rank_distance<EPI>(g[i], a.bits), INFINITY) : INFINITY;
                             float4 *to = reinterpret_cast<float4 *>(a.minima + size_t(query) * a.groups + (w_lo + u) * 64 +
                                                                     (cs * CH + ch) * 8);
                             to[0] = make_float4(g[0], g[1], g[2], g[3]);
                             to[1] = make_float4(g[4], g[5], g[6], g[7]);
                         }
-                        gm[ch] = fmin8(g);
                     } else T.chunk(r[c], row0 + ch * CS * 32, cols, al + ch * 8, al + CH * 8 + ch * 8);
                 }
             }
             if (++b == NACC) { b = 0; ph ^= 1; }
-            if constexpr (SEED && ORDER == STORED) {
-                if (T.valid && a.per_tile != 64) {
-                    float *g = a.minima + size_t(query) * a.groups;
-                    const int64_t at = w_lo + u;
-                    if (a.per_tile == 8) {
+            if constexpr (SPREAD) {
+                // a warp's minima go to its wide tile's four slots, or those of
+                // four wide tiles to a slot of each (fewer at a split's end
+                // join places)
+                const int in = a.per_tile == 8 ? 1 : (u & 3) + 1;
+                if (a.per_tile != 64 && (a.per_tile == 8 || in == 4 || u + 1 == W)) {
+                    if (T.valid) {
+                        float *to = a.minima + size_t(query) * a.groups + (w_lo + u + 1 - in) * a.per_tile;
 #pragma unroll
-                        for (int ch = 0; ch < CH; ++ch) g[at * 8 + cs * CH + ch] = gm[ch];
-                    } else {
-                        float v = gm[0];
+                        for (int i = 0; i < 4; ++i) place[i] = fminf(rank_distance<EPI>(place[i], a.bits), INFINITY);  // (a NaN: +inf)
+                        if (a.per_tile == 8) {
+                            *reinterpret_cast<float4 *>(to + cs * 4) = make_float4(place[0], place[1], place[2], place[3]);
+                        } else {
+                            if (in == 1) place[0] = fminf(place[0], place[1]);
+                            if (in <= 2) place[0] = fminf(place[0], place[2]);
+                            if (in == 2) place[1] = fminf(place[1], place[3]);
+                            else if (in < 4) place[0] = fminf(place[0], place[3]);
 #pragma unroll
-                        for (int ch = 1; ch < CH; ++ch) v = fminf(v, gm[ch]);
-                        g[at * CS + cs] = v;
+                            for (int t = 0; t < 4; ++t)
+                                if (t < in) to[t * CS + cs] = place[t];
+                        }
                     }
+                    T.no_places(place);
                 }
             }
             if constexpr (!SEED) {

@@ -176,3 +176,66 @@ def test_sample_is_distinct_rows_from_everywhere(plans, tmp_path):
         assert ok == 1
         assert reach > n - tile_rows * (tile_rows // 8) - tile_rows  # less than a span of tiles is left out
         assert gap <= 2 * (reach // (2 * samples * 8 * (tile_rows // 8))) * 8 + 16  # evenly spread
+
+
+VISIT_DRIVER = r"""
+#include "list_plan.h"
+#include <cstdio>
+#include <vector>
+// The wide tiles' first units, from any tile on: every one of them once; prints
+// their stride and the shortest way between any two of four visited in a row.
+int main() {
+    long long samples;
+    while (std::scanf("%lld", &samples) == 1) {
+        const ssg::SampleRows s = ssg::sample_rows(256 * 4 * samples, 128, samples);
+        std::vector<int> at(static_cast<size_t>(samples));
+        std::vector<bool> seen(static_cast<size_t>(samples));
+        bool ok = true;
+        int v = ssg::sample_first(s, 0);
+        for (long long w = 0; ok && w < samples; ++w, v = ssg::sample_next(s, v)) {
+            ok = v >= 0 && v < samples && !seen[size_t(v)] && v == ssg::sample_first(s, w);
+            if (ok) seen[size_t(v)] = true;
+            at[size_t(w)] = v;
+        }
+        long long least = samples;
+        for (long long w = 0; w < samples; ++w)
+            for (long long x = w + 1; x < w + 4 && x < samples; ++x) {
+                const long long d = at[size_t(w)] > at[size_t(x)] ? at[size_t(w)] - at[size_t(x)] : at[size_t(x)] - at[size_t(w)];
+                least = d < least ? d : least;
+            }
+        std::printf("%d %d %lld\n", int(ok), s.stride, least);
+    }
+    return 0;
+}
+"""
+
+
+def test_sample_visits_every_unit_once_and_far_apart(tmp_path):
+    gxx = shutil.which("g++")
+    if not gxx:
+        pytest.skip("g++ not found")
+    src = tmp_path / "visit.cpp"
+    src.write_text(VISIT_DRIVER)
+    exe = tmp_path / "visit"
+    subprocess.run([gxx, "-std=c++17", "-O1", "-I", CSRC, str(src), "-o", str(exe)], check=True)
+    sizes = list(range(1, 400)) + [651, 1389, 7812, 65_537, 262_144]
+    out = subprocess.run([str(exe)], input="\n".join(map(str, sizes)), capture_output=True, text=True, check=True).stdout
+    for s, line in zip(sizes, out.splitlines()):
+        ok, stride, least = map(int, line.split())
+        assert ok == 1
+        # three golden sections g = 0.618 come to 1.854: four in a row are 0.146
+        # of the sample apart at least, less three times the way to a coprime stride
+        off = stride - 0.618034 * s
+        assert 0 <= off + 1 < 12
+        assert least >= min(s, 0.1458 * s - 3 * abs(off))
+
+
+def test_large_groups_have_the_tiles_to_keep_places_apart(plans):
+    calls = [(n, m, kk, wide, 0, splits, 76, 0) for n in N for m in M for kk in (1, 10, 100) for wide in (240, 256)
+             for splits in (0, 1, 5)]
+    seen = set()
+    for c, p in zip(calls, plans(calls)):
+        if p["ok"]:
+            seen.add(p["per_tile"])
+            assert p["per_tile"] != 2 or p["samples"] >= 4 * p["splits"]
+    assert {2, 8} <= seen
