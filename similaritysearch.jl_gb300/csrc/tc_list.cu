@@ -56,6 +56,7 @@ constexpr int kTileColumns = 256 / CS;     // columns of a wide tile that one li
 constexpr int kBufCap = 12;                // raw candidates buffered per lane
 constexpr int kBufStride = CS * TILE * 8;  // bytes between a lane's buffer slots
 constexpr int kBufBytes = kBufCap * kBufStride;
+constexpr int kNextBytes = CS * TILE * 4;  // per lane, the entries beyond which make_room has work
 
 enum { EPI_DOT = LIST_DOT, EPI_SQ = LIST_SQ, EPI_COS = LIST_COS, EPI_AFF = LIST_AFFINE, EPI_HAM = LIST_HAMMING,
        EPI_SCALE = LIST_SCALE };
@@ -90,12 +91,16 @@ struct KernelArgs {
 // side every query of a tile comes here at once, so registers for lists of 384
 // entries have a variant of their own (1,000 queries x 1e5 sketches of two
 // words in clusters of 1,000: 348 us, 218 with it and warp_limit).
-// ONE_ZERO: no distance is -0; a largest key at +0 is given as -0's, below
-// which no row of another +0 passes (half a database of zero rows, allknn of
-// 13,094 x 96 in FP8 5.0 -> 2.3 ms: the lists were full of them tile after tile).
-template <int PER, bool ONE_ZERO>
-__device__ __noinline__ int compact_lists(uint64_t *list, int nb, int room, int kk, uint64_t *top) {
+// BELOW: *top is for a limit just below it.  A lane with more than `next`
+// entries, but room for more, then keeps them, and *top is the key `at` of its
+// limit; and a distance of +0 is given as -0, which a limit of the next smaller
+// float would let through (half a database of zero rows had its lists full
+// tile after tile).
+template <int PER, bool BELOW>
+__device__ __noinline__ int compact_lists(uint64_t *list, int nb, int next, int room, int kk, uint64_t at, uint64_t *top) {
     const int lane = threadIdx.x % 32;
+    constexpr uint64_t one = 1ull << 32;
+    if (BELOW && nb > next && nb <= room) *top = at >> 32 == 0x80000000u ? at - one : at;
     uint32_t todo = __ballot_sync(0xffffffffu, nb > room);
     while (todo) {
         const int who = __ffs(todo) - 1;
@@ -114,9 +119,9 @@ __device__ __noinline__ int compact_lists(uint64_t *list, int nb, int room, int 
         for (int i = 0; i < PER; ++i) {
             const bool take = key[i] < below;
             const uint32_t vote = __ballot_sync(0xffffffffu, take);
-            const int at = base + __popc(vote & ((1u << lane) - 1u));
-            if (take && at < kk) {
-                l[at] = key[i];
+            const int place = base + __popc(vote & ((1u << lane) - 1u));
+            if (take && place < kk) {
+                l[place] = key[i];
                 mx = key[i] > mx ? key[i] : mx;
             }
             base += __popc(vote);
@@ -128,7 +133,7 @@ __device__ __noinline__ int compact_lists(uint64_t *list, int nb, int room, int 
         __syncwarp();
         if (lane == who) {
             nb = kk;
-            *top = ONE_ZERO && uint32_t(mx >> 32) == 0x80000000u ? mx - (1ull << 32) : mx;
+            *top = BELOW && mx >> 32 == 0x80000000u ? mx - one : mx;
         }
     }
     return nb;
@@ -257,23 +262,30 @@ struct RowList {
     }
     // Between tiles (nothing of an accumulator in registers): makes room for
     // another tile's columns in every list of the warp.
-    __device__ __forceinline__ bool make_room() {
+    // Where rows come as stored a list is looked at once before, when it has kk
+    // entries: equal rows would fill it first (2,563 queries x 29,191 equal
+    // sketches 444 -> 184 us; allknn of 51,601 BF16 rows of 11, half of them
+    // zeros, 15.7 -> 1.2 ms).  next_at is the shared address of the lane's
+    // threshold: as a register it cost a scan of sketches 9 %.
+    __device__ __forceinline__ bool make_room(uint32_t next_at) {
         const int room = cap - kTileColumns - kBufCap;
-        if (!__any_sync(0xffffffffu, nb > room)) return false;
+        int next = room;
+        if (ORDER == STORED) asm volatile("ld.shared.b32 %0, [%1];" : "=r"(next) : "r"(next_at));
+        if (!__any_sync(0xffffffffu, nb > next)) return false;
         drain();
-        const bool full = nb > room;
+        if (ORDER == STORED && nb > next) asm volatile("st.shared.b32 [%0], %1;" ::"r"(next_at), "r"(room) : "memory");
         uint64_t t = 0;
-        // (|x|^2 - 2 x.q and s x.q + 0 are no -0)
-        constexpr bool one_zero = ORDER == STORED && (EPI == EPI_SQ || EPI == EPI_AFF || EPI == EPI_SCALE);
-        nb = cap <= 384 ? compact_lists<12, one_zero>(list, nb, room, kk, &t)
-                        : compact_lists<kListMaxCap / 32, one_zero>(list, nb, room, kk, &t);
-        if (full) {
-            // kk keys up to t are kept.  Ids only grow from here where rows come
-            // as stored: an equal distance no longer counts.  Positions of a
-            // locality order have any ids: the drain compares the keys.
+        const uint64_t at = ORDER == STORED ? make_key(limit(), 0) : 0;
+        nb = cap <= 384 ? compact_lists<12, ORDER == STORED>(list, nb, next, room, kk, at, &t)
+                        : compact_lists<kListMaxCap / 32, ORDER == STORED>(list, nb, next, room, kk, at, &t);
+        if (t) {
+            // kk keys up to t are kept, or there are kk within the limit.  Ids
+            // only grow from here where rows come as stored: an equal distance
+            // no longer counts.  Positions of a locality order have any ids:
+            // the drain compares the keys.
             if (ORDER != STORED) top = t;
             const float d = key_dist(t);
-            const float e = ORDER != STORED ? d : EPI == EPI_HAM ? d - 0.5f : ordered_to_float(float_to_ordered(d) - 1u);
+            const float e = ORDER != STORED ? d : EPI == EPI_HAM ? d - 0.5f : ordered_to_float(uint32_t(t >> 32) - 1u);
             const float v = EPI == EPI_HAM ? bits - 2.0f * e : EPI == EPI_DOT ? -e : e;
             lim_v = raw_rank(EPI) ? fmaxf(lim_v, v) : fminf(lim_v, v);
         }
@@ -347,7 +359,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     // per epilogue warp, two buffers of its 64 columns' coefficients
     float4 *coef = reinterpret_cast<float4 *>(sB + size_t(stages) * stage_bytes);
     uint64_t *bufs = reinterpret_cast<uint64_t *>(coef + coefs(EPI) * kCoefBytes / 16);  // raw candidates
-    uint64_t *bars = bufs + (SEED ? 0 : kBufBytes / 8);
+    uint64_t *bars = bufs + (SEED ? 0 : (kBufBytes + kNextBytes) / 8);
     uint64_t *a_full = bars;                  // this CTA's query tile landed
     uint64_t *pa_full = a_full + 1;           // (even CTA) the odd CTA's query tile landed
     uint64_t *full = pa_full + 1;             // (even CTA) both halves of stage s landed
@@ -546,6 +558,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
         T.perm = a.perm;
         T.bits = a.bits;
         T.gamma = ((EPI == EPI_AFF || EPI == EPI_SCALE) && a.gamma && T.valid) ? a.gamma[query] : 1.0f;
+        // the lane's word behind the buffers, half of its slots' stride
+        const uint32_t next_at = (T.buf >> 1) + (tc::smem_u32(bufs) + kBufBytes - (tc::smem_u32(bufs) >> 1));
+        if (!SEED && ORDER == STORED) asm volatile("st.shared.b32 [%0], %1;" ::"r"(next_at), "r"(a.kk - 1) : "memory");
         T.set((!SEED && T.valid) ? bound_read(a.bound + query) : INFINITY);
         const bool warp_live = qx * TILE + quarter * 32 < a.m;
         // this warp's columns of a wide tile: the 32-column chunks cs, cs + CS, ...;
@@ -671,7 +686,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
                 }
             }
             if constexpr (!SEED) {
-                const bool tighter = T.make_room();
+                const bool tighter = T.make_room(next_at);
                 if (ORDER == LOCAL_SHARED) {
                     if (tighter) T.publish(a.bound + query);
                     else if ((u & 15) == 15) T.refresh(a.bound + query);
@@ -812,7 +827,7 @@ cudaError_t sample_map(const uint8_t *base, int tile_rows, int swb, int kblocks,
 }
 
 size_t list_smem(int query_bytes, int stage_bytes, int stages, int epi) {
-    return 1024 + size_t(query_bytes) + size_t(stages) * stage_bytes + coefs(epi) * kCoefBytes + kBufBytes +
+    return 1024 + size_t(query_bytes) + size_t(stages) * stage_bytes + coefs(epi) * kCoefBytes + kBufBytes + kNextBytes +
            (2 + 2 * kMaxStages + 2 * NACC + 1) * 8 + 16;
 }
 
