@@ -270,7 +270,11 @@ struct RowList {
     __device__ __forceinline__ bool make_room(uint32_t next_at) {
         const int room = cap - kTileColumns - kBufCap;
         int next = room;
-        if (ORDER == STORED) asm volatile("ld.shared.b32 %0, [%1];" : "=r"(next) : "r"(next_at));
+        if (ORDER == STORED) {
+            // (most lists never have kk: the load waits 1 % of a tile)
+            if (!__any_sync(0xffffffffu, nb >= kk)) return false;
+            asm volatile("ld.shared.b32 %0, [%1];" : "=r"(next) : "r"(next_at));
+        }
         if (!__any_sync(0xffffffffu, nb > next)) return false;
         drain();
         if (ORDER == STORED && nb > next) asm volatile("st.shared.b32 [%0], %1;" ::"r"(next_at), "r"(room) : "memory");
